@@ -559,17 +559,26 @@ __device__ __forceinline__ int cal_max_gap(const AlnOpt &o, int qlen)         //
 
 template <int C>
 __device__ KswResult run_ext(const KswParams &P, int qlen, int tlen, int h0, int w, int eb, const ReadRefAcc &acc,
-                             int lane)
+                             int lane, bool count_cells)
 {
-    return ksw_warp<C>(P, qlen, tlen, h0, w, eb, acc, lane);
+    return ksw_warp<C>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
 }
 
 // A warp tile (C columns per lane) that holds qlen + 1 columns; a kernel compiled for
 // reads of at most 32 * MaxC - 1 bases only instantiates C <= MaxC.
 template <int MaxC>
-__device__ KswResult extend_any(const KswParams &P, int qlen, int tlen, int h0, int w, int eb, const ReadRefAcc &acc,
-                                int lane)
+__device__ KswResult extend_any(const KswParams &P, const int8_t *tab, int qlen, int tlen, int h0, int w, int eb,
+                                const ReadRefAcc &acc, int lane, bool count_cells)
 {
+    // most extensions of a read are its own bases with a mismatch at most: no DP (ksw_core.cuh)
+    if (!count_cells) {
+        int best, best_j, last;
+        if (ksw_diagonal<32>(tab, P.mat_max, diagonal_limit(P, h0), qlen, tlen, h0, acc, lane, best, best_j, last)) {
+            KswResult r;
+            r.score = best, r.qle = r.tle = best_j + 1, r.gtle = qlen, r.gscore = last, r.max_off = 0, r.cells = 0;
+            return r;
+        }
+    }
     // One width per kernel where it can be: each width is a fully unrolled copy of the
     // DP, and the warps of an SM run extensions of every length at once, so extra copies
     // cost more in instruction-cache misses than the columns a tighter fit saves
@@ -577,14 +586,14 @@ __device__ KswResult extend_any(const KswParams &P, int qlen, int tlen, int h0, 
     // reference with repeats and 2x150 reads, and by 2 % on a 2 Mb one with 2x100).
     const int need = (qlen + 32) >> 5;
     if constexpr (MaxC <= 8) {
-        return run_ext<MaxC>(P, qlen, tlen, h0, w, eb, acc, lane);
+        return run_ext<MaxC>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
     } else if constexpr (MaxC <= 16) {
-        if (need <= 8) return run_ext<8>(P, qlen, tlen, h0, w, eb, acc, lane);
-        return run_ext<16>(P, qlen, tlen, h0, w, eb, acc, lane);
+        if (need <= 8) return run_ext<8>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
+        return run_ext<16>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
     } else {                 // reads of 512-1023 bases: extensions past 511 columns need 32 per lane
-        if (need <= 8) return run_ext<8>(P, qlen, tlen, h0, w, eb, acc, lane);
-        if (need <= 16) return run_ext<16>(P, qlen, tlen, h0, w, eb, acc, lane);
-        return run_ext<32>(P, qlen, tlen, h0, w, eb, acc, lane);
+        if (need <= 8) return run_ext<8>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
+        if (need <= 16) return run_ext<16>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
+        return run_ext<32>(P, qlen, tlen, h0, w, eb, acc, lane, count_cells);
     }
 }
 
@@ -601,6 +610,9 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                  bsb_reg_t *__restrict__ regs, int *__restrict__ n_regs, int *__restrict__ next,
                  const int *__restrict__ order, int64_t *__restrict__ read_cells)
 {
+    __shared__ int8_t tab[kScoreTable];
+    load_score_table(P, tab);
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     for (;;) {
         int k = 0;
@@ -726,7 +738,8 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                     for (int i = 0; i < 2; ++i) {
                         const int prev = a.score;
                         aw0 = opt.w << i;
-                        x = extend_any<MaxC>(P, s.qbeg, tlen, s.len * opt.a, aw0, opt.pen_clip5, acc, lane);
+                        x = extend_any<MaxC>(P, tab, s.qbeg, tlen, s.len * opt.a, aw0, opt.pen_clip5, acc, lane,
+                                             read_cells != nullptr);
                         cells += x.cells;
                         a.score = x.score;
                         if (a.score == prev || x.max_off < (aw0 >> 1) + (aw0 >> 2)) break;
@@ -748,7 +761,8 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                     for (int i = 0; i < 2; ++i) {
                         const int prev = a.score;
                         aw1 = opt.w << i;
-                        x = extend_any<MaxC>(P, l_query - qe, tlen, sc0, aw1, opt.pen_clip3, acc, lane);
+                        x = extend_any<MaxC>(P, tab, l_query - qe, tlen, sc0, aw1, opt.pen_clip3, acc, lane,
+                                             read_cells != nullptr);
                         cells += x.cells;
                         a.score = x.score;
                         if (a.score == prev || x.max_off < (aw1 >> 1) + (aw1 >> 2)) break;

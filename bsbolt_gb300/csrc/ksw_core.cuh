@@ -47,6 +47,95 @@ __device__ __forceinline__ uint32_t sext_selector(int byte)
     return b | r << 4 | r << 8 | r << 12;
 }
 
+// The scoring matrix as a shared table, score of target base t against query base q at
+// t << 3 | q (bases above 4 are N, as in profile_word).
+constexpr int kScoreTable = 40;
+__device__ __forceinline__ void load_score_table(const KswParams &P, int8_t *tab)
+{
+    if (threadIdx.x < 25) {
+        int v = 0;
+#pragma unroll
+        for (int k = 0; k < 25; ++k) v = (int)threadIdx.x == k ? P.mat[k] : v;
+        tab[(threadIdx.x / 5) << 3 | threadIdx.x % 5] = (int8_t)v;
+    }
+}
+
+// The loss a job's main diagonal must stay below for its result to be known without the DP
+// (ksw_diagonal), 0 when the scoring never allows it.
+__device__ __forceinline__ int diagonal_limit(const KswParams &P, int h0)
+{
+    int lim = min(P.o_del + P.e_del, P.o_ins + P.e_ins);
+    if (P.zdrop > 0) lim = min(lim, P.zdrop + 1);
+    return P.mat_max > 0 ? min(lim, h0 + P.mat_max) : 0;
+}
+
+// ksw_extend2 of a job whose query lies on its target's main diagonal with little loss, in one
+// pass over the diagonal and no DP.  Let a = max(mat), D(i) = h0 + a(i+1) - L(i) the score of the
+// diagonal through row i, L(i) what its columns lose against a.  Every other cell (i, j) pays at
+// least one gap: H(i,j) <= h0 + a(min(i,j)+1) - (o + e|i-j|).  So while L stays below o + e of
+// both gaps, D(i) is the strict maximum of row i (no tie), the band (which follows the non-zero
+// cells) holds it, max_off stays 0, no row after the query's end and no other row's last column
+// reaches D(qlen-1), and with L below h0 + a no D(i) is 0 and with L <= zdrop none drops far
+// enough to stop: score is the diagonal's best prefix (the first one, since later ones have to
+// exceed it), gscore = D(qlen-1) at row qlen-1.  Needs tlen >= qlen >= 1.  Returns false where the
+// diagonal loses too much.  A group of G lanes takes a job, 32 columns a step (column k*G + lane of
+// the group in slot k); all lanes of the warp call it, the groups with a job each (lim <= 0: none).
+template <int G, class Acc>
+__device__ __forceinline__ bool ksw_diagonal(const int8_t *tab, int a, int lim, int qlen, int tlen, int h0,
+                                             const Acc &acc, int lane, int &best, int &best_j, int &last)
+{
+    constexpr int K = 32 / G;
+    const int gl = lane & (G - 1), g0 = lane & ~(G - 1);
+    bool on = lim > 0 && qlen >= 1 && tlen >= qlen;
+    int loss = 0;
+    best = h0, best_j = -1;
+    for (int c0 = 0; __any_sync(BSB_FULL_MASK, on && c0 < qlen); c0 += 32) {
+        int l[K];
+        unsigned m = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int j = c0 + k * G + gl;
+            l[k] = on && j < qlen ? a - tab[min(acc.t(j), 4) << 3 | min(acc.q(j), 4)] : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const unsigned v = __ballot_sync(BSB_FULL_MASK, l[k] != 0);
+            m |= G == 32 ? v : ((v >> g0) & ((1u << (G & 31)) - 1)) << (k * G & 31);
+        }
+        while (__any_sync(BSB_FULL_MASK, m != 0)) {          // the columns that lose, in order
+            const int b = m ? __ffs(m) - 1 : 0;
+            int x = l[0];
+#pragma unroll
+            for (int k = 1; k < K; ++k) x = b / G == k ? l[k] : x;
+            x = __shfl_sync(BSB_FULL_MASK, x, b & (G - 1), G);
+            if (m) {
+                const int v = h0 + a * (c0 + b) - loss;      // the diagonal just before this column
+                if (v > best) best = v, best_j = c0 + b - 1;
+                loss += x;
+                on = loss < lim;
+                m = on ? m & (m - 1) : 0;
+            }
+        }
+    }
+    last = h0 + a * qlen - loss;
+    if (last > best) best = last, best_j = qlen - 1;
+    return on;
+}
+
+// Rows that can no longer change a result.  After row i every cell of a later row is reached from
+// H(i, j-1) or E(i+1, j) of some column j (stale cells beyond the band included: the band can grow
+// back over them), gaining at most a = max(mat) per remaining column, and from nothing where both
+// are 0.  So with U the largest max(H, E) + a(qlen - j) over the non-zero columns, U < gscore means
+// that no later row can raise gscore, tie with it (a tie moves gtle) or raise the score, which is
+// at least gscore: the six results are final and only the cell count would go on.  The test costs
+// a pass over the columns, so a row runs it only when its own maximum m at mj does not already
+// show a larger U.  Of a job that aligns to its end this leaves out the target's flank: 100 of
+// about 175 rows of the batched jobs.
+__device__ __forceinline__ bool rows_may_be_done(int gscore, int m, int mj, int qlen, int a)
+{
+    return gscore > 0 && (mj == qlen - 1 || m + a * (qlen - 1 - mj) < gscore);
+}
+
 // Extends one job with the calling warp (every lane returns the same tuple).
 // All control values are warp-uniform.  Acc supplies query base j and target
 // base i (q(j), t(i)), so jobs can read a byte buffer or the 2-bit reference.
@@ -61,7 +150,7 @@ __device__ __forceinline__ uint32_t sext_selector(int byte)
 // beg instead, the cells it passes are zeroed explicitly.
 template <int C, class Acc>
 __device__ __forceinline__ KswResult ksw_warp(const KswParams &P, int qlen, int tlen, int h0, int w_in,
-                                              int end_bonus, const Acc &acc, int lane)
+                                              int end_bonus, const Acc &acc, int lane, bool count_cells)
 {
     const int o_del = P.o_del, e_del = P.e_del, o_ins = P.o_ins, e_ins = P.e_ins;
     const int oe_del = o_del + e_del, oe_ins = o_ins + e_ins;
@@ -226,6 +315,15 @@ __device__ __forceinline__ KswResult ksw_warp(const KswParams &P, int qlen, int 
             } else {
                 if (best - m - (dj - di) * e_ins > P.zdrop) break;
             }
+        }
+        if (!count_cells && rows_may_be_done(gscore, m, mj, qlen, P.mat_max)) {
+            int U = 0;
+#pragma unroll
+            for (int s = 0; s < C; ++s) {
+                const int X = max(Hs[s], Es[s]);
+                if (X > 0) U = max(U, X + P.mat_max * (qlen - base - s));
+            }
+            if (__reduce_max_sync(BSB_FULL_MASK, U) < gscore) break;
         }
         // shrink to the non-zero cells (ksw.c:466-469); columns left of beg are zero
         const int lfirst = nzb ? base + __ffs(nzb) - 1 : INT_MAX;

@@ -74,16 +74,42 @@ constexpr int kRejectKey = kNumTiles * kClasses;
 constexpr int kHistSlots = kNumTiles * kClasses + 1;
 constexpr int kScanThreads = 1024;
 
-__global__ void ksw_sched_hist(const bsb_ext_job_t *__restrict__ jobs, int n, long long seq_bytes,
-                               const int32_t *__restrict__ cost, const uint8_t *__restrict__ map, int pack16,
-                               int mat_max, int *__restrict__ hist, int32_t *__restrict__ key_out)
+// A job of the byte buffer, as ksw_diagonal reads it.
+struct BytesAcc {
+    const uint8_t *qs, *ts;
+    __device__ __forceinline__ int q(int j) const { return __ldg(qs + j); }
+    __device__ __forceinline__ int t(int i) const { return __ldg(ts + i); }
+};
+
+// Keys and their histogram; and, unless cells are counted, the jobs whose result the main
+// diagonal decides (ksw_diagonal): these are answered here, get the key kDoneKey and are never
+// issued.  A warp takes `per` jobs at a time: a lane each for the checks and the key, then four
+// diagonals at once, eight lanes each (2M jobs of 10-140 bases: 0.38 ms, 26 us without the
+// diagonals; one diagonal after the other by the whole warp 0.52 ms; 64 jobs 9 against 46 us).
+// Half of those jobs end here: with the rows left out (ksw_core.cuh) the batch takes 8.0 ms
+// instead of 23.4.
+constexpr int32_t kDoneKey = -1;
+constexpr int kHistThreads = 256;
+__global__ void __launch_bounds__(kHistThreads)
+ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long long seq_bytes,
+               const uint8_t *__restrict__ seq, const int32_t *__restrict__ cost, const uint8_t *__restrict__ map,
+               int diagonals, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist, int32_t *__restrict__ key_out)
 {
     __shared__ int sh[kHistSlots];
+    __shared__ int8_t tab[kScoreTable];
     for (int i = threadIdx.x; i < kHistSlots; i += blockDim.x) sh[i] = 0;
+    load_score_table(P, tab);
     __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const bsb_ext_job_t jb = jobs[i];
-        const bool ok = jb.qlen >= 0 && jb.qlen < kMaxNeed && jb.tlen >= 0 && jb.w >= 0 && jb.h0 > 0 &&
+    const int lane = threadIdx.x & 31;
+    const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+    for (long long i0 = (long long)((int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; i0 < n;
+         i0 += (long long)warps * per) {
+        const int i = (int)(i0 + lane);
+        const bool in = lane < per && i0 + lane < n;
+        bsb_ext_job_t jb;
+        jb.qoff = jb.toff = 0, jb.qlen = jb.tlen = jb.h0 = jb.w = jb.end_bonus = jb.flags = 0;
+        if (in) jb = jobs[i];
+        const bool ok = in && jb.qlen >= 0 && jb.qlen < kMaxNeed && jb.tlen >= 0 && jb.w >= 0 && jb.h0 > 0 &&
                         jb.h0 <= (1 << 20) && jb.flags == 0 && jb.qoff >= 0 && jb.toff >= 0 &&
                         jb.qoff + jb.qlen <= seq_bytes && jb.toff + jb.tlen <= seq_bytes;
         int key;
@@ -99,14 +125,38 @@ __global__ void ksw_sched_hist(const bsb_ext_job_t *__restrict__ jobs, int n, lo
                 const long long c = (long long)jb.qlen * max(span, 0LL);
                 k = (uint32_t)min(c, (long long)0x7fffffff);
             }
-            const bool wide = pack16 && (kPack16Tiles >> t & 1) &&
-                              (long long)jb.h0 + (long long)jb.qlen * mat_max > kPack16MaxH;
+            const bool wide = P.pack16 && (kPack16Tiles >> t & 1) &&
+                              (long long)jb.h0 + (long long)jb.qlen * P.mat_max > kPack16MaxH;
             key = t >= kNumTiles ? kRejectKey
                   : wide         ? t * kClasses + kWideClass
                                  : t * kClasses + (kWideClass - 1 - cost_class(k));
         }
-        key_out[i] = key;
-        atomicAdd(&sh[key], 1);
+        if (diagonals) {
+            const int lim = key != kRejectKey && in ? diagonal_limit(P, jb.h0) : 0;
+            const uint8_t *qp = seq + jb.qoff, *tp = seq + jb.toff;
+            for (int r = 0; r < per; r += 4) {
+                const int b = r + (lane >> 3);
+                BytesAcc acc;
+                acc.qs = (const uint8_t *)__shfl_sync(BSB_FULL_MASK, (unsigned long long)qp, b);
+                acc.ts = (const uint8_t *)__shfl_sync(BSB_FULL_MASK, (unsigned long long)tp, b);
+                const int qlen = __shfl_sync(BSB_FULL_MASK, jb.qlen, b), tlen = __shfl_sync(BSB_FULL_MASK, jb.tlen, b);
+                const int h0 = __shfl_sync(BSB_FULL_MASK, jb.h0, b), lm = __shfl_sync(BSB_FULL_MASK, lim, b);
+                int best, best_j, last;
+                const bool known = ksw_diagonal<8>(tab, P.mat_max, lm, qlen, tlen, h0, acc, lane, best, best_j, last);
+                if (known && (lane & 7) == 0) {
+                    bsb_ext_out_t o;
+                    o.score = best; o.qle = o.tle = best_j + 1;
+                    o.gtle = qlen; o.gscore = last; o.max_off = 0;
+                    out[i0 + b] = o;
+                }
+                const unsigned done = __ballot_sync(BSB_FULL_MASK, known);
+                if (lane >= r && lane < r + 4 && (done >> ((lane - r) * 8) & 1)) key = kDoneKey;
+            }
+        }
+        if (in) {
+            key_out[i] = key;
+            if (key != kDoneKey) atomicAdd(&sh[key], 1);
+        }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kHistSlots; i += blockDim.x)
@@ -164,8 +214,9 @@ __global__ void ksw_sched_scatter(const int32_t *__restrict__ key, int n, int *_
                                   int32_t *__restrict__ order)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int pos = atomicAdd(&cursor[key[i]], 1);
-        order[pos] = i;
+        const int k = key[i];
+        if (k == kDoneKey) continue;
+        order[atomicAdd(&cursor[k], 1)] = i;
     }
 }
 
@@ -231,8 +282,12 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
     if (e != cudaSuccess) return e;
     if (n > 0) {
         const int nb = (int)min((int64_t)n_sm * 8, (n + 255) / 256);
-        ksw_sched_hist<<<nb, 256, 0, st>>>(d_jobs, (int)n, (long long)seq_bytes, d_cost, d_map, Q.pack16,
-                                           Q.mat_max, hist, key);
+        // jobs a warp takes at a time: 32, or 4 where that still leaves warps free (the diagonals of
+        // a warp's jobs are a chain of dependent loads, four at a time)
+        const int per = n >= (int64_t)n_sm * 8 * (kHistThreads / 32) * 4 ? 32 : 4;
+        const int hb = (int)min((int64_t)n_sm * 8, (n + per * (kHistThreads / 32) - 1) / (per * (kHistThreads / 32)));
+        ksw_sched_hist<<<hb, kHistThreads, 0, st>>>(Q, d_jobs, (int)n, (long long)seq_bytes, d_seq, d_cost, d_map,
+                                                    d_cells == nullptr, per, d_out, hist, key);
         ksw_sched_scan<<<1, kScanThreads, 0, st>>>(hist, cursor, ranges, rejected);
         ksw_sched_scatter<<<nb, 256, 0, st>>>(key, (int)n, cursor, order);
         e = cudaGetLastError();

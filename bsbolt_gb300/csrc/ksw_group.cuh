@@ -251,6 +251,21 @@ __device__ __forceinline__ void ksw_group_run(const KswParams &P, const bsb_ext_
             max_off = max_off > d ? max_off : d;
         }
 
+        // rows that can no longer change the result (ksw_core.cuh); not where cells are counted
+        bool fin = false;
+        if (!cells) {
+            const bool want = live && rows_may_be_done(gscore, m, mj, qlen, P.mat_max);
+            if (__any_sync(act, want)) {
+                int U = 0;
+#pragma unroll
+                for (int s = 0; s < C; ++s) {
+                    const int X = max(Hs[s], Es[s]);
+                    if (X > 0) U = max(U, X + P.mat_max * (qlen - base - s));
+                }
+                fin = group_max<G>(act, U) < gscore && want;
+            }
+        }
+
         // shrink to the non-zero cells (ksw.c:466-469)
         // first and last non-zero column, reduced together as (2047 - first, last + 1)
         int fnz, lnz;
@@ -267,7 +282,7 @@ __device__ __forceinline__ void ksw_group_run(const KswParams &P, const bsb_ext_
         beg = fnz < end ? fnz : end;
         end = jj + 2 < qlen ? jj + 2 : qlen;
         ++i;
-        const bool done = !live || zd || i >= tlen;
+        const bool done = !live || zd || fin || i >= tlen;
         if (done) {
             if (gl == 0) {
                 bsb_ext_out_t o;

@@ -325,6 +325,28 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
             max_off = max_off > d ? max_off : d;
         }
 
+        // rows that can no longer change the result (ksw_core.cuh); not where cells are counted.
+        // Per half the maximum of X + a(C2 - 1 - u) over the registers with X = max(H, E) > 0,
+        // then the half's first column is put in: at most 2047 + 15 * 15, inside 16 bits.
+        bool fin = false;
+        if (!cells) {
+            const int a = P.mat_max;
+            const bool want = live && rows_may_be_done(gscore, m, mj, qlen, a);
+            if (__any_sync(act, want)) {
+                uint32_t um = 0;
+#pragma unroll
+                for (int u = 0; u < C2; ++u) {
+                    const uint32_t X = __vimax_s16x2_relu(Hs[u], Es[u]);
+                    const uint32_t nz = __viaddmin_s16x2_relu(X, 0u, 0x00010001u) * 0xffffu;
+                    um = __vimax_s16x2_relu(um, (X + (uint32_t)(a * (C2 - 1 - u)) * 0x00010001u) & nz);
+                }
+                const int lo = lo16(um), hi = hi16(um);
+                const int U = max(lo > 0 ? lo + a * (qlen - base - C2 + 1) : 0,
+                                  hi > 0 ? hi + a * (qlen - base - 2 * C2 + 1) : 0);
+                fin = group_max<G>(act, U) < gscore && want;
+            }
+        }
+
         // shrink to the non-zero cells (ksw.c:466-469), as in ksw_group_run
         int fnz, lnz;
         if constexpr (G == 32) {
@@ -340,7 +362,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         beg = fnz < end ? fnz : end;
         end = jj + 2 < qlen ? jj + 2 : qlen;
         ++i;
-        const bool done = !live || zd || i >= tlen;
+        const bool done = !live || zd || fin || i >= tlen;
         if (done) {
             if (gl == 0) {
                 bsb_ext_out_t o;
