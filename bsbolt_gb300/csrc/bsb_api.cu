@@ -295,7 +295,7 @@ static void scan_pieces(const bsb_ext_job_t *jobs, int64_t n, int64_t per, int n
 // the context's map uses when the caller cannot tell which are needed).
 static int extend_device(bsb_ctx *ctx, const bsb_ext_param_t *param, const bsb_ext_job_t *d_jobs,
                          int64_t n_jobs, const uint8_t *d_seq, int64_t seq_bytes, const int32_t *d_cost,
-                         bsb_ext_out_t *d_out, int64_t *d_cells, uint64_t tiles, cudaEvent_t e0 = nullptr,
+                         bsb_ext_out_t *d_out, int64_t *d_cells, int builtin, uint64_t tiles, cudaEvent_t e0 = nullptr,
                          cudaEvent_t e1 = nullptr)
 {
     if (!ctx) return BSB_EINVAL;
@@ -308,7 +308,7 @@ static int extend_device(bsb_ctx *ctx, const bsb_ext_param_t *param, const bsb_e
     if ((rc = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice"))) return rc;
     if ((rc = bsb_ensure(ctx, &ctx->scratch, &ctx->scratch_bytes, ksw_scratch_bytes(n_jobs), "extension scratch")))
         return rc;
-    cudaError_t e = ksw_launch(P, d_jobs, n_jobs, seq_bytes, d_seq, d_cost, ctx->d_tile_map, tiles, d_out, d_cells,
+    cudaError_t e = ksw_launch(P, d_jobs, n_jobs, seq_bytes, d_seq, d_cost, ctx->d_tile_map, builtin, tiles, d_out, d_cells,
                                ctx->scratch, ctx->n_sm, ctx->stream, e0 ? e0 : ctx->ev0, e1 ? e1 : ctx->ev1,
                                ctx->tile_ev, &ctx->ms);
     ctx->pending_ksw = 1;
@@ -322,7 +322,9 @@ extern "C" int bsb_extend_batch_device(bsb_ctx *ctx, const bsb_ext_param_t *para
                                        const int32_t *d_cost, bsb_ext_out_t *d_out, int64_t *d_cells)
 {
     if (!ctx) return BSB_EINVAL;
-    return extend_device(ctx, param, d_jobs, n_jobs, d_seq, seq_bytes, d_cost, d_out, d_cells, ctx->map_tiles);
+    const int builtin = ksw_builtin(n_jobs, ctx->n_sm);
+    const uint64_t tiles = ctx->d_tile_map ? ctx->map_tiles : ksw_map_tiles(ksw_builtin_tile_map(builtin));
+    return extend_device(ctx, param, d_jobs, n_jobs, d_seq, seq_bytes, d_cost, d_out, d_cells, builtin, tiles);
 }
 
 extern "C" int bsb_tile_shapes(int32_t *G, int32_t *C, int max)
@@ -409,7 +411,9 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     const int64_t per = n_jobs >= kChunkFrom ? (n_jobs + BSB_MAX_CHUNKS - 1) / BSB_MAX_CHUNKS : n_jobs;
     const int nck = (int)((n_jobs + per - 1) / per);
     JobScan piece[BSB_MAX_CHUNKS];
-    scan_pieces(jobs, n_jobs, per, nck, seq_bytes, ctx->tile_map, piece);
+    const int builtin = ksw_builtin(per, ctx->n_sm);      // one map for all pieces
+    const uint8_t *map = ctx->d_tile_map ? ctx->tile_map : ksw_builtin_tile_map(builtin);
+    scan_pieces(jobs, n_jobs, per, nck, seq_bytes, map, piece);
     for (int k = 0; k < nck; ++k)          // every job is checked before any device work
         if (piece[k].first_bad < n_jobs) return check_jobs(ctx, jobs + piece[k].first_bad, 1, seq_bytes,
                                                            piece[k].first_bad);
@@ -448,7 +452,7 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
             (rc = bsb_cuda(ctx, cudaStreamWaitEvent(ctx->stream, ev[0], 0), "event")))
             return rc;
         if ((rc = extend_device(ctx, param, d_jobs + lo, cnt, d_seq, seq_bytes, nullptr, d_out + lo,
-                                d_cells ? d_cells + lo : nullptr, tiles, ev[2], ev[3])))
+                                d_cells ? d_cells + lo : nullptr, builtin, tiles, ev[2], ev[3])))
             return rc;
         if ((rc = bsb_cuda(ctx, cudaEventRecord(ev[1], ctx->stream), "event")) ||
             (rc = bsb_cuda(ctx, cudaStreamWaitEvent(ctx->d2h, ev[1], 0), "event")) ||

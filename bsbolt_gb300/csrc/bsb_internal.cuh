@@ -134,19 +134,22 @@ int ksw_max_qlen();
 // Device word counting the jobs the last launch rejected (precondition failures).
 int *ksw_rejected_counter(void *scratch);
 // d_map: the tile map in device memory (BSB_TILE_MAP_LEN bytes), or NULL for
-// the built-in default; tiles: bit t set = launch tile shape t (the shapes the
-// batch's query lengths map to; a shape left out leaves its jobs unrun).
+// the built-in map number `builtin`; tiles: bit t set = launch tile shape t (the shapes that
+// map gives the batch's query lengths; a shape left out leaves its jobs unrun).
 // tile_ev (optional, 2 * BSB_NUM_TILES events): per-shape timing marks as in bsb_ctx.
 // ms (optional): run the shape kernels of batches below ksw_concurrent_below() jobs
 // on st and ms->aux (joined back into st before ev1).
 cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
-                       const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, uint64_t tiles,
+                       const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
                        cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev = nullptr,
                        const KswStreams *ms = nullptr);
 int64_t ksw_concurrent_below();
-// The built-in tile map (host copy, BSB_TILE_MAP_LEN entries).
+// The built-in tile map (host copy, BSB_TILE_MAP_LEN entries); the number of the built-in map a
+// batch of n jobs runs on where the caller has set none, and that map.
 const uint8_t *ksw_default_tile_map();
+int ksw_builtin(int64_t n, int n_sm);
+const uint8_t *ksw_builtin_tile_map(int builtin);
 // Shape of tile t; -1 if t is out of range.
 int ksw_tile_shape(int t, int *G, int *C);
 // Set of tile shapes a map uses (bit t).

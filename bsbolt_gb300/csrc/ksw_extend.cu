@@ -37,7 +37,8 @@
 #include "ksw_group16.cuh"
 #include "ksw_tiles.cuh"
 
-__constant__ KswTileMap c_default_tile_map = kDefaultTileMap;
+__constant__ KswTileMap c_tile_maps[kBuiltinMaps] = {kBuiltinTileMaps[0], kBuiltinTileMaps[1], kBuiltinTileMaps[2],
+                                                     kBuiltinTileMaps[3]};
 
 namespace {
 
@@ -93,7 +94,7 @@ constexpr int kHistThreads = 256;
 __global__ void __launch_bounds__(kHistThreads)
 ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long long seq_bytes,
                const uint8_t *__restrict__ seq, const int32_t *__restrict__ cost, const uint8_t *__restrict__ map,
-               int diagonals, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist, int32_t *__restrict__ key_out)
+               int builtin, int diagonals, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist, int32_t *__restrict__ key_out)
 {
     __shared__ int sh[kHistSlots];
     __shared__ int8_t tab[kScoreTable];
@@ -117,7 +118,7 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
             key = kRejectKey;
         } else {
             const int need = jb.qlen + 1;
-            const int t = map ? map[need] : c_default_tile_map.tile[need];
+            const int t = map ? map[need] : c_tile_maps[builtin].tile[need];
             uint32_t k;
             if (cost) k = (uint32_t)max(cost[i], 0);
             else {
@@ -240,6 +241,10 @@ int64_t ksw_concurrent_below() { return (int64_t)1 << 20; }
 
 int *ksw_rejected_counter(void *scratch) { return (int *)scratch + 3 * kNumTiles; }
 
+int ksw_builtin(int64_t n, int n_sm) { return ksw_builtin_of(n, n_sm); }
+
+const uint8_t *ksw_builtin_tile_map(int builtin) { return kBuiltinTileMaps[builtin].tile; }
+
 const uint8_t *ksw_default_tile_map() { return kDefaultTileMap.tile; }
 
 int ksw_tile_shape(int t, int *G, int *C)
@@ -258,7 +263,7 @@ uint64_t ksw_map_tiles(const uint8_t *map)
 }
 
 cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
-                       const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, uint64_t tiles,
+                       const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
                        cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev, const KswStreams *ms)
 {
@@ -287,7 +292,7 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
         const int per = n >= (int64_t)n_sm * 8 * (kHistThreads / 32) * 4 ? 32 : 4;
         const int hb = (int)min((int64_t)n_sm * 8, (n + per * (kHistThreads / 32) - 1) / (per * (kHistThreads / 32)));
         ksw_sched_hist<<<hb, kHistThreads, 0, st>>>(Q, d_jobs, (int)n, (long long)seq_bytes, d_seq, d_cost, d_map,
-                                                    d_cells == nullptr, per, d_out, hist, key);
+                                                    builtin, d_cells == nullptr, per, d_out, hist, key);
         ksw_sched_scan<<<1, kScanThreads, 0, st>>>(hist, cursor, ranges, rejected);
         ksw_sched_scatter<<<nb, 256, 0, st>>>(key, (int)n, cursor, order);
         e = cudaGetLastError();

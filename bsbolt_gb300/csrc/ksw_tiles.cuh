@@ -78,6 +78,31 @@ constexpr KswTileMap make_default_tile_map()
 
 constexpr KswTileMap kDefaultTileMap = make_default_tile_map();
 
+// The built-in maps by batch size.  The default map fills the GPU with 4-lane groups only from a
+// few hundred thousand jobs on; a smaller batch is bound by the rows of its longest jobs, one after
+// the other, and a row takes the fewer cycles the more lanes share it (a 4x32 group about 1600, a
+// 32x6 warp 600).  So the fewer jobs, the wider the groups, and few shapes, so that few launches
+// follow one another.  Jobs of 10-140 bases, us (default map in brackets): 64 jobs 129 (328), 3000
+// 181 (490), 10,000 220 (537), 30,000 300 (586), 130,000 774 (792), 260,000 1362 (1349).
+// Queries beyond the bands given here keep the default's shapes.
+constexpr int kBuiltinMaps = 4;
+constexpr KswTileMap with_band(KswTileMap m, int lo, int hi, int G, int C)
+{
+    for (int need = lo; need <= hi; ++need) m.tile[need] = (uint8_t)tile_index(G, C);
+    return m;
+}
+constexpr KswTileMap kBuiltinTileMaps[kBuiltinMaps] = {
+    kDefaultTileMap,
+    with_band(with_band(kDefaultTileMap, 1, 64, 4, 16), 65, 144, 8, 18),
+    with_band(kDefaultTileMap, 1, 160, 16, 10),
+    with_band(with_band(kDefaultTileMap, 1, 192, 32, 6), 193, 256, 32, 8),
+};
+// The built-in map of a batch of n jobs (lines between the measured sizes where two maps meet).
+inline int ksw_builtin_of(int64_t n, int n_sm)
+{
+    return n <= 50 * (int64_t)n_sm ? 3 : n <= 90 * (int64_t)n_sm ? 2 : n <= 1300 * (int64_t)n_sm ? 1 : 0;
+}
+
 // Launches the persistent kernel of one tile shape over a range of the scheduled
 // order: the jobs order[range[0] .. range[1]), drawn through *counter.
 typedef cudaError_t (*KswTileLaunch)(const KswParams &P, const bsb_ext_job_t *jobs, const uint8_t *seq,

@@ -54,3 +54,26 @@ def test_diagonal_jobs_and_left_out_rows(gpu_ctx, scoring):
     assert np.array_equal(out, ref)
     out, cells = extend.ksw_extend2_batch(gpu_ctx, jobs, seq, mat, o_del, e_del, o_ins, e_ins, zdrop, want_cells=True)
     assert np.array_equal(out, ref) and np.array_equal(cells, rcells)
+
+
+@pytest.mark.parametrize("per_sm", [50, 90, 1300])
+@pytest.mark.parametrize("past", [0, 1])
+@pytest.mark.parametrize("device", [False, True], ids=["host", "device"])
+def test_built_in_maps_by_batch_size(gpu_ctx, per_sm, past, device):
+    """Both sides of each line between two built-in tile maps, host and device entry."""
+    torch = pytest.importorskip("torch")
+    n = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + past
+    jobs, seq = synth.ksw_jobs(n, seed=n, qmin=1, qmax=300)
+    mat = synth.fill_scmat(1, 4)
+    ref, _ = oracle.ksw_batch(jobs, seq, mat, 6, 1, 6, 1, 100, n_threads=16)
+    if not device:
+        out = extend.ksw_extend2_batch(gpu_ctx, jobs, seq, mat, 6, 1, 6, 1, 100)
+    else:
+        dj, ds = torch.from_numpy(jobs.view(np.uint8).copy()).cuda(), torch.from_numpy(seq).cuda()
+        do = torch.zeros((n, 6), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        extend.ksw_extend2_device(gpu_ctx, dj.data_ptr(), n, ds.data_ptr(), len(seq),
+                                  extend.make_param(mat, 6, 1, 6, 1, 100), do.data_ptr())
+        torch.cuda.synchronize()
+        out = do.cpu().numpy()
+    assert np.array_equal(out, ref)
