@@ -819,8 +819,7 @@ def pipeline_ref1gb(ctx, n_pairs=200_000, batch_bases=10_000_000, tag="1gb", lea
                     f", 45% repeats), {n_reads // 2} directional pairs: 70% 2x150, "
                     f"30% 2x250, 2% adapter read-through; -K 10M batches ({len(batches)}); BWA defaults",
         "seq_len": int(bi.l_pac) * 2,
-        "occ_layout": ("64-symbol sectors (0.5 B/row)" if os.environ.get("BSB_OCC_SYM64") == "1"
-                       else "32-symbol sectors (1 B/row)"),
+        "occ_layout": "64-symbol sectors (0.5 B/row)",
         "gpu_mem_align1_read_pairs_per_s": round(n_reads / 2 / gpu_s, 1),
         "cpu_oracle_read_pairs_per_s": round(ns / 2 / cpu_s, 1), "cpu_oracle_sample_reads": ns,
         "regions_bit_exact_vs_oracle_on_sample": exact})

@@ -4,7 +4,7 @@
 // (64-byte occurrence blocks, uint64 sampled SA, 2-bit pac), so the BWA driver
 // can hand over what bwa_idx_load already read (bwa.c:363-524) or the library
 // can read the files itself (bwt_restore_bwt / bwt_restore_sa, bwt.c:420-457).
-// On the device the occurrence array is re-cut into 32-symbol sectors
+// On the device the occurrence array is re-cut into 64-symbol sectors
 // (fm_index.cuh); the SA and pac stay as they are.
 
 #include <algorithm>
@@ -16,10 +16,8 @@
 #include "fm_index.cuh"
 #include "scan.cuh"
 
-size_t seed_scratch_bytes(int n_threads, int max_len);
 size_t seed_padded_entries(int64_t total_bases, int n_reads, int mult);
-size_t seed_queue_entries(int64_t total_bases, int n_reads, int mult);
-int seed_threads(int n_sm, int max_len, int n_reads, uint64_t seq_len);
+size_t seed_queue_bytes(int64_t total_bases, int n_reads, int mult, int64_t *entries);
 cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, int split_width, int max_mem_intv,
                         int n_reads, const uint8_t *d_seqs, const int64_t *d_offs, int max_len,
                         void *d_padded, int *d_count, int64_t *d_out_off, void *d_out,
@@ -51,7 +49,6 @@ static DevFM dev_fm(const bsb_ctx *ctx)
     DevFM F;
     F.blk = (const uint4 *)ctx->idx_bwt;
     F.sb = (const uint64_t *)ctx->idx_sb;
-    F.sym64 = ctx->idx_sym64;
     F.sa = (const uint64_t *)ctx->idx_sa;
     F.sa_full = (const uint64_t *)ctx->idx_sa_full;
     F.primary = ctx->primary;
@@ -104,26 +101,21 @@ extern "C" int bsb_index_full_sa(bsb_ctx *ctx, int enable)
     return ctx->idx_sa_full ? 0 : bsb_fail(ctx, BSB_ENOMEM, "the full suffix array does not fit in device memory");
 }
 
-// Re-cuts the reference's occurrence array (64-byte blocks of 128 symbols: four uint64
-// counts, eight symbol words) into the 32-byte sectors occ_at reads; one thread per sector.
-__global__ void occ_sectors_kernel(const uint32_t *__restrict__ ref, uint64_t n_sectors, uint4 *__restrict__ out)
+// The even bits of x, packed.
+__device__ __forceinline__ uint32_t even_bits(uint32_t x)
 {
-    const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (s >= n_sectors) return;
-    const uint32_t *b = ref + (s >> 2) * 16;
-    const int q = (int)(s & 3);
-    uint32_t a = 0, c = 0, g = 0;
-    for (int w = 0; w < 2 * q; ++w) word_counts(b[8 + w], 16, a, c, g);
-    const uint64_t ca = ((uint64_t)b[1] << 32 | b[0]) + a;
-    const uint64_t cc = ((uint64_t)b[3] << 32 | b[2]) + c;
-    const uint64_t cg = ((uint64_t)b[5] << 32 | b[4]) + g;
-    out[2 * s] = make_uint4((uint32_t)ca, (uint32_t)(ca >> 32), (uint32_t)cc, (uint32_t)(cc >> 32));
-    out[2 * s + 1] = make_uint4((uint32_t)cg, (uint32_t)(cg >> 32), b[8 + 2 * q], b[9 + 2 * q]);
+    x &= 0x55555555u;
+    x = (x | x >> 1) & 0x33333333u;
+    x = (x | x >> 2) & 0x0f0f0f0fu;
+    x = (x | x >> 4) & 0x00ff00ffu;
+    return (x | x >> 8) & 0x0000ffffu;
 }
 
-// The same re-cut into 64-symbol sectors: counts relative to the sector's 2^32-row
-// superblock (whose block starts at word ((s >> 26) << 25) * 16), four symbol words.
-__global__ void occ_sectors64_kernel(const uint32_t *__restrict__ ref, uint64_t n_sectors, uint4 *__restrict__ out)
+// Re-cuts the reference's occurrence array (64-byte blocks of 128 symbols: four uint64
+// counts, eight symbol words) into the sectors of fm_index.cuh; one thread per sector.  The counts
+// are relative to the sector's 2^32-row superblock (whose block starts at word
+// ((s >> 26) << 25) * 16).
+__global__ void occ_sectors_kernel(const uint32_t *__restrict__ ref, uint64_t n_sectors, uint4 *__restrict__ out)
 {
     const uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (s >= n_sectors) return;
@@ -132,23 +124,18 @@ __global__ void occ_sectors64_kernel(const uint32_t *__restrict__ ref, uint64_t 
     const int h = (int)(s & 1);
     uint32_t a = 0, c = 0, g = 0;
     for (int w = 0; w < 4 * h; ++w) word_counts(b[8 + w], 16, a, c, g);
-    const uint64_t ca = ((uint64_t)b[1] << 32 | b[0]) + a - ((uint64_t)sbk[1] << 32 | sbk[0]);
-    const uint64_t cc = ((uint64_t)b[3] << 32 | b[2]) + c - ((uint64_t)sbk[3] << 32 | sbk[2]);
-    const uint64_t cg = ((uint64_t)b[5] << 32 | b[4]) + g - ((uint64_t)sbk[5] << 32 | sbk[4]);
-    out[2 * s] = make_uint4((uint32_t)ca, (uint32_t)cc, (uint32_t)cg, 0u);
-    out[2 * s + 1] = make_uint4(b[8 + 4 * h], b[9 + 4 * h], b[10 + 4 * h], b[11 + 4 * h]);
-}
-
-// Occurrence layout: 32-symbol sectors (one byte per row), or with BSB_OCC_SYM64=1 64-symbol
-// sectors (half a byte per row, for an index whose 32-symbol array would not fit the device).
-// Measured on GB300 the 32-symbol layout seeds faster even with the array far beyond L2: one
-// sector fetch per occurrence query either way, and half the counting (100 Mb reference, 400 MB
-// array: 3.08 against 3.30 ms per -K batch; 1 Gb reference, 4 GB array: 6.04 against 6.47 ms).
-static int occ_layout_sym64(uint64_t seq_len)
-{
-    const char *e = getenv("BSB_OCC_SYM64");
-    (void)seq_len;
-    return e && e[0] == '1';
+    uint64_t n[4];
+    for (int k = 0; k < 4; ++k)
+        n[k] = ((uint64_t)b[2 * k + 1] << 32 | b[2 * k]) - ((uint64_t)sbk[2 * k + 1] << 32 | sbk[2 * k]);
+    const uint64_t nc = n[1] + c, ng = n[2] + g, nt = n[3] + (64 * h - a - c - g);
+    uint32_t lo[2], hi[2];
+    for (int w = 0; w < 2; ++w) {
+        const uint32_t r0 = __brev(b[8 + 4 * h + 2 * w]), r1 = __brev(b[9 + 4 * h + 2 * w]);   // hi bits even, lo odd
+        hi[w] = even_bits(r0) | even_bits(r1) << 16;
+        lo[w] = even_bits(r0 >> 1) | even_bits(r1 >> 1) << 16;
+    }
+    out[2 * s] = make_uint4((uint32_t)(nc + ng + nt), (uint32_t)(ng + nt), (uint32_t)nt, 0u);
+    out[2 * s + 1] = make_uint4(lo[0], lo[1], hi[0], hi[1]);
 }
 
 extern "C" int bsb_index_upload(bsb_ctx *ctx, const bsb_index_view_t *v)
@@ -169,40 +156,33 @@ extern "C" int bsb_index_upload(bsb_ctx *ctx, const bsb_index_view_t *v)
     bsb_index_release(ctx);
     {
         // the reference blocks go to a zero-padded staging buffer of whole blocks, then are re-cut
-        // into sectors (four or two per block, one extra block of padding past the last symbol)
+        // into sectors (two per block, one extra block of padding past the last symbol)
         const size_t ref_bytes = n_blocks * 64, copy = std::min<size_t>(v->bwt_size * 4, ref_bytes);
-        const int sym64 = occ_layout_sym64(seq_len);
-        const uint64_t n_sectors = n_blocks * (sym64 ? 2 : 4);
+        const uint64_t n_sectors = n_blocks * 2;
         void *stage = nullptr;
         if ((rc = bsb_cuda(ctx, cudaMalloc(&ctx->idx_bwt, n_sectors * 32), "index: occurrence array"))) return rc;
         if ((rc = bsb_cuda(ctx, cudaMalloc(&stage, ref_bytes), "index: occurrence staging"))) return rc;
         rc = bsb_cuda(ctx, cudaMemsetAsync(stage, 0, ref_bytes, ctx->stream), "index memset");
         if (!rc) rc = bsb_cuda(ctx, cudaMemcpyAsync(stage, v->bwt, copy, cudaMemcpyHostToDevice, ctx->stream),
                                "index: occurrence upload");
-        if (!rc && sym64) {
-            // the A, C, G counts before each 2^32-row superblock: the header of its first block
-            const uint64_t n_sb = (seq_len >> 32) + 1;
-            std::vector<uint64_t> sb(3 * n_sb, 0);
-            for (uint64_t k = 1; k < n_sb; ++k) {
-                const uint64_t w = (k << 25) * 16;
-                if (w + 6 > (uint64_t)v->bwt_size) break;
-                for (int c = 0; c < 3; ++c) sb[3 * k + c] = (uint64_t)v->bwt[w + 2 * c + 1] << 32 | v->bwt[w + 2 * c];
-            }
-            rc = bsb_cuda(ctx, cudaMalloc(&ctx->idx_sb, sb.size() * 8), "index: superblock counts");
-            if (!rc) rc = bsb_cuda(ctx, cudaMemcpyAsync(ctx->idx_sb, sb.data(), sb.size() * 8, cudaMemcpyHostToDevice,
-                                                        ctx->stream), "index: superblock counts");
-            if (!rc) rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "index: superblock counts");
+        // the counts of symbols above A, C, G before each 2^32-row superblock, from its first block's header
+        const uint64_t n_sb = (seq_len >> 32) + 1;
+        std::vector<uint64_t> sb(3 * n_sb, 0);
+        for (uint64_t k = 1; k < n_sb; ++k) {
+            const uint64_t w = (k << 25) * 16;
+            if (w + 8 > (uint64_t)v->bwt_size) break;
+            uint64_t above = 0;
+            for (int c = 3; c >= 1; --c)
+                sb[3 * k + c - 1] = above += (uint64_t)v->bwt[w + 2 * c + 1] << 32 | v->bwt[w + 2 * c];
         }
+        if (!rc) rc = bsb_cuda(ctx, cudaMalloc(&ctx->idx_sb, sb.size() * 8), "index: superblock counts");
+        if (!rc) rc = bsb_cuda(ctx, cudaMemcpyAsync(ctx->idx_sb, sb.data(), sb.size() * 8, cudaMemcpyHostToDevice,
+                                                    ctx->stream), "index: superblock counts");
         if (!rc) {
-            if (sym64)
-                occ_sectors64_kernel<<<(unsigned)((n_sectors + 255) / 256), 256, 0, ctx->stream>>>(
-                    (const uint32_t *)stage, n_sectors, (uint4 *)ctx->idx_bwt);
-            else
-                occ_sectors_kernel<<<(unsigned)((n_sectors + 255) / 256), 256, 0, ctx->stream>>>(
-                    (const uint32_t *)stage, n_sectors, (uint4 *)ctx->idx_bwt);
+            occ_sectors_kernel<<<(unsigned)((n_sectors + 255) / 256), 256, 0, ctx->stream>>>(
+                (const uint32_t *)stage, n_sectors, (uint4 *)ctx->idx_bwt);
             rc = bsb_cuda(ctx, cudaGetLastError(), "index: occurrence sectors");
         }
-        ctx->idx_sym64 = sym64;
         if (!rc) rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "index: occurrence sectors");
         cudaFree(stage);
         if (rc) return rc;
@@ -354,10 +334,11 @@ int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_r
     const size_t padded = seed_padded_entries(total_bases, n_reads, mult) * sizeof(DevIntv);
     if (max_len > BSB_SEED_MAX_LEN) return bsb_fail(ctx, BSB_ETOOLONG, "max_len %d > %d", max_len, BSB_SEED_MAX_LEN);
     const DevFM F = dev_fm(ctx);
-    const size_t lists = seed_scratch_bytes(seed_threads(ctx->n_sm, max_len, n_reads, F.seq_len), max_len);
-    const size_t qn = seed_queue_entries(total_bases, n_reads, mult);
+    const size_t lists = seed_plan(ctx->n_sm, max_len, n_reads, F.seq_len).list_bytes;
+    int64_t qn = 0;
+    const size_t queue_b = (seed_queue_bytes(total_bases, n_reads, mult, &qn) + 255) & ~(size_t)255;
     const size_t tot_b = (sizeof(int) * (size_t)n_reads + 255) & ~(size_t)255;
-    const size_t need = padded + lists + 256 * 6 + sizeof(int) * (2 * (size_t)n_reads + 64) + 8 * qn + tot_b +
+    const size_t need = padded + lists + 256 * 6 + sizeof(int) * (2 * (size_t)n_reads + 128) + queue_b + tot_b +
                         sizeof(int64_t) * (size_t)scan_tmp_words(n_reads);
     if ((rc = bsb_ensure(ctx, &ctx->seed_scratch, &ctx->seed_scratch_bytes, need, "seed scratch"))) return rc;
     char *s = (char *)ctx->seed_scratch;
@@ -365,12 +346,12 @@ int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_r
     void *d_lists = s + ((padded + 255) & ~(size_t)255);
     int *d_count = (int *)((char *)d_lists + ((lists + 255) & ~(size_t)255));
     int *d_ctrl = d_count + ((2 * n_reads + 63) & ~63);     // two counts per read (seed_kernel's two parts)
-    void *d_queue = d_ctrl + 64;                              // pass-2 work items (int2)
-    int *d_tot = (int *)((char *)d_queue + ((8 * qn + 255) & ~(size_t)255));     // seeds kept per read
+    void *d_queue = d_ctrl + 64;                              // pass-2 work items
+    int *d_tot = (int *)((char *)d_queue + queue_b);         // seeds kept per read
     int64_t *d_scan_tmp = (int64_t *)((char *)d_tot + tot_b);
     cudaError_t e = seed_launch(F, opt->min_seed_len, opt->split_factor, opt->split_width, opt->max_mem_intv, n_reads,
                                 d_seqs, d_offs, max_len, d_padded, d_count, d_out_off, d_out, d_lists, d_ctrl,
-                                d_queue, (int64_t)qn, d_tot, d_scan_tmp, mult, ctx->n_sm, ctx->stream);
+                                d_queue, qn, d_tot, d_scan_tmp, mult, ctx->n_sm, ctx->stream);
     ctx->seed_ctrl = d_ctrl;
     return bsb_cuda(ctx, e, "seed launch");
 }

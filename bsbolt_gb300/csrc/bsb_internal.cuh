@@ -48,8 +48,7 @@ struct bsb_ctx {
     // device-resident FM-index (reference layout) and its scalars
     int has_index = 0;
     void *idx_bwt = nullptr, *idx_sa = nullptr, *idx_pac = nullptr;
-    void *idx_sb = nullptr;       // superblock counts of the 64-symbol occurrence layout
-    int idx_sym64 = 0;            // occurrence layout: 1 = 64 symbols per sector, 0 = 32
+    void *idx_sb = nullptr;       // superblock counts of the occurrence array
     void *idx_sa_full = nullptr;  // every row's SA value (built at upload when it fits), or NULL
     void *idx_opac = nullptr;     // original (unconverted) reference, 2-bit, for the methylation calls
     uint64_t primary = 0, seq_len = 0, n_sa = 0;
@@ -170,3 +169,10 @@ constexpr int kSeedSlotMultMax = 64;
 int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_reads, const uint8_t *d_seqs,
                             const int64_t *d_offs, int64_t total_bases, int32_t max_len, bsb_intv_t *d_out,
                             int64_t *d_out_off, int mult);
+
+// The launch shape of a seeding batch (seed.cu).
+struct SeedPlan {
+    int blocks, rho, region_cap;
+    size_t list_bytes;
+};
+SeedPlan seed_plan(int n_sm, int max_len, int n_reads, uint64_t seq_len);

@@ -2,18 +2,25 @@
 //
 // The occurrence array holds the reference's information (bwt.h:70-78,
 // bwtindex.c:151-173: per 128 BWT symbols four uint64 cumulative counts and
-// eight uint32 words of 2-bit symbols) re-cut at upload into 32-byte sectors of
-// 32 or 64 symbols that carry their own counts, so an occurrence query touches
-// one 32-byte sector and counts inside two or four words instead of a 64-byte
-// block and up to eight words.  Nothing else of the index is touched by a query.
+// eight uint32 words of 2-bit symbols) re-cut at upload (occ_sectors_kernel) into one
+// 32-byte sector per 64 symbols, so an occurrence query reads one sector: two 16-byte
+// loads of one transaction, at the reference's density (0.5 byte per row).
+//
+// What a query wants is not a base's count alone: bwt_extend by base c needs the
+// occurrences of c and, for the other strand's interval, of the bases above c.  Both follow
+// from two cumulative counts, the symbols >= c and the symbols > c, so a sector holds the
+// counts of symbols > A, > C and > G before it, and its symbols as two bit planes (lo, hi; the
+// first symbol in bit 0): "symbol >= k" is one expression of the planes, and each cumulative
+// count two population counts.  Against 32-symbol sectors with a count per base and symbols two
+// bits apart: half the bytes (more of the index in L2), 8 population counts an extension
+// instead of 12, and no 64-bit arithmetic for an index below 2^32 rows.
 #pragma once
 
 #include <stdint.h>
 
 struct DevFM {
-    const uint4 *blk;        // 32-byte occurrence sectors (layouts below)
-    const uint64_t *sb;      // 64-symbol layout: A, C, G counts before each 2^32-row superblock
-    int sym64;               // 1: 64-symbol sectors, 0: 32-symbol sectors
+    const uint4 *blk;        // 32-byte occurrence sectors
+    const uint64_t *sb;      // symbols > A, > C, > G before each 2^32-row superblock
     const uint64_t *sa;      // sampled suffix array, sa[0] = (uint64_t)-1
     const uint64_t *sa_full; // every row's bwt_sa value (seq_len + 1 entries), or NULL
     uint64_t primary;
@@ -26,25 +33,12 @@ struct DevIntv {             // bwtintv_t (bwt.h:60-62)
     uint64_t x0, x1, x2, info;
 };
 
-struct Occ4 {
-    uint64_t c[4];
-};
+// Sector s: {symbols > A, > C, > G in the rows of its superblock before it, 0},
+// {lo plane of symbols 0-31, lo of 32-63, hi of 0-31, hi of 32-63}.
+constexpr int kSectorSyms = 64;
 
-// Device layouts of the occurrence array, built from the reference's at upload
-// (occ_sectors_kernel / occ_sectors64_kernel, bsb_index.cu); either way an occurrence
-// query reads one 32-byte sector (two 16-byte loads of one transaction) and T follows
-// from the row:
-//  - 32 symbols per sector (1 byte per symbol): the uint64 counts of A, C and G in the
-//    rows before the sector's first symbol, then its two uint32 words of 2-bit symbols,
-//    most significant pair first; a query counts inside at most two words.
-//  - 64 symbols per sector (0.5 byte per symbol, the reference's density): the uint32
-//    counts of A, C and G before the sector relative to its 2^32-row superblock (whose
-//    uint64 counts sit in a small array, sb), one unused word, then four symbol words; a
-//    query counts inside at most four words.  Half the bytes of the first layout, so an
-//    index that would outgrow L2 keeps more of itself there.
-constexpr int kSectorSyms = 32;
-
-// Counts of A, C, G among the first n (0..16) symbols of x.
+// Counts of A, C, G among the first n (0..16) symbols of x, a word of the reference's array (most
+// significant pair first).
 __device__ __forceinline__ void word_counts(uint32_t x, int n, uint32_t &a, uint32_t &c, uint32_t &g)
 {
     const uint32_t keep = n >= 16 ? 0xffffffffu : ~(0xffffffffu >> (2 * n));
@@ -54,90 +48,49 @@ __device__ __forceinline__ void word_counts(uint32_t x, int n, uint32_t &a, uint
     g += __popc(hi & ~lo & keep);
 }
 
-// Occurrences of each base in rows [0, kk] of the $-free BWT (bwt_occ4, bwt.c:169-187);
-// kk is k after the $ adjustment.  *word receives the symbol word holding kk.
-__device__ __forceinline__ Occ4 occ_at64(const DevFM &F, uint64_t kk, uint32_t *word)
-{
-    const uint4 *p = F.blk + (kk >> 6) * 2;
-    const uint4 v0 = __ldg(p), v1 = __ldg(p + 1);
-    const int n = (int)(kk & 63) + 1;                  // symbols counted in this sector
-    uint32_t a = 0, c = 0, g = 0;
-    word_counts(v1.x, n >= 16 ? 16 : n, a, c, g);
-    word_counts(v1.y, n >= 32 ? 16 : n > 16 ? n - 16 : 0, a, c, g);
-    word_counts(v1.z, n >= 48 ? 16 : n > 32 ? n - 32 : 0, a, c, g);
-    word_counts(v1.w, n > 48 ? n - 48 : 0, a, c, g);
-    uint64_t ba = 0, bc = 0, bg = 0;
-    if (kk >> 32) {                                    // past the first 2^32 rows
-        const uint64_t *b = F.sb + 3 * (kk >> 32);
-        ba = __ldg(b), bc = __ldg(b + 1), bg = __ldg(b + 2);
-    }
-    Occ4 o;
-    o.c[0] = ba + v0.x + a;
-    o.c[1] = bc + v0.y + c;
-    o.c[2] = bg + v0.z + g;
-    o.c[3] = kk + 1 - o.c[0] - o.c[1] - o.c[2];
-    if (word) {
-        const int wi = (int)(kk & 63) >> 4;
-        *word = wi == 0 ? v1.x : wi == 1 ? v1.y : wi == 2 ? v1.z : v1.w;
-    }
-    return o;
-}
-
-__device__ __forceinline__ Occ4 occ_at(const DevFM &F, uint64_t kk, uint32_t *word = nullptr)
-{
-    if (F.sym64) return occ_at64(F, kk, word);
-    const uint4 *p = F.blk + (kk >> 5) * 2;
-    const uint4 v0 = __ldg(p), v1 = __ldg(p + 1);
-    const int pos = (int)(kk & 31);
-    uint32_t a = 0, c = 0, g = 0;
-    word_counts(v1.z, pos >= 16 ? 16 : pos + 1, a, c, g);
-    word_counts(v1.w, pos >= 16 ? pos - 15 : 0, a, c, g);
-    Occ4 o;
-    o.c[0] = ((uint64_t)v0.y << 32 | v0.x) + a;
-    o.c[1] = ((uint64_t)v0.w << 32 | v0.z) + c;
-    o.c[2] = ((uint64_t)v1.y << 32 | v1.x) + g;
-    o.c[3] = kk + 1 - o.c[0] - o.c[1] - o.c[2];
-    if (word) *word = pos >= 16 ? v1.w : v1.z;
-    return o;
-}
-
-__device__ __forceinline__ Occ4 occ4(const DevFM &F, uint64_t k)
-{
-    if (k == (uint64_t)-1) {
-        Occ4 z;
-        z.c[0] = z.c[1] = z.c[2] = z.c[3] = 0;
-        return z;
-    }
-    return occ_at(F, k - (k >= F.primary));
-}
-
-// bwt_2occ4 (bwt.c:189-220) without branches, so the threads of a warp never split over
-// whether k and l share a block.
-__device__ __forceinline__ void occ4_pair(const DevFM &F, uint64_t k, uint64_t l, Occ4 &ok, Occ4 &ol)
-{
-    const bool kz = k == (uint64_t)-1, lz = l == (uint64_t)-1;
-    const uint64_t kk = kz ? 0 : k - (k >= F.primary), ll = lz ? 0 : l - (l >= F.primary);
-    ok = occ_at(F, kk);
-    ol = occ_at(F, ll);
-    if (kz) ok.c[0] = ok.c[1] = ok.c[2] = ok.c[3] = 0;
-    if (lz) ol.c[0] = ol.c[1] = ol.c[2] = ol.c[3] = 0;
-}
-
 // F.L2[i] for i = 0..4, indexed with constants only (a dynamic index would copy the
 // kernel parameter to local memory).
-__device__ __forceinline__ uint64_t l2_at(const DevFM &F, int i)
+template <class P = uint64_t>
+__device__ __forceinline__ P l2_at(const DevFM &F, int i)
 {
-    return i == 0 ? F.L2[0] : i == 1 ? F.L2[1] : i == 2 ? F.L2[2] : i == 3 ? F.L2[3] : F.L2[4];
+    return i == 0   ? (P)F.L2[0]
+           : i == 1 ? (P)F.L2[1]
+           : i == 2 ? (P)F.L2[2]
+           : i == 3 ? (P)F.L2[3]
+                    : (P)F.L2[4];
 }
 
-__device__ __forceinline__ DevIntv set_intv(const DevFM &F, int c)   // bwt.h:80
+// Row k of the BWT as a position of its $-free array (bwt_occ4's adjustment, bwt.c:176), held inside
+// the array: k is at most seq_len on a valid index, so the clamp then changes nothing.
+template <class P>
+__device__ __forceinline__ P sym_row(const DevFM &F, P k)
 {
-    DevIntv r;
-    r.x0 = l2_at(F, c) + 1;
-    r.x2 = l2_at(F, c + 1) - l2_at(F, c);
-    r.x1 = l2_at(F, 3 - c) + 1;
-    r.info = 0;
-    return r;
+    k -= k >= (P)F.primary;
+    return k < (P)F.seq_len ? k : (P)F.seq_len - 1;
+}
+
+// Symbols >= c and > c in rows [0, kk] of the $-free BWT (bwt_occ4, bwt.c:169-187).  P: uint32_t
+// for an index below 2^32 rows, which has one superblock, else uint64_t.
+template <class P>
+__device__ __forceinline__ void occ_cumulative(const DevFM &F, P kk, int c, P &ge, P &gt)
+{
+    const uint4 *p = F.blk + (uint64_t)(kk >> 6) * 2;
+    const uint4 v = __ldg(p), s = __ldg(p + 1);
+    const uint64_t keep = ~0ull >> (63 - (int)(kk & 63));
+    const uint32_t k0 = (uint32_t)keep, k1 = (uint32_t)(keep >> 32);
+    // [symbol >= t] = (hi | lo & x) & (lo | y): hi|lo for t = 1, hi for 2, hi&lo for 3
+    const uint32_t xe = c == 1 ? ~0u : 0u, ye = c <= 2 ? ~0u : 0u;       // t = c (c = 0 counts every symbol)
+    const uint32_t xg = c == 0 ? ~0u : 0u, yg = c <= 1 ? ~0u : 0u;       // t = c + 1 (c = 3 counts none)
+    const uint32_t ne = __popc((s.z | (s.x & xe)) & (s.x | ye) & k0) + __popc((s.w | (s.y & xe)) & (s.y | ye) & k1);
+    const uint32_t ng = __popc((s.z | (s.x & xg)) & (s.x | yg) & k0) + __popc((s.w | (s.y & xg)) & (s.y | yg) & k1);
+    P be = c == 1 ? v.x : c == 2 ? v.y : v.z, bg = c == 0 ? v.x : c == 1 ? v.y : v.z;
+    if (sizeof(P) == 8) {
+        const uint64_t *b = F.sb + 3 * ((uint64_t)kk >> 32);
+        be += (P)__ldg(b + (c == 0 ? 0 : c - 1));
+        bg += (P)__ldg(b + (c == 3 ? 2 : c));
+    }
+    ge = c == 0 ? kk + 1 : be + ne;
+    gt = c == 3 ? 0 : bg + ng;
 }
 
 // One LF step of bwt_sa (bwt_invPsi, bwt.c:53-59): the row of the suffix one text
@@ -145,10 +98,13 @@ __device__ __forceinline__ DevIntv set_intv(const DevFM &F, int c)   // bwt.h:80
 __device__ __forceinline__ uint64_t lf_step(const DevFM &F, uint64_t k)
 {
     if (k == F.primary) return 0;
-    // the symbol row (bwt_invPsi uses k > primary, bwt.c:55) equals kk here, so one word serves both
-    const uint64_t kk = k - (k >= F.primary);
-    uint32_t x;
-    const Occ4 o = occ_at(F, kk, &x);
-    const int c = (int)(x >> ((~kk & 15) << 1) & 3);
-    return l2_at(F, c) + (c == 0 ? o.c[0] : c == 1 ? o.c[1] : c == 2 ? o.c[2] : o.c[3]);
+    // the symbol row (bwt_invPsi uses k > primary, bwt.c:55) equals the counted row here
+    const uint64_t kk = sym_row<uint64_t>(F, k);
+    const uint4 s = __ldg(F.blk + (kk >> 6) * 2 + 1);
+    const int n = (int)(kk & 31);
+    const uint32_t lo = (kk & 32) ? s.y : s.x, hi = (kk & 32) ? s.w : s.z;
+    const int c = (int)(lo >> n & 1u) | (int)(hi >> n & 1u) << 1;
+    uint64_t ge, gt;
+    occ_cumulative<uint64_t>(F, kk, c, ge, gt);
+    return l2_at(F, c) + ge - gt;
 }

@@ -1,22 +1,39 @@
 // seed.cu -- SMEM seeding (mem_collect_intv) and suffix-array lookups on sm_103a.
 //
-// mem_collect_intv (bsbolt/External/BWA/bwamem.c:118-166) runs its three passes as
-// independent work items of one persistent kernel (seed_kernel, state machine below):
+// mem_collect_intv (bsbolt/External/BWA/bwamem.c:118-166) runs three passes:
 //   pass 1  bwt_smem1 from every x (bwt.c:289-356), keep SMEMs >= min_seed_len;
-//   pass 2  re-seed from the middle of SMEMs >= split_len with <= split_width hits
-//           (a second launch: one item per such SMEM);
+//   pass 2  re-seed from the middle of SMEMs >= split_len with <= split_width hits;
 //   pass 3  bwt_seed_strategy1 (bwt.c:358-379) from every x;
-// compact_seeds then sorts each read's seeds by info.  Equal info means the same
-// substring and so the same interval, so the sort needs no tie rule.  The interval
-// lists of bwt_smem1 live in a per-thread slice of device scratch (they are short in
-// practice, but a repeat can make them as long as the read).  Every occurrence query
-// reads one 32-byte sector of the occurrence array (fm_index.cuh).  An index of fewer
-// than 2^32 - 2 rows runs the kernel on 32-bit intervals (96 registers, 5 blocks per SM,
-// 16-byte list entries); a larger one on 64-bit intervals (128 registers, 4 blocks).
+// then sorts each read's seeds by info.  Equal info means the same substring and so the same
+// interval, so the sort needs no tie rule and the order seeds are found in does not matter.
+//
+// What bounds it is the chain of dependent sector fetches: an interval can be extended by its next
+// base only once its two occurrence sectors have arrived.  bwt_smem1 keeps its matches in lock step
+// (all forward matches from x, then one round over all of them per base to the left), which makes
+// the chain of a read several hundred extensions long.  The matches are independent, though.  A
+// match [x, e) that the forward phase pushed can be extended to the left on its own until it has
+// fewer than min_intv occurrences, say to [b, e); it is an SMEM exactly if it cannot be extended
+// to the right there either, which is one extension more and asked only of matches long enough to be
+// seeds.  (bwt_smem1 emits the first match that fails in a round, and nothing for those behind it:
+// a shorter match [x, e') never stops before a longer one, b(e') <= b(e), and stops at the same b
+// exactly if [b, e') can still grow to the right.  Matches it drops for having the size of a longer
+// one are of the second kind.  It emits nothing but the longest match where the base left of x is
+// missing or an N.)
+//
+// So a warp takes a few reads: a lane each for the forward phases, every lane with one extension a
+// step, and the pushed matches go to a list of the warp; then the lanes take matches from the
+// list, one after the other, each extending its own to the left.  The re-seeds of pass 2 are
+// a second launch of the same two phases, with their threshold on the occurrences; pass 3 is a forward
+// phase of its own.  Against the lock-step form, a state machine with one thread per read and pass
+// (11-13 of 32 lanes active; now 20), one GB300, seeding stage of a batch with its copies: 64 reads
+// 0.76 -> 0.14 ms, 40k reads of 100 bases on a 2 Mb reference 1.51 -> 0.57, 67k of 150 on 100 Mb
+// 3.6 -> 1.73, 114k RRBS reads 3.2 -> 1.6; 15 % more extensions.
 //
 // bwt_sa (bwt.c:86-96) is one thread per suffix-array row: one load from the full
 // suffix array when it is resident, else LF steps until a sampled row, each step
 // one 32-byte sector.
+
+#include <algorithm>
 
 #include "bsb_internal.cuh"
 #include "fm_index.cuh"
@@ -24,117 +41,78 @@
 
 namespace {
 
-constexpr int kSeedBlock = 128;
+constexpr int kSeedBlock = 128, kSeedWarps = kSeedBlock / 32;
+constexpr int kSeedRho = 16;            // most reads (re-seeds) a warp takes at once
 
 struct SeedOpt {
     int min_seed_len, split_len, split_width, max_mem_intv;
 };
 
-// The interval a seeding thread works with: bwtintv_t's fields in 64 bits (DevIntv), or, for
-// an index of fewer than 2^32 - 2 rows, in 32 bits (SeedIntv32, info = qbeg << 16 | qend with
-// read positions below 2^16), which halves the registers and the scratch bytes an interval
-// costs.  IvT gives the info field's parts and the conversions to the output's DevIntv.
-struct SeedIntv32 {
-    uint32_t x0, x1, x2, info;
+// A bi-interval (bwtintv_t without info) in the width the index needs: 32 bits below
+// 2^32 - 2 rows, else 64.
+template <class P>
+struct Iv {
+    P x0, x1, x2;
 };
+constexpr uint64_t kNarrowRows = 0xfffffffdull;
 
-template <class IV> struct IvT;
-template <> struct IvT<DevIntv> {
-    using pos_t = uint64_t;
-    static constexpr uint64_t kMaxRows = ~0ull;
-    __device__ static uint64_t info(int qb, int qe) { return (uint64_t)(uint32_t)qb << 32 | (uint32_t)qe; }
-    __device__ static int qbeg(const DevIntv &v) { return (int)(v.info >> 32); }
-    __device__ static int qend(const DevIntv &v) { return (int)(uint32_t)v.info; }
-    __device__ static DevIntv out(const DevIntv &v) { return v; }
-    __device__ static DevIntv in(const DevIntv &v) { return v; }
+// A match on a warp's list: its interval, and slot of the read << 21 | start << 11 | end (reads
+// have at most 1024 bases, so a start is below 2^10 and an end below 2^11).
+struct alignas(16) Match32 {
+    uint32_t x0, x1, x2, pos;
 };
-template <> struct IvT<SeedIntv32> {
-    using pos_t = uint32_t;
-    static constexpr uint64_t kMaxRows = 0xfffffffdull;
-    __device__ static uint32_t info(int qb, int qe) { return (uint32_t)qb << 16 | (uint32_t)qe; }
-    __device__ static int qbeg(const SeedIntv32 &v) { return (int)(v.info >> 16); }
-    __device__ static int qend(const SeedIntv32 &v) { return (int)(v.info & 0xffffu); }
-    __device__ static DevIntv out(const SeedIntv32 &v)
-    {
-        DevIntv d;
-        d.x0 = v.x0, d.x1 = v.x1, d.x2 = v.x2;
-        d.info = (uint64_t)(v.info >> 16) << 32 | (v.info & 0xffffu);
-        return d;
-    }
-    __device__ static SeedIntv32 in(const DevIntv &d)
-    {
-        SeedIntv32 v;
-        v.x0 = (uint32_t)d.x0, v.x1 = (uint32_t)d.x1, v.x2 = (uint32_t)d.x2;
-        v.info = (uint32_t)(d.info >> 32) << 16 | ((uint32_t)d.info & 0xffffu);
-        return v;
-    }
+struct alignas(16) Match64 {
+    uint64_t x0, x1, x2;
+    uint32_t pos, pad;
 };
+template <class P> struct MatchOf;
+template <> struct MatchOf<uint32_t> { using type = Match32; };
+template <> struct MatchOf<uint64_t> { using type = Match64; };
+static_assert(BSB_SEED_MAX_LEN <= 1024, "match positions are packed");
 
-template <class IV>
-__device__ __forceinline__ int seed_len(const IV &p)
+template <class P>
+__device__ __forceinline__ Iv<P> set_intv(const DevFM &F, int c)   // bwt.h:80
 {
-    return IvT<IV>::qend(p) - IvT<IV>::qbeg(p);
+    Iv<P> r;
+    r.x0 = l2_at<P>(F, c) + 1;
+    r.x1 = l2_at<P>(F, 3 - c) + 1;
+    r.x2 = l2_at<P>(F, c + 1) - l2_at<P>(F, c);
+    return r;
 }
 
 // bwt_extend (bwt.c:262-275) of ik by the single base c: the reference computes all
 // four extensions and its callers keep ok[c] only, so only that one is formed here.
-template <class IV>
-__device__ __forceinline__ IV extend_one(const DevFM &F, const IV &ik, bool is_back, int c)
+template <class P>
+__device__ __forceinline__ Iv<P> extend_one(const DevFM &F, const Iv<P> &ik, bool is_back, int c)
 {
-    const uint64_t xf = is_back ? ik.x0 : ik.x1;     // x[!is_back]
-    const uint64_t xb = is_back ? ik.x1 : ik.x0;     // x[is_back]
-    const uint64_t x2 = ik.x2;
-    Occ4 tk, tl;
-    occ4_pair(F, xf - 1, xf - 1 + x2, tk, tl);        // in 64 bits whatever IV holds
-    const uint64_t s0 = tl.c[0] - tk.c[0], s1 = tl.c[1] - tk.c[1], s2 = tl.c[2] - tk.c[2], s3 = tl.c[3] - tk.c[3];
-    const uint64_t tkc = c == 0 ? tk.c[0] : c == 1 ? tk.c[1] : c == 2 ? tk.c[2] : tk.c[3];
-    const uint64_t szc = c == 0 ? s0 : c == 1 ? s1 : c == 2 ? s2 : s3;
-    const uint64_t above = c == 0 ? s1 + s2 + s3 : c == 1 ? s2 + s3 : c == 2 ? s3 : 0;   // bases > c
-    const uint64_t l2c = l2_at(F, c);
-    const uint64_t fw = l2c + 1 + tkc;
-    const uint64_t bk = xb + (xf <= F.primary && xf + x2 - 1 >= F.primary) + above;
-    IV o;
-    o.x0 = (typename IvT<IV>::pos_t)(is_back ? fw : bk);
-    o.x1 = (typename IvT<IV>::pos_t)(is_back ? bk : fw);
-    o.x2 = (typename IvT<IV>::pos_t)szc;
-    o.info = 0;
+    const P xf = is_back ? ik.x0 : ik.x1;     // x[!is_back]
+    const P xb = is_back ? ik.x1 : ik.x0;     // x[is_back]
+    P kge, kgt, lge, lgt;
+    occ_cumulative<P>(F, sym_row<P>(F, xf - 1), c, kge, kgt);
+    occ_cumulative<P>(F, sym_row<P>(F, xf - 1 + ik.x2), c, lge, lgt);
+    const P fw = l2_at<P>(F, c) + 1 + (kge - kgt);
+    const P bk = xb + (xf <= (P)F.primary && xf + ik.x2 - 1 >= (P)F.primary) + (lgt - kgt);   // bases > c come first
+    Iv<P> o;
+    o.x0 = is_back ? fw : bk;
+    o.x1 = is_back ? bk : fw;
+    o.x2 = (lge - lgt) - (kge - kgt);
     return o;
 }
 
-// Seeding state machine.  Each loop iteration, every thread first runs its read's
-// bookkeeping up to the next bwt_extend it needs (divergent, cheap), then all
-// threads perform that extend together (converged, the expensive part), then apply
-// its result.  The bookkeeping is mem_collect_intv (bwamem.c:118-166):
-//   pass 1  bwt_smem1 from every x (bwt.c:289-356), keep SMEMs >= min_seed_len;
-//   pass 2  re-seed from the middle of SMEMs >= split_len with <= split_width hits;
-//   pass 3  bwt_seed_strategy1 (bwt.c:358-379) from every x;
-// then the read's seeds are sorted by info (equal info = the same substring and so
-// the same interval: no tie rule is needed, and the order seeds are found in does
-// not matter -- compact_seeds sorts them).  Pass 2 depends only on pass 1's SMEMs,
-// so it runs as a second launch with one work item per SMEM it re-seeds, in parallel
-// with the other re-seeds instead of after them.  bwt_smem1 runs as:
-//   FWD  extend ik forward from x, pushing ik whenever its size is about to change;
-//        the pushes go down from the top of list A, so read upwards they are the
-//        reference's reversed curr list;
-//   BWD  one round per position i = x-1 .. -1: extend every prev entry backward by
-//        q[i]; entries that fail may emit an SMEM (only while nothing has survived
-//        this round), survivors are deduplicated by size into curr.
-enum SeedState : int {
-    kNeedRead, kP1X, kFwd, kFwdEnd, kBwdRound, kBwdEntry, kSmemDone, kP3X, kP3Fwd, kExit
-};
-
-// Launch control words: [0] next item of the first launch, [1] overflow (read + 1),
-// [2] pass-2 items queued, [3] next item of the second launch, [4..5] the bwt_extend
+// Launch control words: [0] next chunk of the first launch, [1] overflow (read + 1),
+// [2] pass-2 items queued, [3] next chunk of the second launch, [4..5] the bwt_extend
 // calls of both launches (uint64; each is one bwt_2occ4, two occurrence queries).
 enum { kCtrlNext1 = 0, kCtrlOverflow = 1, kCtrlQueued = 2, kCtrlNext2 = 3, kCtrlExt = 4, kCtrlWords = 8 };
 
-// Persistent: each thread takes work items from a counter.
-//   mode 0: item r < n_reads runs pass 1 of read r and queues its pass-2 re-seeds;
-//           item n_reads + r runs pass 3 of read r (independent of passes 1-2);
-//   mode 1: item w runs the pass-2 re-seed queue[w] = (read, index of the SMEM).
+// A pass-2 item: bwt_smem1 of read r from x with min_intv occurrences.
+struct Reseed {
+    int r, x;
+    int64_t min_intv;
+};
+
 // out holds, per read r, mult * (2*len(r) + 32) slots starting at mult * (2*(offs[r]-offs[0]) +
-// 32*r): the first part_cap0(len, mult) for passes 1-2 (pass 2 appends with an atomic
-// counter), the last part_cap1(len) (len/2 + 8: pass 3 finds at most one seed per
+// 32*r): the first part_cap0(len, mult) for passes 1-2 (filled in any order through an atomic
+// count), the last part_cap1(len) (len/2 + 8: pass 3 finds at most one seed per
 // min_seed_len + 1 >= 2 bases) for pass 3; count[2r + part] counts each part.  Passes 1-2
 // have no such bound (every re-seed of a repeat can add SMEMs): a batch in which a read
 // overflows runs again with mult doubled.
@@ -145,289 +123,259 @@ __device__ __host__ __forceinline__ int64_t part_base(int64_t rel_off, int r, in
     return (int64_t)mult * (2 * rel_off + 32 * (int64_t)r);
 }
 
-// 4 blocks of 128 threads per SM on 64-bit intervals (128 registers), 5 on 32-bit ones.
-template <class IV>
-__global__ void __launch_bounds__(kSeedBlock, sizeof(IV) == sizeof(DevIntv) ? 4 : 5)
-seed_kernel(DevFM F, SeedOpt opt, int mode, int n_reads, const uint8_t *__restrict__ seqs,
-            const int64_t *__restrict__ offs, DevIntv *__restrict__ out, int *__restrict__ count,
-            IV *__restrict__ scratch, int list_cap, int *__restrict__ ctrl, int2 *__restrict__ queue,
-            int queue_cap, int mult)
+// What the emission of a seed needs, apart from the seed.
+struct SeedOut {
+    DevIntv *out;
+    int *count, *ctrl;
+    Reseed *queue;
+    int queue_cap, mult;
+    const int64_t *offs;
+};
+
+// Passes 1-2: one SMEM [b, e) of read r; from pass 1 a long, rare one is queued for pass 2.
+template <class P, int Pass>
+__device__ __noinline__ void emit_smem(const SeedOpt &opt, const SeedOut &S, int r, int len, int b, int e, Iv<P> v)
 {
-    using T = IvT<IV>;
-    using pos_t = typename T::pos_t;
-    int *const next_item = ctrl + (mode ? kCtrlNext2 : kCtrlNext1);
-    int *const overflow = ctrl + kCtrlOverflow;
-    const int n_items = mode ? min(*(volatile int *)(ctrl + kCtrlQueued), queue_cap) : 2 * n_reads;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    IV *const listA = scratch + (size_t)tid * 3 * list_cap;          // forward pushes / curr and prev rounds
-    IV *const listB = listA + list_cap;
-    IV *const mem = listB + list_cap;                                // SMEMs of one bwt_smem1 call
-    const int64_t base_off = offs[0];
+    const int slot = atomicAdd(&S.count[2 * r], 1);
+    if (slot < part_cap0(len, S.mult)) {
+        DevIntv d;
+        d.x0 = v.x0, d.x1 = v.x1, d.x2 = v.x2;
+        d.info = (uint64_t)(uint32_t)b << 32 | (uint32_t)e;
+        S.out[part_base(S.offs[r] - S.offs[0], r, S.mult) + slot] = d;
+    } else {
+        atomicMax(S.ctrl + kCtrlOverflow, r + 1);
+    }
+    if (Pass == 1 && e - b >= opt.split_len && (uint64_t)v.x2 <= (uint64_t)(int64_t)opt.split_width) {
+        const int q = atomicAdd(S.ctrl + kCtrlQueued, 1);
+        if (q < S.queue_cap) S.queue[q] = Reseed{r, (b + e) >> 1, (int64_t)v.x2 + 1};
+        else atomicMax(S.ctrl + kCtrlOverflow, r + 1);
+    }
+}
 
-    int st = kNeedRead;
-    // read
-    int r = 0, part = 0, len = 0, cap = 0, n = 0;
-    const uint8_t *q = nullptr;
+// The reads of a warp's chunk.
+struct ChunkRead {
+    const uint8_t *q;
+    int len, r;
+    int64_t min_intv;
+};
+
+// Pass 3 of read r by one lane of a converged warp (has: the lane has a read).
+template <class P>
+__device__ __forceinline__ unsigned pass3(const DevFM &F, const SeedOpt &opt, const SeedOut &S, bool has, int r, int len,
+                                          const uint8_t *q)
+{
     DevIntv *dst = nullptr;
-    // bwt_smem1
-    int pass = 1, x = 0, i = 0, min_intv = 1, n_curr = 0, n_prev = 0, n_mem = 0, j = 0, c = 0, ret = 0;
-    int last_mem_start = 0;
-    pos_t last_x2 = 0;
-    IV ik, p;
-    IV *prev = listA, *curr = listB;
-    // bwt_seed_strategy1
-    int x0 = 0;
-    // values loaded one step ahead, so their latency overlaps the extension in flight:
-    // qi = q[i] (forward phases), qb = q[i] of the next backward round, pn = prev[j]
-    int qi = 4, qb = 4;
-    IV pn;
-    ik.x0 = ik.x1 = ik.x2 = ik.info = 0;
-    p = ik;
-    pn = ik;
+    int cap = 0, n = 0, i = 0, x = 0;
+    if (has) {
+        dst = S.out + part_base(S.offs[r] - S.offs[0], r, S.mult) + part_cap0(len, S.mult);
+        cap = part_cap1(len);
+    }
+    bool in = false;
+    Iv<P> ik;
+    ik.x0 = ik.x1 = ik.x2 = 0;
+    int qc = has && i < len ? q[i] : 4;
     unsigned n_ext = 0;
-
-    for (;;) {
-        // ---- bookkeeping up to the next extension (or the end of the work)
-        IV e_ik;
-        bool e_back = false;
-        int e_c = 0;
-        bool need = false;
-        while (!need && st != kExit) {
-            switch (st) {
-            case kNeedRead: {
-                // all pass-1 items first, then all pass-3 items: the warps that take
-                // them hold items of similar length, so fewer lanes idle behind a long one
-                const int w = atomicAdd(next_item, 1);
-                if (w >= n_items) { st = kExit; break; }
-                int k = 0;
-                if (mode) {
-                    const int2 it = queue[w];
-                    r = it.x;
-                    k = it.y;
-                    part = 0;
-                } else {
-                    part = w >= n_reads;
-                    r = part ? w - n_reads : w;
-                }
-                const int64_t o = offs[r];
-                const int64_t len64 = offs[r + 1] - o;
-                if (len64 < 0 || len64 > list_cap - 2) {    // outside the scratch the launch sized: refuse
-                    count[2 * r + part] = 0;
-                    atomicMax(overflow, r + 1);
-                    break;
-                }
-                len = (int)len64;
-                q = seqs + o;
-                dst = out + part_base(o - base_off, r, mult) + (part ? part_cap0(len, mult) : 0);
-                cap = part ? part_cap1(len) : part_cap0(len, mult);
-                n = 0;
-                if (mode) {                                  // re-seed in the middle of a long, rare SMEM
-                    const DevIntv sm = dst[k];
-                    pass = 2;
-                    x = (int)(((sm.info >> 32) + (uint32_t)sm.info) >> 1);
-                    min_intv = (int)sm.x2 + 1;
-                    if (q[x] > 3) break;                     // bwt_smem1 returns at once: no SMEM
-                    goto smem_start;
-                }
-                if (len < opt.min_seed_len || (part && opt.max_mem_intv <= 0)) {
-                    count[2 * r + part] = 0;                 // mem_chain returns before seeding (bwamem.c:266)
-                    break;
-                }
-                x = 0;
-                st = part ? kP3X : kP1X;
-                break;
-            }
-            case kP1X:
-                if (x >= len) {                             // pass 1 done: queue the pass-2 re-seeds
-                    if (n > cap) {
-                        atomicMax(overflow, r + 1);
-                        n = cap;
-                    }
-                    for (int t = 0; t < n; ++t) {
-                        const DevIntv sm = dst[t];
-                        const int start = (int)(sm.info >> 32), end = (int)(uint32_t)sm.info;
-                        if (end - start < opt.split_len || sm.x2 > (uint64_t)opt.split_width) continue;
-                        const int slot = atomicAdd(ctrl + kCtrlQueued, 1);
-                        if (slot < queue_cap) queue[slot] = make_int2(r, t);
-                        else atomicMax(overflow, r + 1);
-                    }
-                    count[2 * r] = n;
-                    st = kNeedRead;
-                    break;
-                }
-                if (q[x] > 3) { ++x; break; }
-                pass = 1;
-                min_intv = 1;
-                goto smem_start;
-            smem_start:
-                if (min_intv < 1) min_intv = 1;
-                ik = T::in(set_intv(F, q[x]));
-                ik.info = T::info(0, x + 1);
-                n_curr = 0;
-                i = x + 1;
-                qi = i < len ? q[i] : 4;
-                st = kFwd;
-                break;
-            case kFwd:
-                if (i < len && qi < 4) {
-                    e_ik = ik; e_back = false; e_c = 3 - qi;
-                    qi = i + 1 < len ? q[i + 1] : 4;         // for the next step
-                    need = true;
-                    break;
-                }
-                listA[list_cap - 1 - n_curr++] = ik;        // an N or the read end stops the match
-                st = kFwdEnd;
-                break;
-            case kFwdEnd:
-                prev = listA + list_cap - n_curr;            // reversed forward list
-                curr = listB;
-                n_prev = n_curr;
-                ret = T::qend(prev[0]);
-                n_mem = 0;
-                i = x - 1;
-                qb = i >= 0 ? q[i] : 4;
-                st = kBwdRound;
-                break;
-            case kBwdRound:
-                c = i < 0 ? -1 : (qb < 4 ? qb : -1);
-                qb = i - 1 >= 0 ? q[i - 1] : 4;              // for the next round
-                n_curr = 0;
-                j = 0;
-                pn = prev[0];
-                st = kBwdEntry;
-                break;
-            case kBwdEntry:
-                if (j >= n_prev) {
-                    if (n_curr == 0) { st = kSmemDone; break; }
-                    // this round's curr becomes the next prev; the list the old prev lived in
-                    // (the forward pushes sit at the top of A) takes the next curr
-                    IV *const was_prev = prev;
-                    prev = curr;
-                    curr = was_prev < listB ? listA : listB;
-                    n_prev = n_curr;
-                    --i;
-                    st = kBwdRound;
-                    break;
-                }
-                p = pn;
-                if (j + 1 < n_prev) pn = prev[j + 1];       // for the next entry
-                if (c >= 0) {
-                    e_ik = p; e_back = true; e_c = c;
-                    need = true;
-                    break;
-                }
-                // no base to extend by: p cannot grow, and is maximal if nothing survived yet
-                if (n_curr == 0 && (n_mem == 0 || i + 1 < last_mem_start)) {
-                    IV m = p;
-                    m.info |= T::info(i + 1, 0);
-                    mem[n_mem++] = m;
-                    last_mem_start = i + 1;
-                }
-                ++j;
-                break;
-            case kSmemDone:
-                for (int t = 0; t < n_mem; ++t) {
-                    const IV m = mem[t];
-                    if (seed_len(m) >= opt.min_seed_len) {
-                        if (pass == 1) {
-                            if (n < cap) dst[n] = T::out(m);
-                            ++n;
-                        } else {                            // re-seeds of one read arrive from many threads
-                            const int slot = atomicAdd(&count[2 * r], 1);
-                            if (slot < cap) dst[slot] = T::out(m);
-                            else atomicMax(overflow, r + 1);
-                        }
-                    }
-                }
-                if (pass == 1) { x = ret; st = kP1X; }
-                else st = kNeedRead;
-                break;
-            case kP3X:
-                if (x >= len) {                             // pass 3 done
-                    if (n > cap) {
-                        atomicMax(overflow, r + 1);
-                        n = cap;
-                    }
-                    count[2 * r + 1] = n;
-                    st = kNeedRead;
-                    break;
-                }
-                if (q[x] > 3) { ++x; break; }
-                ik = T::in(set_intv(F, q[x]));
-                x0 = x;
-                i = x + 1;
-                qi = i < len ? q[i] : 4;
-                st = kP3Fwd;
-                break;
-            case kP3Fwd:
-                if (i >= len) { x = len; st = kP3X; break; }
-                if (qi > 3) { x = i + 1; st = kP3X; break; }
-                e_ik = ik; e_back = false; e_c = 3 - qi;
-                qi = i + 1 < len ? q[i + 1] : 4;             // for the next step
-                need = true;
-                break;
-            default:
-                st = kExit;
-                break;
-            }
-        }
-        if (!__any_sync(BSB_FULL_MASK, need)) {
-            if (st == kExit) break;
-            continue;
-        }
-        n_ext += need;
-
-        // ---- the extension, converged across the warp
-        IV ok;
-        if (need) ok = extend_one(F, e_ik, e_back, e_c);
-
-        // ---- apply it
-        if (!need) continue;
-        switch (st) {
-        case kFwd:
-            if (ok.x2 != ik.x2) {
-                listA[list_cap - 1 - n_curr++] = ik;
-                if (ok.x2 < (pos_t)min_intv) { st = kFwdEnd; break; }
-            }
+    while (__any_sync(BSB_FULL_MASK, has && i < len)) {
+        const bool act = has && i < len;
+        const int qn = act && i + 1 < len ? q[i + 1] : 4;      // for the next step, under this one's fetches
+        if (act && in && qc < 4) {
+            const Iv<P> ok = extend_one<P>(F, ik, false, 3 - qc);
+            ++n_ext;
             ik = ok;
-            ik.info = T::info(0, i + 1);
-            ++i;
-            break;
-        case kBwdEntry:
-            if (ok.x2 < (pos_t)min_intv) {
-                if (n_curr == 0 && (n_mem == 0 || i + 1 < last_mem_start)) {
-                    IV m = p;
-                    m.info |= T::info(i + 1, 0);
-                    mem[n_mem++] = m;
-                    last_mem_start = i + 1;
-                }
-            } else if (n_curr == 0 || ok.x2 != last_x2) {
-                ok.info = p.info;
-                curr[n_curr++] = ok;
-                last_x2 = ok.x2;
-            }
-            ++j;
-            break;
-        case kP3Fwd:
-            if (ok.x2 < (pos_t)opt.max_mem_intv && i - x0 >= opt.min_seed_len) {
-                if (ok.x2 > 0) {                            // an empty interval is not kept (bwamem.c:160)
-                    IV m = ok;
-                    m.info = T::info(x0, i + 1);
-                    if (n < cap) dst[n] = T::out(m);
+            if (ok.x2 < (P)opt.max_mem_intv && i - x >= opt.min_seed_len) {
+                if (ok.x2 > 0) {                               // an empty interval is not kept (bwamem.c:160)
+                    if (n < cap) {
+                        DevIntv d;
+                        d.x0 = ok.x0, d.x1 = ok.x1, d.x2 = ok.x2;
+                        d.info = (uint64_t)(uint32_t)x << 32 | (uint32_t)(i + 1);
+                        dst[n] = d;
+                    }
                     ++n;
                 }
-                x = i + 1;
-                st = kP3X;
-                break;
+                in = false;
             }
-            ik = ok;
-            ++i;
-            break;
-        default:
-            break;
+        } else if (act) {
+            in = qc < 4;
+            if (in) ik = set_intv<P>(F, qc), x = i;
         }
+        ++i;
+        qc = qn;
     }
-    if (n_ext) atomicAdd((unsigned long long *)(ctrl + kCtrlExt), (unsigned long long)n_ext);
+    if (has) {
+        if (n > cap) atomicMax(S.ctrl + kCtrlOverflow, r + 1);
+        S.count[2 * r + 1] = n < cap ? n : cap;
+    }
+    return n_ext;
+}
+
+// Mode 0: chunks of rho reads for pass 1, then chunks of 32 reads for pass 3.  Mode 1: chunks of
+// the queued re-seeds of pass 2, as many a chunk as spread them over all warps (at most rho).
+// matches: region_cap entries per warp.  A read (a re-seed) pushes at most one match per end
+// position, so rho * (max_len + 1) entries always hold a chunk.
+template <class P, int Mode>
+__global__ void __launch_bounds__(kSeedBlock, sizeof(P) == 4 ? 7 : 5)
+seed_kernel(DevFM F, SeedOpt opt, int n_reads, int max_len, const uint8_t *__restrict__ seqs, SeedOut S,
+            typename MatchOf<P>::type *__restrict__ matches, int region_cap, int rho)
+{
+    using Match = typename MatchOf<P>::type;
+    __shared__ ChunkRead chunk_reads[kSeedWarps][32];
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    ChunkRead *const CR = chunk_reads[wb];
+    Match *const list = matches + (size_t)(blockIdx.x * kSeedWarps + wb) * region_cap;
+    const int64_t *const offs = S.offs;
+    int *const next = S.ctrl + (Mode ? kCtrlNext2 : kCtrlNext1);
+    const int n_items = Mode ? min(*(volatile int *)(S.ctrl + kCtrlQueued), S.queue_cap) : n_reads;
+    if (Mode) {
+        const int warps = gridDim.x * kSeedWarps;
+        rho = min(rho, max(1, (n_items + warps - 1) / warps));
+    }
+    const int n1 = (n_items + rho - 1) / rho;
+    const int n_chunks = n1 + (Mode == 0 && opt.max_mem_intv > 0 ? (n_reads + 31) / 32 : 0);
+    unsigned n_ext = 0;
+    for (;;) {
+        int ch = 0;
+        if (lane == 0) ch = atomicAdd(next, 1);
+        ch = __shfl_sync(BSB_FULL_MASK, ch, 0);
+        if (ch >= n_chunks) break;
+        // ---- the chunk's reads, a lane each
+        const bool p3 = Mode == 0 && ch >= n1;
+        const int item = p3 ? (ch - n1) * 32 + lane : ch * rho + lane;
+        bool act = item < n_items && (p3 || lane < rho);
+        int r = 0, len = 0, x = 0;
+        P mi = 1;
+        const uint8_t *q = seqs;
+        if (act) {
+            r = item;
+            if (Mode) {
+                const Reseed it = S.queue[item];
+                r = it.r, x = it.x, mi = (P)it.min_intv;
+            }
+            const int64_t o = offs[r], l = offs[r + 1] - o;
+            q = seqs + o;
+            len = (int)l;
+            if (l < 0 || l > max_len) {                 // outside what the launch was sized for: refuse
+                atomicMax(S.ctrl + kCtrlOverflow, r + 1);
+                act = false;
+            } else if (len < opt.min_seed_len) {        // mem_chain returns before seeding (bwamem.c:266)
+                act = false;
+            }
+        }
+        if (p3) {
+            n_ext += pass3<P>(F, opt, S, act, r, len, q);
+            continue;
+        }
+        __syncwarp();
+        CR[lane] = ChunkRead{q, len, r, (int64_t)mi};
+        __syncwarp();
+        // ---- forward (bwt.c:300-319): every lane one extension a step, matches pushed when their
+        // size is about to change.  lb: the leftmost base a match from x can reach (no N before x)
+        int total = 0;
+        {
+            int i = 0, lb = 0;
+            bool in = false;
+            Iv<P> ik;
+            ik.x0 = ik.x1 = ik.x2 = 0;
+            if (Mode && act) {
+                if (q[x] > 3) act = false;              // bwt_smem1 returns at once: no SMEM
+                else {
+                    ik = set_intv<P>(F, q[x]);
+                    lb = x == 0 || q[x - 1] > 3 ? x : 0;
+                    in = true;
+                    i = x + 1;
+                }
+            }
+            int qc = act && i < len ? q[i] : 4;
+            while (__any_sync(BSB_FULL_MASK, act)) {
+                const int qn = act && i + 1 < len ? q[i + 1] : 4;
+                const bool ext = act && in && qc < 4;
+                Iv<P> ok = ik;
+                if (ext) ok = extend_one<P>(F, ik, false, 3 - qc);
+                n_ext += ext;
+                bool push = false, stop = false;
+                if (act && in) {
+                    push = qc > 3 || ok.x2 != ik.x2;      // an N or the read's end stops the match
+                    stop = qc > 3 || (push && ok.x2 < mi);
+                }
+                const Iv<P> pv = ik;
+                const int px = x, pe = i;
+                const bool enq = push && px > lb && pe - lb >= opt.min_seed_len;
+                // nothing to the left of x: only the longest match, and it is an SMEM
+                const bool seed = push && stop && px == lb && pe - px >= opt.min_seed_len;
+                if (act) {
+                    if (ext && !stop) ik = ok;
+                    if (!in || stop) {
+                        in = qc < 4 && !(Mode && stop);
+                        if (in) ik = set_intv<P>(F, qc), x = i;
+                        else lb = i + 1;
+                        if (i >= len || (Mode && stop)) act = false;
+                    }
+                    ++i;
+                }
+                qc = qn;
+                const unsigned m = __ballot_sync(BSB_FULL_MASK, enq);
+                if (enq) {
+                    const int slot = total + __popc(m & below);
+                    Match e;
+                    e.x0 = pv.x0, e.x1 = pv.x1, e.x2 = pv.x2;
+                    e.pos = (uint32_t)lane << 21 | (uint32_t)px << 11 | (uint32_t)pe;
+                    if (slot < region_cap) list[slot] = e;
+                }
+                total += __popc(m);
+                if (seed) emit_smem<P, Mode + 1>(opt, S, r, len, px, pe, pv);
+            }
+            total = min(total, region_cap);
+        }
+        __syncwarp();
+        // ---- backward: the lanes take the list's matches, the next one loaded ahead
+        int taken = 0;
+        bool have = false, spare = false, right = false;
+        Iv<P> v;
+        v.x0 = v.x1 = v.x2 = 0;
+        Match sp;
+        sp.x0 = sp.x1 = sp.x2 = 0, sp.pos = 0;
+        int i = 0, e = 0, c = 4, slot = 0;
+        q = seqs, len = 0, mi = 1;
+        for (;;) {
+            if (!have && spare) {
+                v.x0 = sp.x0, v.x1 = sp.x1, v.x2 = sp.x2;
+                slot = (int)(sp.pos >> 21);
+                i = (int)(sp.pos >> 11 & 1023u) - 1, e = (int)(sp.pos & 2047u);
+                q = CR[slot].q, len = CR[slot].len, mi = (P)CR[slot].min_intv;
+                c = q[i];                               // x > lb: there is a base to the left
+                have = true, spare = right = false;
+            }
+            if (taken < total) {
+                const unsigned m = __ballot_sync(BSB_FULL_MASK, !spare);
+                const int k = taken + __popc(m & below);
+                if (!spare && k < total) sp = list[k], spare = true;
+                taken += __popc(m);
+            }
+            if (!__any_sync(BSB_FULL_MASK, have || spare)) break;
+            if (!have) continue;
+            const int qn = !right && i > 0 ? q[i - 1] : 4;
+            const bool ext = right || c < 4;
+            Iv<P> ok = v;
+            if (ext) ok = extend_one<P>(F, v, !right, right ? 3 - c : c);
+            n_ext += ext;
+            const bool grows = ext && ok.x2 >= mi;
+            if (right) {                                // asked whether [i + 1, e) can grow to the right
+                have = false;
+                if (!grows) emit_smem<P, Mode + 1>(opt, S, CR[slot].r, len, i + 1, e, v);
+            } else if (grows) {
+                v = ok;
+                --i;
+                c = i >= 0 ? qn : 4;
+            } else if (e - (i + 1) >= opt.min_seed_len) {   // [i + 1, e) is as long as it gets to the left
+                c = e < len ? q[e] : 4;
+                right = true;
+            } else {
+                have = false;
+            }
+        }
+        __syncwarp();
+    }
+    if (n_ext) atomicAdd((unsigned long long *)(S.ctrl + kCtrlExt), (unsigned long long)n_ext);
 }
 
 // Seeds of read r in the two parts of its padded region (a part that overflowed holds
@@ -548,51 +496,68 @@ __global__ void sa_fill_kernel(DevFM F, int64_t n_sa, uint64_t *__restrict__ ful
 
 }  // namespace
 
-size_t seed_scratch_bytes(int n_threads, int max_len)
-{
-    return (size_t)n_threads * 3 * (size_t)(max_len + 2) * sizeof(DevIntv);
-}
+static bool seed_narrow(uint64_t seq_len) { return seq_len < kNarrowRows; }
 
-// The 32-bit interval variant serves indexes of fewer than 2^32 - 2 rows.
-static bool seed_narrow(uint64_t seq_len) { return seq_len < IvT<SeedIntv32>::kMaxRows; }
-
-// Persistent seeding threads for an index of seq_len rows: as many as fit on the GPU at once
-// (the variant the index runs sets the blocks per SM), no more than the reads need, and fewer
-// when long reads would make the per-thread interval lists exceed ~1 GB of scratch.  The
-// scratch of seed_scratch_bytes is sized by this count.
-int seed_threads(int n_sm, int max_len, int n_reads, uint64_t seq_len)
+// The launch shape of a batch: warps that are resident at once, reads a chunk of pass 1 takes, and
+// the match list each warp needs.
+// rho: as few reads a warp as still occupy every warp, so that the matches of a read spread over the
+// warp's lanes, and at most kSeedRho (67k reads of 150 bases: 2.5 ms at 2, 1.93 at 4, 1.73 at 8 and
+// 16, 1.86 at 24, 2.1 at 32, where the forward phases fill the lanes but half the warps stay empty).
+SeedPlan seed_plan(int n_sm, int max_len, int n_reads, uint64_t seq_len)
 {
     const bool narrow = seed_narrow(seq_len);
     static int resident[2] = {0, 0};
     if (!resident[narrow]) {
-        int b = 0;
+        int b = 0, b2 = 0;
         const cudaError_t e =
-            narrow ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_kernel<SeedIntv32>, kSeedBlock, 0)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_kernel<DevIntv>, kSeedBlock, 0);
-        if (e != cudaSuccess || b < 1) b = 4;
+            narrow ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_kernel<uint32_t, 0>, kSeedBlock, 0)
+                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_kernel<uint64_t, 0>, kSeedBlock, 0);
+        const cudaError_t e2 =
+            narrow ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, seed_kernel<uint32_t, 1>, kSeedBlock, 0)
+                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, seed_kernel<uint64_t, 1>, kSeedBlock, 0);
+        b = std::min(b, b2);
+        if (e != cudaSuccess || e2 != cudaSuccess || b < 1) b = 4;
         resident[narrow] = b;
     }
-    const int res = resident[narrow];
-    const size_t per_block = (size_t)kSeedBlock * 3 * (size_t)(max_len + 2) * sizeof(DevIntv);
-    size_t blocks = (size_t)n_sm * res;
-    const size_t want = ((size_t)2 * (n_reads > 0 ? n_reads : 1) + kSeedBlock - 1) / kSeedBlock;   // two items per read
-    if (blocks > want) blocks = want;
-    const size_t budget = (size_t)1 << 30;
-    if (blocks * per_block > budget) blocks = budget / per_block;
-    if (blocks < 1) blocks = 1;
-    return (int)blocks * kSeedBlock;
+    SeedPlan p;
+    const int64_t warps = (int64_t)n_sm * resident[narrow] * kSeedWarps;
+    p.rho = (int)std::min<int64_t>(kSeedRho, std::max<int64_t>(1, (n_reads + warps - 1) / warps));
+    const size_t entry = narrow ? sizeof(Match32) : sizeof(Match64);
+    const size_t budget = (size_t)1 << 30;              // long reads: fewer reads a warp
+    const size_t fit = budget / ((size_t)warps * (size_t)(max_len + 1) * entry);
+    if ((size_t)p.rho > fit) p.rho = (int)std::max<size_t>(1, fit);
+    // no more warps than the first launch has chunks (pass 1 and pass 3) or the second can use
+    const int64_t chunks = (n_reads + p.rho - 1) / p.rho + (n_reads + 31) / 32;
+    p.blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)n_sm * resident[narrow],
+                                                           std::max<int64_t>((chunks + kSeedWarps - 1) / kSeedWarps,
+                                                                             std::min<int64_t>(n_reads, n_sm))));
+    p.region_cap = p.rho * (max_len + 1);
+    p.list_bytes = (size_t)p.blocks * kSeedWarps * (size_t)p.region_cap * entry;
+    return p;
 }
 
 // Pass-2 work items a batch can queue: at most one per SMEM of pass 1, i.e. per read
 // position.
-size_t seed_queue_entries(int64_t total_bases, int n_reads, int mult)
+size_t seed_queue_bytes(int64_t total_bases, int n_reads, int mult, int64_t *entries)
 {
-    return (size_t)mult * ((size_t)total_bases + (size_t)n_reads) + 64;
+    *entries = (int64_t)mult * (total_bases + n_reads) + 64;
+    return (size_t)*entries * sizeof(Reseed);
 }
 
 size_t seed_padded_entries(int64_t total_bases, int n_reads, int mult)
 {
     return (size_t)mult * (2 * (size_t)total_bases + 32 * (size_t)n_reads);
+}
+
+template <class P>
+static void seed_passes(const DevFM &F, const SeedOpt &o, int n_reads, int max_len, const uint8_t *d_seqs,
+                        const SeedOut &S, void *d_lists, const SeedPlan &p, cudaStream_t st)
+{
+    using Match = typename MatchOf<P>::type;
+    seed_kernel<P, 0><<<p.blocks, kSeedBlock, 0, st>>>(F, o, n_reads, max_len, d_seqs, S, (Match *)d_lists,
+                                                       p.region_cap, p.rho);
+    seed_kernel<P, 1><<<p.blocks, kSeedBlock, 0, st>>>(F, o, n_reads, max_len, d_seqs, S, (Match *)d_lists,
+                                                       p.region_cap, p.rho);
 }
 
 cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, int split_width, int max_mem_intv,
@@ -608,19 +573,18 @@ cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, in
     o.max_mem_intv = max_mem_intv;
     cudaError_t e = cudaMemsetAsync(d_ctrl, 0, kCtrlWords * sizeof(int), st);
     if (e != cudaSuccess) return e;
-    const bool narrow = seed_narrow(F.seq_len);
-    const int blocks = seed_threads(n_sm, max_len, n_reads, F.seq_len) / kSeedBlock;
-    const int qcap = (int)(queue_cap < 0x7fffffff ? queue_cap : 0x7fffffff);
-    for (int mode = 0; mode < 2; ++mode) {      // passes 1 and 3, then the pass-2 re-seeds
-        if (narrow)
-            seed_kernel<SeedIntv32><<<blocks, kSeedBlock, 0, st>>>(F, o, mode, n_reads, d_seqs, d_offs,
-                                                                   (DevIntv *)d_padded, d_count, (SeedIntv32 *)d_lists,
-                                                                   max_len + 2, d_ctrl, (int2 *)d_queue, qcap, mult);
-        else
-            seed_kernel<DevIntv><<<blocks, kSeedBlock, 0, st>>>(F, o, mode, n_reads, d_seqs, d_offs,
-                                                                (DevIntv *)d_padded, d_count, (DevIntv *)d_lists,
-                                                                max_len + 2, d_ctrl, (int2 *)d_queue, qcap, mult);
-    }
+    e = cudaMemsetAsync(d_count, 0, sizeof(int) * 2 * (size_t)n_reads, st);
+    if (e != cudaSuccess) return e;
+    SeedOut S;
+    S.out = (DevIntv *)d_padded;
+    S.count = d_count, S.ctrl = d_ctrl;
+    S.queue = (Reseed *)d_queue;
+    S.queue_cap = (int)(queue_cap < 0x7fffffff ? queue_cap : 0x7fffffff);
+    S.mult = mult;
+    S.offs = d_offs;
+    const SeedPlan p = seed_plan(n_sm, max_len, n_reads, F.seq_len);
+    if (seed_narrow(F.seq_len)) seed_passes<uint32_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, p, st);
+    else seed_passes<uint64_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, p, st);
     read_totals<<<n_sm * 4, 256, 0, st>>>(d_count, d_offs, n_reads, mult, d_tot);
     e = scan_i32_i64(d_tot, n_reads, d_out_off, d_scan_tmp, st);
     if (e != cudaSuccess) return e;
