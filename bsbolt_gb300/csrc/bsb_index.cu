@@ -21,8 +21,10 @@ size_t seed_queue_bytes(int64_t total_bases, int n_reads, int mult, int64_t *ent
 cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, int split_width, int max_mem_intv,
                         int n_reads, const uint8_t *d_seqs, const int64_t *d_offs, int max_len,
                         void *d_padded, int *d_count, int64_t *d_out_off, void *d_out,
-                        void *d_lists, int *d_ctrl, void *d_queue, int64_t queue_cap, int *d_tot,
+                        const SeedPlan &p, void *d_lists, void *d_list_counts, int *d_ctrl, void *d_queue, int64_t queue_cap, int *d_tot,
                         int64_t *d_scan_tmp, int mult, int n_sm, cudaStream_t st);
+size_t kmer_bytes(uint64_t seq_len);
+cudaError_t kmer_build(const DevFM &F, void *out, cudaStream_t st);
 cudaError_t sa_launch(const DevFM &F, const uint64_t *d_rows, int64_t n, uint64_t *d_pos, int n_sm, cudaStream_t st);
 cudaError_t sa_full_build(const DevFM &F, int64_t n_sa, uint64_t *full, int *failed, int n_sm, cudaStream_t st);
 
@@ -31,6 +33,8 @@ void bsb_index_release(bsb_ctx *ctx)
     if (ctx->idx_bwt) cudaFree(ctx->idx_bwt);
     if (ctx->idx_sb) cudaFree(ctx->idx_sb);
     ctx->idx_sb = nullptr;
+    if (ctx->idx_kmers) cudaFree(ctx->idx_kmers);
+    ctx->idx_kmers = nullptr;
     if (ctx->idx_sa) cudaFree(ctx->idx_sa);
     if (ctx->idx_pac) cudaFree(ctx->idx_pac);
     if (ctx->idx_sa_full) cudaFree(ctx->idx_sa_full);
@@ -49,6 +53,7 @@ static DevFM dev_fm(const bsb_ctx *ctx)
     DevFM F;
     F.blk = (const uint4 *)ctx->idx_bwt;
     F.sb = (const uint64_t *)ctx->idx_sb;
+    F.kmers = (const uint4 *)ctx->idx_kmers;
     F.sa = (const uint64_t *)ctx->idx_sa;
     F.sa_full = (const uint64_t *)ctx->idx_sa_full;
     F.primary = ctx->primary;
@@ -217,6 +222,17 @@ extern "C" int bsb_index_upload(bsb_ctx *ctx, const bsb_index_view_t *v)
     ctx->l_pac = v->l_pac;
     if ((rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "index upload"))) return rc;
     if ((rc = build_sa_full(ctx))) return rc;
+    // the k-mer table, where it fits (seeding goes base by base without it); a text too short for
+    // every base to occur has none
+    if (seq_len > 0 && cudaMalloc(&ctx->idx_kmers, kmer_bytes(seq_len)) == cudaSuccess) {
+        const DevFM F = dev_fm(ctx);
+        if ((rc = bsb_cuda(ctx, kmer_build(F, ctx->idx_kmers, ctx->stream), "index: k-mer table")) ||
+            (rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "index: k-mer table")))
+            return rc;
+    } else {
+        ctx->idx_kmers = nullptr;
+        cudaGetLastError();       // an allocation that did not fit is not an error
+    }
     ctx->has_index = 1;
     return 0;
 }
@@ -334,11 +350,12 @@ int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_r
     const size_t padded = seed_padded_entries(total_bases, n_reads, mult) * sizeof(DevIntv);
     if (max_len > BSB_SEED_MAX_LEN) return bsb_fail(ctx, BSB_ETOOLONG, "max_len %d > %d", max_len, BSB_SEED_MAX_LEN);
     const DevFM F = dev_fm(ctx);
-    const size_t lists = seed_plan(ctx->n_sm, max_len, n_reads, F.seq_len).list_bytes;
+    const SeedPlan plan = seed_plan(ctx->n_sm, total_bases, max_len, n_reads, F.seq_len);
+    const size_t lists = plan.list_bytes, counts_b = (plan.counts_bytes + 255) & ~(size_t)255;
     int64_t qn = 0;
     const size_t queue_b = (seed_queue_bytes(total_bases, n_reads, mult, &qn) + 255) & ~(size_t)255;
     const size_t tot_b = (sizeof(int) * (size_t)n_reads + 255) & ~(size_t)255;
-    const size_t need = padded + lists + 256 * 6 + sizeof(int) * (2 * (size_t)n_reads + 128) + queue_b + tot_b +
+    const size_t need = padded + lists + 256 * 6 + sizeof(int) * (2 * (size_t)n_reads + 128) + queue_b + tot_b + counts_b +
                         sizeof(int64_t) * (size_t)scan_tmp_words(n_reads);
     if ((rc = bsb_ensure(ctx, &ctx->seed_scratch, &ctx->seed_scratch_bytes, need, "seed scratch"))) return rc;
     char *s = (char *)ctx->seed_scratch;
@@ -348,9 +365,10 @@ int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_r
     int *d_ctrl = d_count + ((2 * n_reads + 63) & ~63);     // two counts per read (seed_kernel's two parts)
     void *d_queue = d_ctrl + 64;                              // pass-2 work items
     int *d_tot = (int *)((char *)d_queue + queue_b);         // seeds kept per read
-    int64_t *d_scan_tmp = (int64_t *)((char *)d_tot + tot_b);
+    void *d_list_counts = (char *)d_tot + tot_b;
+    int64_t *d_scan_tmp = (int64_t *)((char *)d_list_counts + counts_b);
     cudaError_t e = seed_launch(F, opt->min_seed_len, opt->split_factor, opt->split_width, opt->max_mem_intv, n_reads,
-                                d_seqs, d_offs, max_len, d_padded, d_count, d_out_off, d_out, d_lists, d_ctrl,
+                                d_seqs, d_offs, max_len, d_padded, d_count, d_out_off, d_out, plan, d_lists, d_list_counts, d_ctrl,
                                 d_queue, qn, d_tot, d_scan_tmp, mult, ctx->n_sm, ctx->stream);
     ctx->seed_ctrl = d_ctrl;
     return bsb_cuda(ctx, e, "seed launch");

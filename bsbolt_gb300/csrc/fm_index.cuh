@@ -21,6 +21,7 @@
 struct DevFM {
     const uint4 *blk;        // 32-byte occurrence sectors
     const uint64_t *sb;      // symbols > A, > C, > G before each 2^32-row superblock
+    const uint4 *kmers;      // bi-interval of every kKmer-base string (KmerOf<P>), or NULL
     const uint64_t *sa;      // sampled suffix array, sa[0] = (uint64_t)-1
     const uint64_t *sa_full; // every row's bwt_sa value (seq_len + 1 entries), or NULL
     uint64_t primary;
@@ -36,6 +37,19 @@ struct DevIntv {             // bwtintv_t (bwt.h:60-62)
 // Sector s: {symbols > A, > C, > G in the rows of its superblock before it, 0},
 // {lo plane of symbols 0-31, lo of 32-63, hi of 0-31, hi of 32-63}.
 constexpr int kSectorSyms = 64;
+
+// The table of bi-intervals (x0, x1, x2) by string, the first base in the code's highest bits: 16
+// bytes an entry (0.27 GB) for an index below 2^32 rows, else 32.
+constexpr int kKmer = 12;
+constexpr uint32_t kKmers = 1u << (2 * kKmer);
+
+// 32 bytes in one transaction.
+__device__ __forceinline__ void load32(const uint4 *p, uint32_t (&v)[8])
+{
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
+}
 
 // Counts of A, C, G among the first n (0..16) symbols of x, a word of the reference's array (most
 // significant pair first).
@@ -69,13 +83,18 @@ __device__ __forceinline__ P sym_row(const DevFM &F, P k)
     return k < (P)F.seq_len ? k : (P)F.seq_len - 1;
 }
 
-// Symbols >= c and > c in rows [0, kk] of the $-free BWT (bwt_occ4, bwt.c:169-187).  P: uint32_t
-// for an index below 2^32 rows, which has one superblock, else uint64_t.
 template <class P>
-__device__ __forceinline__ void occ_cumulative(const DevFM &F, P kk, int c, P &ge, P &gt)
+__device__ __forceinline__ const uint4 *sector_of(const DevFM &F, P kk)
 {
-    const uint4 *p = F.blk + (uint64_t)(kk >> 6) * 2;
-    const uint4 v = __ldg(p), s = __ldg(p + 1);
+    return F.blk + (uint64_t)(kk >> 6) * 2;
+}
+
+// Symbols >= c and > c in rows [0, kk] of the $-free BWT (bwt_occ4, bwt.c:169-187), w the sector of
+// kk.  P: uint32_t for an index below 2^32 rows, which has one superblock, else uint64_t.
+template <class P>
+__device__ __forceinline__ void occ_cumulative(const DevFM &F, const uint32_t (&w)[8], P kk, int c, P &ge, P &gt)
+{
+    const uint4 v = make_uint4(w[0], w[1], w[2], w[3]), s = make_uint4(w[4], w[5], w[6], w[7]);
     const uint64_t keep = ~0ull >> (63 - (int)(kk & 63));
     const uint32_t k0 = (uint32_t)keep, k1 = (uint32_t)(keep >> 32);
     // [symbol >= t] = (hi | lo & x) & (lo | y): hi|lo for t = 1, hi for 2, hi&lo for 3
@@ -100,11 +119,12 @@ __device__ __forceinline__ uint64_t lf_step(const DevFM &F, uint64_t k)
     if (k == F.primary) return 0;
     // the symbol row (bwt_invPsi uses k > primary, bwt.c:55) equals the counted row here
     const uint64_t kk = sym_row<uint64_t>(F, k);
-    const uint4 s = __ldg(F.blk + (kk >> 6) * 2 + 1);
+    uint32_t w[8];
+    load32(sector_of<uint64_t>(F, kk), w);
     const int n = (int)(kk & 31);
-    const uint32_t lo = (kk & 32) ? s.y : s.x, hi = (kk & 32) ? s.w : s.z;
+    const uint32_t lo = (kk & 32) ? w[5] : w[4], hi = (kk & 32) ? w[7] : w[6];
     const int c = (int)(lo >> n & 1u) | (int)(hi >> n & 1u) << 1;
     uint64_t ge, gt;
-    occ_cumulative<uint64_t>(F, kk, c, ge, gt);
+    occ_cumulative<uint64_t>(F, w, kk, c, ge, gt);
     return l2_at(F, c) + ge - gt;
 }

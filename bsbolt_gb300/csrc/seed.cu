@@ -20,14 +20,18 @@
 // one are of the second kind.  It emits nothing but the longest match where the base left of x is
 // missing or an N.)
 //
-// So a warp takes a few reads: a lane each for the forward phases, every lane with one extension a
-// step, and the pushed matches go to a list of the warp; then the lanes take matches from the
-// list, one after the other, each extending its own to the left.  The re-seeds of pass 2 are
-// a second launch of the same two phases, with their threshold on the occurrences; pass 3 is a forward
-// phase of its own.  Against the lock-step form, a state machine with one thread per read and pass
-// (11-13 of 32 lanes active; now 20), one GB300, seeding stage of a batch with its copies: 64 reads
-// 0.76 -> 0.14 ms, 40k reads of 100 bases on a 2 Mb reference 1.51 -> 0.57, 67k of 150 on 100 Mb
-// 3.6 -> 1.73, 114k RRBS reads 3.2 -> 1.6; 15 % more extensions.
+// So pass 1 is two kernels: forward phases, 32 reads a warp, one extension a step for every lane
+// (pass 3 is a forward phase of its own, in the same launch), which list their matches; then
+// warps whose lanes take matches from the lists, one after the other, each extending its own to the
+// left.  The re-seeds of pass 2 run both phases in one kernel, a few a warp, with their threshold on
+// the occurrences.  A table of the bi-intervals of all 12-base strings stands in for the first 11
+// extensions of every forward phase and of every short match.  One GB300, seeding stage of a batch
+// with its copies: 64 reads 0.76 -> 0.165 ms, 40k reads of 100 bases on a 2 Mb reference 1.51 -> 0.38,
+// 67k of 150 on 100 Mb 3.6 -> 1.24, 114k RRBS reads 3.2 -> 1.2 (the lock-step form, a state machine
+// with one thread per read and pass and 11-13 of 32 lanes active, against this one; with both phases
+// in one kernel and no table 0.14, 0.57, 1.73 and 1.6).  Of the 39M extensions of the third a
+// forward step runs at 3.5 TB/s of DRAM, half the device's copy rate; the rest waits for sectors
+// (L2 serves 24-37 %) with 20 of 64 warps per SM and 22 of 32 lanes.
 //
 // bwt_sa (bwt.c:86-96) is one thread per suffix-array row: one load from the full
 // suffix array when it is resident, else LF steps until a sampled row, each step
@@ -42,7 +46,6 @@
 namespace {
 
 constexpr int kSeedBlock = 128, kSeedWarps = kSeedBlock / 32;
-constexpr int kSeedRho = 16;            // most reads (re-seeds) a warp takes at once
 
 struct SeedOpt {
     int min_seed_len, split_len, split_width, max_mem_intv;
@@ -81,15 +84,23 @@ __device__ __forceinline__ Iv<P> set_intv(const DevFM &F, int c)   // bwt.h:80
 }
 
 // bwt_extend (bwt.c:262-275) of ik by the single base c: the reference computes all
-// four extensions and its callers keep ok[c] only, so only that one is formed here.
+// four extensions and its callers keep ok[c] only, so only that one is formed here.  In two
+// halves, around the load of the two rows' sectors (wk, wl): extend_rows and extend_with.
 template <class P>
-__device__ __forceinline__ Iv<P> extend_one(const DevFM &F, const Iv<P> &ik, bool is_back, int c)
+__device__ __forceinline__ void extend_rows(const DevFM &F, const Iv<P> &ik, bool is_back, P &kk, P &ll)
 {
     const P xf = is_back ? ik.x0 : ik.x1;     // x[!is_back]
-    const P xb = is_back ? ik.x1 : ik.x0;     // x[is_back]
+    kk = sym_row<P>(F, xf - 1);
+    ll = sym_row<P>(F, xf - 1 + ik.x2);
+}
+template <class P>
+__device__ __forceinline__ Iv<P> extend_with(const DevFM &F, const Iv<P> &ik, bool is_back, int c, P kk, P ll,
+                                             const uint32_t (&wk)[8], const uint32_t (&wl)[8])
+{
+    const P xf = is_back ? ik.x0 : ik.x1, xb = is_back ? ik.x1 : ik.x0;
     P kge, kgt, lge, lgt;
-    occ_cumulative<P>(F, sym_row<P>(F, xf - 1), c, kge, kgt);
-    occ_cumulative<P>(F, sym_row<P>(F, xf - 1 + ik.x2), c, lge, lgt);
+    occ_cumulative<P>(F, wk, kk, c, kge, kgt);
+    occ_cumulative<P>(F, wl, ll, c, lge, lgt);
     const P fw = l2_at<P>(F, c) + 1 + (kge - kgt);
     const P bk = xb + (xf <= (P)F.primary && xf + ik.x2 - 1 >= (P)F.primary) + (lgt - kgt);   // bases > c come first
     Iv<P> o;
@@ -99,10 +110,63 @@ __device__ __forceinline__ Iv<P> extend_one(const DevFM &F, const Iv<P> &ik, boo
     return o;
 }
 
-// Launch control words: [0] next chunk of the first launch, [1] overflow (read + 1),
-// [2] pass-2 items queued, [3] next chunk of the second launch, [4..5] the bwt_extend
-// calls of both launches (uint64; each is one bwt_2occ4, two occurrence queries).
-enum { kCtrlNext1 = 0, kCtrlOverflow = 1, kCtrlQueued = 2, kCtrlNext2 = 3, kCtrlExt = 4, kCtrlWords = 8 };
+// Entry `code` of the k-mer table out of its 32 bytes.
+template <class P>
+__device__ __forceinline__ const uint4 *kmer_at(const DevFM &F, uint32_t code)
+{
+    return F.kmers + (sizeof(P) == 4 ? (code & ~1u) : 2 * (uint64_t)code);
+}
+template <class P>
+__device__ __forceinline__ Iv<P> kmer_of(const uint32_t (&w)[8], uint32_t code)
+{
+    Iv<P> r;
+    if (sizeof(P) == 4) {
+        const bool odd = code & 1;
+        r.x0 = odd ? w[4] : w[0], r.x1 = odd ? w[5] : w[1], r.x2 = odd ? w[6] : w[2];
+    } else {
+        r.x0 = (P)((uint64_t)w[1] << 32 | w[0]), r.x1 = (P)((uint64_t)w[3] << 32 | w[2]);
+        r.x2 = (P)((uint64_t)w[5] << 32 | w[4]);
+    }
+    return r;
+}
+
+// The k-mer table, one thread per string of kKmer - 2 bases and the 16 strings it starts.
+template <class P>
+__device__ __forceinline__ Iv<P> extend_one(const DevFM &F, const Iv<P> &ik, int base)
+{
+    P kk, ll;
+    uint32_t wk[8], wl[8];
+    extend_rows<P>(F, ik, false, kk, ll);
+    load32(sector_of<P>(F, kk), wk);
+    load32(sector_of<P>(F, ll), wl);
+    return extend_with<P>(F, ik, false, 3 - base, kk, ll, wk, wl);
+}
+template <class P>
+__global__ void kmer_kernel(DevFM F, uint4 *__restrict__ out)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= kKmers / 16) return;
+    Iv<P> v = set_intv<P>(F, (int)(t >> (2 * kKmer - 6)) & 3);
+    for (int k = kKmer - 4; k >= 0; --k) v = extend_one<P>(F, v, (int)(t >> (2 * k)) & 3);
+    for (int a = 0; a < 4; ++a) {
+        const Iv<P> va = extend_one<P>(F, v, a);
+        for (int b = 0; b < 4; ++b) {
+            const Iv<P> e = extend_one<P>(F, va, b);
+            const uint32_t code = t << 4 | a << 2 | b;
+            if (sizeof(P) == 4) {
+                out[code] = make_uint4((uint32_t)e.x0, (uint32_t)e.x1, (uint32_t)e.x2, 0u);
+            } else {
+                const uint64_t x0 = e.x0, x1 = e.x1, x2 = e.x2;
+                out[2 * (uint64_t)code] = make_uint4((uint32_t)x0, (uint32_t)(x0 >> 32), (uint32_t)x1, (uint32_t)(x1 >> 32));
+                out[2 * (uint64_t)code + 1] = make_uint4((uint32_t)x2, (uint32_t)(x2 >> 32), 0u, 0u);
+            }
+        }
+    }
+}
+
+// Control words: [1] overflow (read + 1), [2] pass-2 items queued, [3] next chunk of pass 2, [4..5]
+// the bwt_extend calls of the batch (uint64; each is one bwt_2occ4, two occurrence queries).
+enum { kCtrlOverflow = 1, kCtrlQueued = 2, kCtrlNext = 3, kCtrlExt = 4, kCtrlWords = 8 };
 
 // A pass-2 item: bwt_smem1 of read r from x with min_intv occurrences.
 struct Reseed {
@@ -132,37 +196,106 @@ struct SeedOut {
     const int64_t *offs;
 };
 
-// Passes 1-2: one SMEM [b, e) of read r; from pass 1 a long, rare one is queued for pass 2.
-template <class P, int Pass>
-__device__ __noinline__ void emit_smem(const SeedOpt &opt, const SeedOut &S, int r, int len, int b, int e, Iv<P> v)
-{
-    const int slot = atomicAdd(&S.count[2 * r], 1);
-    if (slot < part_cap0(len, S.mult)) {
-        DevIntv d;
-        d.x0 = v.x0, d.x1 = v.x1, d.x2 = v.x2;
-        d.info = (uint64_t)(uint32_t)b << 32 | (uint32_t)e;
-        S.out[part_base(S.offs[r] - S.offs[0], r, S.mult) + slot] = d;
-    } else {
-        atomicMax(S.ctrl + kCtrlOverflow, r + 1);
-    }
-    if (Pass == 1 && e - b >= opt.split_len && (uint64_t)v.x2 <= (uint64_t)(int64_t)opt.split_width) {
-        const int q = atomicAdd(S.ctrl + kCtrlQueued, 1);
-        if (q < S.queue_cap) S.queue[q] = Reseed{r, (b + e) >> 1, (int64_t)v.x2 + 1};
-        else atomicMax(S.ctrl + kCtrlOverflow, r + 1);
-    }
-}
-
-// The reads of a warp's chunk.
+// The reads of a warp's chunk, beside their packed bases.
 struct ChunkRead {
-    const uint8_t *q;
     int len, r;
     int64_t min_intv;
 };
 
-// Pass 3 of read r by one lane of a converged warp (has: the lane has a read).
+// Passes 1-2: the first n (<= 32) SMEMs of a warp's buffer go out, a lane each, so that the wait for
+// a read's slot counter is paid once for 32 of them; from pass 1 the long, rare ones are queued for
+// pass 2.
+template <class P, int Pass>
+__device__ __forceinline__ void flush_smems(const SeedOpt &opt, const SeedOut &S, const ChunkRead *CR,
+                                            const typename MatchOf<P>::type *buf, int n, int lane)
+{
+    bool again = false;
+    Reseed rs;
+    rs.r = rs.x = 0, rs.min_intv = 0;
+    if (lane < n) {
+        const typename MatchOf<P>::type v = buf[lane];
+        const int k = (int)(v.pos >> 21 & 31u), b = (int)(v.pos >> 11 & 1023u), e = (int)(v.pos & 2047u);
+        const int r = CR[k].r;
+        const int slot = atomicAdd(&S.count[2 * r], 1);
+        if (slot < part_cap0(CR[k].len, S.mult)) {
+            DevIntv d;
+            d.x0 = v.x0, d.x1 = v.x1, d.x2 = v.x2;
+            d.info = (uint64_t)(uint32_t)b << 32 | (uint32_t)e;
+            S.out[part_base(S.offs[r] - S.offs[0], r, S.mult) + slot] = d;
+        } else {
+            atomicMax(S.ctrl + kCtrlOverflow, r + 1);
+        }
+        again = Pass == 1 && e - b >= opt.split_len && (uint64_t)v.x2 <= (uint64_t)(int64_t)opt.split_width;
+        rs.r = r, rs.x = (b + e) >> 1, rs.min_intv = (int64_t)v.x2 + 1;
+    }
+    if (Pass == 1) {
+        const unsigned m = __ballot_sync(BSB_FULL_MASK, again);
+        if (m) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(S.ctrl + kCtrlQueued, __popc(m));
+            at = __shfl_sync(BSB_FULL_MASK, at, 0) + __popc(m & ((1u << lane) - 1u));
+            if (again) {
+                if (at < S.queue_cap) S.queue[at] = rs;
+                else atomicMax(S.ctrl + kCtrlOverflow, rs.r + 1);
+            }
+        }
+    }
+}
+
+// The reads of a warp's chunk, in shared memory: per read nw words of 16 bases (first base in the
+// top bits, 0 for an N) and nm words of N bits (first base in bit 0; set from the read's end on),
+// both strides odd so that the lanes' reads lie in different banks.
+__host__ __device__ __forceinline__ int chunk_words(int max_len) { return (max_len / 16 + 2) | 1; }
+__host__ __device__ __forceinline__ int chunk_masks(int max_len) { return (max_len / 32 + 2) | 1; }
+
+struct PackedReads {
+    const uint32_t *w, *m;
+    int nw, nm;
+    // base i of read k, 4 for an N and past the end
+    __device__ __forceinline__ int base(int k, int i) const
+    {
+        const uint32_t v = w[k * nw + (i >> 4)], n = m[k * nm + (i >> 5)];
+        return (n >> (i & 31) & 1u) ? 4 : (int)(v >> (30 - 2 * (i & 15)) & 3u);
+    }
+    // the code of the kKmer bases from i on; false where an N or the read's end is among them
+    __device__ __forceinline__ bool kmer(int k, int i, uint32_t &code) const
+    {
+        const uint32_t *p = w + k * nw + (i >> 4), *q = m + k * nm + (i >> 5);
+        code = __funnelshift_l(p[1], p[0], 2 * (i & 15)) >> (32 - 2 * kKmer);
+        return !(__funnelshift_r(q[0], q[1], i & 31) & ((1u << kKmer) - 1u));
+    }
+};
+
+// Packs the chunk's reads (lane k < n holds read k's bytes and length; a lane without a read: 0),
+// 16 bases a lane and step.
+__device__ __forceinline__ void pack_reads(uint32_t *w, uint32_t *m, int nw, int nm, int n, const uint8_t *q, int len,
+                                           int lane)
+{
+    const int per = 2 * nm;                             // 16-bit halves of a read's N bits, at least nw
+    for (int t0 = 0; t0 < n * per; t0 += 32) {
+        const int t = t0 + lane, k = min(t / per, 31), word = t - t / per * per;
+        const uint8_t *p = (const uint8_t *)__shfl_sync(BSB_FULL_MASK, (unsigned long long)q, k);
+        const int l = __shfl_sync(BSB_FULL_MASK, len, k) - word * 16;
+        uint32_t b[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) b[j] = j < l ? __ldg(p + word * 16 + j) : 4u;
+        uint32_t v = 0, none = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            v |= (b[j] < 4 ? b[j] : 0u) << (30 - 2 * j);
+            none |= (uint32_t)(b[j] > 3) << j;
+        }
+        if (t < n * per) {
+            if (word < nw) w[k * nw + word] = v;
+            ((uint16_t *)m)[k * per + word] = (uint16_t)none;
+        }
+    }
+}
+
+// Pass 3 of read r, packed read k, by one lane of a converged warp (has: the lane has a read).
 template <class P>
 __device__ __forceinline__ unsigned pass3(const DevFM &F, const SeedOpt &opt, const SeedOut &S, bool has, int r, int len,
-                                          const uint8_t *q)
+                                          const PackedReads &R, int k, bool tab)
 {
     DevIntv *dst = nullptr;
     int cap = 0, n = 0, i = 0, x = 0;
@@ -173,33 +306,43 @@ __device__ __forceinline__ unsigned pass3(const DevFM &F, const SeedOpt &opt, co
     bool in = false;
     Iv<P> ik;
     ik.x0 = ik.x1 = ik.x2 = 0;
-    int qc = has && i < len ? q[i] : 4;
     unsigned n_ext = 0;
     while (__any_sync(BSB_FULL_MASK, has && i < len)) {
         const bool act = has && i < len;
-        const int qn = act && i + 1 < len ? q[i + 1] : 4;      // for the next step, under this one's fetches
-        if (act && in && qc < 4) {
-            const Iv<P> ok = extend_one<P>(F, ik, false, 3 - qc);
-            ++n_ext;
-            ik = ok;
-            if (ok.x2 < (P)opt.max_mem_intv && i - x >= opt.min_seed_len) {
-                if (ok.x2 > 0) {                               // an empty interval is not kept (bwamem.c:160)
-                    if (n < cap) {
-                        DevIntv d;
-                        d.x0 = ok.x0, d.x1 = ok.x1, d.x2 = ok.x2;
-                        d.info = (uint64_t)(uint32_t)x << 32 | (uint32_t)(i + 1);
-                        dst[n] = d;
+        const int qc = act ? R.base(k, i) : 4;
+        uint32_t code = 0;
+        const bool jump = act && !in && tab && R.kmer(k, i, code), ext = act && in && qc < 4;
+        if (jump || ext) {
+            P kk = 0, ll = 0;
+            uint32_t wk[8], wl[8];
+            if (ext) extend_rows<P>(F, ik, false, kk, ll);
+            load32(jump ? kmer_at<P>(F, code) : sector_of<P>(F, kk), wk);
+            load32(jump ? kmer_at<P>(F, code) : sector_of<P>(F, ll), wl);
+            if (jump) {
+                ik = kmer_of<P>(wk, code);
+                in = true, x = i;
+                i += kKmer - 1;
+            } else {
+                ik = extend_with<P>(F, ik, false, 3 - qc, kk, ll, wk, wl);
+                ++n_ext;
+                if (ik.x2 < (P)opt.max_mem_intv && i - x >= opt.min_seed_len) {
+                    if (ik.x2 > 0) {                           // an empty interval is not kept (bwamem.c:160)
+                        if (n < cap) {
+                            DevIntv d;
+                            d.x0 = ik.x0, d.x1 = ik.x1, d.x2 = ik.x2;
+                            d.info = (uint64_t)(uint32_t)x << 32 | (uint32_t)(i + 1);
+                            dst[n] = d;
+                        }
+                        ++n;
                     }
-                    ++n;
+                    in = false;
                 }
-                in = false;
             }
         } else if (act) {
             in = qc < 4;
             if (in) ik = set_intv<P>(F, qc), x = i;
         }
         ++i;
-        qc = qn;
     }
     if (has) {
         if (n > cap) atomicMax(S.ctrl + kCtrlOverflow, r + 1);
@@ -208,174 +351,372 @@ __device__ __forceinline__ unsigned pass3(const DevFM &F, const SeedOpt &opt, co
     return n_ext;
 }
 
-// Mode 0: chunks of rho reads for pass 1, then chunks of 32 reads for pass 3.  Mode 1: chunks of
-// the queued re-seeds of pass 2, as many a chunk as spread them over all warps (at most rho).
-// matches: region_cap entries per warp.  A read (a re-seed) pushes at most one match per end
-// position, so rho * (max_len + 1) entries always hold a chunk.
-template <class P, int Mode>
-__global__ void __launch_bounds__(kSeedBlock, sizeof(P) == 4 ? 7 : 5)
-seed_kernel(DevFM F, SeedOpt opt, int n_reads, int max_len, const uint8_t *__restrict__ seqs, SeedOut S,
-            typename MatchOf<P>::type *__restrict__ matches, int region_cap, int rho)
+// With a k-mer table (and min_seed_len >= kKmer) a match of fewer than kKmer bases is never formed:
+// the forward phase starts at length kKmer, and what would be the matches [x, e) with e < x + kKmer
+// is one record of x (a fan); such a match to the left has to reach [e - kKmer, e) to become a
+// seed, so it starts from that string's entry.  (An end whose size does not change there is tried
+// too; its match can grow to the right, so it is not emitted.)  Where the string from x has fewer
+// than min_intv occurrences the forward phase goes base by base, and the short matches it lists are
+// marked kTable to start the same way.  kSeed: the match is an SMEM as it stands.
+constexpr uint32_t kTable = 1u << 31, kSeed = 1u << 30;
+constexpr int kFan = kKmer - 1;
+
+// The forward phases of bwt_smem1 (bwt.c:300-319) for the reads of a warp's chunk, a lane each, one
+// extension a step; matches are listed when their size is about to change.  Reseed false: all
+// matches of a read, the next one from where the longest ended; true: one from x with mi
+// occurrences.  Matches go to list[0 ..), fans to list[cap - 1], list[cap - 2] ..: together at most one
+// per read and end position, so a cap of the reads' bases and one more each always holds them.
+template <class P, bool Reseed>
+__device__ __forceinline__ unsigned forward_phase(const DevFM &F, const SeedOpt &opt, const PackedReads &R, bool act,
+                                                  int len, int x, P mi, bool tab, typename MatchOf<P>::type *list, int cap,
+                                                  int lane, int &n_list, int &n_fans)
 {
     using Match = typename MatchOf<P>::type;
-    __shared__ ChunkRead chunk_reads[kSeedWarps][32];
-    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
-    ChunkRead *const CR = chunk_reads[wb];
-    Match *const list = matches + (size_t)(blockIdx.x * kSeedWarps + wb) * region_cap;
-    const int64_t *const offs = S.offs;
-    int *const next = S.ctrl + (Mode ? kCtrlNext2 : kCtrlNext1);
-    const int n_items = Mode ? min(*(volatile int *)(S.ctrl + kCtrlQueued), S.queue_cap) : n_reads;
-    if (Mode) {
-        const int warps = gridDim.x * kSeedWarps;
-        rho = min(rho, max(1, (n_items + warps - 1) / warps));
-    }
-    const int n1 = (n_items + rho - 1) / rho;
-    const int n_chunks = n1 + (Mode == 0 && opt.max_mem_intv > 0 ? (n_reads + 31) / 32 : 0);
+    int i = Reseed ? x : 0, lb = 0;       // lb: the leftmost base a match from x can reach (no N before x)
+    bool in = false, slow = false;        // slow: this match base by base from its start
+    Iv<P> ik;
+    ik.x0 = ik.x1 = ik.x2 = 0;
     unsigned n_ext = 0;
+    n_list = n_fans = 0;
+    if (Reseed && act) {
+        act = R.base(lane, x) < 4;        // bwt_smem1 returns at once: no SMEM
+        lb = x == 0 || R.base(lane, x - 1) > 3 ? x : 0;
+    }
+    while (__any_sync(BSB_FULL_MASK, act)) {
+        const int qc = act ? R.base(lane, i) : 4;
+        uint32_t code = 0;
+        const bool jump = act && !in && !slow && tab && R.kmer(lane, i, code), ext = act && in && qc < 4;
+        Iv<P> ok = ik;
+        if (jump || ext) {
+            P kk = 0, ll = 0;
+            uint32_t wk[8], wl[8];
+            if (ext) extend_rows<P>(F, ik, false, kk, ll);
+            load32(jump ? kmer_at<P>(F, code) : sector_of<P>(F, kk), wk);
+            load32(jump ? kmer_at<P>(F, code) : sector_of<P>(F, ll), wl);
+            ok = jump ? kmer_of<P>(wk, code) : extend_with<P>(F, ik, false, 3 - qc, kk, ll, wk, wl);
+        }
+        n_ext += ext;
+        const bool push = act && in && (qc > 3 || ok.x2 != ik.x2);    // an N or the read's end stops the match
+        const bool stop = push && (qc > 3 || ok.x2 < mi);
+        // nothing to the left of x: only the longest match, and it is an SMEM
+        const bool seed = stop && x == lb;
+        const bool put = (seed || (push && x > lb)) && i - lb >= opt.min_seed_len;
+        const unsigned m = __ballot_sync(BSB_FULL_MASK, put);
+        if (put) {
+            const int slot = n_list + __popc(m & below);
+            Match e;
+            e.x0 = ik.x0, e.x1 = ik.x1, e.x2 = ik.x2;
+            e.pos = (uint32_t)lane << 21 | (uint32_t)x << 11 | (uint32_t)i;
+            if (seed) e.pos |= kSeed;
+            else if (tab && i - x < kKmer) e.pos |= kTable;
+            if (slot < cap) list[slot] = e;
+        }
+        n_list += __popc(m);
+        const bool hit = jump && ok.x2 >= mi, fan = hit && i > lb && i + kKmer - 1 >= lb + opt.min_seed_len;
+        const unsigned mf = __ballot_sync(BSB_FULL_MASK, fan);
+        if (fan) {
+            const int slot = cap - 1 - n_fans - __popc(mf & below);
+            if (slot >= 0)
+                list[slot].pos = (uint32_t)lane << 21 | (uint32_t)i << 11 | (uint32_t)max(i + 1, lb + opt.min_seed_len);
+        }
+        n_fans += __popc(mf);
+        if (hit) {
+            in = true, x = i, ik = ok, i += kKmer;
+        } else if (jump) {
+            slow = true;
+        } else if (act) {
+            if (Reseed && stop) {
+                act = false;
+            } else if (stop && tab && qc < 4) {           // a new match from i, which is looked up first
+                in = slow = false;
+            } else {
+                if (!in || stop) {
+                    in = qc < 4, slow = false;
+                    if (in) ik = set_intv<P>(F, qc), x = i;
+                    else lb = i + 1, act = i < len;
+                } else {
+                    ik = ok;
+                }
+                ++i;
+            }
+        }
+    }
+    n_list = min(n_list, cap);
+    n_fans = min(n_fans, cap);
+    return n_ext;
+}
+
+// The listed matches to the left (bwt.c:320-353): the lanes take them one after the other, the next
+// one loaded ahead; of the units k = 32 * (j * stride + first) + l (fans first, kFan each) for all
+// j and l.  buf: 64 SMEMs of shared memory.
+template <class P, bool Reseed>
+__device__ __forceinline__ unsigned backward_phase(const DevFM &F, const SeedOpt &opt, const SeedOut &S,
+                                                   const PackedReads &R, const ChunkRead *CR, bool tab,
+                                                   const typename MatchOf<P>::type *list, int cap, int n_list, int n_fans,
+                                                   int first, int stride, typename MatchOf<P>::type *buf, int lane)
+{
+    using Match = typename MatchOf<P>::type;
+    const unsigned below = (1u << lane) - 1u;
+    const int fans = n_fans * kFan, total = fans + n_list;
+    unsigned n_ext = 0;
+    int taken = 0, n_buf = 0;
+    bool have = false, spare = false, right = false, jump = false, done = false;
+    Iv<P> v;
+    v.x0 = v.x1 = v.x2 = 0;
+    Match sp;
+    sp.x0 = sp.x1 = sp.x2 = 0, sp.pos = 0;
+    int i = 0, e = 0, slot = 0;
+    P mi = 1;
+    bool more = 32 * first < total;
     for (;;) {
-        int ch = 0;
-        if (lane == 0) ch = atomicAdd(next, 1);
-        ch = __shfl_sync(BSB_FULL_MASK, ch, 0);
-        if (ch >= n_chunks) break;
-        // ---- the chunk's reads, a lane each
-        const bool p3 = Mode == 0 && ch >= n1;
-        const int item = p3 ? (ch - n1) * 32 + lane : ch * rho + lane;
-        bool act = item < n_items && (p3 || lane < rho);
-        int r = 0, len = 0, x = 0;
-        P mi = 1;
-        const uint8_t *q = seqs;
-        if (act) {
-            r = item;
-            if (Mode) {
-                const Reseed it = S.queue[item];
-                r = it.r, x = it.x, mi = (P)it.min_intv;
-            }
-            const int64_t o = offs[r], l = offs[r + 1] - o;
-            q = seqs + o;
-            len = (int)l;
-            if (l < 0 || l > max_len) {                 // outside what the launch was sized for: refuse
-                atomicMax(S.ctrl + kCtrlOverflow, r + 1);
-                act = false;
-            } else if (len < opt.min_seed_len) {        // mem_chain returns before seeding (bwamem.c:266)
-                act = false;
-            }
+        if (!have && spare) {
+            v.x0 = sp.x0, v.x1 = sp.x1, v.x2 = sp.x2;
+            slot = (int)(sp.pos >> 21 & 31u);
+            e = (int)(sp.pos & 2047u);
+            jump = sp.pos & kTable, done = sp.pos & kSeed;
+            i = jump ? e - kKmer : (int)(sp.pos >> 11 & 1023u) - 1;
+            if (Reseed) mi = (P)CR[slot].min_intv;
+            have = true, spare = right = false;
         }
-        if (p3) {
-            n_ext += pass3<P>(F, opt, S, act, r, len, q);
-            continue;
+        if (more) {
+            const unsigned m = __ballot_sync(BSB_FULL_MASK, !spare);
+            const int t = taken + __popc(m & below), k = ((t >> 5) * stride + first) * 32 + (t & 31);
+            if (!spare && k < total) {
+                if (k < fans) {                         // end x + 1 + k % kFan of fan k / kFan
+                    const uint32_t f = list[cap - 1 - k / kFan].pos;
+                    const uint32_t end = (f >> 11 & 1023u) + 1 + (uint32_t)(k % kFan);
+                    sp.pos = (f & ~2047u) | kTable | end;
+                    spare = end >= (f & 2047u);
+                } else {
+                    sp = list[k - fans], spare = true;
+                }
+            }
+            taken += __popc(m);
+            more = ((taken >> 5) * stride + first) * 32 < total;
         }
-        __syncwarp();
-        CR[lane] = ChunkRead{q, len, r, (int64_t)mi};
-        __syncwarp();
-        // ---- forward (bwt.c:300-319): every lane one extension a step, matches pushed when their
-        // size is about to change.  lb: the leftmost base a match from x can reach (no N before x)
-        int total = 0;
-        {
-            int i = 0, lb = 0;
-            bool in = false;
-            Iv<P> ik;
-            ik.x0 = ik.x1 = ik.x2 = 0;
-            if (Mode && act) {
-                if (q[x] > 3) act = false;              // bwt_smem1 returns at once: no SMEM
-                else {
-                    ik = set_intv<P>(F, q[x]);
-                    lb = x == 0 || q[x - 1] > 3 ? x : 0;
-                    in = true;
-                    i = x + 1;
-                }
-            }
-            int qc = act && i < len ? q[i] : 4;
-            while (__any_sync(BSB_FULL_MASK, act)) {
-                const int qn = act && i + 1 < len ? q[i + 1] : 4;
-                const bool ext = act && in && qc < 4;
-                Iv<P> ok = ik;
-                if (ext) ok = extend_one<P>(F, ik, false, 3 - qc);
-                n_ext += ext;
-                bool push = false, stop = false;
-                if (act && in) {
-                    push = qc > 3 || ok.x2 != ik.x2;      // an N or the read's end stops the match
-                    stop = qc > 3 || (push && ok.x2 < mi);
-                }
-                const Iv<P> pv = ik;
-                const int px = x, pe = i;
-                const bool enq = push && px > lb && pe - lb >= opt.min_seed_len;
-                // nothing to the left of x: only the longest match, and it is an SMEM
-                const bool seed = push && stop && px == lb && pe - px >= opt.min_seed_len;
-                if (act) {
-                    if (ext && !stop) ik = ok;
-                    if (!in || stop) {
-                        in = qc < 4 && !(Mode && stop);
-                        if (in) ik = set_intv<P>(F, qc), x = i;
-                        else lb = i + 1;
-                        if (i >= len || (Mode && stop)) act = false;
-                    }
-                    ++i;
-                }
-                qc = qn;
-                const unsigned m = __ballot_sync(BSB_FULL_MASK, enq);
-                if (enq) {
-                    const int slot = total + __popc(m & below);
-                    Match e;
-                    e.x0 = pv.x0, e.x1 = pv.x1, e.x2 = pv.x2;
-                    e.pos = (uint32_t)lane << 21 | (uint32_t)px << 11 | (uint32_t)pe;
-                    if (slot < region_cap) list[slot] = e;
-                }
-                total += __popc(m);
-                if (seed) emit_smem<P, Mode + 1>(opt, S, r, len, px, pe, pv);
-            }
-            total = min(total, region_cap);
-        }
-        __syncwarp();
-        // ---- backward: the lanes take the list's matches, the next one loaded ahead
-        int taken = 0;
-        bool have = false, spare = false, right = false;
-        Iv<P> v;
-        v.x0 = v.x1 = v.x2 = 0;
-        Match sp;
-        sp.x0 = sp.x1 = sp.x2 = 0, sp.pos = 0;
-        int i = 0, e = 0, c = 4, slot = 0;
-        q = seqs, len = 0, mi = 1;
-        for (;;) {
-            if (!have && spare) {
-                v.x0 = sp.x0, v.x1 = sp.x1, v.x2 = sp.x2;
-                slot = (int)(sp.pos >> 21);
-                i = (int)(sp.pos >> 11 & 1023u) - 1, e = (int)(sp.pos & 2047u);
-                q = CR[slot].q, len = CR[slot].len, mi = (P)CR[slot].min_intv;
-                c = q[i];                               // x > lb: there is a base to the left
-                have = true, spare = right = false;
-            }
-            if (taken < total) {
-                const unsigned m = __ballot_sync(BSB_FULL_MASK, !spare);
-                const int k = taken + __popc(m & below);
-                if (!spare && k < total) sp = list[k], spare = true;
-                taken += __popc(m);
-            }
-            if (!__any_sync(BSB_FULL_MASK, have || spare)) break;
-            if (!have) continue;
-            const int qn = !right && i > 0 ? q[i - 1] : 4;
-            const bool ext = right || c < 4;
+        if (!__any_sync(BSB_FULL_MASK, have || spare || more)) break;
+        uint32_t code = 0;
+        if (have && jump && !R.kmer(slot, i, code)) have = jump = false;   // an N among the last kKmer bases: too short
+        bool put = have && done;
+        if (have && !done) {
+            const int c = jump || (!right && i < 0) ? 4 : R.base(slot, right ? e : i);
+            const bool ext = c < 4;
             Iv<P> ok = v;
-            if (ext) ok = extend_one<P>(F, v, !right, right ? 3 - c : c);
+            if (jump || ext) {
+                P kk = 0, ll = 0;
+                uint32_t wk[8], wl[8];
+                if (ext) extend_rows<P>(F, v, !right, kk, ll);
+                load32(jump ? kmer_at<P>(F, code) : sector_of<P>(F, kk), wk);
+                load32(jump ? kmer_at<P>(F, code) : sector_of<P>(F, ll), wl);
+                ok = jump ? kmer_of<P>(wk, code) : extend_with<P>(F, v, !right, right ? 3 - c : c, kk, ll, wk, wl);
+            }
             n_ext += ext;
-            const bool grows = ext && ok.x2 >= mi;
+            const bool grows = (jump || ext) && ok.x2 >= mi;
             if (right) {                                // asked whether [i + 1, e) can grow to the right
-                have = false;
-                if (!grows) emit_smem<P, Mode + 1>(opt, S, CR[slot].r, len, i + 1, e, v);
+                have = false, put = !grows;
             } else if (grows) {
                 v = ok;
                 --i;
-                c = i >= 0 ? qn : 4;
-            } else if (e - (i + 1) >= opt.min_seed_len) {   // [i + 1, e) is as long as it gets to the left
-                c = e < len ? q[e] : 4;
+            } else if (!jump && e - (i + 1) >= opt.min_seed_len) {   // [i + 1, e) is as long as it gets to the left
                 right = true;
             } else {
                 have = false;
             }
+            jump = false;
         }
-        __syncwarp();
+        const unsigned mp = __ballot_sync(BSB_FULL_MASK, put);
+        if (mp) {
+            if (put) {
+                Match o;
+                o.x0 = v.x0, o.x1 = v.x1, o.x2 = v.x2;
+                o.pos = (uint32_t)slot << 21 | (uint32_t)(i + 1) << 11 | (uint32_t)e;
+                buf[n_buf + __popc(mp & below)] = o;
+                have = false;
+            }
+            n_buf += __popc(mp);
+            if (n_buf >= 32) {
+                __syncwarp();
+                flush_smems<P, Reseed ? 2 : 1>(opt, S, CR, buf, 32, lane);
+                n_buf -= 32;
+                Match o = sp;
+                if (lane < n_buf) o = buf[32 + lane];
+                __syncwarp();
+                if (lane < n_buf) buf[lane] = o;
+            }
+        }
     }
-    if (n_ext) atomicAdd((unsigned long long *)(S.ctrl + kCtrlExt), (unsigned long long)n_ext);
+    __syncwarp();
+    flush_smems<P, Reseed ? 2 : 1>(opt, S, CR, buf, n_buf, lane);
+    __syncwarp();
+    return n_ext;
+}
+
+// The warp's share of a block's dynamic shared memory: packed reads, then 64 SMEMs.
+template <class P>
+__device__ __forceinline__ typename MatchOf<P>::type *warp_smem(uint32_t *smem, int slots, int max_len, int wb,
+                                                                uint32_t *&pw, uint32_t *&pm, PackedReads &R)
+{
+    using Match = typename MatchOf<P>::type;
+    R.nw = chunk_words(max_len), R.nm = chunk_masks(max_len);
+    Match *const bufs = (Match *)smem;
+    uint32_t *const reads = (uint32_t *)(bufs + 64 * kSeedWarps) + (size_t)wb * slots * (R.nw + R.nm);
+    pw = reads, pm = reads + slots * R.nw;
+    R.w = pw, R.m = pm;
+    return bufs + 64 * wb;
+}
+
+__device__ __forceinline__ void count_extensions(const SeedOut &S, unsigned n_ext, int lane)
+{
+    n_ext = __reduce_add_sync(BSB_FULL_MASK, n_ext);
+    if (lane == 0 && n_ext) atomicAdd((unsigned long long *)(S.ctrl + kCtrlExt), (unsigned long long)n_ext);
+}
+
+// The list of reads r0 .. r1 - 1 among pass 1's: an entry per base and one more per read, from their
+// first base's place on; kept inside the list_cap entries whatever the offsets say.
+__device__ __forceinline__ int list_of(const SeedOut &S, int r0, int r1, int slots, int max_len, int64_t list_cap,
+                                       int64_t &at)
+{
+    at = S.offs[r0] - S.offs[0] + r0;
+    int64_t cap = min(S.offs[r1] - S.offs[r0], (int64_t)slots * max_len) + (r1 - r0);
+    cap = min(cap, list_cap - at);
+    if (at < 0 || cap < 0) at = cap = 0;
+    return (int)cap;
+}
+
+// A lane's read of a chunk: false where there is none or mem_chain returns before seeding it
+// (bwamem.c:266); a length the launch was not sized for is refused.
+__device__ __forceinline__ bool chunk_read(const SeedOut &S, const SeedOpt &opt, const uint8_t *seqs, int r, int max_len,
+                                           const uint8_t *&q, int &len)
+{
+    const int64_t o = S.offs[r], l = S.offs[r + 1] - o;
+    q = seqs + o;
+    len = 0;
+    if (l < 0 || l > max_len) {
+        atomicMax(S.ctrl + kCtrlOverflow, r + 1);
+        return false;
+    }
+    if (l < opt.min_seed_len) return false;
+    len = (int)l;
+    return true;
+}
+
+// Pass 1's forward phases (a warp each for reads 32c ..) and pass 3 (the warps after these, `slots`
+// reads each).  A warp's list: as many entries as its reads have bases, and one more per read.
+// counts[c]: its matches and fans.
+template <class P>
+__global__ void __launch_bounds__(kSeedBlock, sizeof(P) == 4 ? 8 : 6)
+seed_forward_kernel(DevFM F, SeedOpt opt, int n_reads, int max_len, int slots, const uint8_t *__restrict__ seqs,
+                    SeedOut S, typename MatchOf<P>::type *__restrict__ lists, int64_t list_cap,
+                    int2 *__restrict__ counts)
+{
+    extern __shared__ __align__(16) uint32_t smem[];
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const bool tab = F.kmers != nullptr && opt.min_seed_len >= kKmer;
+    const int n1 = (n_reads + slots - 1) / slots;
+    int c = blockIdx.x * kSeedWarps + wb;
+    const bool p3 = c >= n1;
+    if (p3) c -= n1;
+    if (c >= n1 || (p3 && opt.max_mem_intv <= 0)) return;
+    uint32_t *pw, *pm;
+    PackedReads R;
+    warp_smem<P>(smem, slots, max_len, wb, pw, pm, R);
+    const int r = c * slots + lane;
+    const uint8_t *q = seqs;
+    int len = 0;
+    const bool act = lane < slots && r < n_reads && chunk_read(S, opt, seqs, r, max_len, q, len);
+    pack_reads(pw, pm, R.nw, R.nm, slots, q, len, lane);
+    __syncwarp();
+    unsigned n_ext;
+    if (p3) {
+        n_ext = pass3<P>(F, opt, S, act, r, len, R, lane, tab);
+    } else {
+        int64_t b0;
+        const int cap = list_of(S, c * slots, min((c + 1) * slots, n_reads), slots, max_len, list_cap, b0);
+        int n_list, n_fans;
+        n_ext = forward_phase<P, false>(F, opt, R, act, len, 0, (P)1, tab, lists + b0, cap, lane, n_list, n_fans);
+        if (lane == 0) counts[c] = make_int2(n_list, n_fans);
+    }
+    count_extensions(S, n_ext, lane);
+}
+
+// Pass 1's backward phases: `split` warps share a list.
+template <class P>
+__global__ void __launch_bounds__(kSeedBlock, sizeof(P) == 4 ? 8 : 6)
+seed_backward_kernel(DevFM F, SeedOpt opt, int n_reads, int max_len, int slots, int split,
+                     const uint8_t *__restrict__ seqs, SeedOut S, const typename MatchOf<P>::type *__restrict__ lists,
+                     int64_t list_cap, const int2 *__restrict__ counts)
+{
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ ChunkRead chunk_reads[kSeedWarps][32];
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const bool tab = F.kmers != nullptr && opt.min_seed_len >= kKmer;
+    const int u = blockIdx.x * kSeedWarps + wb, c = u / split;
+    if (c * slots >= n_reads) return;
+    const int2 n = counts[c];
+    if (32 * (u - c * split) >= n.x + n.y * kFan) return;
+    uint32_t *pw, *pm;
+    PackedReads R;
+    typename MatchOf<P>::type *const buf = warp_smem<P>(smem, slots, max_len, wb, pw, pm, R);
+    const int r = c * slots + lane;
+    const uint8_t *q = seqs;
+    int len = 0;
+    if (lane < slots && r < n_reads) chunk_read(S, opt, seqs, r, max_len, q, len);
+    chunk_reads[wb][lane] = ChunkRead{len, r, 1};
+    pack_reads(pw, pm, R.nw, R.nm, slots, q, len, lane);
+    __syncwarp();
+    int64_t b0;
+    const int cap = list_of(S, c * slots, min((c + 1) * slots, n_reads), slots, max_len, list_cap, b0);
+    const unsigned n_ext = backward_phase<P, false>(F, opt, S, R, chunk_reads[wb], tab, lists + b0, cap, n.x, n.y,
+                                                    u - c * split, split, buf, lane);
+    count_extensions(S, n_ext, lane);
+}
+
+// Pass 2: chunks of the queued re-seeds, as many a chunk as spread them over all warps (at most
+// slots), both phases; lists of slots * (max_len + 1) entries per warp.
+template <class P>
+__global__ void __launch_bounds__(kSeedBlock, sizeof(P) == 4 ? 8 : 5)
+seed_again_kernel(DevFM F, SeedOpt opt, int max_len, int slots, const uint8_t *__restrict__ seqs, SeedOut S,
+                  typename MatchOf<P>::type *__restrict__ lists)
+{
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ ChunkRead chunk_reads[kSeedWarps][32];
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const bool tab = F.kmers != nullptr && opt.min_seed_len >= kKmer;
+    ChunkRead *const CR = chunk_reads[wb];
+    uint32_t *pw, *pm;
+    PackedReads R;
+    typename MatchOf<P>::type *const buf = warp_smem<P>(smem, slots, max_len, wb, pw, pm, R);
+    const int cap = slots * (max_len + 1);
+    typename MatchOf<P>::type *const list = lists + (size_t)(blockIdx.x * kSeedWarps + wb) * cap;
+    const int n_items = min(*(volatile int *)(S.ctrl + kCtrlQueued), S.queue_cap);
+    const int warps = gridDim.x * kSeedWarps;
+    const int per = min(slots, max(1, (n_items + warps - 1) / warps));
+    unsigned n_ext = 0;
+    for (;;) {
+        int ch = 0;
+        if (lane == 0) ch = atomicAdd(S.ctrl + kCtrlNext, 1);
+        ch = __shfl_sync(BSB_FULL_MASK, ch, 0);
+        if ((int64_t)ch * per >= n_items) break;
+        const int item = ch * per + lane;
+        bool act = lane < per && item < n_items;
+        Reseed it;
+        it.r = it.x = 0, it.min_intv = 1;
+        const uint8_t *q = seqs;
+        int len = 0;
+        if (act) {
+            it = S.queue[item];
+            act = chunk_read(S, opt, seqs, it.r, max_len, q, len);
+        }
+        CR[lane] = ChunkRead{len, it.r, it.min_intv};
+        pack_reads(pw, pm, R.nw, R.nm, per, q, len, lane);
+        __syncwarp();
+        int n_list, n_fans;
+        n_ext += forward_phase<P, true>(F, opt, R, act, len, it.x, (P)it.min_intv, tab, list, cap, lane, n_list, n_fans);
+        __syncwarp();
+        n_ext += backward_phase<P, true>(F, opt, S, R, CR, tab, list, cap, n_list, n_fans, 0, 1, buf, lane);
+    }
+    count_extensions(S, n_ext, lane);
 }
 
 // Seeds of read r in the two parts of its padded region (a part that overflowed holds
@@ -498,41 +839,49 @@ __global__ void sa_fill_kernel(DevFM F, int64_t n_sa, uint64_t *__restrict__ ful
 
 static bool seed_narrow(uint64_t seq_len) { return seq_len < kNarrowRows; }
 
-// The launch shape of a batch: warps that are resident at once, reads a chunk of pass 1 takes, and
-// the match list each warp needs.
-// rho: as few reads a warp as still occupy every warp, so that the matches of a read spread over the
-// warp's lanes, and at most kSeedRho (67k reads of 150 bases: 2.5 ms at 2, 1.93 at 4, 1.73 at 8 and
-// 16, 1.86 at 24, 2.1 at 32, where the forward phases fill the lanes but half the warps stay empty).
-SeedPlan seed_plan(int n_sm, int max_len, int n_reads, uint64_t seq_len)
+// Builds the k-mer table of an index (kmer_bytes(seq_len) bytes) on the stream.
+size_t kmer_bytes(uint64_t seq_len) { return (size_t)kKmers * (seed_narrow(seq_len) ? 16 : 32); }
+cudaError_t kmer_build(const DevFM &F, void *out, cudaStream_t st)
+{
+    const unsigned blocks = kKmers / 16 / 128;
+    if (seed_narrow(F.seq_len)) kmer_kernel<uint32_t><<<blocks, 128, 0, st>>>(F, (uint4 *)out);
+    else kmer_kernel<uint64_t><<<blocks, 128, 0, st>>>(F, (uint4 *)out);
+    return cudaGetLastError();
+}
+
+template <class P>
+static int again_blocks_per_sm(size_t smem)
+{
+    int b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_again_kernel<P>, kSeedBlock, smem) != cudaSuccess || b < 1)
+        b = 4;
+    return b;
+}
+
+// The launch shape of a batch.  slots: reads a warp packs and runs side by side (32, 16 where that
+// would take more than 48 KB of shared memory a block).  split: warps that share a list of pass 1
+// matches: enough to fill the GPU, and at least four, which even out the lists (67k reads of 150
+// bases, seeding stage: 1.28 ms at 2, 1.30 at 3, 1.24 at 4, 1.26 at 6 and 8).  32 warps per SM at 64
+// registers: 40 at 48 registers 1.29, 48 at 40 2.1.  The lists of pass 1 and 2 share the memory.
+SeedPlan seed_plan(int n_sm, int64_t total_bases, int max_len, int n_reads, uint64_t seq_len)
 {
     const bool narrow = seed_narrow(seq_len);
-    static int resident[2] = {0, 0};
-    if (!resident[narrow]) {
-        int b = 0, b2 = 0;
-        const cudaError_t e =
-            narrow ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_kernel<uint32_t, 0>, kSeedBlock, 0)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seed_kernel<uint64_t, 0>, kSeedBlock, 0);
-        const cudaError_t e2 =
-            narrow ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, seed_kernel<uint32_t, 1>, kSeedBlock, 0)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, seed_kernel<uint64_t, 1>, kSeedBlock, 0);
-        b = std::min(b, b2);
-        if (e != cudaSuccess || e2 != cudaSuccess || b < 1) b = 4;
-        resident[narrow] = b;
-    }
-    SeedPlan p;
-    const int64_t warps = (int64_t)n_sm * resident[narrow] * kSeedWarps;
-    p.rho = (int)std::min<int64_t>(kSeedRho, std::max<int64_t>(1, (n_reads + warps - 1) / warps));
     const size_t entry = narrow ? sizeof(Match32) : sizeof(Match64);
-    const size_t budget = (size_t)1 << 30;              // long reads: fewer reads a warp
-    const size_t fit = budget / ((size_t)warps * (size_t)(max_len + 1) * entry);
-    if ((size_t)p.rho > fit) p.rho = (int)std::max<size_t>(1, fit);
-    // no more warps than the first launch has chunks (pass 1 and pass 3) or the second can use
-    const int64_t chunks = (n_reads + p.rho - 1) / p.rho + (n_reads + 31) / 32;
-    p.blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)n_sm * resident[narrow],
-                                                           std::max<int64_t>((chunks + kSeedWarps - 1) / kSeedWarps,
-                                                                             std::min<int64_t>(n_reads, n_sm))));
-    p.region_cap = p.rho * (max_len + 1);
-    p.list_bytes = (size_t)p.blocks * kSeedWarps * (size_t)p.region_cap * entry;
+    SeedPlan p;
+    p.slots = max_len <= 512 ? 32 : 16;
+    p.smem = kSeedWarps * (64 * entry + sizeof(uint32_t) * (size_t)p.slots *
+                                            (size_t)(chunk_words(max_len) + chunk_masks(max_len)));
+    const int64_t lists = (n_reads + p.slots - 1) / p.slots, warps = (int64_t)n_sm * 32;
+    p.split = (int)std::min<int64_t>(32, std::max<int64_t>(4, (warps + lists - 1) / lists));
+    // pass 2: no more warps than there are re-seeds to expect (a few a read), fewer for long reads,
+    // whose lists would take more than 1 GB
+    const size_t per_block = (size_t)kSeedWarps * p.slots * (size_t)(max_len + 1) * entry, budget = (size_t)1 << 30;
+    int64_t blocks = (int64_t)n_sm * (narrow ? again_blocks_per_sm<uint32_t>(p.smem) : again_blocks_per_sm<uint64_t>(p.smem));
+    blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, (int64_t)(budget / per_block)));
+    p.again_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, n_reads));
+    p.counts_bytes = sizeof(int2) * (size_t)lists;
+    p.list_entries = total_bases + n_reads;
+    p.list_bytes = std::max((size_t)p.again_blocks * per_block, (size_t)p.list_entries * entry);
     return p;
 }
 
@@ -551,19 +900,22 @@ size_t seed_padded_entries(int64_t total_bases, int n_reads, int mult)
 
 template <class P>
 static void seed_passes(const DevFM &F, const SeedOpt &o, int n_reads, int max_len, const uint8_t *d_seqs,
-                        const SeedOut &S, void *d_lists, const SeedPlan &p, cudaStream_t st)
+                        const SeedOut &S, void *d_lists, int2 *d_counts, const SeedPlan &p, cudaStream_t st)
 {
     using Match = typename MatchOf<P>::type;
-    seed_kernel<P, 0><<<p.blocks, kSeedBlock, 0, st>>>(F, o, n_reads, max_len, d_seqs, S, (Match *)d_lists,
-                                                       p.region_cap, p.rho);
-    seed_kernel<P, 1><<<p.blocks, kSeedBlock, 0, st>>>(F, o, n_reads, max_len, d_seqs, S, (Match *)d_lists,
-                                                       p.region_cap, p.rho);
+    const int lists = (n_reads + p.slots - 1) / p.slots;
+    const auto blocks = [](int64_t warps) { return (unsigned)((warps + kSeedWarps - 1) / kSeedWarps); };
+    seed_forward_kernel<P><<<blocks(2 * (int64_t)lists), kSeedBlock, p.smem, st>>>(F, o, n_reads, max_len, p.slots, d_seqs,
+                                                                                   S, (Match *)d_lists, p.list_entries, d_counts);
+    seed_backward_kernel<P><<<blocks((int64_t)lists * p.split), kSeedBlock, p.smem, st>>>(
+        F, o, n_reads, max_len, p.slots, p.split, d_seqs, S, (const Match *)d_lists, p.list_entries, d_counts);
+    seed_again_kernel<P><<<p.again_blocks, kSeedBlock, p.smem, st>>>(F, o, max_len, p.slots, d_seqs, S, (Match *)d_lists);
 }
 
 cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, int split_width, int max_mem_intv,
                         int n_reads, const uint8_t *d_seqs, const int64_t *d_offs, int max_len,
                         void *d_padded, int *d_count, int64_t *d_out_off, void *d_out,
-                        void *d_lists, int *d_ctrl, void *d_queue, int64_t queue_cap, int *d_tot,
+                        const SeedPlan &p, void *d_lists, void *d_list_counts, int *d_ctrl, void *d_queue, int64_t queue_cap, int *d_tot,
                         int64_t *d_scan_tmp, int mult, int n_sm, cudaStream_t st)
 {
     SeedOpt o;
@@ -582,9 +934,9 @@ cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, in
     S.queue_cap = (int)(queue_cap < 0x7fffffff ? queue_cap : 0x7fffffff);
     S.mult = mult;
     S.offs = d_offs;
-    const SeedPlan p = seed_plan(n_sm, max_len, n_reads, F.seq_len);
-    if (seed_narrow(F.seq_len)) seed_passes<uint32_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, p, st);
-    else seed_passes<uint64_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, p, st);
+    int2 *const d_counts = (int2 *)d_list_counts;
+    if (seed_narrow(F.seq_len)) seed_passes<uint32_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, d_counts, p, st);
+    else seed_passes<uint64_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, d_counts, p, st);
     read_totals<<<n_sm * 4, 256, 0, st>>>(d_count, d_offs, n_reads, mult, d_tot);
     e = scan_i32_i64(d_tot, n_reads, d_out_off, d_scan_tmp, st);
     if (e != cudaSuccess) return e;
