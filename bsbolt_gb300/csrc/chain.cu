@@ -5,16 +5,18 @@
 //   rows_count / rows_fill  the SA rows mem_chain samples per seed interval
 //                           (bwamem.c:280-283), then sa_kernel (seed.cu) maps them
 //                           to reference positions;
-//   chain_kernel            one thread per read: mem_chain with the reference's
-//                           B-tree of chains (kbtree.h, t = 5) so equal keys land
-//                           where the reference puts them, then mem_chain_weight
-//                           and mem_chain_flt with ks_introsort's exact order;
+//   chain_warp_kernel       one warp per read: mem_chain, mem_chain_weight and
+//                           mem_chain_flt with ks_introsort's exact order;
+//   chain_kernel            the same by one thread, with the reference's B-tree of
+//                           chains (kbtree.h, t = 5), for reads where two chains start
+//                           at the same place and the tree's nodes decide;
 //   chain2aln_kernel        one warp per read: mem_chain2aln (bwamem.c:636-790),
 //                           each ksw_extend2 run by the warp (ksw_core.cuh) on the
 //                           read and the device 2-bit reference directly, so no
 //                           reversed copies or target windows are materialised.
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -314,23 +316,21 @@ struct FltLt {
     __device__ bool operator()(int x, int y) const { return w[x] > w[y]; }
 };
 
-// One thread per read.  Per-read scratch is carved from arrays sized by the
-// read's SA-row count R (a read never has more chains, seeds or tree nodes
-// than rows).  Outputs the kept chains in mem_chain_flt's order and their
-// seeds (in insertion order) at the read's row offset.
+// The reads that chain_warp_kernel leaves (two chains start at the same place, so their order
+// follows the tree's nodes): one thread per read, with the tree itself.  Per-read scratch is carved
+// from arrays sized by the read's SA-row count R (a read never has more chains, seeds or tree nodes
+// than rows).  Outputs the kept chains in mem_chain_flt's order and their seeds (in insertion
+// order) at the read's row offset.
 __global__ void __launch_bounds__(128)
-chain_kernel(AlnOpt opt, DevBns B, int n_reads, const int64_t *__restrict__ read_off,
-             const DevIntv *__restrict__ seeds, const int64_t *__restrict__ seed_off,
-             const int64_t *__restrict__ row_off_of_seed, const uint64_t *__restrict__ pos,
-             ChainRec *__restrict__ chains, BtNode *__restrict__ nodes, int *__restrict__ row_chain,
-             int *__restrict__ iwork, DevSeed *__restrict__ out_seeds, DevChain *__restrict__ out_chains,
-             int *__restrict__ n_chains, int *__restrict__ next)
+chain_kernel(AlnOpt opt, DevBns B, const int *__restrict__ list, const int *__restrict__ n_list,
+             const int64_t *__restrict__ read_off, const DevIntv *__restrict__ seeds,
+             const int64_t *__restrict__ seed_off, const int64_t *__restrict__ row_off_of_seed,
+             const uint64_t *__restrict__ pos, ChainRec *__restrict__ chains, BtNode *__restrict__ nodes,
+             int *__restrict__ row_chain, int *__restrict__ iwork, DevSeed *__restrict__ out_seeds,
+             DevChain *__restrict__ out_chains, int *__restrict__ n_chains)
 {
-    // reads in batch order: neighbouring threads' scratch (carved at the reads' row offsets)
-    // shares cache lines; taking reads by row count instead ran 1.6 -> 3.8 ms on a 100 Mb batch
-    for (;;) {
-        const int r = atomicAdd(next, 1);
-        if (r >= n_reads) break;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < *n_list; t += gridDim.x * blockDim.x) {
+        const int r = list[t];
         const int len = (int)(read_off[r + 1] - read_off[r]);
         const int64_t s0 = seed_off[r], s1 = seed_off[r + 1];
         const int64_t R0 = row_off_of_seed[s0], R = row_off_of_seed[s1] - R0;
@@ -530,6 +530,691 @@ chain_kernel(AlnOpt opt, DevBns B, int n_reads, const int64_t *__restrict__ read
                 if (oc[i].kept != 0) oc[k++] = oc[i];
             n_chains[r] = k;
         }
+    }
+}
+
+// ---------------------------------------------------------------- chaining, a warp per read
+
+// mem_chain, mem_chain_weight and mem_chain_flt with a warp per read.  The tree serves two
+// purposes, the chain with the largest pos at or before a row, and the chains in order of pos; while
+// no two chains of a read have the same pos neither depends on the tree's nodes.  A read where a
+// second chain would start at a pos that another one has (a seed that fails test_and_merge against
+// the chain it found there) goes to chain_kernel.
+//
+// chain_fast, up to kFastRows rows and 64 chains (of the 100 Mb workload's reads all but a few in a
+// thousand): the chains' places lie sorted over the lanes' registers, two a lane, so a row's
+// chain is one ballot and an insertion one shuffle; the chains' fields lie in shared memory.  Rows are
+// taken in order, one after the other (each sees the chains of those before), but their seed, contig
+// and place are found 32 at a time.  ks_introsort: a partition step's swaps follow from two
+// ballots over its segment, and the closing insertion sort is a stable sort, i.e. ranks.
+// mem_chain_flt: one step per kept chain, all others compared with it at once, in place of one
+// step per chain.
+// chain_general, any size: the same on arrays in the read's slices of the scratch, the sort on one lane.
+//
+// One thread per read walking the tree in global memory took 2.27 ms for 67k reads of 150 bases (36
+// rows, 20 chains a read), some 20,000 cycles a row; a warp per read with chain_general on shared
+// memory 1.03 ms (75,000 cycles a read: 960 a row, 12,500 the sort, 14,800 the filter); this 0.63 ms
+// (114k RRBS reads 1.78 -> 0.74 ms, 64 reads 78 -> 19 us), 6000 instructions a read with the issue
+// slots 71 % busy.  40 warps per SM (48 registers): 24 at 80 registers 0.68, 32 at 64 0.65.
+constexpr int kFastRows = 128, kFastChains = 64, kChainWarps = 4;
+
+struct FastChain {
+    int64_t pos, last_rbeg;             // first seed's rbeg, last seed's
+    int rid, first_qbeg, last_q, n;     // last_q: last seed's qbeg << 16 | len
+};
+struct ChainSmem {
+    FastChain ch[kFastChains];
+    int row[kFastRows], row_q[kFastRows];           // chain << 16 | place in it, or -1; qbeg << 16 | len
+    int order[kFastChains], weight[kFastChains], start[kFastChains];
+};
+
+// ks_introsort (ksort.h:146-226) of order[0 .. n), n <= 64, by weight[] (of the same places),
+// descending: the permutation it leaves, ties included.
+__device__ __forceinline__ void sort_places(int *order, int *weight, int n, int lane)
+{
+    const auto swap2 = [&](int x, int y) {
+        const int c = order[x], w = weight[x];
+        order[x] = order[y], weight[x] = weight[y];
+        order[y] = c, weight[y] = w;
+    };
+    if (n > 2) {
+        int d, top = 0, s = 0, t = n - 1;
+        int stk[8];                                     // s | t << 8 | d << 16; segments of more than 16 only
+        for (d = 2; 1 << d < n; ++d) ;
+        d <<= 1;
+        for (;;) {
+            if (s < t) {
+                if (--d == 0) {                         // the reference's combsort
+                    if (lane == 0) {
+                        const double shrink_factor = 1.2473309501039786540366528676643;
+                        const int m = t - s + 1;
+                        int swapped, gap = m;
+                        do {
+                            if (gap > 2) {
+                                gap = (int)(gap / shrink_factor);
+                                if (gap == 9 || gap == 10) gap = 11;
+                            }
+                            swapped = 0;
+                            for (int i = s; i + gap < s + m; ++i)
+                                if (weight[i + gap] > weight[i]) swap2(i, i + gap), swapped = 1;
+                        } while (swapped || gap > 2);
+                        if (gap != 1)
+                            for (int i = s + 1; i < s + m; ++i)
+                                for (int j = i; j > s && weight[j] > weight[j - 1]; --j) swap2(j, j - 1);
+                    }
+                    __syncwarp();
+                    t = s;
+                    continue;
+                }
+                int k = s + ((t - s) >> 1) + 1;
+                const int ws = weight[s], wt = weight[t], wm = weight[k];
+                if (wm > ws) {
+                    if (wm > wt) k = t;
+                } else {
+                    k = wt > ws ? s : t;
+                }
+                const int wp = weight[k];
+                __syncwarp();
+                if (lane == 0 && k != t) swap2(k, t);
+                __syncwarp();
+                // from the left the places not above the pivot, from the right those not below it
+                const int w0 = lane < n ? weight[lane] : 0, w1 = lane + 32 < n ? weight[lane + 32] : 0;
+                const uint64_t in = (~0ull >> (63 - t)) & (~0ull << s);
+                uint64_t L = in & ((uint64_t)__ballot_sync(BSB_FULL_MASK, w1 <= wp) << 32 |
+                                   __ballot_sync(BSB_FULL_MASK, w0 <= wp));
+                const uint64_t Rm = in & ((uint64_t)__ballot_sync(BSB_FULL_MASK, w1 >= wp) << 32 |
+                                          __ballot_sync(BSB_FULL_MASK, w0 >= wp));
+                int i = s, j = t, x = -1, y = -1;       // lane q swaps the q-th pair
+                for (int q = 0;; ++q) {
+                    i = __ffsll((long long)(L & (~0ull << i << 1))) - 1;         // t is among them
+                    const uint64_t below = Rm & ((1ull << j) - 1ull);
+                    const int p = 63 - __clzll((long long)below);               // -1: none
+                    if (p <= i) break;
+                    j = p;
+                    L |= 1ull << j;                     // it takes place i's, which is not above the pivot
+                    if (lane == q) x = i, y = j;
+                }
+                __syncwarp();
+                if (x >= 0) swap2(x, y);
+                __syncwarp();
+                if (lane == 0) swap2(i, t);
+                __syncwarp();
+                if (i - s > t - i) {
+                    if (i - s > 16) stk[top++] = s | (i - 1) << 8 | d << 16;
+                    s = t - i > 16 ? i + 1 : t;
+                } else {
+                    if (t - i > 16) stk[top++] = (i + 1) | t << 8 | d << 16;
+                    t = i - s > 16 ? i - 1 : s;
+                }
+            } else {
+                if (top == 0) break;
+                --top;
+                s = stk[top] & 255, t = stk[top] >> 8 & 255, d = stk[top] >> 16;
+            }
+        }
+    }
+    // insertion sort: stable
+    int c[2], w[2], rank[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int k = lane + 32 * h;
+        c[h] = k < n ? order[k] : 0, w[h] = k < n ? weight[k] : 0, rank[h] = 0;
+    }
+    for (int e = 0; e < n; ++e) {
+        const int u = weight[e];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) rank[h] += u > w[h] || (u == w[h] && e < lane + 32 * h);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if (lane + 32 * h < n) order[rank[h]] = c[h], weight[rank[h]] = w[h];
+    __syncwarp();
+}
+
+// -1: more than 64 chains (chain_general takes the read); 0: left to chain_kernel; 1: done, n_out
+// kept chains.
+__device__ __forceinline__ int chain_fast(const AlnOpt &opt, const DevBns &B, float frac_rep, const DevIntv *seeds, int ns,
+                                          const int64_t *roff, int64_t R0, int R, const uint64_t *pos, ChainSmem &S,
+                                          DevSeed *sd, DevChain *oc, int lane, int &n_out)
+{
+    constexpr int64_t kNone = INT64_MAX;
+    n_out = 0;
+    // mem_chain (bwamem.c:279-305).  p[h], c[h]: the chain with the (lane + 32 h)-th smallest pos
+    int64_t p[2] = {kNone, kNone};
+    int c[2] = {0, 0}, n = 0;
+    for (int base = 0; base < R; base += 32) {
+        const int k = base + lane;
+        int64_t rb = 0;
+        int q = 0, rid = -1;
+        // the seed of row k: the last with roff <= R0 + k, 32 seeds at a time over the lanes
+        int at = 0;
+        for (int s0 = 0; s0 < ns; s0 += 32) {
+            const int first = s0 + lane < ns ? (int)min(roff[s0 + lane] - R0, (int64_t)INT_MAX) : INT_MAX;
+            int lo = 0, hi = 32;                        // seeds of these that start at or before k
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                const int mid = (lo + hi) >> 1, f = __shfl_sync(BSB_FULL_MASK, first, min(mid, 31));
+                if (lo < hi) {
+                    if (f <= k) lo = mid + 1;
+                    else hi = mid;
+                }
+            }
+            at += lo;
+            if (__all_sync(BSB_FULL_MASK, lo < 32 || k >= R)) break;
+        }
+        if (k < R) {
+            const uint64_t info = seeds[at - 1].info;
+            const int qb = (int)(info >> 32), sl = (int)(uint32_t)info - qb;
+            q = qb << 16 | sl;
+            rb = (int64_t)pos[R0 + k];
+            rid = intv2rid(B, rb, rb + sl);
+            S.row[k] = -1;
+            S.row_q[k] = q;
+        }
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(BSB_FULL_MASK, rid >= 0); todo; todo &= todo - 1) {
+            const int j = __ffs(todo) - 1;
+            const int64_t rbeg = __shfl_sync(BSB_FULL_MASK, rb, j);
+            const int id = __shfl_sync(BSB_FULL_MASK, rid, j), qs = __shfl_sync(BSB_FULL_MASK, q, j);
+            const int qbeg = qs >> 16, slen = qs & 0xffff;
+            int below = __popc(__ballot_sync(BSB_FULL_MASK, p[0] <= rbeg));
+            if (n > 32) below += __popc(__ballot_sync(BSB_FULL_MASK, p[1] <= rbeg));
+            if (below) {                                // test_and_merge (bwamem.c:203-227)
+                const int e = below - 1, ci = __shfl_sync(BSB_FULL_MASK, e < 32 ? c[0] : c[1], e & 31);
+                const FastChain f = S.ch[ci];
+                const int lq = f.last_q >> 16, ll = f.last_q & 0xffff;
+                const int64_t y = rbeg - f.last_rbeg;
+                const int x = qbeg - lq;
+                bool add = true;
+                if (id != f.rid) {
+                } else if (qbeg >= f.first_qbeg && qbeg + slen <= lq + ll && rbeg >= f.pos && y + slen <= ll) {
+                    add = false;                        // contained: the seed is dropped
+                } else if ((f.last_rbeg < B.l_pac || f.pos < B.l_pac) && rbeg >= B.l_pac) {
+                } else if (y >= 0 && x - y <= opt.w && y - x <= opt.w && x - ll < opt.max_chain_gap &&
+                           y - ll < opt.max_chain_gap) {
+                    __syncwarp();
+                    if (lane == 0) {
+                        S.ch[ci].last_rbeg = rbeg, S.ch[ci].last_q = qs, S.ch[ci].n = f.n + 1;
+                        S.row[base + j] = ci << 16 | f.n;
+                    }
+                    add = false;
+                }
+                if (!add) {
+                    __syncwarp();
+                    continue;
+                }
+                if (f.pos == rbeg) return 0;
+            }
+            if (n == kFastChains) return -1;
+            if (lane == 0) {
+                FastChain f;
+                f.pos = f.last_rbeg = rbeg;
+                f.rid = id, f.first_qbeg = qbeg, f.last_q = qs, f.n = 1;
+                S.ch[n] = f;
+                S.row[base + j] = n << 16;
+            }
+            if (n >= 32) {
+                const int64_t up = __shfl_up_sync(BSB_FULL_MASK, p[1], 1), over = __shfl_sync(BSB_FULL_MASK, p[0], 31);
+                const int cu = __shfl_up_sync(BSB_FULL_MASK, c[1], 1), co = __shfl_sync(BSB_FULL_MASK, c[0], 31);
+                if (lane + 32 > below) p[1] = lane ? up : over, c[1] = lane ? cu : co;
+                else if (lane + 32 == below) p[1] = rbeg, c[1] = n;
+            }
+            if (below < 32) {
+                const int64_t up = __shfl_up_sync(BSB_FULL_MASK, p[0], 1);
+                const int cu = __shfl_up_sync(BSB_FULL_MASK, c[0], 1);
+                if (lane > below) p[0] = up, c[0] = cu;
+                else if (lane == below) p[0] = rbeg, c[0] = n;
+            }
+            ++n;
+            __syncwarp();
+        }
+    }
+    if (n == 0) return 1;
+    // where the chains' seeds start, in order of pos; the seeds
+    int acc = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const bool has = lane + 32 * h < n;
+        const int v = has ? S.ch[c[h]].n : 0;
+        int incl = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(BSB_FULL_MASK, incl, d);
+            if (lane >= d) incl += u;
+        }
+        if (has) S.start[c[h]] = acc + incl - v;
+        acc += __shfl_sync(BSB_FULL_MASK, incl, 31);
+    }
+    __syncwarp();
+    for (int k = lane; k < R; k += 32) {
+        const int t = S.row[k];
+        if (t < 0) continue;
+        DevSeed s;
+        s.rbeg = (int64_t)pos[R0 + k];
+        s.qbeg = S.row_q[k] >> 16;
+        s.len = s.score = S.row_q[k] & 0xffff;
+        s.pad = 0;
+        sd[S.start[t >> 16] + (t & 0xffff)] = s;
+    }
+    __syncwarp();
+    // mem_chain_weight (bwamem.c:229-250); mem_chain_flt (bwamem.c:331-389): light chains dropped
+    int m = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        int w = -1;
+        if (lane + 32 * h < n) {
+            const DevSeed *s = sd + S.start[c[h]];
+            const int cn = S.ch[c[h]].n;
+            int64_t qe = 0, re = 0;
+            int wq = 0, wr = 0;
+            for (int j = 0; j < cn; ++j) {
+                const DevSeed t = s[j];
+                if (t.qbeg >= qe) wq += t.len;
+                else if (t.qbeg + t.len > qe) wq += (int)(t.qbeg + t.len - qe);
+                qe = qe > t.qbeg + t.len ? qe : t.qbeg + t.len;
+                if (t.rbeg >= re) wr += t.len;
+                else if (t.rbeg + t.len > re) wr += (int)(t.rbeg + t.len - re);
+                re = re > t.rbeg + t.len ? re : t.rbeg + t.len;
+            }
+            w = wr < wq ? wr : wq;
+        }
+        const bool heavy = lane + 32 * h < n && w >= opt.min_chain_weight;
+        const unsigned hm = __ballot_sync(BSB_FULL_MASK, heavy);
+        if (heavy) {
+            const int at = m + __popc(hm & ((1u << lane) - 1u));
+            S.order[at] = c[h], S.weight[at] = w;
+        }
+        m += __popc(hm);
+    }
+    n = m;
+    if (n == 0) return 1;
+    __syncwarp();
+    if (n > 1) sort_places(S.order, S.weight, n, lane);
+    // the kept chains one after the other (each the first that none before it dropped), all chains
+    // behind it at once
+    int b[2], e[2], w[2], mark[2] = {0, 0}, first[2] = {-1, -1};      // mark: 1 overlaps a kept chain, 2 is a first
+    bool alive[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int k = lane + 32 * h;
+        alive[h] = k < n;
+        c[h] = k < n ? S.order[k] : 0, w[h] = k < n ? S.weight[k] : 0;
+        b[h] = S.ch[c[h]].first_qbeg;
+        const int lq = S.ch[c[h]].last_q;
+        e[h] = (lq >> 16) + (lq & 0xffff);
+    }
+    for (int j = 0; j < n;) {
+        const int jl = j & 31, bj = __shfl_sync(BSB_FULL_MASK, j < 32 ? b[0] : b[1], jl);
+        const int ej = __shfl_sync(BSB_FULL_MASK, j < 32 ? e[0] : e[1], jl);
+        const int wj = __shfl_sync(BSB_FULL_MASK, j < 32 ? w[0] : w[1], jl);
+        uint64_t over = 0, live = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            bool ovl = false;
+            if (alive[h] && lane + 32 * h > j) {
+                const int b_max = bj > b[h] ? bj : b[h], e_min = ej < e[h] ? ej : e[h];
+                if (e_min > b_max) {                     // no ALT contigs: the is_alt test always passes
+                    const int li = e[h] - b[h], lj = ej - bj, min_l = li < lj ? li : lj;
+                    if (e_min - b_max >= min_l * opt.mask_level && min_l < opt.max_chain_gap) {
+                        ovl = true;
+                        mark[h] |= 1;
+                        if (w[h] < wj * opt.drop_ratio && wj - w[h] >= opt.min_seed_len << 1) alive[h] = false;
+                    }
+                }
+            }
+            over |= (uint64_t)__ballot_sync(BSB_FULL_MASK, ovl) << (32 * h);
+            live |= (uint64_t)__ballot_sync(BSB_FULL_MASK, alive[h]) << (32 * h);
+        }
+        const int f = __ffsll((long long)over) - 1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (lane + 32 * h == j) first[h] = f;
+            if (lane + 32 * h == f) mark[h] |= 2;
+        }
+        const uint64_t rest = j == 63 ? 0ull : live & (~0ull << (j + 1));
+        j = rest ? __ffsll((long long)rest) - 1 : n;
+    }
+    int kept[2];
+    uint64_t weak = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        kept[h] = mark[h] & 2 ? 1 : !alive[h] ? 0 : mark[h] & 1 ? 2 : 3;
+        weak |= (uint64_t)__ballot_sync(BSB_FULL_MASK, kept[h] == 1 || kept[h] == 2) << (32 * h);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int k = lane + 32 * h;
+        // from the max_chain_extend-th of these on, only the strongest stay
+        if (kept[h] < 3 && __popcll(weak & (~0ull >> (63 - k))) >= opt.max_chain_extend) kept[h] = 0;
+        const unsigned km = __ballot_sync(BSB_FULL_MASK, kept[h] != 0);
+        if (kept[h] != 0) {
+            DevChain d;
+            d.n = S.ch[c[h]].n, d.rid = S.ch[c[h]].rid, d.w = w[h];
+            d.kept = kept[h], d.first = first[h], d.seed_off = S.start[c[h]];
+            d.frac_rep = frac_rep, d.pad = 0;
+            oc[n_out + __popc(km & ((1u << lane) - 1u))] = d;
+        }
+        n_out += __popc(km);
+    }
+    return 1;
+}
+
+struct ChainArrays {                    // of one read; R entries each
+    int64_t *pos, *last_rbeg;           // per chain: first seed's rbeg, last seed's
+    int *rid, *first_qbeg, *last_qbeg, *last_len, *n;
+    int *row_chain, *row_at, *row_q;    // per row: its chain (-1: none), place in it, qbeg << 16 | len
+    int *order, *start, *weight;        // per chain
+};
+
+// frac_rep (bwamem.c:271-278): only seeds with more than max_occ hits count.
+__device__ __forceinline__ float repeat_share(const AlnOpt &opt, int len, const DevIntv *seeds, int ns, int lane)
+{
+    int l_rep = 0;
+    bool many = false;
+    for (int i = lane; i < ns; i += 32) many |= seeds[i].x2 > (uint64_t)opt.max_occ;
+    if (__any_sync(BSB_FULL_MASK, many)) {
+        int b = 0, e = 0;
+        for (int i = 0; i < ns; ++i) {
+            const int sb = (int)(seeds[i].info >> 32), se = (int)(uint32_t)seeds[i].info;
+            if (seeds[i].x2 <= (uint64_t)opt.max_occ) continue;
+            if (sb > e) l_rep += e - b, b = sb, e = se;
+            else e = e > se ? e : se;
+        }
+        l_rep += e - b;
+    }
+    return (float)l_rep / len;
+}
+
+// False: left to chain_kernel.  n_out: kept chains.
+__device__ __noinline__ bool chain_general(const AlnOpt &opt, const DevBns &B, float frac_rep, const DevIntv *seeds,
+                                           int ns, const int64_t *roff, int64_t R0, int R, const uint64_t *pos,
+                                           ChainArrays A, DevSeed *sd, DevChain *oc, int lane, int *n_kept_out)
+{
+    const unsigned below = (1u << lane) - 1u;
+    int n_out = 0;
+    *n_kept_out = 0;
+    // mem_chain (bwamem.c:279-305)
+    int n_chn = 0;
+    for (int base = 0; base < R; base += 32) {
+        const int k = base + lane;
+        int64_t rb = 0;
+        int qb = 0, sl = 0, rid = -1;
+        if (k < R) {
+            int lo = 0, hi = ns - 1;                     // the seed of row k: the last with roff <= R0 + k
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (roff[mid] <= R0 + k) lo = mid;
+                else hi = mid - 1;
+            }
+            const uint64_t info = seeds[lo].info;
+            qb = (int)(info >> 32), sl = (int)(uint32_t)info - qb;
+            rb = (int64_t)pos[R0 + k];
+            rid = intv2rid(B, rb, rb + sl);
+            A.row_chain[k] = -1;
+            A.row_q[k] = qb << 16 | sl;
+        }
+        __syncwarp();
+        const int rows = min(32, R - base);
+        for (int j = 0; j < rows; ++j) {
+            const int id = __shfl_sync(BSB_FULL_MASK, rid, j);
+            if (id < 0) continue;
+            const int64_t rbeg = __shfl_sync(BSB_FULL_MASK, rb, j);
+            const int qbeg = __shfl_sync(BSB_FULL_MASK, qb, j), slen = __shfl_sync(BSB_FULL_MASK, sl, j);
+            // the chain with the largest pos <= rbeg: high words first, then low words among the highest
+            int64_t bp = -1;
+            int bc = -1;
+            for (int c = lane; c < n_chn; c += 32) {
+                const int64_t p = A.pos[c];
+                if (p <= rbeg && p > bp) bp = p, bc = c;
+            }
+            const int hi = (int)(bp >> 32), mh = __reduce_max_sync(BSB_FULL_MASK, hi);
+            bool add = true;
+            if (mh >= 0) {
+                const uint32_t lw = hi == mh ? (uint32_t)bp : 0u, ml = __reduce_max_sync(BSB_FULL_MASK, lw);
+                const unsigned m = __ballot_sync(BSB_FULL_MASK, hi == mh && (uint32_t)bp == ml);
+                const int c = __shfl_sync(BSB_FULL_MASK, bc, __ffs(m) - 1);
+                // test_and_merge (bwamem.c:203-227)
+                const int64_t first_rbeg = A.pos[c], last_rbeg = A.last_rbeg[c];
+                const int lq = A.last_qbeg[c], ll = A.last_len[c];
+                const int64_t qend = lq + ll, rend = last_rbeg + ll;
+                if (id != A.rid[c]) {
+                } else if (qbeg >= A.first_qbeg[c] && qbeg + slen <= qend && rbeg >= first_rbeg && rbeg + slen <= rend) {
+                    add = false;                         // contained: the seed is dropped
+                } else if ((last_rbeg < B.l_pac || first_rbeg < B.l_pac) && rbeg >= B.l_pac) {
+                } else {
+                    const int64_t x = qbeg - lq, y = rbeg - last_rbeg;
+                    if (y >= 0 && x - y <= opt.w && y - x <= opt.w && x - ll < opt.max_chain_gap &&
+                        y - ll < opt.max_chain_gap) {
+                        const int at = A.n[c];
+                        __syncwarp();
+                        if (lane == 0) {
+                            A.last_qbeg[c] = qbeg, A.last_rbeg[c] = rbeg, A.last_len[c] = slen;
+                            A.n[c] = at + 1;
+                            A.row_chain[base + j] = c, A.row_at[base + j] = at;
+                        }
+                        add = false;
+                    }
+                }
+                if (add && first_rbeg == rbeg) return false;
+            }
+            if (add) {
+                if (lane == 0) {
+                    A.pos[n_chn] = A.last_rbeg[n_chn] = rbeg;
+                    A.first_qbeg[n_chn] = A.last_qbeg[n_chn] = qbeg, A.last_len[n_chn] = slen;
+                    A.n[n_chn] = 1, A.rid[n_chn] = id;
+                    A.row_chain[base + j] = n_chn, A.row_at[base + j] = 0;
+                }
+                ++n_chn;
+            }
+            __syncwarp();
+        }
+    }
+    if (n_chn == 0) return true;
+    // the chains in order of pos, and where their seeds start
+    for (int c = lane; c < n_chn; c += 32) {
+        const int64_t p = A.pos[c];
+        int rank = 0;
+        for (int d = 0; d < n_chn; ++d) rank += A.pos[d] < p;
+        A.order[rank] = c;
+    }
+    for (int base = 0, acc = 0; base < n_chn; base += 32) {
+        const int c = base + lane, v = c < n_chn ? A.n[c] : 0;
+        int incl = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(BSB_FULL_MASK, incl, d);
+            if (lane >= d) incl += u;
+        }
+        if (c < n_chn) A.start[c] = acc + incl - v;
+        acc += __shfl_sync(BSB_FULL_MASK, incl, 31);
+    }
+    __syncwarp();
+    for (int k = lane; k < R; k += 32) {
+        const int c = A.row_chain[k];
+        if (c < 0) continue;
+        DevSeed s;
+        s.rbeg = (int64_t)pos[R0 + k];
+        s.qbeg = A.row_q[k] >> 16;
+        s.len = s.score = A.row_q[k] & 0xffff;
+        s.pad = 0;
+        sd[A.start[c] + A.row_at[k]] = s;
+    }
+    __syncwarp();
+    // mem_chain_weight (bwamem.c:229-250)
+    for (int c = lane; c < n_chn; c += 32) {
+        const DevSeed *s = sd + A.start[c];
+        const int n = A.n[c];
+        int64_t qe = 0, re = 0;
+        int wq = 0, wr = 0;
+        for (int j = 0; j < n; ++j) {
+            const DevSeed t = s[j];
+            if (t.qbeg >= qe) wq += t.len;
+            else if (t.qbeg + t.len > qe) wq += (int)(t.qbeg + t.len - qe);
+            qe = qe > t.qbeg + t.len ? qe : t.qbeg + t.len;
+            if (t.rbeg >= re) wr += t.len;
+            else if (t.rbeg + t.len > re) wr += (int)(t.rbeg + t.len - re);
+            re = re > t.rbeg + t.len ? re : t.rbeg + t.len;
+        }
+        const int w = wr < wq ? wr : wq;
+        A.weight[c] = w < (1 << 30) ? w : (1 << 30) - 1;
+    }
+    __syncwarp();
+    // mem_chain_flt (bwamem.c:331-389): drop light chains, sort by weight, mark kept
+    int n = 0;
+    for (int base = 0; base < n_chn; base += 32) {
+        const int k = base + lane, c = k < n_chn ? A.order[k] : 0;
+        const bool heavy = k < n_chn && A.weight[c] >= opt.min_chain_weight;
+        const unsigned m = __ballot_sync(BSB_FULL_MASK, heavy);
+        if (heavy) A.order[n + __popc(m & below)] = c;
+        n += __popc(m);
+        __syncwarp();
+    }
+    if (n == 0) return true;
+    if (n > 1) {
+        // by weight, descending: ranks where the weights differ, ks_introsort's steps where some
+        // are equal.  (row_at and row_chain are free from here on.)
+        bool equal = false;
+        for (int k = lane; k < n; k += 32) {
+            const int c = A.order[k], w = A.weight[c];
+            int rank = 0;
+            for (int d = 0; d < n; ++d) {
+                const int u = A.weight[A.order[d]];
+                rank += u > w;
+                equal |= u == w && d != k;
+            }
+            A.row_at[rank] = c;
+        }
+        equal = __any_sync(BSB_FULL_MASK, equal);
+        __syncwarp();
+        if (!equal) {
+            for (int k = lane; k < n; k += 32) A.order[k] = A.row_at[k];
+        } else if (lane == 0) {
+            int stk_l[64], stk_r[64], stk_d[64];
+            KsSort<FltLt> fs{A.order, FltLt{A.weight}};
+            fs.sort(n, stk_l, stk_r, stk_d);
+        }
+        __syncwarp();
+    }
+    int *const kept = A.row_chain, *const first = A.row_at, *const list = A.row_q;
+    for (int k = lane; k < n; k += 32) kept[k] = 0, first[k] = -1;
+    __syncwarp();
+    if (lane == 0) kept[0] = 3, list[0] = 0;
+    __syncwarp();
+    int n_kept = 1;
+    for (int i = 1; i < n; ++i) {
+        const int ci = A.order[i], wi = A.weight[ci];
+        const int bi = A.first_qbeg[ci], ei = A.last_qbeg[ci] + A.last_len[ci];
+        bool large = false, drop = false;
+        for (int base = 0; base < n_kept && !drop; base += 32) {
+            bool ovl = false, end = false;
+            int j = 0;
+            if (base + lane < n_kept) {
+                j = list[base + lane];
+                const int cj = A.order[j], wj = A.weight[cj];
+                const int bj = A.first_qbeg[cj], ej = A.last_qbeg[cj] + A.last_len[cj];
+                const int b_max = bj > bi ? bj : bi, e_min = ej < ei ? ej : ei;
+                if (e_min > b_max) {                     // no ALT contigs: the is_alt test always passes
+                    const int li = ei - bi, lj = ej - bj, min_l = li < lj ? li : lj;
+                    if (e_min - b_max >= min_l * opt.mask_level && min_l < opt.max_chain_gap) {
+                        ovl = true;
+                        end = wi < wj * opt.drop_ratio && wj - wi >= opt.min_seed_len << 1;
+                    }
+                }
+            }
+            // the reference stops at the first chain that drops this one: those after it see nothing
+            const unsigned me = __ballot_sync(BSB_FULL_MASK, end);
+            const unsigned seen = me ? (2u << (__ffs(me) - 1)) - 1u : 0xffffffffu;
+            ovl = ovl && (seen >> lane & 1u);
+            if (ovl && first[j] < 0) first[j] = i;
+            large |= __any_sync(BSB_FULL_MASK, ovl);
+            drop = me != 0;
+        }
+        if (!drop) {
+            if (lane == 0) list[n_kept] = i, kept[i] = large ? 2 : 3;
+            ++n_kept;
+        }
+        __syncwarp();
+    }
+    for (int k = lane; k < n_kept; k += 32) {
+        const int f = first[list[k]];
+        if (f >= 0) kept[f] = 1;
+    }
+    __syncwarp();
+    if (n >= opt.max_chain_extend) {
+        if (lane == 0) {
+            int i, k = 0;
+            for (i = 0; i < n; ++i) {
+                if (kept[i] == 0 || kept[i] == 3) continue;
+                if (++k >= opt.max_chain_extend) break;
+            }
+            for (; i < n; ++i)
+                if (kept[i] < 3) kept[i] = 0;
+        }
+        __syncwarp();
+    }
+    for (int base = 0; base < n; base += 32) {
+        const int i = base + lane;
+        const bool keep = i < n && kept[i] != 0;
+        const unsigned m = __ballot_sync(BSB_FULL_MASK, keep);
+        if (keep) {
+            const int c = A.order[i];
+            DevChain d;
+            d.n = A.n[c], d.rid = A.rid[c], d.w = A.weight[c];
+            d.kept = kept[i], d.first = first[i], d.seed_off = A.start[c];
+            d.frac_rep = frac_rep, d.pad = 0;
+            oc[n_out + __popc(m & below)] = d;
+        }
+        n_out += __popc(m);
+    }
+    *n_kept_out = n_out;
+    return true;
+}
+
+__global__ void __launch_bounds__(kChainWarps * 32, 10)
+chain_warp_kernel(AlnOpt opt, DevBns B, int n_reads, const int64_t *__restrict__ read_off,
+                  const DevIntv *__restrict__ seeds, const int64_t *__restrict__ seed_off,
+                  const int64_t *__restrict__ row_off_of_seed, const uint64_t *__restrict__ pos,
+                  ChainRec *__restrict__ chains, BtNode *__restrict__ nodes, int *__restrict__ row_chain,
+                  int *__restrict__ iwork, DevSeed *__restrict__ out_seeds, DevChain *__restrict__ out_chains,
+                  int *__restrict__ n_chains, int *__restrict__ left, int *__restrict__ n_left)
+{
+    __shared__ ChainSmem sm[kChainWarps];
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const int r = blockIdx.x * kChainWarps + wb;
+    if (r >= n_reads) return;
+    const int len = (int)(read_off[r + 1] - read_off[r]);
+    const int64_t s0 = seed_off[r], s1 = seed_off[r + 1];
+    const int64_t R0 = row_off_of_seed[s0];
+    const int R = (int)(row_off_of_seed[s1] - R0);
+    int n_out = 0;
+    bool done = true;
+    if (len >= opt.min_seed_len && R > 0) {
+        DevSeed *const sd = out_seeds + R0;
+        DevChain *const oc = out_chains + R0;
+        const int ns = (int)(s1 - s0);
+        const float frac_rep = repeat_share(opt, len, seeds + s0, ns, lane);
+        int how = -1;
+        if (R <= kFastRows)
+            how = chain_fast(opt, B, frac_rep, seeds + s0, ns, row_off_of_seed + s0, R0, R, pos, sm[wb], sd, oc, lane, n_out);
+        done = how != 0;
+        if (how < 0) {
+            static_assert(sizeof(ChainRec) >= 2 * 8 + 5 * 4 && sizeof(BtNode) >= 2 * 4, "the read's scratch slices");
+            ChainArrays A;
+            A.pos = (int64_t *)(chains + R0), A.last_rbeg = A.pos + R;
+            int *const ai = (int *)(A.last_rbeg + R);
+            A.rid = ai, A.first_qbeg = ai + R, A.last_qbeg = ai + 2 * (int64_t)R, A.last_len = ai + 3 * (int64_t)R;
+            A.n = ai + 4 * (int64_t)R;
+            A.row_chain = row_chain + R0;
+            A.row_at = (int *)(nodes + R0), A.row_q = A.row_at + R;
+            A.order = iwork + R0 * 3, A.start = A.order + R, A.weight = A.order + 2 * (int64_t)R;
+            __syncwarp();
+            done = chain_general(opt, B, frac_rep, seeds + s0, ns, row_off_of_seed + s0, R0, R, pos, A, sd, oc, lane, &n_out);
+        }
+    }
+    if (lane == 0) {
+        n_chains[r] = n_out;
+        if (!done) left[atomicAdd(n_left, 1)] = r;
     }
 }
 
@@ -1445,8 +2130,12 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     for (int i = 0; i < 25; ++i) mx = mx > o->mat[i] ? mx : o->mat[i];
     P.mat_max = mx;
     P.pack16 = 0;
-    chain_kernel<<<ctx->n_sm * 8, 128, 0, st>>>(ao, B, n_reads, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff,
-                                                 pos, chains, nodes, row_chain, iwork, cseeds, cchains, n_chains, ctrl);
+    int *const left = (int *)(A + o_order);                  // reads for chain_kernel (the read order comes after)
+    chain_warp_kernel<<<(n_reads + kChainWarps - 1) / kChainWarps, kChainWarps * 32, 0, st>>>(
+        ao, B, n_reads, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos, chains, nodes, row_chain, iwork,
+        cseeds, cchains, n_chains, left, ctrl);
+    chain_kernel<<<ctx->n_sm, 128, 0, st>>>(ao, B, left, ctrl, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos,
+                                            chains, nodes, row_chain, iwork, cseeds, cchains, n_chains);
     if (h_min_hsp &&
         (rc = seed_sw_filter(ctx, o, B, n_reads, h_min_hsp, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
                              n_chains, ao)))
