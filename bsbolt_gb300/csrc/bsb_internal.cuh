@@ -90,6 +90,9 @@ struct bsb_ctx {
     // batch's own reads and seeds occupy d_in / d_out meanwhile)
     void *flt_in = nullptr, *flt_out = nullptr, *flt_dev = nullptr;
     size_t flt_in_bytes = 0, flt_out_bytes = 0, flt_dev_bytes = 0;
+    // the chains' first extensions of an alignment batch: jobs, bytes, results, scheduler scratch
+    void *pre_buf = nullptr;
+    size_t pre_bytes = 0;
     // learned read order of the alignment batches: the cost model (caller's device memory,
     // or NULL for the chain-count order), and the per-read features and extension cells of
     // the last batch when logging
@@ -124,7 +127,23 @@ struct KswParams {
     int o_del, e_del, o_ins, e_ins, zdrop;
     int mat_max;
     int pack16;        // set by ksw_launch: the penalties allow 16-bit cells
+    // Jobs of an alignment batch read the reference itself (pac: 2-bit forward text of l_pac bases;
+    // NULL: jobs of a byte buffer), on 16-bit cells and a built-in map only.  Their qoff is the place of query base 0 in the buffer, toff the
+    // place of target base 0 in the forward-reverse text; both run backwards with kExtBack in flags, and
+    // kExtNone marks a job that is passed over.
+    const uint8_t *pac = nullptr;
+    int64_t l_pac = 0;
 };
+constexpr int kExtNone = 1, kExtBack = 2;
+
+// Base at position p of the forward-reverse text (bns_get_seq, bntseq.c:414-434).
+__device__ __forceinline__ int packed_text_base(const uint8_t *pac, int64_t l_pac, int64_t p)
+{
+    const bool rev = p >= l_pac;
+    if (rev) p = (l_pac << 1) - 1 - p;
+    const int b = __ldg(pac + (p >> 2)) >> ((~p & 3) << 1) & 3;
+    return rev ? 3 - b : b;
+}
 
 // Launches the extension of n jobs (device buffers) on stream, scheduled by
 // tile bin and cost key (d_cost, or the plain bound when NULL).
@@ -143,7 +162,11 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
                        const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
                        cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev = nullptr,
-                       const KswStreams *ms = nullptr);
+                       const KswStreams *ms = nullptr, bool all_narrow = false);
+// all_narrow: the caller knows that no job's h0 + qlen * max(mat) exceeds this, so that no job needs
+// 32-bit cells where the scoring allows 16-bit ones.
+int ksw_pack16_max();
+bool ksw_pack16(const KswParams &P);      // the penalties and scores allow 16-bit cells
 int64_t ksw_concurrent_below();
 // The built-in tile map (host copy, BSB_TILE_MAP_LEN entries); the number of the built-in map a
 // batch of n jobs runs on where the caller has set none, and that map.

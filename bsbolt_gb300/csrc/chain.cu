@@ -1282,6 +1282,133 @@ __device__ KswResult extend_any(const KswParams &P, const int8_t *tab, int qlen,
     }
 }
 
+// The target span of a chain's extensions: the widest that any seed can use (bwamem.c:646-661),
+// clipped to the contig of the first seed as bns_fetch_seq does (bntseq.c:436-461).
+__device__ __forceinline__ void chain_window(const AlnOpt &opt, const DevBns &B, int l_query, const DevSeed *cs, int n,
+                                             int64_t &rmax0, int64_t &rmax1)
+{
+    const int64_t l_pac = B.l_pac;
+    rmax0 = l_pac << 1, rmax1 = 0;
+    for (int i = 0; i < n; ++i) {
+        const DevSeed t = cs[i];
+        const int64_t b = t.rbeg - (t.qbeg + cal_max_gap(opt, t.qbeg));
+        const int64_t e = t.rbeg + t.len + ((l_query - t.qbeg - t.len) + cal_max_gap(opt, l_query - t.qbeg - t.len));
+        rmax0 = rmax0 < b ? rmax0 : b;
+        rmax1 = rmax1 > e ? rmax1 : e;
+    }
+    rmax0 = rmax0 > 0 ? rmax0 : 0;
+    rmax1 = rmax1 < l_pac << 1 ? rmax1 : l_pac << 1;
+    if (rmax0 < l_pac && l_pac < rmax1) {
+        if (cs[0].rbeg < l_pac) rmax1 = l_pac;
+        else rmax0 = l_pac;
+    }
+    int is_rev;
+    const int rid = pos2rid(B, depos(B, cs[0].rbeg, is_rev));
+    int64_t far_beg = B.ann_offset[rid], far_end = far_beg + B.ann_len[rid];
+    if (is_rev) {
+        const int64_t t = far_beg;
+        far_beg = (l_pac << 1) - far_end;
+        far_end = (l_pac << 1) - t;
+    }
+    rmax0 = rmax0 > far_beg ? rmax0 : far_beg;
+    rmax1 = rmax1 < far_end ? rmax1 : far_end;
+}
+
+// ---------------------------------------------------------------- the chains' first extensions, batched
+
+// mem_chain2aln takes a chain's seeds from the highest score down, and most chains are one seed, or
+// one whose region then covers the others.  So the extensions of every chain's first seed are nearly
+// all there are, and they need nothing of the read's other chains: they run as two batches of the
+// job-parallel extension (ksw_extend.cu: the main diagonal first, then 4 to 32 lanes a job on 16-bit
+// cells), left ends and then right ends, whose h0 is the left ends' score.  chain2aln_kernel takes the
+// results where it comes to such a seed; what it passes over (a seed inside an earlier region) was
+// extended for nothing.  A warp per extension of a few dozen rows took 8,100 warp instructions a
+// region.  One GB300, everything from the read order to the regions: 114k RRBS reads (450k regions)
+// 4.62 -> 1.98 ms, of which chain2aln_kernel 0.60; 67k reads of 150 bases 2.21 -> 1.18; 40k of 100 on
+// 2 Mb 0.46 -> 0.42.  (With the jobs' bytes written out first, RRBS 2.54.)
+struct PreChain {
+    int64_t rmax0, rmax1;
+    int seed, pad;                      // the first seed to extend
+};
+struct PreResults {                     // chains: NULL where there are none
+    const PreChain *chains;
+    const int64_t *off;                 // per read, its first chain's place
+    const bsb_ext_out_t *left, *right;  // score < 0: not run
+};
+
+// One thread per kept chain: its window, its first seed and the two jobs, on the reads and the 2-bit
+// reference as they lie.  Rows from qlen + w + 1 on are never reached (the band is then right of the
+// query), so targets end there.
+__global__ void pre_plan_kernel(AlnOpt opt, DevBns B, int64_t n_chains, int n_reads,
+                                const int64_t *__restrict__ chain_off, const int64_t *__restrict__ read_off,
+                                const int64_t *__restrict__ seed_off, const int64_t *__restrict__ row_off_of_seed,
+                                const DevSeed *__restrict__ seeds, const DevChain *__restrict__ chains,
+                                PreChain *__restrict__ pre, bsb_ext_job_t *__restrict__ left,
+                                bsb_ext_job_t *__restrict__ right)
+{
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n_chains) return;
+    int lo = 0, hi = n_reads - 1;                     // the chain's read: the last with chain_off <= t
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (chain_off[mid] <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    const int64_t R0 = row_off_of_seed[seed_off[lo]];
+    const int l_query = (int)(read_off[lo + 1] - read_off[lo]);
+    const DevChain c = chains[R0 + (t - chain_off[lo])];
+    const DevSeed *cs = seeds + R0 + c.seed_off;
+    PreChain p;
+    bsb_ext_job_t L, R;
+    memset(&p, 0, sizeof p);
+    memset(&L, 0, sizeof L);
+    L.flags = kExtNone;
+    R = L;
+    if (c.n > 0) {
+        chain_window(opt, B, l_query, cs, c.n, p.rmax0, p.rmax1);
+        for (int i = 1; i < c.n; ++i)
+            if (cs[i].score >= cs[p.seed].score) p.seed = i;
+        const DevSeed s = cs[p.seed];
+        const int qe = s.qbeg + s.len;
+        L.qlen = s.qbeg, R.qlen = l_query - qe;
+        L.tlen = (int)min(s.rbeg - p.rmax0, (int64_t)L.qlen + opt.w + 1);
+        R.tlen = (int)min(p.rmax1 - (s.rbeg + s.len), (int64_t)R.qlen + opt.w + 1);
+        L.qoff = read_off[lo] + s.qbeg - 1, L.toff = s.rbeg - 1;
+        R.qoff = read_off[lo] + qe, R.toff = s.rbeg + s.len;
+        L.h0 = R.h0 = s.len * opt.a;
+        L.w = R.w = opt.w;
+        L.end_bonus = opt.pen_clip5, R.end_bonus = opt.pen_clip3;
+        L.flags = L.qlen < 1 ? kExtNone : kExtBack, R.flags = R.qlen < 1 ? kExtNone : 0;
+    }
+    pre[t] = p;
+    left[t] = L;
+    right[t] = R;
+}
+
+// A result that mem_chain2aln would take without trying a wider band (bwamem.c:727,756).
+__device__ __forceinline__ bool pre_usable(const AlnOpt &opt, const bsb_ext_out_t &x)
+{
+    return x.score >= 0 && x.max_off < (opt.w >> 1) + (opt.w >> 2);
+}
+
+__device__ __forceinline__ bool pre_result(const AlnOpt &opt, const bsb_ext_out_t &o, KswResult &x)
+{
+    x.score = o.score, x.qle = o.qle, x.tle = o.tle, x.gtle = o.gtle, x.gscore = o.gscore, x.max_off = o.max_off;
+    x.cells = 0;
+    return pre_usable(opt, o);
+}
+
+// The right ends' h0, or no job where the left end is not decided.
+__global__ void pre_right_kernel(AlnOpt opt, int64_t n_chains, const bsb_ext_job_t *__restrict__ left,
+                                 const bsb_ext_out_t *__restrict__ left_out, bsb_ext_job_t *__restrict__ right)
+{
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n_chains || (left[t].flags & kExtNone)) return;       // no left end: h0 as planned
+    const bsb_ext_out_t x = left_out[t];
+    if (pre_usable(opt, x)) right[t].h0 = x.score;
+    else right[t].flags |= kExtNone;
+}
+
 // One warp per read.  regs: the read's region slots start at its row offset.
 // MaxC = 4, 5, 8 serve batches whose reads are at most 127, 159, 255 bases long (one DP
 // copy of that width), 16 every read the batch accepts; the 4- and 5-column variants are
@@ -1293,7 +1420,7 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                  const int64_t *__restrict__ row_off_of_seed, const DevSeed *__restrict__ seeds,
                  const DevChain *__restrict__ chains, const int *__restrict__ n_chains, uint64_t *__restrict__ srt_buf,
                  bsb_reg_t *__restrict__ regs, int *__restrict__ n_regs, int *__restrict__ next,
-                 const int *__restrict__ order, int64_t *__restrict__ read_cells)
+                 const int *__restrict__ order, int64_t *__restrict__ read_cells, PreResults pre)
 {
     __shared__ int8_t tab[kScoreTable];
     load_score_table(P, tab);
@@ -1320,33 +1447,9 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
             const DevChain c = chn[ci];
             const DevSeed *cs = sd + c.seed_off;
             if (c.n == 0) continue;
-            // the widest target span any seed can use (bwamem.c:646-661)
-            int64_t rmax0 = l_pac << 1, rmax1 = 0;
-            for (int i = 0; i < c.n; ++i) {
-                const DevSeed t = cs[i];
-                const int64_t b = t.rbeg - (t.qbeg + cal_max_gap(opt, t.qbeg));
-                const int64_t e = t.rbeg + t.len + ((l_query - t.qbeg - t.len) + cal_max_gap(opt, l_query - t.qbeg - t.len));
-                rmax0 = rmax0 < b ? rmax0 : b;
-                rmax1 = rmax1 > e ? rmax1 : e;
-            }
-            rmax0 = rmax0 > 0 ? rmax0 : 0;
-            rmax1 = rmax1 < l_pac << 1 ? rmax1 : l_pac << 1;
-            if (rmax0 < l_pac && l_pac < rmax1) {
-                if (cs[0].rbeg < l_pac) rmax1 = l_pac;
-                else rmax0 = l_pac;
-            }
-            {   // bns_fetch_seq's clip to the contig of the first seed (bntseq.c:436-461)
-                int is_rev;
-                const int rid = pos2rid(B, depos(B, cs[0].rbeg, is_rev));
-                int64_t far_beg = B.ann_offset[rid], far_end = far_beg + B.ann_len[rid];
-                if (is_rev) {
-                    const int64_t t = far_beg;
-                    far_beg = (l_pac << 1) - far_end;
-                    far_end = (l_pac << 1) - t;
-                }
-                rmax0 = rmax0 > far_beg ? rmax0 : far_beg;
-                rmax1 = rmax1 < far_end ? rmax1 : far_end;
-            }
+            int64_t rmax0, rmax1;
+            if (pre.chains) rmax0 = pre.chains[pre.off[r] + ci].rmax0, rmax1 = pre.chains[pre.off[r] + ci].rmax1;
+            else chain_window(opt, B, l_query, cs, c.n, rmax0, rmax1);
             // seeds by (score, index) ascending; keys are distinct, so ranks give ks_introsort_64's order
             for (int i = lane; i < c.n; i += 32) {
                 const uint64_t ki = (uint64_t)(uint32_t)cs[i].score << 32 | (uint32_t)i;
@@ -1416,11 +1519,14 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                 a.w = opt.w;
                 a.score = a.truesc = -1;
                 a.rid = c.rid;
+                const bool first_seed = pre.chains && k == c.n - 1;
                 if (s.qbeg) {      // left extension (bwamem.c:715-748)
                     ReadRefAcc acc{query, s.qbeg - 1, -1, s.rbeg - 1, -1, B};
                     const int tlen = (int)(s.rbeg - rmax0);
                     KswResult x;
-                    for (int i = 0; i < 2; ++i) {
+                    const bool known = first_seed && pre_result(opt, pre.left[pre.off[r] + ci], x);
+                    if (known) a.score = x.score;
+                    for (int i = 0; i < 2 && !known; ++i) {
                         const int prev = a.score;
                         aw0 = opt.w << i;
                         x = extend_any<MaxC>(P, tab, s.qbeg, tlen, s.len * opt.a, aw0, opt.pen_clip5, acc, lane,
@@ -1443,7 +1549,10 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                     ReadRefAcc acc{query, qe, 1, rmax0 + re, 1, B};
                     const int tlen = (int)(rmax1 - rmax0 - re);
                     KswResult x;
-                    for (int i = 0; i < 2; ++i) {
+                    // (the right end's job started from the left end's score where that was known)
+                    const bool known = first_seed && pre_result(opt, pre.right[pre.off[r] + ci], x);
+                    if (known) a.score = x.score;
+                    for (int i = 0; i < 2 && !known; ++i) {
                         const int prev = a.score;
                         aw1 = opt.w << i;
                         x = extend_any<MaxC>(P, tab, l_query - qe, tlen, sc0, aw1, opt.pen_clip3, acc, lane,
@@ -1677,51 +1786,69 @@ __device__ __forceinline__ int key_bin(int32_t key)
     const int half = 2 * msb + (msb > 0 ? (int)(k >> (msb - 1) & 1u) : 0);
     return 63 - (half < 63 ? half : 63);
 }
-__global__ void order_hist_key(const int32_t *__restrict__ key, int n_reads, int *__restrict__ cnt)
+// Counting sort into 64 bins in two kernels: the bins' sizes, then the places.  A block counts in shared
+// memory and touches each global counter once (one global atomic per read on a few busy counters took
+// 84 us for 67k reads, the two kernels together).
+constexpr int kOrderBins = 64, kOrderThreads = 256;
+template <class Bin>
+__device__ __forceinline__ void order_count(int n_reads, int *__restrict__ cnt, Bin bin)
 {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_reads; r += gridDim.x * blockDim.x)
-        atomicAdd(&cnt[key_bin(key[r])], 1);
-}
-__global__ void order_scatter_key(const int32_t *__restrict__ key, int n_reads, const int *__restrict__ cnt,
-                                  int *__restrict__ cur, int *__restrict__ order)
-{
-    __shared__ int off[64];
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int b = 0; b < 64; ++b) off[b] = acc, acc += cnt[b];
-    }
+    __shared__ int sh[kOrderBins];
+    if (threadIdx.x < kOrderBins) sh[threadIdx.x] = 0;
     __syncthreads();
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_reads; r += gridDim.x * blockDim.x) {
-        const int b = key_bin(key[r]);
-        order[off[b] + atomicAdd(&cur[b], 1)] = r;
-    }
+    for (int r = blockIdx.x * kOrderThreads + threadIdx.x; r < n_reads; r += gridDim.x * kOrderThreads)
+        atomicAdd(&sh[bin(r)], 1);
+    __syncthreads();
+    if (threadIdx.x < kOrderBins && sh[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], sh[threadIdx.x]);
 }
-
-// The order chain2aln_kernel takes reads in: most chains first (reads are independent, so the
-// order changes no result; it shortens the tail a few repeat-laden reads would otherwise set).
-constexpr int kOrderBins = 64;
-
-__device__ __forceinline__ int order_bin(int nc) { return kOrderBins - 1 - (nc < kOrderBins - 1 ? nc : kOrderBins - 1); }
-
-__global__ void order_hist(const int *__restrict__ n_chains, int n_reads, int *__restrict__ cnt)
+template <class Bin>
+__device__ __forceinline__ void order_place(int n_reads, const int *__restrict__ cnt, int *__restrict__ cur,
+                                            int *__restrict__ order, Bin bin)
 {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_reads; r += gridDim.x * blockDim.x)
-        atomicAdd(&cnt[order_bin(n_chains[r])], 1);
-}
-
-__global__ void order_scatter(const int *__restrict__ n_chains, int n_reads, const int *__restrict__ cnt,
-                              int *__restrict__ cur, int *__restrict__ order)
-{
-    __shared__ int off[kOrderBins];
+    __shared__ int off[kOrderBins], sh[kOrderBins];
     if (threadIdx.x == 0) {
         int acc = 0;
         for (int b = 0; b < kOrderBins; ++b) off[b] = acc, acc += cnt[b];
     }
-    __syncthreads();
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_reads; r += gridDim.x * blockDim.x) {
-        const int b = order_bin(n_chains[r]);
-        order[off[b] + atomicAdd(&cur[b], 1)] = r;
+    for (int base = blockIdx.x * kOrderThreads; base < n_reads; base += gridDim.x * kOrderThreads) {
+        if (threadIdx.x < kOrderBins) sh[threadIdx.x] = 0;
+        __syncthreads();
+        const int r = base + threadIdx.x, b = r < n_reads ? bin(r) : -1;
+        const int at = b < 0 ? 0 : atomicAdd(&sh[b], 1);
+        __syncthreads();
+        if (threadIdx.x < kOrderBins && sh[threadIdx.x])
+            sh[threadIdx.x] = off[threadIdx.x] + atomicAdd(&cur[threadIdx.x], sh[threadIdx.x]);
+        __syncthreads();
+        if (b >= 0) order[sh[b] + at] = r;
+        __syncthreads();
     }
+}
+__global__ void __launch_bounds__(kOrderThreads)
+order_hist_key(const int32_t *__restrict__ key, int n_reads, int *__restrict__ cnt)
+{
+    order_count(n_reads, cnt, [=](int r) { return key_bin(key[r]); });
+}
+__global__ void __launch_bounds__(kOrderThreads)
+order_scatter_key(const int32_t *__restrict__ key, int n_reads, const int *__restrict__ cnt, int *__restrict__ cur,
+                  int *__restrict__ order)
+{
+    order_place(n_reads, cnt, cur, order, [=](int r) { return key_bin(key[r]); });
+}
+
+// The order chain2aln_kernel takes reads in: most chains first (reads are independent, so the
+// order changes no result; it shortens the tail a few repeat-laden reads would otherwise set).
+__device__ __forceinline__ int order_bin(int nc) { return kOrderBins - 1 - (nc < kOrderBins - 1 ? nc : kOrderBins - 1); }
+
+__global__ void __launch_bounds__(kOrderThreads)
+order_hist(const int *__restrict__ n_chains, int n_reads, int *__restrict__ cnt)
+{
+    order_count(n_reads, cnt, [=](int r) { return order_bin(n_chains[r]); });
+}
+__global__ void __launch_bounds__(kOrderThreads)
+order_scatter(const int *__restrict__ n_chains, int n_reads, const int *__restrict__ cnt, int *__restrict__ cur,
+              int *__restrict__ order)
+{
+    order_place(n_reads, cnt, cur, order, [=](int r) { return order_bin(n_chains[r]); });
 }
 
 // One warp per read (reads hold a few regions each).
@@ -2047,6 +2174,62 @@ static int seed_sw_filter(bsb_ctx *ctx, const bsb_align_opt_t *o, const DevBns &
     return bsb_cuda(ctx, cudaStreamSynchronize(st), "seed SW filter");
 }
 
+// Batches of fewer reads run their extensions inside chain2aln_kernel: it then has warps to spare,
+// and the batches' some 20 launches would take longer.
+constexpr int kPreReads = 4096;
+
+// The extensions of every chain's first seed as two batches (pre_plan_kernel); chain_off receives the
+// offsets of the reads' chains.  Leaves pre empty where the scoring or the reads' length need 32-bit
+// cells.
+static int first_extensions(bsb_ctx *ctx, const bsb_align_opt_t *o, const AlnOpt &ao, const DevBns &B,
+                            const KswParams &P, int n_reads, int max_len, const uint8_t *d_reads,
+                            const int64_t *d_read_off, const int64_t *d_seed_off, const int64_t *roff,
+                            const DevSeed *cseeds, const DevChain *cchains, const int *n_chains, int64_t *chain_off,
+                            int64_t *scan_tmp, PreResults *pre)
+{
+    cudaStream_t st = ctx->stream;
+    int rc;
+    for (int k = 0; k < 25; ++k)
+        if (o->mat[k] > 63 || o->mat[k] < -63) return 0;
+    if (!ksw_pack16(P) || o->w > 4096 || (int64_t)max_len * (o->a + P.mat_max) > ksw_pack16_max()) return 0;
+    int64_t T = 0;
+    if ((rc = bsb_cuda(ctx, scan_i32_i64(n_chains, n_reads, chain_off, scan_tmp, st), "chain offsets")) ||
+        (rc = bsb_cuda(ctx, cudaMemcpyAsync(&T, chain_off + n_reads, 8, cudaMemcpyDeviceToHost, st), "chain total")) ||
+        (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "chain total")))
+        return rc;
+    if (T == 0 || T > 0x7fffffff) return 0;
+    size_t off = 0;
+    const size_t o_pre = off; off += al(sizeof(PreChain) * T);
+    const size_t o_left = off; off += al(sizeof(bsb_ext_job_t) * T);
+    const size_t o_right = off; off += al(sizeof(bsb_ext_job_t) * T);
+    const size_t o_out = off; off += al(sizeof(bsb_ext_out_t) * 2 * T);
+    const size_t o_scr = off; off += al(ksw_scratch_bytes(T));
+    if ((rc = bsb_ensure(ctx, &ctx->pre_buf, &ctx->pre_bytes, off, "chain extensions"))) return rc;
+    char *const D = (char *)ctx->pre_buf;
+    PreChain *const pc = (PreChain *)(D + o_pre);
+    bsb_ext_job_t *const left = (bsb_ext_job_t *)(D + o_left), *const right = (bsb_ext_job_t *)(D + o_right);
+    bsb_ext_out_t *const out = (bsb_ext_out_t *)(D + o_out);
+    const unsigned tb = (unsigned)((T + 127) / 128);
+    pre_plan_kernel<<<tb, 128, 0, st>>>(ao, B, T, n_reads, chain_off, d_read_off, d_seed_off, roff, cseeds, cchains, pc,
+                                        left, right);
+    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(out, 0x80, sizeof(bsb_ext_out_t) * 2 * T, st), "chain extensions"))) return rc;
+    KswParams Q = P;
+    Q.pac = B.pac, Q.l_pac = B.l_pac;
+    const int builtin = ksw_builtin(T, ctx->n_sm);
+    const uint8_t *const map = ksw_builtin_tile_map(builtin);
+    uint64_t tiles = 0;
+    for (int need = 1; need <= max_len + 1 && need < BSB_TILE_MAP_LEN; ++need) tiles |= 1ull << map[need];
+    for (int side = 0; side < 2; ++side) {
+        if (side) pre_right_kernel<<<tb, 128, 0, st>>>(ao, T, left, out, right);
+        if ((rc = bsb_cuda(ctx, ksw_launch(Q, side ? right : left, T, 0, d_reads, nullptr, nullptr, builtin, tiles,
+                                           out + side * T, nullptr, D + o_scr, ctx->n_sm, st, nullptr, nullptr, nullptr,
+                                           &ctx->ms, true), "chain extensions")))
+            return rc;
+    }
+    pre->chains = pc, pre->off = chain_off, pre->left = out, pre->right = out + T;
+    return 0;
+}
+
 static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_reads, const uint8_t *d_reads,
                        const int64_t *d_read_off, const bsb_intv_t *d_seeds, const int64_t *d_seed_off,
                        int64_t n_seeds, int max_len, bool dedup, bsb_reg_t **d_regs_out, int64_t **d_reg_off_out,
@@ -2173,36 +2356,41 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
                 (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "read order keys")))
                 return rc;
             ctx->order_keys.clear();
-            order_hist_key<<<ob, 256, 0, st>>>(d_rkey, n_reads, ocnt);
-            order_scatter_key<<<ob, 256, 0, st>>>(d_rkey, n_reads, ocnt, ocnt + kOrderBins, order);
+            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt);
+            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt, ocnt + kOrderBins, order);
         } else if (learned) {   // predicted cells of every read, most expensive first
             if ((rc = bsb_mlp_forward(ctx, (const bsb_mlp_weights_t *)ctx->read_model, d_feat, n_reads, nullptr,
                                       d_rkey)))
                 return rc;
-            order_hist_key<<<ob, 256, 0, st>>>(d_rkey, n_reads, ocnt);
-            order_scatter_key<<<ob, 256, 0, st>>>(d_rkey, n_reads, ocnt, ocnt + kOrderBins, order);
+            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt);
+            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt, ocnt + kOrderBins, order);
         } else {
-            order_hist<<<ob, 256, 0, st>>>(n_chains, n_reads, ocnt);
-            order_scatter<<<ob, 256, 0, st>>>(n_chains, n_reads, ocnt, ocnt + kOrderBins, order);
+            order_hist<<<ob, kOrderThreads, 0, st>>>(n_chains, n_reads, ocnt);
+            order_scatter<<<ob, kOrderThreads, 0, st>>>(n_chains, n_reads, ocnt, ocnt + kOrderBins, order);
         }
     }
     int64_t *const rcells_out = logging ? d_rcells : nullptr;
+    PreResults pre{};
+    if (!logging && n_reads >= kPreReads &&
+        (rc = first_extensions(ctx, o, ao, B, P, n_reads, max_len, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
+                               n_chains, reg_off, scan_tmp, &pre)))
+        return rc;
     // every extension of these reads fits (max_len + 1) columns: the narrowest variant that holds them
     if (max_len <= 127)
         chain2aln_kernel<4><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out);
+                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
     else if (max_len <= 159)
         chain2aln_kernel<5><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out);
+                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
     else if (max_len <= 255)
         chain2aln_kernel<8><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out);
+                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
     else if (max_len <= 511)
         chain2aln_kernel<16><<<ctx->n_sm * 4, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out);
+                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
     else
         chain2aln_kernel<32><<<ctx->n_sm * 2, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out);
+                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
     if ((rc = bsb_cuda(ctx, cudaEventRecord(ctx->stage_ev[4], st), "stage mark")) ||
         (rc = bsb_cuda(ctx, scan_i32_i64(n_regs, n_reads, reg_off, scan_tmp, st), "region offsets")))
         return rc;

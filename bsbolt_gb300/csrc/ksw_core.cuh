@@ -47,6 +47,40 @@ __device__ __forceinline__ uint32_t sext_selector(int byte)
     return b | r << 4 | r << 8 | r << 12;
 }
 
+// A job's query or target: bytes, or for the jobs of an alignment batch (Packed, see KswParams) the
+// read's bytes and places of the forward-reverse text, either of them run backwards.
+template <bool Packed> struct JobText;
+template <> struct JobText<false> {
+    const uint8_t *p = nullptr;
+    __device__ __forceinline__ int byte(int i) const { return p[i]; }
+    __device__ __forceinline__ uint32_t base(const KswParams &, int i) const { return p[i]; }
+};
+template <> struct JobText<true> {
+    int64_t at = 0;
+    int back = 0;
+    __device__ __forceinline__ int byte(int i) const { return *(const uint8_t *)(at + (back ? -i : i)); }
+    __device__ __forceinline__ uint32_t base(const KswParams &P, int i) const
+    {
+        return (uint32_t)packed_text_base(P.pac, P.l_pac, at + (back ? -i : i));
+    }
+};
+template <bool Packed>
+__device__ __forceinline__ JobText<Packed> job_query(const uint8_t *seq, const bsb_ext_job_t &jb)
+{
+    JobText<Packed> t;
+    if constexpr (Packed) t.at = (int64_t)(seq + jb.qoff), t.back = jb.flags & kExtBack;
+    else t.p = seq + jb.qoff;
+    return t;
+}
+template <bool Packed>
+__device__ __forceinline__ JobText<Packed> job_target(const uint8_t *seq, const bsb_ext_job_t &jb)
+{
+    JobText<Packed> t;
+    if constexpr (Packed) t.at = jb.toff, t.back = jb.flags & kExtBack;
+    else t.p = seq + jb.toff;
+    return t;
+}
+
 // The scoring matrix as a shared table, score of target base t against query base q at
 // t << 3 | q (bases above 4 are N, as in profile_word).
 constexpr int kScoreTable = 40;

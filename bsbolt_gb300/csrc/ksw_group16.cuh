@@ -96,7 +96,7 @@ __device__ __forceinline__ void ksw16_pass2(const uint32_t (&Mv)[C2], uint32_t (
     if (C2 & 1) kmx = __vimax_s16x2_relu(kmx, kprev);
 }
 
-template <int C2, int G>
+template <int C2, int G, bool Packed = false>
 __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ext_job_t *__restrict__ jobs,
                                                 const uint8_t *__restrict__ seq, const int32_t *__restrict__ order,
                                                 int lo, int hi, int *__restrict__ counter,
@@ -116,7 +116,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
 
     // per-group job state
     int qlen = 0, tlen = 0, h0 = 0, w = 0, job = -1;
-    const uint8_t *t = nullptr;
+    JobText<Packed> t;
     uint32_t prof[C];
     uint32_t profN[(C + 3) / 4];
     uint32_t Hs[C2], Es[C2];
@@ -141,8 +141,8 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                 job = order[idx];
                 const bsb_ext_job_t jb = jobs[job];
                 qlen = jb.qlen; tlen = jb.tlen; h0 = jb.h0;
-                const uint8_t *q = seq + jb.qoff;
-                t = seq + jb.toff;
+                const JobText<Packed> q = job_query<Packed>(seq, jb);
+                t = job_target<Packed>(seq, jb);
                 const int h1run = max(h0 - oe_ins, 0);
 #pragma unroll
                 for (int s = 0; s < (C + 3) / 4; ++s) profN[s] = 0;
@@ -150,7 +150,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
 #pragma unroll
                 for (int s = 0; s < C; ++s) {
                     const int j = base + s;
-                    const int qc = j < qlen ? q[j] : 0;
+                    const int qc = j < qlen ? q.byte(j) : 0;
                     prof[s] = profile_word(P, qc);
                     profN[s >> 2] |= (uint32_t)(uint8_t)profile_n(P, qc) << ((s & 3) * 8);
                     h_init[s] = j == 0 ? h0 : (j <= qlen ? max(h1run - e_ins * (j - 1), 0) : 0);   // ksw.c:395-397
@@ -169,8 +169,8 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                 best = h0; best_i = best_j = -1; max_ie = -1; gscore = -1; max_off = 0;
                 beg = 0; end = qlen; i = 0; ncell = 0;
                 q_lane = qlen / C; q_slot = qlen % C;
-                tch = gl < tlen ? t[gl] : 4u;
-                tnext = G + gl < tlen ? t[G + gl] : 4u;
+                tch = gl < tlen ? t.base(P, gl) : 4u;
+                tnext = G + gl < tlen ? t.base(P, G + gl) : 4u;
                 have = tlen > 0;
                 if (!have && gl == 0) {        // no target: the reference returns h0 untouched
                     bsb_ext_out_t o;
@@ -192,7 +192,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         if ((i & (G - 1)) == G - 1) {
             tch = tnext;
             const int ti = i + G + 1 + gl;
-            tnext = ti < tlen ? t[ti] : 4u;
+            tnext = ti < tlen ? t.base(P, ti) : 4u;
         }
         const bool bump = beg < i - w;         // band edge (ksw.c:416-419)
         beg = bump ? i - w : beg;

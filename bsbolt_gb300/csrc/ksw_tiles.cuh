@@ -118,6 +118,15 @@ KswTileLaunch ksw_tiles16_g8(int C);
 KswTileLaunch ksw_tiles16_g16(int C);
 KswTileLaunch ksw_tiles16_g32(int C);
 
+// The kernels of an alignment batch's jobs exist for the shapes of the built-in maps.
+KswTileLaunch ksw_packed16_g4(int C);
+KswTileLaunch ksw_packed16_wide(int G, int C);
+inline KswTileLaunch ksw_packed16_launcher(int t)
+{
+    if (t < 0 || t >= kNumTiles) return nullptr;
+    return kTileList[t].G == 4 ? ksw_packed16_g4(kTileList[t].C) : ksw_packed16_wide(kTileList[t].G, kTileList[t].C);
+}
+
 // The 32-bit cell kernel of tile t (every shape has one).
 inline KswTileLaunch ksw_tile_launcher(int t)
 {

@@ -39,6 +39,16 @@ ksw_tile16_kernel(KswParams P, const bsb_ext_job_t *__restrict__ jobs, const uin
     ksw_group16_run<C2, G>(P, jobs, seq, order, range[0], range[1], counter, out, cells);
 }
 
+// The same for the jobs of an alignment batch, which read the 2-bit reference (KswParams::pac).
+template <int C2, int G>
+__global__ void __launch_bounds__(kKswBlock, ksw16_min_blocks(C2, G))
+ksw_packed16_kernel(KswParams P, const bsb_ext_job_t *__restrict__ jobs, const uint8_t *__restrict__ seq,
+                    const int32_t *__restrict__ order, const int32_t *__restrict__ range, int *__restrict__ counter,
+                    bsb_ext_out_t *__restrict__ out, int64_t *__restrict__ cells)
+{
+    ksw_group16_run<C2, G, true>(P, jobs, seq, order, range[0], range[1], counter, out, cells);
+}
+
 // One resident wave of blocks; the warps drain the range's queue.  n_sm < 0 asks for
 // one block per SM (-n_sm blocks), for a range that is expected to be short.
 template <typename K>
@@ -74,5 +84,15 @@ cudaError_t ksw_tile16_launch(const KswParams &P, const bsb_ext_job_t *jobs, con
 {
     static int blocks_per_sm = 0;
     return ksw_launch_wave(ksw_tile16_kernel<C2, G>, blocks_per_sm, P, jobs, seq, order, range, counter, out,
+                           cells, n_sm, st);
+}
+
+template <int C2, int G>
+cudaError_t ksw_packed16_launch(const KswParams &P, const bsb_ext_job_t *jobs, const uint8_t *seq,
+                                const int32_t *order, const int32_t *range, int *counter, bsb_ext_out_t *out,
+                                int64_t *cells, int n_sm, cudaStream_t st)
+{
+    static int blocks_per_sm = 0;
+    return ksw_launch_wave(ksw_packed16_kernel<C2, G>, blocks_per_sm, P, jobs, seq, order, range, counter, out,
                            cells, n_sm, st);
 }

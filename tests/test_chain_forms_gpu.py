@@ -78,3 +78,30 @@ def test_regions_equal_the_oracle(loaded, changes):
     assert np.array_equal(roff, want["regs_off"])
     for f in want["regs"].dtype.names:
         assert np.array_equal(regs[f], want["regs"][f]), f"reg.{f}"
+
+
+@pytest.mark.parametrize("changes", [{}, {"pen_clip5": 30, "pen_clip3": 30, "zdrop": 20}, {"w": 6, "zdrop": 0},
+                                     {"a": 2, "b": 3, "o_del": 4, "e_del": 2}, {"o_ins": 9000}],
+                         ids=lambda c: ",".join(c) or "defaults")
+def test_large_batches_equal_small_ones(loaded, changes):
+    """From 4096 reads on the chains' first extensions run as batches of their own (on 16-bit cells;
+    scorings that need 32-bit ones stay with the read's warp); the regions are those of small batches."""
+    ctx, bi = loaded
+    pac = bi.pac_codes()
+    rng = np.random.Generator(np.random.PCG64(21))
+    reads = []
+    for k in range(11):
+        reads += make_reads(pac, rng)
+    offs = np.zeros(len(reads) + 1, np.int64)
+    offs[1:] = np.cumsum([len(r) for r in reads])
+    seqs = np.concatenate(reads)
+    opt = _lib.AlignOpt.bwa_defaults(a=changes.get("a", 1), b=changes.get("b", 4))
+    for k, v in changes.items():
+        setattr(opt, k, v)
+    assert len(reads) >= 4096
+    regs, roff = seed.align_regs(ctx, seqs, offs, opt)
+    for lo in range(0, len(reads), 2000):
+        hi = min(lo + 2000, len(reads))
+        part, poff = seed.align_regs(ctx, seqs[offs[lo]:offs[hi]], offs[lo:hi + 1] - offs[lo], opt)
+        assert np.array_equal(roff[lo:hi + 1] - roff[lo], poff)
+        assert regs[roff[lo]:roff[hi]].tobytes() == part.tobytes()
