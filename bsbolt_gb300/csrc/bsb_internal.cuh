@@ -93,6 +93,9 @@ struct bsb_ctx {
     // the chains' first extensions of an alignment batch: jobs, bytes, results, scheduler scratch
     void *pre_buf = nullptr;
     size_t pre_bytes = 0;
+    // workspace of bsb_build_bwt for texts that need at most 4 GB
+    void *build_buf = nullptr;
+    size_t build_bytes = 0;
     // learned read order of the alignment batches: the cost model (caller's device memory,
     // or NULL for the chain-count order), and the per-read features and extension cells of
     // the last batch when logging

@@ -95,7 +95,8 @@ __global__ void widen_rows(const uint32_t *__restrict__ idx, int64_t m, uint64_t
 
 struct DevBuf {                          // freed on every return (after the stream is idle or failed)
     void *p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
+    bool lent = false;                   // a part of a buffer that stays
+    ~DevBuf() { if (p && !lent) cudaFree(p); }
 };
 
 }  // namespace
@@ -192,6 +193,7 @@ extern "C" int bsb_build_suffix_array(bsb_ctx *ctx, const uint8_t *pac, int64_t 
 
 namespace {
 
+constexpr size_t kBuildKept = (size_t)4 << 30;   // largest workspace the context keeps between builds
 constexpr uint64_t kAlone = 1ull << 63;     // rank flag: the suffix's group has one member
 constexpr int kBucketSyms = 5, kBuckets = 3125;    // 5^5 buckets of round 0
 constexpr int kBinBits = 13;                 // rounds >= 1: up to 2^13 rank bins
@@ -315,13 +317,18 @@ __global__ void tails_rev(const uint64_t *__restrict__ key, int64_t N, int from,
 // New ranks of a sorted chunk, the position of the last row of each suffix's group: base + that
 // row in round 0 (base = the chunk's first position); later, the old group's rank (its last row)
 // less the rows of the old group after the new group's last row.
-__global__ void write_ranks(const uint64_t *__restrict__ key, const uint64_t *__restrict__ val, int64_t N,
+// list (optional): receives the suffixes whose group has more members, n_open counting them.
+template <class V>
+__global__ void write_ranks(const uint64_t *__restrict__ key, const V *__restrict__ val, int64_t N,
                             const uint32_t *__restrict__ ek, const uint32_t *__restrict__ eo, int rbits,
                             uint64_t base, int round0, uint64_t *__restrict__ rank,
-                            unsigned long long *__restrict__ n_open)
+                            unsigned long long *__restrict__ n_open, V *__restrict__ list)
 {
     unsigned open = 0;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; j0 < N; j0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = min(j0 + lane, N - 1);
+        const bool in = j0 + lane < N;
         const uint64_t k = key[j];
         const int64_t end = N - 1 - (int64_t)ek[N - 1 - j];
         const bool alone = end == j && (j == 0 || key[j - 1] != k);
@@ -332,11 +339,49 @@ __global__ void write_ranks(const uint64_t *__restrict__ key, const uint64_t *__
             const int64_t oend = N - 1 - (int64_t)eo[N - 1 - j];
             r = base + (k >> rbits) - (uint64_t)(oend - end);
         }
-        rank[val[j]] = r | (alone ? kAlone : 0);
-        open += !alone;
+        const V i = val[j];
+        if (in) rank[i] = r | (alone ? kAlone : 0);
+        if (list) {
+            const unsigned m = __ballot_sync(BSB_FULL_MASK, in && !alone);
+            unsigned long long at = 0;
+            if (m && lane == 0) at = atomicAdd(n_open, (unsigned long long)__popc(m));
+            at = __shfl_sync(BSB_FULL_MASK, at, 0) + __popc(m & ((1u << lane) - 1u));
+            if (in && !alone) list[at] = i;
+        } else {
+            open += in && !alone;
+        }
     }
     open = __reduce_add_sync(0xffffffffu, open);
     if ((threadIdx.x & 31) == 0 && open) atomicAdd(n_open, (unsigned long long)open);
+}
+
+// ---- one chunk holds all suffixes
+// Every suffix's first key, eight suffixes a thread (a key is the one before, shifted by a symbol).
+__global__ void all_keys(const uint8_t *__restrict__ text, int64_t n, uint64_t *__restrict__ keys,
+                         uint32_t *__restrict__ vals)
+{
+    constexpr int kRun = 8;
+    const int64_t m = n + 1;
+    for (int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * kRun; i0 < m;
+         i0 += (int64_t)gridDim.x * blockDim.x * kRun) {
+        uint64_t k = key21(text, n, i0);
+#pragma unroll
+        for (int j = 0; j < kRun; ++j) {
+            if (i0 + j < m) keys[i0 + j] = k, vals[i0 + j] = (uint32_t)(i0 + j);
+            k = (k << 3 & ~0ull >> 1) | code_at(text, n, i0 + j + kPrefixSyms);
+        }
+    }
+}
+
+// A later round's keys of the suffixes still open, straight from their list.
+__global__ void open_keys(const uint64_t *__restrict__ rank, int64_t m, int64_t h, int rbits,
+                          const uint32_t *__restrict__ list, int64_t N, uint64_t *__restrict__ keys)
+{
+    const uint64_t mask = (1ull << rbits) - 1;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = list[j];
+        keys[j] = rank[i] << rbits | (i + h < m ? rank[i + h] & mask : 0);
+    }
 }
 
 // BWT symbols (2 bits, 16 to a word, first symbol in the top bits) and sampled rows, from the ranks
@@ -372,31 +417,67 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
     const size_t pb = (size_t)(l_pac + 3) / 4;
     const int64_t n_words = (n + 15) / 16, n_sa = (n + sa_intv) / sa_intv;
     DevBuf d_pac, d_text, d_rank, d_hist, d_cnt, k0, k1, v0, v1, s0, s1, d_tmp;
-    if ((rc = bsb_cuda(ctx, cudaMalloc(&d_text.p, (size_t)n + 64), "BWT build: text")) ||
+    // A text whose suffixes one chunk holds in kBuildKept bytes: everything in one buffer that the
+    // context keeps (allocating and freeing 1 GB in 13 pieces took more than the sort of a 10 Mb text),
+    // no bins, after each round only the suffixes still open are looked at again, and suffixes are 32-bit
+    // values of the sorts.  10 Mb text of three letters with repeats: 9.65 -> 5.5 ms, of which the sorts
+    // are half (0.15 ms a pass of the first, 10-30 us of the later ones).
+    size_t lent_tmp = 0;
+    bool whole = false;
+    if (m <= 0x7fffffffLL / 2 && (chunk <= 0 || chunk >= m)) {
+        cub::DoubleBuffer<uint64_t> kk((uint64_t *)nullptr, (uint64_t *)nullptr);
+        cub::DoubleBuffer<uint32_t> vv((uint32_t *)nullptr, (uint32_t *)nullptr);
+        size_t ts = 0, tc = 0;
+        if (cub::DeviceRadixSort::SortPairs(nullptr, ts, kk, vv, (int)m, 0, 64, st) != cudaSuccess ||
+            cub::DeviceScan::InclusiveScan(nullptr, tc, (uint32_t *)nullptr, (uint32_t *)nullptr, cuda::maximum<>(),
+                                           (int)m, st) != cudaSuccess)
+            return bsb_fail(ctx, BSB_ECUDA, "BWT build: sort set-up");
+        lent_tmp = std::max(ts, tc);
+        struct Part { DevBuf *b; size_t bytes; };
+        const size_t mm = (size_t)m;
+        const Part parts[] = {{&d_text, (size_t)n + 64}, {&d_rank, 8 * mm}, {&d_hist, 64}, {&d_cnt, 64}, {&d_pac, pb + 16},
+                              {&k0, 8 * mm}, {&k1, 8 * mm}, {&v0, 4 * mm}, {&v1, 4 * mm}, {&s0, 4 * mm}, {&s1, 4 * mm},
+                              {&d_tmp, lent_tmp + 256}};
+        size_t need = 0;
+        for (const Part &q : parts) need += (q.bytes + 255) & ~(size_t)255;
+        if (need <= kBuildKept && !bsb_ensure(ctx, &ctx->build_buf, &ctx->build_bytes, need, "BWT build")) {
+            char *at = (char *)ctx->build_buf;
+            for (const Part &q : parts) q.b->p = at, q.b->lent = true, at += (q.bytes + 255) & ~(size_t)255;
+            whole = true;
+        } else {
+            cudaGetLastError();          // no room for it: in chunks, as large texts are
+        }
+    }
+    if (!whole && ((rc = bsb_cuda(ctx, cudaMalloc(&d_text.p, (size_t)n + 64), "BWT build: text")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&d_rank.p, 8 * (size_t)m), "BWT build: ranks")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&d_hist.p, 8 * (size_t)std::max(kBuckets, 1 << kBinBits)),
                        "BWT build: histogram")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&d_cnt.p, 64), "BWT build: counters")) ||
-        (rc = bsb_cuda(ctx, cudaMalloc(&d_pac.p, pb + 16), "BWT build: pac")))
+        (rc = bsb_cuda(ctx, cudaMalloc(&d_pac.p, pb + 16), "BWT build: pac"))))
         return rc;
     const int grid = ctx->n_sm * 8;
     if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_pac.p, pac, pb, cudaMemcpyHostToDevice, st), "BWT build: H2D pac")))
         return rc;
     text_kernel<<<grid, 256, 0, st>>>((const uint8_t *)d_pac.p, l_pac, (uint8_t *)d_text.p);
-    if ((rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: text"))) return rc;
-    cudaFree(d_pac.p);
-    d_pac.p = nullptr;
+    if (!whole) {
+        if ((rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: text"))) return rc;
+        cudaFree(d_pac.p);
+        d_pac.p = nullptr;
+    }
     // the chunk: as many suffixes as the free memory holds at 44 bytes each (keys, suffixes, group rows
     // and sort scratch) less 3 GB, at most 2^31 - 1
-    size_t fr = 0, tot = 0;
-    if ((rc = bsb_cuda(ctx, cudaMemGetInfo(&fr, &tot), "BWT build: memory"))) return rc;
-    int64_t cap = (int64_t)((fr > ((size_t)3 << 30) ? fr - ((size_t)3 << 30) : 0) / 44);
-    cap = std::min<int64_t>(cap, 0x7fffffffLL);
-    cap = std::min<int64_t>(cap, m);
-    if (chunk > 0) cap = std::min<int64_t>(cap, chunk);
-    if (cap < std::min<int64_t>(m, 32)) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: no room for a sort chunk");
+    int64_t cap = m;
+    if (!whole) {
+        size_t fr = 0, tot = 0;
+        if ((rc = bsb_cuda(ctx, cudaMemGetInfo(&fr, &tot), "BWT build: memory"))) return rc;
+        cap = (int64_t)((fr > ((size_t)3 << 30) ? fr - ((size_t)3 << 30) : 0) / 44);
+        cap = std::min<int64_t>(cap, 0x7fffffffLL);
+        cap = std::min<int64_t>(cap, m);
+        if (chunk > 0) cap = std::min<int64_t>(cap, chunk);
+        if (cap < std::min<int64_t>(m, 32)) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: no room for a sort chunk");
+    }
     size_t tmp_sort = 0, tmp_scan = 0;
-    {
+    if (!whole) {
         cub::DoubleBuffer<uint64_t> kk((uint64_t *)nullptr, (uint64_t *)nullptr);
         cub::DoubleBuffer<uint64_t> vv((uint64_t *)nullptr, (uint64_t *)nullptr);
         if (cub::DeviceRadixSort::SortPairs(nullptr, tmp_sort, kk, vv, (int)cap, 0, 64, st) != cudaSuccess ||
@@ -404,14 +485,15 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                                            cuda::maximum<>(), (int)cap, st) != cudaSuccess)
             return bsb_fail(ctx, BSB_ECUDA, "BWT build: sort set-up");
     }
-    const size_t tmp_bytes = std::max(tmp_sort, tmp_scan);
-    if ((rc = bsb_cuda(ctx, cudaMalloc(&k0.p, 8 * (size_t)cap), "BWT build: keys")) ||
+    const size_t tmp_bytes = whole ? lent_tmp : std::max(tmp_sort, tmp_scan);
+    if (!whole &&
+        ((rc = bsb_cuda(ctx, cudaMalloc(&k0.p, 8 * (size_t)cap), "BWT build: keys")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&k1.p, 8 * (size_t)cap), "BWT build: keys")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&v0.p, 8 * (size_t)cap), "BWT build: suffixes")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&v1.p, 8 * (size_t)cap), "BWT build: suffixes")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&s0.p, 4 * (size_t)cap), "BWT build: group rows")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&s1.p, 4 * (size_t)cap), "BWT build: group rows")) ||
-        (rc = bsb_cuda(ctx, cudaMalloc(&d_tmp.p, tmp_bytes + 256), "BWT build: sort scratch")))
+        (rc = bsb_cuda(ctx, cudaMalloc(&d_tmp.p, tmp_bytes + 256), "BWT build: sort scratch"))))
         return rc;
     const uint8_t *text = (const uint8_t *)d_text.p;
     uint64_t *rank = (uint64_t *)d_rank.p;
@@ -419,9 +501,9 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
 
     // sorts the gathered chunk of N suffixes on key bits [0, end_bit) and writes their ranks
     unsigned long long h_cnt[2];
-    auto sort_chunk = [&](int64_t N, int end_bit, int round0, uint64_t base) -> int {
+    // (listed: the open ones' list in the spare buffer of vals, suffixes in 32 bits)
+    auto sort_as = [&](auto vals, int64_t N, int end_bit, int round0, uint64_t base, bool listed, void **list) -> int {
         cub::DoubleBuffer<uint64_t> keys((uint64_t *)k0.p, (uint64_t *)k1.p);
-        cub::DoubleBuffer<uint64_t> vals((uint64_t *)v0.p, (uint64_t *)v1.p);
         size_t t = 0;
         int r;
         if ((r = bsb_cuda(ctx, cub::DeviceRadixSort::SortPairs(nullptr, t, keys, vals, (int)N, 0, end_bit, st),
@@ -447,8 +529,14 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                 return r;
         }
         write_ranks<<<g, 256, 0, st>>>(keys.Current(), vals.Current(), N, ek, eo, rbits, base, round0, rank,
-                                       cnt + 1);
+                                       cnt + 1, listed ? vals.Alternate() : nullptr);
+        *list = vals.Alternate();
         return bsb_cuda(ctx, cudaGetLastError(), "BWT build: ranks");
+    };
+    auto sort_chunk = [&](int64_t N, int end_bit, int round0, uint64_t base) -> int {
+        void *list;
+        return sort_as(cub::DoubleBuffer<uint64_t>((uint64_t *)v0.p, (uint64_t *)v1.p), N, end_bit, round0, base, false,
+                       &list);
     };
 
     // the gather of a chunk appended exactly the suffixes its histogram counted
@@ -462,68 +550,91 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                                        (unsigned long long)N);
     };
 
-    // round 0: buckets of the first five symbols, chunks of whole buckets, 21-symbol keys
-    std::vector<unsigned long long> bh(kBuckets);
-    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(hist, 0, 8 * (size_t)kBuckets, st), "BWT build: histogram")) ||
-        (rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters")))
-        return rc;
-    bucket_hist<<<grid, 256, 0, st>>>(text, n, hist);
-    if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(bh.data(), hist, 8 * (size_t)kBuckets, cudaMemcpyDeviceToHost, st),
-                       "BWT build: histogram")) ||
-        (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: histogram")))
-        return rc;
-    {
-        uint64_t pos = 0;
-        for (int b = 0; b < kBuckets;) {
-            if ((int64_t)bh[b] > cap) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: bucket of %llu suffixes", bh[b]);
-            int e = b;
-            uint64_t N = 0;
-            while (e < kBuckets && N + bh[e] <= (uint64_t)cap) N += bh[e++];
-            if (N) {
-                if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 8, st), "BWT build: counters"))) return rc;
-                gather_buckets<<<grid, 256, 0, st>>>(text, n, b, e, cnt, (unsigned long long)cap, (uint64_t *)k0.p,
-                                                     (uint64_t *)v0.p);
-                if ((rc = gathered(N)) || (rc = sort_chunk((int64_t)N, 63, 1, pos))) return rc;
-            }
-            pos += N;
-            b = e;
+    if (whole) {
+        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters"))) return rc;
+        all_keys<<<grid, 256, 0, st>>>(text, n, (uint64_t *)k0.p, (uint32_t *)v0.p);
+        int64_t N = m;
+        for (int64_t h = kPrefixSyms, round = 0;; h *= 2, ++round) {
+            // the open suffixes go to the spare buffer, which becomes the next round's list
+            void *list = nullptr;
+            if ((rc = sort_as(cub::DoubleBuffer<uint32_t>((uint32_t *)v0.p, (uint32_t *)v1.p), N,
+                              round == 0 ? 63 : 2 * rbits, round == 0, 0, true, &list)) ||
+                (rc = bsb_cuda(ctx, cudaMemcpyAsync(h_cnt, cnt, 16, cudaMemcpyDeviceToHost, st), "BWT build: count")) ||
+                (rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters")) ||
+                (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: round")))
+                return rc;
+            N = (int64_t)h_cnt[1];
+            if (N == 0) break;                                      // every suffix is alone: sorted
+            if (round > 40) return bsb_fail(ctx, BSB_EINVAL, "BWT build: no convergence");
+            if (list != v0.p) std::swap(v0.p, v1.p);                 // the next sort takes them from v0
+            open_keys<<<(int)std::min<int64_t>((N + 255) / 256, (int64_t)ctx->n_sm * 16), 256, 0, st>>>(
+                rank, m, h, rbits, (const uint32_t *)list, N, (uint64_t *)k0.p);
         }
     }
-    // rounds 1, 2, ...: the suffixes whose group has more members, by rank bins
-    const int shift = rbits > kBinBits ? rbits - kBinBits : 0;
-    const int n_bins = (int)(((uint64_t)(m - 1) >> shift) + 1);
-    std::vector<unsigned long long> rh(n_bins);
-    for (int64_t h = kPrefixSyms, round = 1;; h *= 2, ++round) {
-        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(h_cnt, cnt, 16, cudaMemcpyDeviceToHost, st), "BWT build: count")) ||
-            (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: round")))
-            return rc;
-        if (h_cnt[1] == 0) break;                                   // every suffix is alone: sorted
-        if (round > 40) return bsb_fail(ctx, BSB_EINVAL, "BWT build: no convergence");
-        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(hist, 0, 8 * (size_t)n_bins, st), "BWT build: histogram")) ||
+    // round 0: buckets of the first five symbols, chunks of whole buckets, 21-symbol keys
+    std::vector<unsigned long long> bh(kBuckets);
+    if (!whole) {
+        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(hist, 0, 8 * (size_t)kBuckets, st), "BWT build: histogram")) ||
             (rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters")))
             return rc;
-        rank_hist<<<grid, 256, 0, st>>>(rank, m, shift, n_bins, hist);
-        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(rh.data(), hist, 8 * (size_t)n_bins, cudaMemcpyDeviceToHost, st),
+        bucket_hist<<<grid, 256, 0, st>>>(text, n, hist);
+        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(bh.data(), hist, 8 * (size_t)kBuckets, cudaMemcpyDeviceToHost, st),
                            "BWT build: histogram")) ||
             (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: histogram")))
             return rc;
-        const uint64_t bins_per_range = std::max<uint64_t>(1, max_range >> shift);
-        for (int b = 0; b < n_bins;) {
-            if ((int64_t)rh[b] > cap) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: rank bin of %llu suffixes", rh[b]);
-            int e = b;
-            uint64_t N = 0;
-            while (e < n_bins && N + rh[e] <= (uint64_t)cap && (uint64_t)(e - b) < bins_per_range) N += rh[e++];
-            if (N) {
-                const uint64_t rlo = (uint64_t)b << shift, rhi = (uint64_t)e << shift;
-                int span = 1;
-                while (span < 63 - rbits && (1ull << span) < rhi - rlo) ++span;
-                if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 8, st), "BWT build: counters"))) return rc;
-                gather_ranks<<<grid, 256, 0, st>>>(rank, m, h, rlo, rhi, rbits, cnt, (unsigned long long)cap,
-                                                   (uint64_t *)k0.p, (uint64_t *)v0.p);
-                if ((rc = gathered(N)) || (rc = sort_chunk((int64_t)N, std::min(64, rbits + span), 0, rlo)))
-                    return rc;
+        {
+            uint64_t pos = 0;
+            for (int b = 0; b < kBuckets;) {
+                if ((int64_t)bh[b] > cap) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: bucket of %llu suffixes", bh[b]);
+                int e = b;
+                uint64_t N = 0;
+                while (e < kBuckets && N + bh[e] <= (uint64_t)cap) N += bh[e++];
+                if (N) {
+                    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 8, st), "BWT build: counters"))) return rc;
+                    gather_buckets<<<grid, 256, 0, st>>>(text, n, b, e, cnt, (unsigned long long)cap, (uint64_t *)k0.p,
+                                                         (uint64_t *)v0.p);
+                    if ((rc = gathered(N)) || (rc = sort_chunk((int64_t)N, 63, 1, pos))) return rc;
+                }
+                pos += N;
+                b = e;
             }
-            b = e;
+        }
+        // rounds 1, 2, ...: the suffixes whose group has more members, by rank bins
+        const int shift = rbits > kBinBits ? rbits - kBinBits : 0;
+        const int n_bins = (int)(((uint64_t)(m - 1) >> shift) + 1);
+        std::vector<unsigned long long> rh(n_bins);
+        for (int64_t h = kPrefixSyms, round = 1;; h *= 2, ++round) {
+            if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(h_cnt, cnt, 16, cudaMemcpyDeviceToHost, st), "BWT build: count")) ||
+                (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: round")))
+                return rc;
+            if (h_cnt[1] == 0) break;                                   // every suffix is alone: sorted
+            if (round > 40) return bsb_fail(ctx, BSB_EINVAL, "BWT build: no convergence");
+            if ((rc = bsb_cuda(ctx, cudaMemsetAsync(hist, 0, 8 * (size_t)n_bins, st), "BWT build: histogram")) ||
+                (rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters")))
+                return rc;
+            rank_hist<<<grid, 256, 0, st>>>(rank, m, shift, n_bins, hist);
+            if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(rh.data(), hist, 8 * (size_t)n_bins, cudaMemcpyDeviceToHost, st),
+                               "BWT build: histogram")) ||
+                (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: histogram")))
+                return rc;
+            const uint64_t bins_per_range = std::max<uint64_t>(1, max_range >> shift);
+            for (int b = 0; b < n_bins;) {
+                if ((int64_t)rh[b] > cap) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: rank bin of %llu suffixes", rh[b]);
+                int e = b;
+                uint64_t N = 0;
+                while (e < n_bins && N + rh[e] <= (uint64_t)cap && (uint64_t)(e - b) < bins_per_range) N += rh[e++];
+                if (N) {
+                    const uint64_t rlo = (uint64_t)b << shift, rhi = (uint64_t)e << shift;
+                    int span = 1;
+                    while (span < 63 - rbits && (1ull << span) < rhi - rlo) ++span;
+                    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 8, st), "BWT build: counters"))) return rc;
+                    gather_ranks<<<grid, 256, 0, st>>>(rank, m, h, rlo, rhi, rbits, cnt, (unsigned long long)cap,
+                                                       (uint64_t *)k0.p, (uint64_t *)v0.p);
+                    if ((rc = gathered(N)) || (rc = sort_chunk((int64_t)N, std::min(64, rbits + span), 0, rlo)))
+                        return rc;
+                }
+                b = e;
+            }
         }
     }
     // the BWT without the row of suffix 0, and the sampled rows
