@@ -8,7 +8,8 @@
 // reading the device pac / opac directly; the ungapped score (bwa.c:222-230) is a
 // warp sum.  What the reference does as one sequential pass -- the DP rows with
 // their F chain, the traceback, and the MD / XB text whose run lengths carry from
-// base to base -- runs on lane 0 out of shared memory.  The bands mem_reg2aln asks
+// base to base -- the warp takes 32 cells or bases at a time (ksw_global.cuh, global_traceback,
+// the mask arithmetic below).  The bands mem_reg2aln asks
 // for are narrow (infer_bw, bwamem.c:1219-1223: 0 for a near-perfect ungapped hit,
 // a few columns per indel), so these passes are a few hundred steps.  Jobs longer
 // than kSmemLen keep their arrays in global scratch instead.
@@ -125,32 +126,63 @@ __global__ void plan_kernel(CigarParams P, const bsb_cigar_job_t *__restrict__ j
     }
 }
 
-// The traceback of ksw_global2 (ksw.c:584-600), one thread: ops come out last-first, then
-// are reversed.  Returns false when a step leaves the band.
+// The traceback of ksw_global2 (ksw.c:584-600) on the warp, all lanes in step: a run of matches is read 32 cells
+// of its diagonal at a time (the band holds a diagonal whole), gaps cell by cell.  Ops come out last-first (lane 0
+// writes), then are reversed.  Returns false when a step leaves the band.
 __device__ __forceinline__ bool global_traceback(const uint8_t *Z, int qlen, int tlen, int w, int stride, uint32_t *cig,
-                                 int &n_cigar)
+                                                 int &n_cigar, int lane)
 {
-    int which = 0, i = tlen - 1, k = (i + w + 1 < qlen ? i + w + 1 : qlen) - 1;
-    n_cigar = 0;
-    auto push = [&](int op, int len) {
-        if (n_cigar && (int)(cig[n_cigar - 1] & 0xf) == op) cig[n_cigar - 1] += (uint32_t)len << 4;
-        else cig[n_cigar++] = (uint32_t)len << 4 | op;
+    int which = 0, i = tlen - 1, k = (i + w + 1 < qlen ? i + w + 1 : qlen) - 1, op = 0, len = 0, n = 0;
+    const auto push = [&](int o, int l) {
+        if (o != op) {
+            if (len) {
+                if (lane == 0) cig[n] = (uint32_t)len << 4 | op;
+                ++n;
+            }
+            op = o, len = 0;
+        }
+        len += l;
     };
+    bool left = false;
     while (i >= 0 && k >= 0) {
         const int beg = i > w ? i - w : 0, end = i + w + 1 < qlen ? i + w + 1 : qlen;
-        if (k < beg || k >= end) return false;
-        which = Z[(size_t)i * stride + (k - beg)] >> (which << 1) & 3;
-        if (which == 0) push(0, 1), --i, --k;
-        else if (which == 1) push(2, 1), --i;
-        else push(1, 1), --k;
+        if (k < beg || k >= end) {
+            left = true;
+            break;
+        }
+        if (which == 0) {
+            const int r = i - lane, c = k - lane;
+            const bool in = r >= 0 && c >= 0;
+            const int z = in ? Z[(size_t)r * stride + (c - (r > w ? r - w : 0))] & 3 : 3;
+            const unsigned stop = __ballot_sync(BSB_FULL_MASK, z != 0);
+            const int run = stop ? __ffs(stop) - 1 : 32;
+            if (run) push(0, run), i -= run, k -= run;
+            if (run == 32 || i < 0 || k < 0) continue;
+            which = __shfl_sync(BSB_FULL_MASK, z, run);
+        } else {
+            which = Z[(size_t)i * stride + (k - beg)] >> (which << 1) & 3;
+            if (which == 0) push(0, 1), --i, --k;
+        }
+        if (which == 1) push(2, 1), --i;
+        else if (which == 2) push(1, 1), --k;
     }
-    if (i >= 0) push(2, i + 1);
-    if (k >= 0) push(1, k + 1);
-    for (int a = 0; a < n_cigar >> 1; ++a) {
-        const uint32_t t = cig[a];
-        cig[a] = cig[n_cigar - 1 - a];
-        cig[n_cigar - 1 - a] = t;
+    if (!left) {
+        if (i >= 0) push(2, i + 1);
+        if (k >= 0) push(1, k + 1);
     }
+    if (len) {
+        if (lane == 0) cig[n] = (uint32_t)len << 4 | op;
+        ++n;
+    }
+    n_cigar = n;
+    if (left) return false;
+    if (lane == 0)
+        for (int a = 0; a < n >> 1; ++a) {
+            const uint32_t t = cig[a];
+            cig[a] = cig[n - 1 - a];
+            cig[n - 1 - a] = t;
+        }
+    __syncwarp();
     return true;
 }
 
@@ -230,14 +262,12 @@ cigar_kernel(CigarParams P, const bsb_cigar_job_t *__restrict__ jobs, int n, con
             score = __reduce_add_sync(BSB_FULL_MASK, sum);
             n_cigar = 1;
             if (lane == 0) cig[0] = (uint32_t)l << 4;
-        } else {                              // ksw_global2: rows on the warp, traceback on lane 0
-            score = global_rows_warp(GlobalPen{P.o_del, P.e_del, P.o_ins, P.e_ins}, smat, qs, l, ts, rlen, p.w, p.stride,
-                                     H, E, Z, lane);
-            if (lane == 0) band_exit = !global_traceback(Z, l, rlen, p.w, p.stride, cig, n_cigar);
+        } else {                              // ksw_global2
+            score = global_warp(GlobalPen{P.o_del, P.e_del, P.o_ins, P.e_ins}, smat, qs, l, (const uint8_t *)ts, rlen,
+                                p.w, p.stride, H, E, Z, lane);
+            band_exit = !global_traceback(Z, l, rlen, p.w, p.stride, cig, n_cigar, lane);
         }
-        score = __shfl_sync(BSB_FULL_MASK, score, 0);
-        n_cigar = __shfl_sync(BSB_FULL_MASK, n_cigar, 0);
-        band_exit = __shfl_sync(BSB_FULL_MASK, band_exit, 0);
+        __syncwarp();
         if (band_exit) {
             if (lane == 0) finish(out, bytes, id, BSB_CIGAR_BAND_EXIT, score, n_cigar, -1, 0, 0, 0, 0, 0);
             __syncwarp();

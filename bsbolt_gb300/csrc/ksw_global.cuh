@@ -1,4 +1,4 @@
-// ksw_global.cuh -- the DP rows of ksw_global2 (bsbolt/External/BWA/ksw.c:504-582) on one warp,
+// ksw_global.cuh -- the DP of ksw_global2 (bsbolt/External/BWA/ksw.c:504-582) on one warp,
 // shared by bwa_gen_cigar2 (cigar.cu) and mem_patch_reg's score-only call (chain.cu).
 #pragma once
 
@@ -83,3 +83,92 @@ __device__ __forceinline__ int global_rows_warp(const GlobalPen &P, const int8_t
     return H[qlen];
 }
 
+// The same cells with the band's diagonals over the lanes, C neighbours to a lane: cell (i, d), j = i + d - w,
+// takes H from its own diagonal's row before, E from diagonal d + 1's row before and F from diagonal d - 1's
+// same row.  Lane k does row s - k in step s: F comes from the lane below's step before, E of a lane's last
+// diagonal from the lane above's first in the same step, so a step is one exchange each way and C cells whose
+// only chain is F's, and a job takes tlen + band / C steps.  H, E and F stay in registers (a diagonal's first
+// H is the border's value; a cell outside leaves E and F at -inf), and scores are fetched a step ahead.
+// Needs 2w + 1 < 32 C.
+template <int C, class TS>
+__device__ __forceinline__ int global_diagonals_warp(const GlobalPen &P, const int8_t *smat, const uint8_t *qs,
+                                                     int qlen, const TS &ts, int tlen, int w, int stride, uint8_t *Z,
+                                                     int lane)
+{
+    const int oe_del = P.o_del + P.e_del, oe_ins = P.o_ins + P.e_ins, e_ins = P.e_ins;
+    const int d0 = lane * C, last = 2 * w;
+    int32_t h[C], e[C], f_out = kNegInf;
+    int sc[C], q[C];                              // this step's scores; the next step's query bases
+    int i = -lane, t = 0;                         // this step's row; the next row's base
+    const auto base_q = [&](int j) { return (unsigned)j < (unsigned)qlen ? (int)qs[j] : 0; };
+    const auto base_t = [&](int r) { return (unsigned)r < (unsigned)tlen ? (int)ts[r] : 0; };
+    t = base_t(i);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const int j = d0 + c - w;
+        h[c] = j > 0 ? -(P.o_ins + e_ins * j) : j < 0 ? -(P.o_del - P.e_del * j) : 0;
+        e[c] = kNegInf;
+        sc[c] = smat[t * 5 + base_q(i + j)];
+        q[c] = base_q(i + j + 1);
+    }
+    t = base_t(i + 1);
+    const int steps = tlen + last / C;
+    for (int s = 0; s < steps; ++s, ++i) {
+        int next[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) next[c] = smat[t * 5 + q[c]];
+        const int j0 = i + d0 - w;
+        t = base_t(i + 2);
+#pragma unroll
+        for (int c = 0; c < C - 1; ++c) q[c] = q[c + 1];
+        q[C - 1] = base_q(j0 + C + 1);
+        int32_t f = __shfl_up_sync(BSB_FULL_MASK, f_out, 1);
+        if (lane == 0) f = kNegInf;
+        const bool row = (unsigned)i < (unsigned)tlen;
+        const int z_at = i * stride + (i >= w ? d0 : j0);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const int32_t e_in = c == C - 1 ? __shfl_down_sync(BSB_FULL_MASK, e[0], 1) : e[c + 1];
+            const bool on = row && (unsigned)(j0 + c) < (unsigned)qlen && d0 + c <= last;
+            const int32_t m = h[c] + sc[c];
+            int32_t best = m;
+            uint32_t dir = 0;
+            if (m < e_in) best = e_in, dir = 1;
+            if (best < f) best = f, dir = 2;
+            const int32_t td = m - oe_del, ed = e_in - P.e_del;
+            if (ed > td) dir |= 1 << 2;
+            const int32_t ti = m - oe_ins, fi = f - e_ins;
+            if (fi > ti) dir |= 2 << 4;
+            e[c] = on ? (ed > td ? ed : td) : kNegInf;
+            f = on ? (fi > ti ? fi : ti) : kNegInf;
+            if (on) {
+                h[c] = best;
+                if (Z) Z[z_at + c] = (uint8_t)dir;
+            }
+            sc[c] = next[c];
+        }
+        f_out = f;
+    }
+    __syncwarp();
+    const int d = qlen - tlen + w;                // the last cell's diagonal
+    int32_t score = h[0];
+#pragma unroll
+    for (int c = 1; c < C; ++c)
+        if (d % C == c) score = h[c];
+    return __shfl_sync(BSB_FULL_MASK, score, d / C);
+}
+
+// Which form: the diagonals' wherever they fit four to a lane, two to a lane where that suffices (half the cells
+// a step).  A row at a time costs a five-step scan and four exchanges per 32 columns one after the other, some
+// 2000 clocks a row for a band of 65 columns against 150 here: bwa_gen_cigar2's kernel on 40k reads of 100 bases
+// 204 us -> 124, and a merge's 150-row alignment in mem_patch_reg 180 us -> 15.  Rows are left for wider bands.
+template <class TS>
+__device__ __forceinline__ int global_warp(const GlobalPen &P, const int8_t *smat, const uint8_t *qs, int qlen,
+                                           const TS &ts, int tlen, int w, int stride, int32_t *H, int32_t *E,
+                                           uint8_t *Z, int lane)
+{
+    const int diagonals = 2 * w + 1;
+    if (diagonals < 64) return global_diagonals_warp<2>(P, smat, qs, qlen, ts, tlen, w, stride, Z, lane);
+    if (diagonals < 128) return global_diagonals_warp<4>(P, smat, qs, qlen, ts, tlen, w, stride, Z, lane);
+    return global_rows_warp(P, smat, qs, qlen, ts, tlen, w, stride, H, E, Z, lane);
+}
