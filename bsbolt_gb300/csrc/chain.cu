@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -1886,12 +1887,29 @@ struct DedupOpt {
     int8_t mat[25];
 };
 
-constexpr int kDedupWarps = 4;
+constexpr int kDedupWarps = 4, kDedupFew = 64;
 
-struct DedupSmem {                    // one warp's global alignment of mem_patch_reg
-    int32_t H[BSB_ALIGN_MAX_LEN + 1], E[BSB_ALIGN_MAX_LEN + 1];
-    uint8_t q[BSB_ALIGN_MAX_LEN];
+struct DedupSmem {                    // one warp's orders, and its global alignment of mem_patch_reg
+    int *order, *weight;              // kDedupFew entries
+    int32_t *H, *E;                   // max_len + 1 entries
+    uint8_t *q;                       // max_len entries
 };
+__host__ __device__ __forceinline__ int dedup_warp_bytes(int max_len)
+{
+    return 4 * (2 * kDedupFew + 2 * (max_len + 1)) + ((max_len + 3) & ~3);
+}
+
+// dst[k] = src[ix ? ix[k] : k] for k < n by the warp, 4 bytes a lane; one_comp: with n_comp = 1.
+__device__ __forceinline__ void copy_regs(bsb_reg_t *dst, const bsb_reg_t *src, const int *ix, int n, bool one_comp,
+                                          int lane)
+{
+    constexpr int kWords = sizeof(bsb_reg_t) / 4, kComp = offsetof(bsb_reg_t, n_comp) / 4;
+    for (int t = lane; t < n * kWords; t += 32) {
+        const int k = t / kWords, f = t - k * kWords;
+        const int v = ((const int *)(src + (ix ? ix[k] : k)))[f];
+        ((int *)dst)[t] = one_comp && f == kComp ? 1 : v;
+    }
+}
 
 // Target base i of [rb, re) after bwa_gen_cigar2's flip (bwa.c:216-221): read backwards on the
 // reverse strand.
@@ -1902,28 +1920,41 @@ struct PatchText {
     __device__ __forceinline__ int operator[](int i) const { return text_base(B, rev ? re - 1 - i : rb + i); }
 };
 
-// mem_patch_reg (bwamem.c:410-439) on the warp: every lane takes the same steps; the global
-// alignment of its bwa_gen_cigar2 call (score only, bwa.c:211-244) runs on the whole warp.  The
-// reference's double expressions are evaluated as written (no fused multiply-adds).
-__device__ int patch_reg_warp(const DedupOpt &O, const int8_t *smat, const DevBns &B, const uint8_t *read,
-                              const bsb_reg_t &a, const bsb_reg_t &b, int *w_out, DedupSmem &S, int lane)
+// mem_patch_reg's tests before its alignment (bwamem.c:413-428).
+__device__ __forceinline__ bool patch_candidate(const DedupOpt &O, int64_t l_pac, const bsb_reg_t &a, const bsb_reg_t &b)
 {
-    const int64_t l_pac = B.l_pac;
-    if (a.rb < l_pac && b.rb >= l_pac) return 0;                       // different strands
-    if (a.qb >= b.qb || a.qe >= b.qe || a.re >= b.re) return 0;       // not colinear
+    if (a.rb < l_pac && b.rb >= l_pac) return false;                   // different strands
+    if (a.qb >= b.qb || a.qe >= b.qe || a.re >= b.re) return false;   // not colinear
     int w = (int)((a.re - b.rb) - (a.qe - b.qb));
     w = w > 0 ? w : -w;
+    const bool apart = a.re < b.rb || a.qe < b.qb;
+    if (w > (apart ? O.w << 1 : O.w << 2)) return false;
     double r = __dsub_rn(__ddiv_rn((double)(a.re - b.rb), (double)(b.re - a.rb)),
                          __ddiv_rn((double)(a.qe - b.qb), (double)(b.qe - a.qb)));
     r = r > 0. ? r : -r;
-    if (a.re < b.rb || a.qe < b.qb) {
-        if (w > O.w << 1 || r >= (double)0.05f) return 0;              // PATCH_MAX_R_BW
-    } else if (w > O.w << 2 || r >= (double)(0.05f * 2)) return 0;
+    return !(r >= (apart ? (double)0.05f : (double)(0.05f * 2)));     // PATCH_MAX_R_BW
+}
+
+// The rest of mem_patch_reg (bwamem.c:410-439) on the warp: every lane takes the same steps; the global
+// alignment of its bwa_gen_cigar2 call (score only, bwa.c:211-244) runs on the whole warp.  The
+// reference's double expressions are evaluated as written (no fused multiply-adds).
+__device__ __noinline__ int patch_reg_warp(const DedupOpt &O, const int8_t *smat, const DevBns &B, const uint8_t *read,
+                                           const bsb_reg_t &a, const bsb_reg_t &b, int *w_out, const DedupSmem &S,
+                                           int lane)
+{
+    const int64_t l_pac = B.l_pac;
+    int w = (int)((a.re - b.rb) - (a.qe - b.qb));
+    w = w > 0 ? w : -w;
     w += a.w + b.w;
     w = w < O.w << 2 ? w : O.w << 2;
     // bwa_gen_cigar2(..., w, l_pac, pac, pac, b.qe - a.qb, query + a.qb, a.rb, b.re, &score, 0, ...)
     const int lq = b.qe - a.qb;
     const int64_t rb = a.rb, re = b.re;
+    const int sc2 = b.score + a.score;
+    const int q_s = (int)__dadd_rn(__dmul_rn(__ddiv_rn((double)(b.qe - a.qb), (double)((b.qe - b.qb) + (a.qe - a.qb))),
+                                             (double)sc2), .499);
+    const int r_s = (int)__dadd_rn(__dmul_rn(__ddiv_rn((double)(b.re - a.rb), (double)((b.re - b.rb) + (a.re - a.rb))),
+                                             (double)sc2), .499);
     int score = 0;
     if (!(lq <= 0 || rb >= re || (rb < l_pac && re > l_pac)) && rb >= 0 && re <= l_pac << 1) {
         const bool rev = rb >= l_pac;
@@ -1931,31 +1962,24 @@ __device__ int patch_reg_warp(const DedupOpt &O, const int8_t *smat, const DevBn
         for (int j = lane; j < lq; j += 32) S.q[j] = read[rev ? b.qe - 1 - j : a.qb + j];
         __syncwarp();
         const PatchText T{B, rb, re, rev};
-        if (lq == rlen && w == 0) {                                    // ungapped (bwa.c:222-230)
+        const int dl = rlen > lq ? rlen - lq : lq - rlen;
+        if (lq == rlen && w == 0) {                                     // without gaps (bwa.c:222-230)
             int part = 0;
             for (int j = lane; j < lq; j += 32) part += smat[T[j] * 5 + S.q[j]];
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(BSB_FULL_MASK, part, d);
-            score = part;
+            score = __reduce_add_sync(BSB_FULL_MASK, part);
         } else {                                                       // the band of bwa.c:232-240
             const int half = ((lq + 1) >> 1) * smat[0];
             const int max_ins = (int)__dadd_rn(__ddiv_rn((double)(half - O.pen.o_ins), (double)O.pen.e_ins), 1.);
             const int max_del = (int)__dadd_rn(__ddiv_rn((double)(half - O.pen.o_del), (double)O.pen.e_del), 1.);
             int max_gap = max_ins > max_del ? max_ins : max_del;
             max_gap = max_gap > 1 ? max_gap : 1;
-            const int dl = rlen > lq ? rlen - lq : lq - rlen;
             int bw = (max_gap + dl + 1) >> 1;
             bw = bw < w ? bw : w;
             bw = bw > dl + 3 ? bw : dl + 3;
-            score = global_rows_warp(O.pen, smat, S.q, lq, T, rlen, bw, 0, S.H, S.E, nullptr, lane);
+            score = global_warp(O.pen, smat, S.q, lq, T, rlen, bw, 0, S.H, S.E, nullptr, lane);
         }
         __syncwarp();
     }
-    const int sc2 = b.score + a.score;
-    const int q_s = (int)__dadd_rn(__dmul_rn(__ddiv_rn((double)(b.qe - a.qb), (double)((b.qe - b.qb) + (a.qe - a.qb))),
-                                             (double)sc2), .499);
-    const int r_s = (int)__dadd_rn(__dmul_rn(__ddiv_rn((double)(b.re - a.rb), (double)((b.re - b.rb) + (a.re - a.rb))),
-                                             (double)sc2), .499);
     if (__ddiv_rn((double)score, (double)(q_s > r_s ? q_s : r_s)) < (double)0.90f) return 0;   // PATCH_MIN_SC_RATIO
     *w_out = w;
     return score;
@@ -1963,20 +1987,30 @@ __device__ int patch_reg_warp(const DedupOpt &O, const int8_t *smat, const DevBn
 
 // mem_sort_dedup_patch (bwamem.c:441-493) per read, one warp per read.  in: the read's
 // pre-dedup regions at reg_off[r]; a: scratch of the same size (the sorted copy that the scan
-// edits); ix: index scratch; out: the kept regions at reg_off[r], n_out[r] of them.  Lane 0 runs
-// the two ks_introsort orders; the redundancy and merge scan is taken by every lane in step
-// (lane 0 writes), so that the warp can run a merge's global alignment.
-__global__ void __launch_bounds__(kDedupWarps * 32)
+// edits); ix: index scratch; out: the kept regions at reg_off[r], n_out[r] of them.  The two
+// ks_introsort orders: each region's count of regions that come before it decides every comparison, so
+// up to 64 regions are sort_places' integers (more: lane 0 on the records).  The redundancy and
+// merge scan is taken by every lane in step (lane 0 writes), so that the warp can run a merge's global
+// alignment, and only at regions that reach the one before.
+// Both sorts on one lane with the records in global memory, all regions scanned: 0.50 ms for 114k RRBS
+// reads (450k regions), 0.20 ms for 67k of 150 bases; as here 0.24 and 0.13.  Time is a warp's own chain
+// (10k clocks a read), so warps resident count up to where registers spill: at 6, 8, 10 and 12 blocks an SM the
+// stage takes 0.315, 0.288, 0.287, 0.350 ms on the RRBS reads and 0.190, 0.181, 0.207, 0.237 on the others.
+__global__ void __launch_bounds__(kDedupWarps * 32, 8)
 dedup_kernel(DedupOpt O, DevBns B, int n_reads, const uint8_t *__restrict__ reads,
              const int64_t *__restrict__ read_off, const int64_t *__restrict__ reg_off,
              const bsb_reg_t *__restrict__ in, bsb_reg_t *a_all, int *ix_all, bsb_reg_t *__restrict__ out,
-             int *__restrict__ n_out)
+             int *__restrict__ n_out, int max_len)
 {
-    __shared__ DedupSmem sm[kDedupWarps];
+    extern __shared__ __align__(16) char dedup_smem[];
     __shared__ int8_t smat[25];
     if (threadIdx.x < 25) smat[threadIdx.x] = O.mat[threadIdx.x];
     __syncthreads();
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    DedupSmem S;
+    S.order = (int *)(dedup_smem + wb * dedup_warp_bytes(max_len)), S.weight = S.order + kDedupFew;
+    S.H = (int32_t *)(S.weight + kDedupFew), S.E = S.H + max_len + 1;
+    S.q = (uint8_t *)(S.E + max_len + 1);
     for (int r = blockIdx.x * kDedupWarps + wb; r < n_reads; r += gridDim.x * kDedupWarps) {
         const int64_t o0 = reg_off[r];
         const int n = (int)(reg_off[r + 1] - o0);
@@ -1984,65 +2018,197 @@ dedup_kernel(DedupOpt O, DevBns B, int n_reads, const uint8_t *__restrict__ read
         bsb_reg_t *a = a_all + o0, *dst = out + o0;
         int *ix = ix_all + o0;
         if (n <= 1) {                                    // bwamem.c:444: returned as they are
-            if (lane == 0) {
-                if (n == 1) dst[0] = a_in[0];
-                n_out[r] = n;
-            }
+            if (n == 1) copy_regs(dst, a_in, nullptr, 1, false, lane);
+            if (lane == 0) n_out[r] = n;
             continue;
         }
-        if (lane == 0) {                                 // sort by end (bwamem.c:445)
-            int stk_l[64], stk_r[64], stk_d[64];
-            for (int k = 0; k < n; ++k) ix[k] = k;
-            KsSort<RegReLt>{ix, RegReLt{a_in}}.sort(n, stk_l, stk_r, stk_d);
+        const bool few = n <= kDedupFew;
+        // which regions the scan has to look at: those that reach the one before (neither its contig and end
+        // nor a region's own start changes before the scan comes to it)
+        uint64_t near = ~0ull;
+        if (few) {                                       // sort by end (bwamem.c:445)
+            int64_t re[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) re[h] = lane + 32 * h < n ? a_in[lane + 32 * h].re : 0;
+            int less[2] = {0, 0};
+            for (int e = 0; e < n; ++e) {
+                const int64_t x = __shfl_sync(BSB_FULL_MASK, e < 32 ? re[0] : re[1], e & 31);
+                less[0] += x < re[0], less[1] += x < re[1];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (lane + 32 * h < n) S.order[lane + 32 * h] = lane + 32 * h, S.weight[lane + 32 * h] = -less[h];
+            __syncwarp();
+            sort_places(S.order, S.weight, n, lane);
+            near = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = lane + 32 * h;
+                bool reach = false;
+                if (k >= 1 && k < n) {
+                    const bsb_reg_t &p = a_in[S.order[k]], &q = a_in[S.order[k - 1]];
+                    reach = p.rid == q.rid && p.rb < q.re + O.max_chain_gap;
+                }
+                near |= (uint64_t)__ballot_sync(BSB_FULL_MASK, reach) << (32 * h);
+            }
+            if (near) copy_regs(a, a_in, S.order, n, true, lane);
+            __syncwarp();
+        } else {
+            if (lane == 0) {
+                int stk_l[64], stk_r[64], stk_d[64];
+                for (int k = 0; k < n; ++k) ix[k] = k;
+                KsSort<RegReLt>{ix, RegReLt{a_in}}.sort(n, stk_l, stk_r, stk_d);
+            }
+            __syncwarp();
+            copy_regs(a, a_in, ix, n, true, lane);
+            __syncwarp();
         }
-        __syncwarp();
-        for (int k = lane; k < n; k += 32) {
-            a[k] = a_in[ix[k]];
-            a[k].n_comp = 1;
-        }
-        __syncwarp();
         const uint8_t *read = reads + read_off[r];
         for (int i = 1; i < n; ++i) {                    // bwamem.c:447-474
+            if (few) {
+                const uint64_t rest = i < 64 ? near >> i : 0ull;
+                if (!rest) break;
+                i += __ffsll((long long)rest) - 1;
+            }
             bsb_reg_t p = a[i];
             if (p.rid != a[i - 1].rid || p.rb >= a[i - 1].re + O.max_chain_gap) continue;
-            for (int j = i - 1; j >= 0 && p.rid == a[j].rid && p.rb < a[j].re + O.max_chain_gap; --j) {
-                const bsb_reg_t q = a[j];
-                if (q.qe == q.qb) continue;                      // a[j] has been excluded
-                const int64_t or_ = q.re - p.rb;
-                const int64_t oq = q.qb < p.qb ? q.qe - p.qb : p.qe - q.qb;
-                const int64_t mr = q.re - q.rb < p.re - p.rb ? q.re - q.rb : p.re - p.rb;
-                const int64_t mq = q.qe - q.qb < p.qe - p.qb ? q.qe - q.qb : p.qe - p.qb;
-                // float, as the reference's float option times an int64
-                if ((float)or_ > __fmul_rn(O.mask_level_redun, (float)mr) &&
-                    (float)oq > __fmul_rn(O.mask_level_redun, (float)mq)) {
-                    if (p.score < q.score) {
+            // The reference goes down from i - 1 until a region is out of reach; here 32 at a time, the lanes
+            // finding what each would do: end the scan, exclude region j, exclude region i and end, or try to
+            // merge.  Exclusions of j change nothing for the others, so only the last two are taken one by one;
+            // a merge changes p, and the regions below it are looked at again.
+            bool ended = false;
+            for (int top = i - 1; top >= 0 && !ended;) {
+                const int j = top - lane;
+                bool out = false, drop_j = false, drop_i = false, merge = false;
+                if (j >= 0) {
+                    const bsb_reg_t q = a[j];
+                    out = p.rid != q.rid || p.rb >= q.re + O.max_chain_gap;
+                    if (!out && q.qe != q.qb) {                  // (else a[j] has been excluded)
+                        const int64_t or_ = q.re - p.rb;
+                        const int64_t oq = q.qb < p.qb ? q.qe - p.qb : p.qe - q.qb;
+                        const int64_t mr = q.re - q.rb < p.re - p.rb ? q.re - q.rb : p.re - p.rb;
+                        const int64_t mq = q.qe - q.qb < p.qe - p.qb ? q.qe - q.qb : p.qe - p.qb;
+                        // float, as the reference's float option times an int64
+                        if ((float)or_ > __fmul_rn(O.mask_level_redun, (float)mr) &&
+                            (float)oq > __fmul_rn(O.mask_level_redun, (float)mq)) {
+                            drop_i = p.score < q.score;
+                            drop_j = !drop_i;
+                        } else {
+                            merge = q.rb < p.rb && patch_candidate(O, B.l_pac, q, p);
+                        }
+                    }
+                }
+                const unsigned mo = __ballot_sync(BSB_FULL_MASK, out || j < 0);
+                unsigned events = __ballot_sync(BSB_FULL_MASK, drop_i || merge);
+                const unsigned reach = mo ? (1u << (__ffs(mo) - 1)) - 1u : 0xffffffffu;
+                events &= reach;
+                int next = mo ? -1 : top - 32, done = 0;        // lanes below `done` have been taken
+                bool again = false;
+                while (!again) {
+                    const int e = events ? __ffs(events) - 1 : 32;
+                    if (drop_j && lane >= done && lane < e && (reach >> lane & 1u)) a[j].qe = a[j].qb;
+                    __syncwarp();
+                    if (e == 32) break;
+                    done = e + 1;
+                    events &= events - 1;
+                    if (__shfl_sync(BSB_FULL_MASK, drop_i, e)) {
                         if (lane == 0) a[i].qe = p.qb;
-                        __syncwarp();
+                        next = -1;
                         break;
                     }
-                    if (lane == 0) a[j].qe = q.qb;
-                    __syncwarp();
-                } else if (q.rb < p.rb) {
+                    const bsb_reg_t q = a[top - e];
                     int w = 0;
-                    const int score = patch_reg_warp(O, smat, B, read, q, p, &w, sm[wb], lane);
+                    const int score = patch_reg_warp(O, smat, B, read, q, p, &w, S, lane);
                     if (score > 0) {                             // merge q into p
                         if (lane == 0) {
-                            p.n_comp += q.n_comp + 1;
-                            p.seedcov = p.seedcov > q.seedcov ? p.seedcov : q.seedcov;
-                            p.qb = q.qb, p.rb = q.rb;
-                            p.truesc = p.score = score;
-                            p.w = w;
-                            a[i] = p;
-                            a[j].qb = q.qe;
+                            bsb_reg_t u = p;
+                            u.n_comp += q.n_comp + 1;
+                            u.seedcov = u.seedcov > q.seedcov ? u.seedcov : q.seedcov;
+                            u.qb = q.qb, u.rb = q.rb;
+                            u.truesc = u.score = score;
+                            u.w = w;
+                            a[i] = u;
+                            a[top - e].qb = q.qe;
                         }
                         __syncwarp();
                         p = a[i];
+                        next = top - e - 1;
+                        again = true;
                     }
                 }
+                __syncwarp();
+                ended = next < 0;
+                top = next;
             }
         }
         __syncwarp();
-        if (lane == 0) {                                 // bwamem.c:475-492
+        if (few) {                                       // bwamem.c:475-492
+            // the regions in order: a's, or where the scan had nothing to do the given ones through S.order
+            const bsb_reg_t *const from_regs = near ? a : a_in;
+            int m = 0, first_reg = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = lane + 32 * h, c = k >= n ? 0 : near ? k : S.order[k];
+                if (h == 0) first_reg = __shfl_sync(BSB_FULL_MASK, c, 0);
+                const bool keep = k < n && from_regs[c].qe > from_regs[c].qb;
+                const unsigned km = __ballot_sync(BSB_FULL_MASK, keep);
+                if (keep) S.order[m + __popc(km & ((1u << lane) - 1u))] = c;
+                m += __popc(km);
+            }
+            __syncwarp();
+            int cnt = 1;
+            if (m == 0) {                                // the reference then returns its first region
+                if (lane == 0) S.order[0] = first_reg;
+                __syncwarp();
+                copy_regs(dst, from_regs, S.order, 1, !near, lane);
+            } else {
+                // by (score down, rb up, qb up); identical ones once
+                int sc[2], qb[2], less[2] = {0, 0};
+                int64_t rb[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const bsb_reg_t &x = from_regs[S.order[lane + 32 * h < m ? lane + 32 * h : 0]];
+                    sc[h] = x.score, rb[h] = x.rb, qb[h] = x.qb;
+                }
+                for (int e = 0; e < m; ++e) {
+                    const int es = __shfl_sync(BSB_FULL_MASK, e < 32 ? sc[0] : sc[1], e & 31);
+                    const int eq = __shfl_sync(BSB_FULL_MASK, e < 32 ? qb[0] : qb[1], e & 31);
+                    const int64_t er = __shfl_sync(BSB_FULL_MASK, e < 32 ? rb[0] : rb[1], e & 31);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        less[h] += es > sc[h] || (es == sc[h] && (er < rb[h] || (er == rb[h] && eq < qb[h])));
+                }
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (lane + 32 * h < m) S.weight[lane + 32 * h] = -less[h];
+                __syncwarp();
+                if (m > 1) sort_places(S.order, S.weight, m, lane);
+                cnt = 0;
+                int at[2], from[2];
+                bool out_[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = lane + 32 * h;
+                    out_[h] = k < m && (k == 0 || S.weight[k] != S.weight[k - 1]);
+                    from[h] = k < m ? S.order[k] : 0;
+                    const unsigned om = __ballot_sync(BSB_FULL_MASK, out_[h]);
+                    at[h] = cnt + __popc(om & ((1u << lane) - 1u));
+                    cnt += __popc(om);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (out_[h]) S.order[at[h]] = from[h];
+                __syncwarp();
+                copy_regs(dst, from_regs, S.order, cnt, !near, lane);
+            }
+            if (lane == 0) n_out[r] = cnt;
+            __syncwarp();
+            continue;
+        }
+        if (lane == 0) {
             int m = 0;
             for (int k = 0; k < n; ++k)
                 if (a[k].qe > a[k].qb) ix[m++] = k;
@@ -2407,8 +2573,8 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
         int *n_kept = (int *)(A + o_dn);
         int64_t *kept_off = (int64_t *)(A + o_doff);
         const int db = (int)((n_reads + kDedupWarps - 1) / kDedupWarps);
-        dedup_kernel<<<db < ctx->n_sm * 8 ? db : ctx->n_sm * 8, kDedupWarps * 32, 0, st>>>(
-            D, B, n_reads, d_reads, d_read_off, reg_off, regs_out, dtmp, iwork, regs, n_kept);
+        dedup_kernel<<<db, kDedupWarps * 32, kDedupWarps * dedup_warp_bytes(max_len), st>>>(
+            D, B, n_reads, d_reads, d_read_off, reg_off, regs_out, dtmp, iwork, regs, n_kept, max_len);
         if ((rc = bsb_cuda(ctx, scan_i32_i64(n_kept, n_reads, kept_off, scan_tmp, st), "kept offsets"))) return rc;
         compact_kept<<<cgrid, 128, 0, st>>>(regs, reg_off, n_reads, n_kept, kept_off, regs_out);
         reg_off = kept_off;

@@ -105,3 +105,25 @@ def test_large_batches_equal_small_ones(loaded, changes):
         part, poff = seed.align_regs(ctx, seqs[offs[lo]:offs[hi]], offs[lo:hi + 1] - offs[lo], opt)
         assert np.array_equal(roff[lo:hi + 1] - roff[lo], poff)
         assert regs[roff[lo]:roff[hi]].tobytes() == part.tobytes()
+
+
+@pytest.mark.parametrize("redun,gap", [(0.95, 10000), (0.5, 10000), (0.95, 60)])
+def test_dedup_equals_the_oracle(loaded, redun, gap):
+    """mem_sort_dedup_patch on reads with one to more than 64 regions, many of them with equal ends or
+    equal scores and starts."""
+    ctx, bi = loaded
+    reads = make_reads(bi.pac_codes(), np.random.Generator(np.random.PCG64(13)))
+    offs = np.zeros(len(reads) + 1, np.int64)
+    offs[1:] = np.cumsum([len(r) for r in reads])
+    seqs = np.concatenate(reads)
+    opt = _lib.AlignOpt.bwa_defaults(max_chain_gap=gap)
+    oo = oracle.Opt.from_list([1, 4, 6, 1, 6, 1, 100, 100, 5, 5, 19, 500, 10, 20, gap])
+    opt.mask_level_redun = oo.mask_level_redun = redun
+    regs, roff = seed.align_regs(ctx, seqs, offs, opt)
+    n = np.diff(roff)
+    assert n.max() > 64 and (n == 1).any() and (n == 2).any()
+    want, woff = oracle.sort_dedup_batch(oo, bi.l_pac, bi.pac, seqs, offs, regs, roff)
+    got, goff = seed.align_regs(ctx, seqs, offs, opt, dedup=True)
+    assert np.array_equal(goff, woff)
+    for f in want.dtype.names:
+        assert np.array_equal(got[f], want[f]), f"reg.{f}"
