@@ -333,7 +333,9 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     constexpr int kLenBins = 64, kKeys8 = kPackMaxSeg8 * kLenBins, kKeys16 = kPackMaxSeg16 * kLenBins;
     const bool w16_ok = S.o_del + S.e_del <= 32767 && S.o_ins + S.e_ins <= 32767;
     // the packed passes read F in closed form, which needs oe_ins >= e_ins as the lanes hold them
-    const bool b8_ok = (uint8_t)(S.o_ins + S.e_ins) >= (uint8_t)S.e_ins;
+    // (and byte lanes a matrix entry <= 0, see sw_pack.cuh)
+    const bool b8_ok = (uint8_t)(S.o_ins + S.e_ins) >= (uint8_t)S.e_ins &&
+                       *std::min_element(S.mat, S.mat + 25) <= 0;
     std::vector<int64_t> boff((size_t)n);
     std::vector<int32_t> key((size_t)n);
     std::vector<int32_t> lists((size_t)n);
@@ -377,28 +379,26 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     S.slen8 = std::max(1, (max8 + 15) / 16), S.slen16 = std::max(1, (max16 + 7) / 8);
     PackParams P8, P16;
     {
-        const uint8_t sh = (uint8_t)S.shift;
         for (int tc = 0; tc < 5; ++tc) {
-            uint8_t b[8], w[8];
-            for (int qc = 0; qc < 5; ++qc) {               // ksw_qinit (ksw.c:80-95)
-                b[qc] = (uint8_t)(p->mat[tc * 5 + qc] + sh);
-                w[qc] = (uint8_t)p->mat[tc * 5 + qc];
-            }
-            b[5] = sh, w[5] = 0;                           // the padding column: score 0
-            P8.plo[tc] = (uint32_t)b[0] | (uint32_t)b[1] << 8 | (uint32_t)b[2] << 16 | (uint32_t)b[3] << 24;
-            P8.phi[tc] = (uint32_t)b[4] | (uint32_t)b[5] << 8;
-            P16.plo[tc] = (uint32_t)w[0] | (uint32_t)w[1] << 8 | (uint32_t)w[2] << 16 | (uint32_t)w[3] << 24;
-            P16.phi[tc] = (uint32_t)w[4];
+            uint8_t w[5];
+            for (int qc = 0; qc < 5; ++qc) w[qc] = (uint8_t)p->mat[tc * 5 + qc];       // ksw_qinit (ksw.c:80-95)
+            P8.prof[tc] = make_uint2((uint32_t)w[0] | (uint32_t)w[1] << 8 | (uint32_t)w[2] << 16 | (uint32_t)w[3] << 24,
+                                     (uint32_t)w[4]);
+            P16.prof[tc] = P8.prof[tc];
         }
-        // the penalties as _mm_set1_epi8 / _mm_set1_epi16 broadcast them, negated in both halves
-        P8.nshift = neg2(S.shift);
-        P8.npe_del = neg2((uint8_t)S.e_del), P8.npoe_del = neg2((uint8_t)(S.o_del + S.e_del));
-        P8.npe_ins = neg2((uint8_t)S.e_ins), P8.npoe_ins = neg2((uint8_t)(S.o_ins + S.e_ins));
-        P8.shift = S.shift, P8.qmax = S.qmax, P8.pe_ins = (uint8_t)S.e_ins;
-        P16.nshift = 0;
-        P16.npe_del = neg2(std::min(S.e_del, 32767)), P16.npoe_del = neg2(std::min(S.o_del + S.e_del, 32767));
-        P16.npe_ins = neg2(std::min(S.e_ins, 32767)), P16.npoe_ins = neg2(std::min(S.o_ins + S.e_ins, 32767));
-        P16.shift = 0, P16.qmax = S.qmax, P16.pe_ins = std::min(S.e_ins, 32767);
+        P8.prof[5] = P16.prof[5] = make_uint2(0u, 0u);
+        // the penalties as _mm_set1_epi8 / _mm_set1_epi16 broadcast them, negated in both halves.  Word lanes: no
+        // H is above 32640, so a penalty beyond what leaves anything is as good as one that just leaves nothing,
+        // and no sum of pack_pass leaves 16 bits
+        const auto set = [](PackParams &Q, int e_del, int oe_del, int e_ins, int oe_ins) {
+            Q.npe_del = neg2(e_del), Q.npoe_del = neg2(oe_del), Q.npe_ins = neg2(e_ins), Q.npoe_ins = neg2(oe_ins);
+            Q.pe_ins = e_ins;
+        };
+        set(P8, (uint8_t)S.e_del, (uint8_t)(S.o_del + S.e_del), (uint8_t)S.e_ins, (uint8_t)(S.o_ins + S.e_ins));
+        const int od = std::min(S.o_del + S.e_del, 32640), oi = std::min(S.o_ins + S.e_ins, 32640);
+        set(P16, std::min(S.e_del, 32640 - od), od, std::min(S.e_ins, 32640 - oi), oi);
+        P8.shift = S.shift, P8.qmax = S.qmax;
+        P16.shift = 0, P16.qmax = S.qmax;
     }
     int rc;
     if ((rc = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice"))) return rc;

@@ -5,17 +5,17 @@
 // lanes, column j + l*slen in lane l of segment j; F carried along a lane's stripe in the first
 // pass, E and the row maximum taken from that pass, the lazy-F loop fixing H for the next row).
 // Here thread t of a group of P/2 plays SIMD lanes t (low 16 bits) and t + P/2 (high 16 bits):
-//   P = 16, byte lanes (ksw_u8): values 0..255 never leave 16 bits, so _mm_adds_epu8 is
-//     min(a + b, 255) (__viaddmin_s16x2), _mm_subs_epu8 is max(a - b, 0) (__viaddmax_s16x2 of a
-//     negated b), _mm_max_epu8 is __vimax_s16x2_relu (every value is non-negative);
-//   P = 8, word lanes (ksw_i16): the same instructions with signed scores, for jobs whose scores
+//   P = 16, byte lanes (ksw_u8), for matrices with an entry <= 0: then shift = -min, and a score that the
+//     reference's bytes would clip puts the row's maximum at 255 - shift or above, where the pass ends with
+//     score 255 whatever the rest of the row holds.  So signed scores in 16 bits, without a clip, are exact;
+//   P = 8, word lanes (ksw_i16): the same instructions, for jobs whose scores
 //     cannot reach the reference's 16-bit saturation (qlen * max score <= 32640) and whose
 //     penalties stay below 32768, so that 16-bit arithmetic without saturation is exact.
 // A job's H and E vectors and its query-profile selectors are register arrays sized by its
 // segment count's bucket (below); the row's scores come from two profile words of its
 // target base by one byte permute per pair of cells.  The lazy-F loop runs in closed form (see
-// pack_pass).  The groups of a warp take consecutive jobs of a list sorted by segment count, so
-// they run the same code for about as many rows.
+// pack_pass).  The groups of a warp take consecutive jobs of a list sorted by segment count and go through
+// their rows in step, so that every exchange and vote is the whole warp's.
 #pragma once
 
 #include <cstdint>
@@ -37,10 +37,9 @@ struct PassOut {
 };
 
 struct PackParams {
-    // per target base: the scores of query bases 0..3 (plo), of base 4, the padding column (score
-    // 0) and zero (phi).  Byte lanes: biased, (uint8)(mat + shift); word lanes: signed bytes.
-    uint32_t plo[5], phi[5];
-    uint32_t nshift;                                       // byte lanes: -shift in both halves
+    // per target base: the scores of query bases 0..3 (x), and of base 4 and the padding column, whose
+    // score is 0 (y), as signed bytes; the last for rows past a target's end: every score 0
+    uint2 prof[6];
     uint32_t npe_del, npoe_del, npe_ins, npoe_ins;         // negated penalties in both halves
     int shift, qmax, pe_ins;
 };
@@ -63,28 +62,29 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)  
 
 __host__ __device__ __forceinline__ uint32_t neg2(int v) { return (uint32_t)(uint16_t)(-v) * 0x10001u; }
 
+constexpr unsigned kAll = 0xffffffffu;
+
 template <int G>
-__device__ __forceinline__ uint32_t lane_up(uint32_t x, int tid, unsigned gm)   // _mm_slli_si128 by one lane
+__device__ __forceinline__ uint32_t lane_up(uint32_t x, int tid)   // _mm_slli_si128 by one lane
 {
-    const uint32_t r = __shfl_sync(gm, x, (tid + G - 1) & (G - 1), G);
-    return tid ? r : r << 16;
+    const uint32_t r = __shfl_sync(kAll, x, (tid + G - 1) & (G - 1), G);
+    return prmt(r, 0u, tid ? 0x3210u : 0x1044u);
 }
 
-// maximum / minimum over the group's threads (G of them): a segmented butterfly, since a
-// reduction with per-group member masks is carried out one mask at a time
+// maximum / minimum over the group's threads (G of them)
 template <int G>
-__device__ __forceinline__ int grp_max(unsigned gm, int v)
+__device__ __forceinline__ int grp_max(int v)
 {
 #pragma unroll
-    for (int d = G / 2; d > 0; d >>= 1) v = max(v, __shfl_xor_sync(gm, v, d, G));
+    for (int d = G / 2; d > 0; d >>= 1) v = max(v, __shfl_xor_sync(kAll, v, d, G));
     return v;
 }
 
 template <int G>
-__device__ __forceinline__ int grp_min(unsigned gm, int v)
+__device__ __forceinline__ int grp_min(int v)
 {
 #pragma unroll
-    for (int d = G / 2; d > 0; d >>= 1) v = min(v, __shfl_xor_sync(gm, v, d, G));
+    for (int d = G / 2; d > 0; d >>= 1) v = min(v, __shfl_xor_sync(kAll, v, d, G));
     return v;
 }
 
@@ -96,153 +96,194 @@ __device__ __forceinline__ int grp_min(unsigned gm, int v)
 template <int P>
 constexpr int kSegBucket = P == 16 ? 2 : 8;
 
-// One ksw_u8 (P = 16) or ksw_i16 (P = 8) pass of a group of P/2 threads on sl segments,
-// SLMAX - kSegBucket < sl <= SLMAX.  hm: the thread's Hmax slots (stride kPackBlock); bbuf: the
-// suboptimal rows (KSW_XSUBO only).
+// The ksw_u8 (P = 16) or ksw_i16 (P = 8) passes of a warp's groups of P/2 threads, each on its own job of sl
+// segments, SLMAX - kSegBucket < sl <= SLMAX (a group without one: qlen = tlen = 0).  hm: the thread's Hmax slots
+// (stride kPackBlock); bbuf: the suboptimal rows (KSW_XSUBO only).
+//
+// Bound by the integer pipe, which takes a warp's instruction every second clock (81 % busy, 117 of its
+// instructions a row of 10 segments).  Hence: no clip and no relu that another instruction implies (7 instructions
+// a segment, 9 before); the groups in step, since an exchange or vote under a group's own mask is carried out
+// group by group with a synchronisation each (40 instructions a row went there); the row's maximum only compared,
+// and reduced where it matters; and registers for the widest instance without spills (4 blocks an SM; at 5, 6 and 7
+// the call below takes 2.08, 2.21 and 2.31 ms).  40k mates of 30-250 bases against 500-base windows, forward
+// passes: 1.76 ms before, 1.22 now, the word-lane mates beside them 1.21 and 0.80; the call 2.72 and 2.00.
 template <int P, int SLMAX>
-__device__ __noinline__ PassOut pack_pass(const PackParams &S, const uint32_t *plo, const uint32_t *phi, int sl,
-                                          int qlen, int tlen, const SwSeq &a, int xtra, uint32_t *hm, int2 *bbuf,
-                                          int tid, unsigned gm)
+__device__ __noinline__ PassOut pack_pass(const PackParams &S, const uint2 *prof, int sl, int qlen, int tlen,
+                                          const SwSeq &a, int xtra, uint32_t *hm, int2 *bbuf, int tid)
 {
     constexpr bool U8 = P == 16;
     constexpr int G = P / 2, SLMIN = SLMAX - kSegBucket<P> + 1;    // segments below SLMIN always exist
-    const uint32_t nshift = S.nshift, npe_del = S.npe_del, npoe_del = S.npoe_del, npe_ins = S.npe_ins,
-                   npoe_ins = S.npoe_ins;
+    const uint32_t npe_del = S.npe_del, npoe_del = S.npoe_del, npe_ins = S.npe_ins, npoe_ins = S.npoe_ins;
+    const uint32_t oe_ins = neg2((int)(int16_t)(npoe_ins & 0xffffu));
     const int shift = S.shift, pe_ins = S.pe_ins;
+    const uint32_t npe_one = 0u - (uint32_t)pe_ins * 0x10001u;     // one e_ins less in both halves of -j * e_ins, j >= 1
     uint32_t sel[SLMAX], H[SLMAX], E[SLMAX];
 #pragma unroll
     for (int j = 0; j < SLMAX; ++j) {              // ksw_qinit's striping; the vectors start at zero
         const int c0 = j + tid * sl, c1 = j + (tid + G) * sl;
         const bool in = j < sl;
         const uint32_t x = in && c0 < qlen ? (uint32_t)a.qc(c0) : 5u, y = in && c1 < qlen ? (uint32_t)a.qc(c1) : 5u;
-        // bytes: score(x), 0 or its sign, score(y), 0 or its sign
-        sel[j] = U8 ? (x | 0x60u | y << 8 | 0x6000u) : (x | (x | 8u) << 4 | y << 8 | (y | 8u) << 12);
+        sel[j] = x | (x | 8u) << 4 | y << 8 | (y | 8u) << 12;      // bytes: score(x), its sign, score(y), its sign
         H[j] = 0, E[j] = 0;
         hm[j * kPackBlock] = 0;
     }
     const int minsc = (xtra & kXSubo) ? xtra & 0xffff : 0x10000;
     const int endsc = (xtra & kXStop) ? xtra & 0xffff : 0x10000;
     int gmax = 0, te = -1, n_b = 0, last_row = -2, last_sc = 0;
-    int tc = tlen > 0 ? a.tc(0) : 0;
+    // rows whose maximum is above lim (in both halves) are looked at: min(gmax, minsc - 1)
+    const int low = min(minsc, 0x8000) - 1;
+    uint32_t lim = (uint32_t)(uint16_t)min(gmax, low) * 0x10001u;
     uint32_t hlast = 0;                            // H of segment sl - 1 in the previous row
-    for (int i = 0; i < tlen; ++i) {
-        const int tn = i + 1 < tlen ? a.tc(i + 1) : 0;
-        const uint32_t xlo = plo[tc], xhi = phi[tc];
-        uint32_t h = lane_up<G>(hlast, tid, gm), f = 0, mx = 0;          // H(i-1, -1), ksw.c:141-142
-        // H = max(a, E, f), a = the diagonal plus the score (ksw.c:149-153); the next f is
-        // max(relu(f - e_ins), relu(H - oe_ins)) = max(relu(f - e_ins), relu(max(a, E) - oe_ins)), as
-        // relu(f - oe_ins) <= relu(f - e_ins): one instruction per segment on the f chain
+    // the lazy F's scan: what a lane's G loses on the way o lanes up (a thread without a lane there: all of it),
+    // and from the last low lane to this thread's high one
+    const int d = pe_ins * sl;
+    uint32_t up[3];
 #pragma unroll
-        for (int j = 0; j < SLMAX; ++j)
-            if (j < SLMIN || j < sl) {
-                const uint32_t s = prmt(xlo, xhi, sel[j]);
-                const uint32_t ae = U8 ? __viaddmax_s16x2(__viaddmin_s16x2(h, s, 0x00ff00ffu), nshift, E[j])
-                                       : __viaddmax_s16x2(h, s, E[j]);
-                const uint32_t fo = __viaddmax_s16x2(ae, npoe_ins, 0u);
-                const uint32_t hv = __vimax_s16x2_relu(ae, f);
-                f = __viaddmax_s16x2(f, npe_ins, fo);
-                mx = __vimax_s16x2_relu(mx, hv);
-                E[j] = __viaddmax_s16x2(E[j], npe_del, __viaddmax_s16x2(hv, npoe_del, 0u));
-                h = H[j];
-                H[j] = hv;
-            }
-        {   // lazy F (ksw.c:166-177, 284-295).  The reference shifts f up one lane per round and
-            // sweeps the segments until no lane can raise an H any more.  The sweep raises H(l, j)
-            // to relu(G(l) - j*e_ins) at most, where G(l) is the F arriving at lane l's first
-            // column: G(0) = 0, G(l) = max(x(l), relu(G(l-1) - sl*e_ins)), x(l) the f leaving lane
-            // l-1; its early exit (Farrar's) leaves out only updates that change nothing.  So: the
-            // reference's own first test, and where a lane fails it, G as a max-plus scan over the
-            // lanes (the group's threads, then the low lanes into the high ones) and one max per
-            // segment, without a vote per segment.  (Segments past sl take values nothing reads.)
-            const uint32_t x = lane_up<G>(f, tid, gm);
-            const uint32_t h0 = __vimax_s16x2_relu(H[0], x);
-            const uint32_t hh = __viaddmax_s16x2(h0, npoe_ins, 0u), fn = __viaddmax_s16x2(x, npe_ins, 0u);
-            if (__any_sync(gm, __vimax_s16x2_relu(fn, hh) != hh)) {
-                const int d = pe_ins * sl;
-                uint32_t g = x;
+    for (int o = 1, k = 0; o < G; o <<= 1, ++k) up[k] = tid >= o ? neg2(min(o * d, 32767)) : 0x80008000u;
+    const uint32_t low_up = neg2(min(d * (tid + 1), 32767)) & 0xffff0000u;
+    const unsigned my_group = ((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+    int tmax = __reduce_max_sync(kAll, tlen);
+    int tb = tid < tlen ? a.tc(tid) : 5;           // a row's base, one a thread for G rows
+    uint2 pr = prof[__shfl_sync(kAll, tb, 0, G)];
+    int i = 0;
+    while (i < tmax) {
+        int tn = i + G + tid < tlen ? a.tc(i + G + tid) : 5;
+#pragma unroll 1
+        for (int r = 0; r < G && i < tmax; ++r, ++i) {
+            const uint32_t xlo = pr.x, xhi = pr.y;
+            pr = prof[__shfl_sync(kAll, r + 1 < G ? tb : tn, (r + 1) & (G - 1), G)];
+            uint32_t h = lane_up<G>(hlast, tid), F = oe_ins, mx = 0;     // H(i-1, -1), ksw.c:141-142
+            // H = max(a, E, f), a = the diagonal plus the score (ksw.c:149-153); the next f is
+            // max(relu(f - e_ins), relu(H - oe_ins)) = relu(max(f - e_ins, max(a, E) - oe_ins)), as
+            // relu(f - oe_ins) <= relu(f - e_ins).  F = f + oe_ins, not held at zero (H is): one instruction a
+            // segment, and one for H
 #pragma unroll
-                for (int o = 1; o < G; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(gm, g, o, G);
-                    if (tid >= o) g = __viaddmax_s16x2(v, neg2(min(o * d, 32767)), g);
+            for (int j = 0; j < SLMAX; ++j)
+                if (j < SLMIN || j < sl) {
+                    const uint32_t ae = __viaddmax_s16x2(h, prmt(xlo, xhi, sel[j]), E[j]);
+                    const uint32_t hv = __viaddmax_s16x2_relu(F, npoe_ins, ae);
+                    F = __viaddmax_s16x2(F, npe_ins, ae);
+                    if (j < SLMIN && (j & 1)) mx = __vimax3_s16x2_relu(mx, hv, H[j - 1]);
+                    else if (j >= SLMIN - (SLMIN & 1)) mx = __vimax_s16x2_relu(mx, hv);
+                    E[j] = __viaddmax_s16x2(E[j], npe_del, __viaddmax_s16x2(hv, npoe_del, 0u));
+                    h = H[j];
+                    H[j] = hv;
                 }
-                const int gl = (int)(__shfl_sync(gm, g, G - 1, G) & 0xffffu);
-                g = __vimax_s16x2_relu(g, (uint32_t)max(gl - d * (tid + 1), 0) << 16);
-#pragma unroll
-                for (int j = 0; j < SLMAX; ++j) {
-                    H[j] = __vimax_s16x2_relu(H[j], g);
-                    g = __viaddmax_s16x2(g, npe_ins, 0u);
-                }
-            } else {
+            {   // lazy F (ksw.c:166-177, 284-295).  The reference shifts f up one lane per round and
+                // sweeps the segments until no lane can raise an H any more.  The sweep raises H(l, j)
+                // to relu(G(l) - j*e_ins) at most, where G(l) is the F arriving at lane l's first
+                // column: G(0) = 0, G(l) = max(x(l), relu(G(l-1) - sl*e_ins)), x(l) the f leaving lane
+                // l-1; its early exit (Farrar's) leaves out only updates that change nothing.  So: the
+                // reference's own first test, and where a lane fails it, G as a max-plus scan over its group's
+                // lanes (the group's threads, then the low lanes into the high ones) and one max per
+                // segment, without a vote per segment.  (Segments past sl take values nothing reads.)
+                const uint32_t x = lane_up<G>(__viaddmax_s16x2(F, npoe_ins, 0u), tid);
+                const uint32_t h0 = __vimax_s16x2_relu(H[0], x);
+                const uint32_t hh = __viaddmax_s16x2(h0, npoe_ins, 0u), fn = __viaddmax_s16x2(x, npe_ins, 0u);
                 H[0] = h0;
-            }
-        }
-        hlast = H[SLMIN - 1];
+                const unsigned fail = __ballot_sync(kAll, __vimax_s16x2_relu(fn, hh) != hh);
+                if (fail) {
+                    uint32_t g = x;
 #pragma unroll
-        for (int j = SLMIN; j < SLMAX; ++j)
-            if (j == sl - 1) hlast = H[j];
-        const int imax = grp_max<G>(gm, max((int)(mx & 0xffffu), (int)(mx >> 16)));
-        if (imax > gmax || imax >= minsc) {
-            if (imax >= minsc) {                  // the rows of the suboptimal score (ksw.c:182-189)
-                if (n_b == 0 || last_row + 1 != i) {
-                    if (tid == 0) bbuf[n_b] = make_int2(imax, i);
-                    ++n_b, last_row = i, last_sc = imax;
-                } else if (last_sc < imax) {
-                    if (tid == 0) bbuf[n_b - 1] = make_int2(imax, i);
-                    last_row = i, last_sc = imax;
+                    for (int o = 1, k = 0; o < G; o <<= 1, ++k)
+                        g = __viaddmax_s16x2(__shfl_up_sync(kAll, g, o, G), up[k], g);
+                    g = __viaddmax_s16x2(__shfl_sync(kAll, g, G - 1, G) << 16, low_up, g);
+                    if (!(fail & my_group)) g = 0;       // a group without a failing lane keeps its H as they are
+                    H[0] = __vimax_s16x2_relu(H[0], g);
+                    if (U8) {                            // at most 15 * 255 down
+                        uint32_t down = npe_ins;
+#pragma unroll
+                        for (int j = 1; j < SLMAX; ++j) {
+                            H[j] = __viaddmax_s16x2(g, down, H[j]);
+                            down += npe_one;
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 1; j < SLMAX; ++j) {
+                            g = __viaddmax_s16x2(g, npe_ins, 0u);
+                            H[j] = __vimax_s16x2_relu(H[j], g);
+                        }
+                    }
                 }
             }
-            if (imax > gmax) {
-                gmax = imax, te = i;
+            hlast = H[SLMIN - 1];
 #pragma unroll
-                for (int j = 0; j < SLMAX; ++j) hm[j * kPackBlock] = H[j];
-                if ((U8 && gmax + shift >= 255) || gmax >= endsc) break;
+            for (int j = SLMIN; j < SLMAX; ++j)
+                if (j == sl - 1) hlast = H[j];
+            if (__any_sync(kAll, __viaddmax_s16x2(mx, 0u, lim) != lim)) {
+#pragma unroll
+                for (int d = G / 2; d > 0; d >>= 1) mx = __vimax_s16x2_relu(mx, __shfl_xor_sync(kAll, mx, d, G));
+                const int imax = max((int)(mx & 0xffffu), (int)(mx >> 16));
+                bool ends = false;
+                if (i < tlen) {
+                    if (imax >= minsc) {              // the rows of the suboptimal score (ksw.c:182-189)
+                        if (n_b == 0 || last_row + 1 != i) {
+                            if (tid == 0) bbuf[n_b] = make_int2(imax, i);
+                            ++n_b, last_row = i, last_sc = imax;
+                        } else if (last_sc < imax) {
+                            if (tid == 0) bbuf[n_b - 1] = make_int2(imax, i);
+                            last_row = i, last_sc = imax;
+                        }
+                    }
+                    if (imax > gmax) {
+                        gmax = imax, te = i;
+                        lim = (uint32_t)(uint16_t)min(gmax, low) * 0x10001u;
+#pragma unroll
+                        for (int j = 0; j < SLMAX; ++j) hm[j * kPackBlock] = H[j];
+                        ends = (U8 && gmax + shift >= 255) || gmax >= endsc;
+                    }
+                } else {                             // past this group's target
+                    lim = 0x7fff7fffu;
+                }
+                if (ends) tlen = i + 1, tb = tn = 5;
+                if (__any_sync(kAll, ends)) tmax = __reduce_max_sync(kAll, tlen);
             }
         }
-        tc = tn;
+        tb = tn;
     }
-    __syncwarp(gm);
+    __syncwarp();
     PassOut r;
     r.score = U8 ? (gmax + shift < 255 ? gmax : 255) : gmax;
     r.te = te, r.qe = -1, r.score2 = -1, r.te2 = -1;
-    if (!U8 || r.score != 255) {
-        int best = -1, col = 0x7fffffff;          // the smallest column holding the best Hmax value
+    const bool whole = !U8 || r.score != 255;
+    int best = -1, col = 0x7fffffff;              // the smallest column holding the best Hmax value
 #pragma unroll 1
-        for (int j = 0; j < sl; ++j) {
-            const uint32_t v = hm[j * kPackBlock];
-            const int v0 = (int)(v & 0xffffu), v1 = (int)(v >> 16), c0 = j + tid * sl, c1 = j + (tid + G) * sl;
-            if (v0 > best || (v0 == best && c0 < col)) best = v0, col = c0;
-            if (v1 > best || (v1 == best && c1 < col)) best = v1, col = c1;
-        }
-        const int gbest = grp_max<G>(gm, best);
-        r.qe = grp_min<G>(gm, best == gbest ? col : 0x7fffffff);
-        if (n_b) {                                 // ksw.c:218-225: the best row outside te +- d
-            const int d = (r.score + S.qmax - 1) / S.qmax, low = te - d, high = te + d;
-            int bs = -1, bk = 0x7fffffff;
+    for (int j = 0; j < sl; ++j) {
+        const uint32_t v = hm[j * kPackBlock];
+        const int v0 = (int)(v & 0xffffu), v1 = (int)(v >> 16), c0 = j + tid * sl, c1 = j + (tid + G) * sl;
+        if (v0 > best || (v0 == best && c0 < col)) best = v0, col = c0;
+        if (v1 > best || (v1 == best && c1 < col)) best = v1, col = c1;
+    }
+    __syncwarp();
+    const int gbest = grp_max<G>(best), qe = grp_min<G>(best == gbest ? col : 0x7fffffff);
+    if (whole) r.qe = qe;
+    if (__any_sync(kAll, n_b != 0)) {              // ksw.c:218-225: the best row outside te +- d
+        const int reach = (r.score + S.qmax - 1) / S.qmax, lo = te - reach, hi = te + reach;
+        int bs = -1, bk = 0x7fffffff;
 #pragma unroll 1
-            for (int k = tid; k < n_b; k += G) {
-                const int2 e = bbuf[k];
-                if ((e.y < low || e.y > high) && e.x > bs) bs = e.x, bk = k;
-            }
-            const int gbs = grp_max<G>(gm, bs);
-            const int gk = grp_min<G>(gm, bs == gbs ? bk : 0x7fffffff);
-            if (gbs > r.score2 && gk != 0x7fffffff) r.score2 = gbs, r.te2 = bbuf[gk].y;
+        for (int k = tid; k < n_b; k += G) {
+            const int2 e = bbuf[k];
+            if ((e.y < lo || e.y > hi) && e.x > bs) bs = e.x, bk = k;
         }
+        __syncwarp();
+        const int gbs = grp_max<G>(bs);
+        const int gk = grp_min<G>(bs == gbs ? bk : 0x7fffffff);
+        if (whole && n_b && gbs > r.score2 && gk != 0x7fffffff) r.score2 = gbs, r.te2 = bbuf[gk].y;
     }
     return r;
 }
 
-// pack_pass of the bucket holding sl, for buckets ending at SLMAX..HI (step kSegBucket<P>).
-// Each instance is a function of its own, so a kernel's registers are those of its largest.
+// pack_pass of the bucket ending at hi (the same in the whole warp), for buckets ending at SLMAX..HI (step
+// kSegBucket<P>).  Each instance is a function of its own, so a kernel's registers are those of its largest.
 template <int P, int SLMAX, int HI>
-__device__ __forceinline__ PassOut pack_range(int sl, const PackParams &S, const uint32_t *plo, const uint32_t *phi,
-                                              int qlen, int tlen, const SwSeq &a, int xtra, uint32_t *hm, int2 *bbuf,
-                                              int tid, unsigned gm)
+__device__ __forceinline__ PassOut pack_range(int hi, const PackParams &S, const uint2 *prof, int sl, int qlen,
+                                              int tlen, const SwSeq &a, int xtra, uint32_t *hm, int2 *bbuf, int tid)
 {
     if constexpr (SLMAX >= HI) {
-        return pack_pass<P, HI>(S, plo, phi, sl, qlen, tlen, a, xtra, hm, bbuf, tid, gm);
+        return pack_pass<P, HI>(S, prof, sl, qlen, tlen, a, xtra, hm, bbuf, tid);
     } else {
-        if (sl <= SLMAX) return pack_pass<P, SLMAX>(S, plo, phi, sl, qlen, tlen, a, xtra, hm, bbuf, tid, gm);
-        return pack_range<P, SLMAX + kSegBucket<P>, HI>(sl, S, plo, phi, qlen, tlen, a, xtra, hm, bbuf, tid, gm);
+        if (hi <= SLMAX) return pack_pass<P, SLMAX>(S, prof, sl, qlen, tlen, a, xtra, hm, bbuf, tid);
+        return pack_range<P, SLMAX + kSegBucket<P>, HI>(hi, S, prof, sl, qlen, tlen, a, xtra, hm, bbuf, tid);
     }
 }
 
@@ -253,18 +294,18 @@ __device__ __forceinline__ PassOut pack_range(int sl, const PackParams &S, const
 // sw_rev_scatter) whose reversed query has LO..HI segments, completing tb and qb.  Each warp
 // takes 64/P consecutive jobs of its list at a time; q is the queue counter.
 template <int P, bool REV, int LO, int HI, int MAXS>
-__global__ void __launch_bounds__(kPackBlock, P == 16 ? 6 : 1)
+__global__ void __launch_bounds__(kPackBlock, P == 16 ? 4 : 1)
 sw_pack_kernel(PackParams S, const bsb_sw_job_t *__restrict__ jobs, const uint8_t *__restrict__ seq,
                const int32_t *__restrict__ list, int n_fwd, const int64_t *__restrict__ boff,
                int2 *__restrict__ bscratch, bsb_kswr_t *__restrict__ out, uint8_t *__restrict__ rsl,
                int *__restrict__ ctr, int *__restrict__ q)
 {
-    constexpr int G = P / 2, NG = 32 / G;
+    constexpr int G = P / 2, NG = 32 / G, B = kSegBucket<P>;
     __shared__ uint32_t hmax_s[HI * kPackBlock];
-    __shared__ uint32_t plo[5], phi[5];
+    __shared__ uint2 prof[6];
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int c = 0; c < 5; ++c) plo[c] = S.plo[c], phi[c] = S.phi[c];
+        for (int c = 0; c < 6; ++c) prof[c] = S.prof[c];
     }
     __syncthreads();
     int total = n_fwd;
@@ -276,26 +317,40 @@ sw_pack_kernel(PackParams S, const bsb_sw_job_t *__restrict__ jobs, const uint8_
         list += skip;
     }
     const int wl = threadIdx.x & 31, g = wl / G, tid = wl % G;
-    const unsigned gm = ((1u << G) - 1) << (G * g);
     uint32_t *hm = hmax_s + threadIdx.x;
     for (;;) {
         int base = 0;
         if (wl == 0) base = atomicAdd(q, NG);
-        base = __shfl_sync(0xffffffffu, base, 0);
+        base = __shfl_sync(kAll, base, 0);
         if (base >= total) break;
         const int k = base + g;
+        int id = 0, left = 0, qlen = 0, tlen = 0, xtra = 0;        // left: the segments of a job still to be run
+        SwSeq a{seq, seq, -1, -1};
+        int2 *bbuf = nullptr;
+        bsb_kswr_t o{};
         if (k < total) {
-            const int id = list[k];
+            id = list[k];
             const bsb_sw_job_t jb = jobs[id];
-            const uint8_t *qp = seq + jb.qoff, *tp = seq + jb.toff;
+            a.q += jb.qoff, a.t += jb.toff;
+            tlen = jb.tlen;
             if (!REV) {
-                const SwSeq a{qp, tp, -1, -1};
-                constexpr int B0 = LO + kSegBucket<P> - 1;
-                const PassOut r = pack_range<P, B0, HI>((jb.qlen + P - 1) / P, S, plo, phi, jb.qlen, jb.tlen, a,
-                                                        jb.xtra, hm, bscratch + boff[id], tid, gm);
-                const bool start = (jb.xtra & kXStart) && !((jb.xtra & kXSubo) && r.score < (jb.xtra & 0xffff));
-                if (tid == 0) {
-                    bsb_kswr_t o;
+                qlen = jb.qlen, xtra = jb.xtra, bbuf = bscratch + boff[id];
+            } else {
+                o = out[id];
+                a.qe = o.qe, a.te = o.te;
+                qlen = o.qe + 1, xtra = kXStop | o.score;
+            }
+            left = (qlen + P - 1) / P;
+        }
+        // a list sorted by segment count gives a warp jobs of one bucket but at the buckets' borders
+        for (int top; (top = __reduce_max_sync(kAll, left)) > 0;) {
+            const int hi = LO + B - 1 + (top - LO) / B * B;
+            const bool mine = left > hi - B;
+            const PassOut r = pack_range<P, LO + B - 1, HI>(hi, S, prof, mine ? left : hi, mine ? qlen : 0,
+                                                            mine ? tlen : 0, a, mine ? xtra : 0, hm, bbuf, tid);
+            if (mine && tid == 0) {
+                if (!REV) {
+                    const bool start = (xtra & kXStart) && !((xtra & kXSubo) && r.score < (xtra & 0xffff));
                     o.score = r.score, o.te = r.te, o.qe = r.qe, o.score2 = r.score2, o.te2 = r.te2;
                     o.tb = -1, o.qb = -1;
                     out[id] = o;
@@ -303,15 +358,11 @@ sw_pack_kernel(PackParams S, const bsb_sw_job_t *__restrict__ jobs, const uint8_
                     const int sl = start && r.qe >= 0 ? (r.qe + P) / P : 0;
                     rsl[id] = (uint8_t)sl;
                     if (sl) atomicAdd(&ctr[kRcnt + sl], 1);
+                } else if (r.score == o.score) {
+                    out[id].tb = o.te - r.te, out[id].qb = o.qe - r.qe;
                 }
-            } else {
-                const bsb_kswr_t o = out[id];
-                const SwSeq a{qp, tp, o.qe, o.te};
-                constexpr int B0 = LO + kSegBucket<P> - 1;
-                const PassOut rr = pack_range<P, B0, HI>((o.qe + P) / P, S, plo, phi, o.qe + 1, jb.tlen, a,
-                                                         kXStop | o.score, hm, nullptr, tid, gm);
-                if (tid == 0 && rr.score == o.score) out[id].tb = o.te - rr.te, out[id].qb = o.qe - rr.qe;
             }
+            if (mine) left = 0;
         }
         __syncwarp();
     }
