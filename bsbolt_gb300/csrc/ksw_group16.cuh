@@ -180,23 +180,25 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                 }
             } else {
                 exhausted = true;
+                tlen = 0, tch = tnext = 0;
             }
         }
-        const unsigned act = __ballot_sync(0xffffffffu, have);
-        if (!act) break;
-        if (!have) continue;
+        __syncwarp();
+        if (!__any_sync(BSB_FULL_MASK, have)) break;
 
         // ---- one target row of this group's job (ksw.c:412-470); per-job decisions
-        // are selects or warp-uniform branches, as in ksw_group_run.
-        const int tc = (int)__shfl_sync(act, tch, i & (G - 1), G);
+        // are selects or warp-uniform branches, as in ksw_group_run.  A group that is out of jobs goes along
+        // on nothing, so that every exchange and vote is the whole warp's: under a mask known only at run
+        // time each of a row's twenty or so needs a synchronisation of its own.
+        const int tc = (int)__shfl_sync(BSB_FULL_MASK, tch, i & (G - 1), G);
         if ((i & (G - 1)) == G - 1) {
             tch = tnext;
             const int ti = i + G + 1 + gl;
-            tnext = ti < tlen ? t.base(P, ti) : 4u;
+            tnext = ti < tlen ? t.base(P, ti) : have ? 4u : 0u;
         }
-        const bool bump = beg < i - w;         // band edge (ksw.c:416-419)
+        const bool bump = have && beg < i - w;         // band edge (ksw.c:416-419)
         beg = bump ? i - w : beg;
-        if (__any_sync(act, bump)) {           // cells left of the band are kept at zero
+        if (__any_sync(BSB_FULL_MASK, bump)) {           // cells left of the band are kept at zero
             // |beg - base| <= 1023 and u < C2: the 16-bit differences below are exact
             const uint32_t tb = pk16(beg - base, beg - base - C2);
 #pragma unroll
@@ -217,7 +219,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         // minimum with H*16, which is >= H + score when H > 0 (scores <= 15).
         uint32_t Mv[C2];
         uint32_t local = 0;
-        if (!__any_sync(act, tc >= 4)) {
+        if (!__any_sync(BSB_FULL_MASK, tc >= 4)) {
             const uint32_t sel = sext2_same((uint32_t)tc);
 #pragma unroll
             for (int u = 0; u < C2; ++u) {
@@ -246,8 +248,8 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         int incl = f_lane;
 #pragma unroll
         for (int d = 1; d < G; d <<= 1)
-            incl = __viaddmax_s32(__shfl_up_sync(act, incl, d, G), -eC * d, incl);
-        const int excl = __shfl_up_sync(act, incl, 1, G);
+            incl = __viaddmax_s32(__shfl_up_sync(BSB_FULL_MASK, incl, d, G), -eC * d, incl);
+        const int excl = __shfl_up_sync(BSB_FULL_MASK, incl, 1, G);
         const int carry = gl == 0 ? 0 : excl;
 
         // pass 2: F (the recurrence F(i,j+1) = max(F(i,j) - e_ins, max(M - oe_ins, 0)) of
@@ -272,7 +274,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         else
             ksw16_pass2<C2, false>(Mv, Es, Hs, F, t_lt, ltm_prev, kmx, Hprev, nE0, lem0, nzw, ne_del, noe_del,
                                    ne_ins, noe_ins);
-        int Hleft = __shfl_up_sync(act, hi16(Hprev), 1, G);
+        int Hleft = __shfl_up_sync(BSB_FULL_MASK, hi16(Hprev), 1, G);
         if (gl == 0) Hleft = h1_init;
         {
             const uint32_t nH = (pk16(Hleft, lo16(Hprev)) & lem0) | (Hs[0] & ~lem0);
@@ -285,13 +287,13 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         const int k_lo = lo16(kmx), k_hi = hi16(kmx);
         const int kmax = (k_hi >> 4) >= (k_lo >> 4) ? (k_hi >> 4) * 1024 + (k_hi & 15) + C2
                                                     : (k_lo >> 4) * 1024 + (k_lo & 15);
-        const int kw = group_max<G>(act, kmax + base);
+        const int kw = group_max<G>(BSB_FULL_MASK, kmax + base);
         const int m = kw >> 10, mj = kw & 1023;
         if (!empty) ncell += end - beg;
 
         // query end reached: eh[qlen].h == H(i, qlen-1), or h1 for an empty band at qlen (ksw.c:450-453)
         int hq = h1_init;
-        if (__any_sync(act, !empty && end == qlen)) {
+        if (__any_sync(BSB_FULL_MASK, have && !empty && end == qlen)) {
             // register qu by a select tree on its bits (C2 - 1 selects)
             const int qu = q_slot < C2 ? q_slot : q_slot - C2;
             uint32_t v[C2];
@@ -305,7 +307,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
             }
             const uint32_t wsel = v[0];
             const int hsel = q_slot < C2 ? lo16(wsel) : hi16(wsel);
-            const int h1 = __shfl_sync(act, hsel, q_lane, G);
+            const int h1 = __shfl_sync(BSB_FULL_MASK, hsel, q_lane, G);
             hq = empty ? hq : h1;
         }
         if (empty ? beg == qlen : end == qlen) {
@@ -314,7 +316,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         }
 
         // row maximum, z-drop (ksw.c:454-464)
-        const bool live = !empty && m != 0;
+        const bool live = have && !empty && m != 0;
         const bool up = live && m > best;
         const int di = i - best_i, dj = mj - best_j;
         const int drop = di > dj ? best - m - (di - dj) * e_del : best - m - (dj - di) * e_ins;
@@ -332,7 +334,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         if (!cells) {
             const int a = P.mat_max;
             const bool want = live && rows_may_be_done(gscore, m, mj, qlen, a);
-            if (__any_sync(act, want)) {
+            if (__any_sync(BSB_FULL_MASK, want)) {
                 uint32_t um = 0;
 #pragma unroll
                 for (int u = 0; u < C2; ++u) {
@@ -343,18 +345,18 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                 const int lo = lo16(um), hi = hi16(um);
                 const int U = max(lo > 0 ? lo + a * (qlen - base - C2 + 1) : 0,
                                   hi > 0 ? hi + a * (qlen - base - 2 * C2 + 1) : 0);
-                fin = group_max<G>(act, U) < gscore && want;
+                fin = group_max<G>(BSB_FULL_MASK, U) < gscore && want;
             }
         }
 
         // shrink to the non-zero cells (ksw.c:466-469), as in ksw_group_run
         int fnz, lnz;
         if constexpr (G == 32) {
-            fnz = __reduce_min_sync(act, nzb ? base + __ffs(nzb) - 1 : INT_MAX);
-            lnz = __reduce_max_sync(act, nzb ? base + 31 - __clz(nzb) : -1);
+            fnz = __reduce_min_sync(BSB_FULL_MASK, nzb ? base + __ffs(nzb) - 1 : INT_MAX);
+            lnz = __reduce_max_sync(BSB_FULL_MASK, nzb ? base + 31 - __clz(nzb) : -1);
         } else {
             const uint32_t pk = nzb ? (uint32_t)(2048 - base - __ffs(nzb)) << 16 | (uint32_t)(base + 32 - __clz(nzb)) : 0u;
-            const uint32_t r = group_max_u16x2<G>(act, pk);
+            const uint32_t r = group_max_u16x2<G>(BSB_FULL_MASK, pk);
             fnz = 2047 - (int)(r >> 16);
             lnz = (int)(r & 0xffffu) - 1;
         }
@@ -363,7 +365,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         end = jj + 2 < qlen ? jj + 2 : qlen;
         ++i;
         const bool done = !live || zd || fin || i >= tlen;
-        if (done) {
+        if (have && done) {
             if (gl == 0) {
                 bsb_ext_out_t o;
                 o.score = best; o.qle = best_j + 1; o.tle = best_i + 1;
