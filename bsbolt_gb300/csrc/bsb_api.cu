@@ -231,10 +231,11 @@ static bool job_ok(const bsb_ext_job_t &j, int64_t seq_bytes, int qmax)
            j.toff + j.tlen <= seq_bytes && (int64_t)j.qlen + j.tlen <= (1 << 30);
 }
 
-static JobScan scan_jobs(const bsb_ext_job_t *jobs, int64_t lo, int64_t hi, int64_t seq_bytes,
-                         const uint8_t *tile_map)
+// builtin: the number of the built-in map, -1 where tile_map is an installed one.
+static JobScan scan_jobs(const KswParams &P, const bsb_ext_job_t *jobs, int64_t lo, int64_t hi, int64_t seq_bytes,
+                         const uint8_t *tile_map, int builtin)
 {
-    const int qmax = ksw_max_qlen();
+    const int qmax = ksw_max_qlen(), ring_from = builtin < 0 ? qmax + 1 : ksw_ring_from(builtin);
     JobScan r{hi, 0, 0};
     for (int64_t i = lo; i < hi; ++i) {
         const bsb_ext_job_t &j = jobs[i];
@@ -242,7 +243,8 @@ static JobScan scan_jobs(const bsb_ext_job_t *jobs, int64_t lo, int64_t hi, int6
             r.first_bad = i;
             break;
         }
-        r.tiles |= 1ull << tile_map[j.qlen + 1];
+        r.tiles |= 1ull << (j.qlen >= ring_from && ksw_takes_ring(P, j, builtin) ? ksw_ring_tile()
+                                                                                 : tile_map[j.qlen + 1]);
         r.need = r.need > j.qoff + j.qlen ? r.need : j.qoff + j.qlen;
         r.need = r.need > j.toff + j.tlen ? r.need : j.toff + j.tlen;
     }
@@ -251,15 +253,15 @@ static JobScan scan_jobs(const bsb_ext_job_t *jobs, int64_t lo, int64_t hi, int6
 
 // scan_jobs over pieces [k*per, (k+1)*per), host threads sharing the work for large
 // batches (the scan is on the host entry's critical path before any device work).
-static void scan_pieces(const bsb_ext_job_t *jobs, int64_t n, int64_t per, int nck, int64_t seq_bytes,
-                        const uint8_t *tile_map, JobScan *piece)
+static void scan_pieces(const KswParams &P, const bsb_ext_job_t *jobs, int64_t n, int64_t per, int nck,
+                        int64_t seq_bytes, const uint8_t *tile_map, int builtin, JobScan *piece)
 {
     const int64_t kSlice = 1 << 16;
     const int64_t n_slices = (n + kSlice - 1) / kSlice;
     std::vector<JobScan> sl((size_t)n_slices);
     auto run = [&](int64_t a, int64_t b) {
         for (int64_t k = a; k < b; ++k)
-            sl[(size_t)k] = scan_jobs(jobs, k * kSlice, std::min(n, (k + 1) * kSlice), seq_bytes, tile_map);
+            sl[(size_t)k] = scan_jobs(P, jobs, k * kSlice, std::min(n, (k + 1) * kSlice), seq_bytes, tile_map, builtin);
     };
     unsigned hw = std::thread::hardware_concurrency();
     int T = (int)std::min<int64_t>(n_slices, hw ? (int64_t)hw : 4);
@@ -282,8 +284,8 @@ static void scan_pieces(const bsb_ext_job_t *jobs, int64_t n, int64_t per, int n
             p.need = std::max(p.need, sl[(size_t)k].need);
         } else {
             for (int c = a; c <= b; ++c) {
-                const JobScan q = scan_jobs(jobs, std::max(lo, c * per), std::min(hi, (c + 1) * per), seq_bytes,
-                                            tile_map);
+                const JobScan q = scan_jobs(P, jobs, std::max(lo, c * per), std::min(hi, (c + 1) * per), seq_bytes,
+                                            tile_map, builtin);
                 JobScan &p = piece[c];
                 p.first_bad = std::min(p.first_bad, q.first_bad < std::min(hi, (c + 1) * per) ? q.first_bad : n);
                 p.tiles |= q.tiles;
@@ -325,7 +327,7 @@ extern "C" int bsb_extend_batch_device(bsb_ctx *ctx, const bsb_ext_param_t *para
 {
     if (!ctx) return BSB_EINVAL;
     const int builtin = ksw_builtin(n_jobs, ctx->n_sm);
-    const uint64_t tiles = ctx->d_tile_map ? ctx->map_tiles : ksw_map_tiles(ksw_builtin_tile_map(builtin));
+    const uint64_t tiles = ctx->d_tile_map ? ctx->map_tiles : ksw_builtin_tiles(builtin);
     return extend_device(ctx, param, d_jobs, n_jobs, d_seq, seq_bytes, d_cost, d_out, d_cells, builtin, tiles);
 }
 
@@ -414,8 +416,10 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     const int nck = (int)((n_jobs + per - 1) / per);
     JobScan piece[BSB_MAX_CHUNKS];
     const int builtin = ksw_builtin(per, ctx->n_sm);      // one map for all pieces
-    const uint8_t *map = ctx->d_tile_map ? ctx->tile_map : ksw_builtin_tile_map(builtin);
-    scan_pieces(jobs, n_jobs, per, nck, seq_bytes, map, piece);
+    P.pack16 = ksw_pack16(P);
+    const bool installed = ctx->d_tile_map != nullptr;
+    scan_pieces(P, jobs, n_jobs, per, nck, seq_bytes, installed ? ctx->tile_map : ksw_builtin_tile_map(builtin),
+                installed ? -1 : builtin, piece);
     for (int k = 0; k < nck; ++k)          // every job is checked before any device work
         if (piece[k].first_bad < n_jobs) return check_jobs(ctx, jobs + piece[k].first_bad, 1, seq_bytes,
                                                            piece[k].first_bad);

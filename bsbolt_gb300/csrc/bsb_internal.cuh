@@ -180,6 +180,12 @@ const uint8_t *ksw_builtin_tile_map(int builtin);
 int ksw_tile_shape(int t, int *G, int *C);
 // Set of tile shapes a map uses (bit t).
 uint64_t ksw_map_tiles(const uint8_t *map);
+// The same for a built-in map, with the place ksw_ring_tile() of the ring's jobs (ksw_tiles.cuh); and whether
+// ksw_launch puts job j there on that map (P.pack16 as ksw_pack16 has it), queries below ksw_ring_from() never.
+uint64_t ksw_builtin_tiles(int builtin);
+int ksw_ring_tile();
+int ksw_ring_from(int builtin);
+bool ksw_takes_ring(const KswParams &P, const bsb_ext_job_t &j, int builtin);
 
 // (int)((double)num / e + 1.), the band caps of ksw.c:400-407, bwamem.c:627-628 and
 // bwa.c:234-235, in integer arithmetic (e >= 1, |num| < 2^30): (num + e) / e truncated

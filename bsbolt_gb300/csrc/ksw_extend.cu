@@ -29,7 +29,8 @@
 // two per register (ksw_group16.cuh); a job whose scores could leave 16 bits
 // (h0 + qlen * max(mat) > kPack16MaxH) is binned last in its shape and runs on
 // the 32-bit kernel.  Results never depend on the shape, the cell width or the
-// order.
+// order.  Long queries with a narrow band run on registers that move along with the band
+// (ksw_ring16.cu) where the scheduler's own maps are in use.
 
 #include <climits>
 #include <cstdio>
@@ -38,7 +39,7 @@
 #include "ksw_tiles.cuh"
 
 __constant__ KswTileMap c_tile_maps[kBuiltinMaps] = {kBuiltinTileMaps[0], kBuiltinTileMaps[1], kBuiltinTileMaps[2],
-                                                     kBuiltinTileMaps[3]};
+                                                     kBuiltinTileMaps[3], kBuiltinTileMaps[4]};
 
 namespace {
 
@@ -97,7 +98,8 @@ template <bool Packed>
 __global__ void __launch_bounds__(kHistThreads)
 ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long long seq_bytes,
                const uint8_t *__restrict__ seq, const int32_t *__restrict__ cost, const uint8_t *__restrict__ map,
-               int builtin, int diagonals, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist, int32_t *__restrict__ key_out)
+               int builtin, int ring, int diagonals, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist,
+               int32_t *__restrict__ key_out)
 {
     __shared__ int sh[kHistSlots];
     __shared__ int8_t tab[kScoreTable];
@@ -123,7 +125,8 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
             key = kRejectKey;
         } else {
             const int need = jb.qlen + 1;
-            const int t = map ? map[need] : c_tile_maps[builtin].tile[need];
+            const int t = !Packed && ring && ksw_ring_fits(P, jb, ring_of(builtin)) ? kRingTile
+                          : map ? map[need] : c_tile_maps[builtin].tile[need];
             uint32_t k;
             if (cost) k = (uint32_t)max(cost[i], 0);
             else {
@@ -307,6 +310,17 @@ uint64_t ksw_map_tiles(const uint8_t *map)
     return m;
 }
 
+uint64_t ksw_builtin_tiles(int builtin) { return ksw_map_tiles(kBuiltinTileMaps[builtin].tile) | 1ull << kRingTile; }
+
+int ksw_ring_from(int builtin) { return ring_cols(ring_of(builtin)); }
+
+bool ksw_takes_ring(const KswParams &P, const bsb_ext_job_t &j, int builtin)
+{
+    return P.pack16 && ksw_ring_fits(P, j, ring_of(builtin));
+}
+
+int ksw_ring_tile() { return kRingTile; }
+
 cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
                        const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
@@ -326,6 +340,8 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
     // kPack16MaxScore (h0 + qlen * max score is checked per job)
     KswParams Q = P;
     Q.pack16 = ksw_pack16(P);
+    const bool ring = !d_map && !Q.pac && Q.pack16 && (tiles >> kRingTile & 1);
+    if (!d_map && !ring) tiles &= ~(1ull << kRingTile);
     cudaError_t e;
     if (ev0) cudaEventRecord(ev0, st);
     e = cudaMemsetAsync(scratch, 0, sizeof(int) * (3 * kNumTiles + 1 + kHistSlots), st);
@@ -338,7 +354,7 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
         const int hb = (int)min((int64_t)n_sm * 8, (n + per * (kHistThreads / 32) - 1) / (per * (kHistThreads / 32)));
         const auto hist_kernel = Q.pac ? ksw_sched_hist<true> : ksw_sched_hist<false>;
         hist_kernel<<<hb, kHistThreads, 0, st>>>(Q, d_jobs, (int)n, (long long)seq_bytes, d_seq, d_cost, d_map, builtin,
-                                                 d_cells == nullptr, per, d_out, hist, key);
+                                                 ring, d_cells == nullptr, per, d_out, hist, key);
         ksw_sched_scan<<<1, kScanThreads, 0, st>>>(hist, cursor, ranges, rejected);
         if (n >= 8 * kScatterTile)
             ksw_sched_scatter_tiles<<<(unsigned)((n + kScatterTile - 1) / kScatterTile), kScatterThreads, 0, st>>>(
@@ -365,7 +381,9 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
             cudaStream_t s = conc && lane ? ms->aux[lane - 1] : st;
             const int32_t *r = ranges + kRangeInts * t;
             if (tile_ev) cudaEventRecord(tile_ev[2 * t], s);
-            if (f16) {
+            if (ring && t == kRingTile) {
+                e = ksw_ring16(ring_of(builtin))(Q, d_jobs, d_seq, order, r + 4, counter + 3 * t, d_out, d_cells, n_sm, s);
+            } else if (f16) {
                 // the wide class is rare (very large h0): one block per SM drains it
                 e = f16(Q, d_jobs, d_seq, order, r, counter + 3 * t, d_out, d_cells, n_sm, s);
                 if (e == cudaSuccess && !all_narrow)

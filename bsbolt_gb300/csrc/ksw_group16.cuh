@@ -20,8 +20,8 @@
 #pragma once
 
 #include "ksw_group.cuh"
+#include "ksw_tiles.cuh"
 
-constexpr int kPack16MaxH = 2047;
 constexpr int kPack16MaxScore = 15;
 
 __device__ __forceinline__ uint32_t pk16(int lo, int hi)
@@ -96,20 +96,52 @@ __device__ __forceinline__ void ksw16_pass2(const uint32_t (&Mv)[C2], uint32_t (
     if (C2 & 1) kmx = __vimax_s16x2_relu(kmx, kprev);
 }
 
-template <int C2, int G, bool Packed = false>
+// Ring: the registers hold G*C columns that move along with the band instead of the whole query.  Column block b
+// (columns b*C ..) lives in lane b % G; once block `first` lies left of the band its lane takes block first + G, whose
+// cells are still as the first row left them: no row has written them while 2w + C + 1 <= G*C (ksw_ring_fits).  The
+// lanes' order is that of their blocks, from lane first % G on.  qbytes: the group's query, base_words: the profile
+// words of base 0..4, in shared memory.
+template <int C2, int G, bool Packed = false, bool Ring = false>
 __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ext_job_t *__restrict__ jobs,
                                                 const uint8_t *__restrict__ seq, const int32_t *__restrict__ order,
                                                 int lo, int hi, int *__restrict__ counter,
-                                                bsb_ext_out_t *__restrict__ out, int64_t *__restrict__ cells)
+                                                bsb_ext_out_t *__restrict__ out, int64_t *__restrict__ cells,
+                                                uint8_t *qbytes = nullptr, const uint2 *base_words = nullptr)
 {
+    static_assert(!(Packed && Ring), "the ring stages a byte query");
     static_assert(C2 <= 16, "the row-maximum key and the non-zero bits hold a column index in 4 bits per half");
     constexpr int C = 2 * C2;
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const unsigned gm = group_mask<G>(lane);
     const int e_del = P.e_del, e_ins = P.e_ins;
     const int oe_del = P.o_del + e_del, oe_ins = P.o_ins + e_ins;
-    const int base = gl * C;
+    int base = gl * C;                    // the lane's first column
     const int eC = e_ins * C;
+    // Ring: the first block held, the lane's place after it, and what F loses on the way from d lanes before
+    int first = 0, place = gl;
+    constexpr int kSteps = G == 4 ? 2 : G == 8 ? 3 : G == 16 ? 4 : 5;
+    int lose[kSteps];
+    const auto set_lose = [&]() {
+#pragma unroll
+        for (int k = 0; k < kSteps; ++k) lose[k] = place >= 1 << k ? -eC * (1 << k) : -(1 << 28);
+    };
+    // the block's profile and its cells as the first row leaves them (ksw.c:395-397)
+    const auto load_block = [&](int qlen, int h0, uint32_t *prof, uint32_t *profN, uint32_t *Hs, uint32_t *Es) {
+        const int h1run = max(h0 - oe_ins, 0);
+        int h_init[C];
+#pragma unroll
+        for (int s = 0; s < (C + 3) / 4; ++s) profN[s] = 0;
+#pragma unroll
+        for (int s = 0; s < C; ++s) {
+            const int j = base + s;
+            const uint2 v = base_words[j < qlen ? qbytes[j] : 0];
+            prof[s] = v.x;
+            profN[s >> 2] |= v.y << ((s & 3) * 8);
+            h_init[s] = j == 0 ? h0 : (j <= qlen ? max(h1run - e_ins * (j - 1), 0) : 0);
+        }
+#pragma unroll
+        for (int u = 0; u < C2; ++u) Hs[u] = pk16(h_init[u], h_init[u + C2]), Es[u] = 0;
+    };
     const uint32_t ne_del = pk16(-e_del, -e_del), ne_ins = pk16(-e_ins, -e_ins);
     const uint32_t noe_del = pk16(-oe_del, -oe_del), noe_ins = pk16(-oe_ins, -oe_ins);
     const bool sym_gaps = oe_del == oe_ins && e_del == e_ins;
@@ -143,20 +175,30 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                 qlen = jb.qlen; tlen = jb.tlen; h0 = jb.h0;
                 const JobText<Packed> q = job_query<Packed>(seq, jb);
                 t = job_target<Packed>(seq, jb);
-                const int h1run = max(h0 - oe_ins, 0);
+                if constexpr (Ring) {
+                    __syncwarp(gm);
+#pragma unroll 4
+                    for (int j = gl; j < qlen; j += G) qbytes[j] = (uint8_t)min(q.byte(j), 4);
+                    __syncwarp(gm);
+                    first = 0, place = gl, base = gl * C;
+                    set_lose();
+                    load_block(qlen, h0, prof, profN, Hs, Es);
+                } else {
+                    const int h1run = max(h0 - oe_ins, 0);
 #pragma unroll
-                for (int s = 0; s < (C + 3) / 4; ++s) profN[s] = 0;
-                int h_init[C];
+                    for (int s = 0; s < (C + 3) / 4; ++s) profN[s] = 0;
+                    int h_init[C];
 #pragma unroll
-                for (int s = 0; s < C; ++s) {
-                    const int j = base + s;
-                    const int qc = j < qlen ? q.byte(j) : 0;
-                    prof[s] = profile_word(P, qc);
-                    profN[s >> 2] |= (uint32_t)(uint8_t)profile_n(P, qc) << ((s & 3) * 8);
-                    h_init[s] = j == 0 ? h0 : (j <= qlen ? max(h1run - e_ins * (j - 1), 0) : 0);   // ksw.c:395-397
+                    for (int s = 0; s < C; ++s) {
+                        const int j = base + s;
+                        const int qc = j < qlen ? q.byte(j) : 0;
+                        prof[s] = profile_word(P, qc);
+                        profN[s >> 2] |= (uint32_t)(uint8_t)profile_n(P, qc) << ((s & 3) * 8);
+                        h_init[s] = j == 0 ? h0 : (j <= qlen ? max(h1run - e_ins * (j - 1), 0) : 0);   // ksw.c:395-397
+                    }
+#pragma unroll
+                    for (int u = 0; u < C2; ++u) Hs[u] = pk16(h_init[u], h_init[u + C2]), Es[u] = 0;
                 }
-#pragma unroll
-                for (int u = 0; u < C2; ++u) Hs[u] = pk16(h_init[u], h_init[u + C2]), Es[u] = 0;
                 w = jb.w;                                                                  // ksw.c:399-407
                 {
                     int max_ins = band_cap(qlen * P.mat_max + jb.end_bonus - P.o_ins, e_ins);
@@ -168,7 +210,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                 }
                 best = h0; best_i = best_j = -1; max_ie = -1; gscore = -1; max_off = 0;
                 beg = 0; end = qlen; i = 0; ncell = 0;
-                q_lane = qlen / C; q_slot = qlen % C;
+                q_lane = qlen / C & (G - 1); q_slot = qlen % C;
                 tch = gl < tlen ? t.base(P, gl) : 4u;
                 tnext = G + gl < tlen ? t.base(P, G + gl) : 4u;
                 have = tlen > 0;
@@ -195,6 +237,20 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
             tch = tnext;
             const int ti = i + G + 1 + gl;
             tnext = ti < tlen ? t.base(P, ti) : have ? 4u : 0u;
+        }
+        if constexpr (Ring) {
+            const bool move = have && (first + 1) * C <= i - w && (first + G) * C <= qlen;
+            if (__any_sync(BSB_FULL_MASK, move)) {
+                if (move) {
+                    if (place == 0) {
+                        base += G * C;
+                        load_block(qlen, h0, prof, profN, Hs, Es);
+                    }
+                    ++first, place = (place - 1) & (G - 1);
+                    set_lose();
+                }
+                __syncwarp();
+            }
         }
         const bool bump = have && beg < i - w;         // band edge (ksw.c:416-419)
         beg = bump ? i - w : beg;
@@ -246,11 +302,19 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         const int f_lo_end = lo16(local);
         const int f_lane = max(f_lo_end - e_ins * C2, hi16(local));
         int incl = f_lane;
+        int excl;
+        if constexpr (Ring) {
 #pragma unroll
-        for (int d = 1; d < G; d <<= 1)
-            incl = __viaddmax_s32(__shfl_up_sync(BSB_FULL_MASK, incl, d, G), -eC * d, incl);
-        const int excl = __shfl_up_sync(BSB_FULL_MASK, incl, 1, G);
-        const int carry = gl == 0 ? 0 : excl;
+            for (int k = 0; k < kSteps; ++k)
+                incl = __viaddmax_s32(__shfl_sync(BSB_FULL_MASK, incl, (gl - (1 << k)) & (G - 1), G), lose[k], incl);
+            excl = __shfl_sync(BSB_FULL_MASK, incl, (gl - 1) & (G - 1), G);
+        } else {
+#pragma unroll
+            for (int d = 1; d < G; d <<= 1)
+                incl = __viaddmax_s32(__shfl_up_sync(BSB_FULL_MASK, incl, d, G), -eC * d, incl);
+            excl = __shfl_up_sync(BSB_FULL_MASK, incl, 1, G);
+        }
+        const int carry = (Ring ? place : gl) == 0 ? 0 : excl;
 
         // pass 2: F (the recurrence F(i,j+1) = max(F(i,j) - e_ins, max(M - oe_ins, 0)) of
         // ksw.c:446-447 from each half's carry-in), H, E(i+1,j), the row maximum key, and the
@@ -274,8 +338,9 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
         else
             ksw16_pass2<C2, false>(Mv, Es, Hs, F, t_lt, ltm_prev, kmx, Hprev, nE0, lem0, nzw, ne_del, noe_del,
                                    ne_ins, noe_ins);
-        int Hleft = __shfl_up_sync(BSB_FULL_MASK, hi16(Hprev), 1, G);
-        if (gl == 0) Hleft = h1_init;
+        int Hleft = Ring ? __shfl_sync(BSB_FULL_MASK, hi16(Hprev), (gl - 1) & (G - 1), G)
+                         : __shfl_up_sync(BSB_FULL_MASK, hi16(Hprev), 1, G);
+        if ((Ring ? place : gl) == 0) Hleft = h1_init;       // (0 once the first block is past column 0)
         {
             const uint32_t nH = (pk16(Hleft, lo16(Hprev)) & lem0) | (Hs[0] & ~lem0);
             Hs[0] = nH;
@@ -343,8 +408,12 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                     um = __vimax_s16x2_relu(um, (X + (uint32_t)(a * (C2 - 1 - u)) * 0x00010001u) & nz);
                 }
                 const int lo = lo16(um), hi = hi16(um);
-                const int U = max(lo > 0 ? lo + a * (qlen - base - C2 + 1) : 0,
-                                  hi > 0 ? hi + a * (qlen - base - 2 * C2 + 1) : 0);
+                int U = max(lo > 0 ? lo + a * (qlen - base - C2 + 1) : 0,
+                            hi > 0 ? hi + a * (qlen - base - 2 * C2 + 1) : 0);
+                if constexpr (Ring) {      // the blocks not held yet, which only the first row has written
+                    const int j = (first + G) * C, x = h0 - oe_ins - e_ins * (j - 1);
+                    if (j <= qlen && x > 0) U = max(U, x + a * (qlen - j));
+                }
                 fin = group_max<G>(BSB_FULL_MASK, U) < gscore && want;
             }
         }

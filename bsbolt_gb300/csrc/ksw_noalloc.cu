@@ -81,7 +81,7 @@ extern "C" int bsb_extend_batch_noalloc(const bsb_ext_param_t *param, const bsb_
     if (rc) return rc;
     if (n_jobs == 0) return 0;
     const int builtin = ksw_builtin(n_jobs, n_sm);
-    const uint64_t tiles = ksw_map_tiles(ksw_builtin_tile_map(builtin));
+    const uint64_t tiles = ksw_builtin_tiles(builtin);
     cudaError_t e = ksw_launch(P, d_jobs, n_jobs, seq_bytes, d_seq, nullptr, nullptr, builtin, tiles, d_out, d_cells, scratch,
                                n_sm, (cudaStream_t)stream, nullptr, nullptr);
     return e == cudaSuccess ? 0 : BSB_ECUDA;

@@ -30,6 +30,7 @@ constexpr KswTile kTileList[] = {
 constexpr int kNumTiles = sizeof(kTileList) / sizeof(kTileList[0]);
 constexpr int kMaxNeed = BSB_TILE_MAP_LEN - 1;    // columns 0..qlen with qlen <= 1023
 constexpr int kKswBlock = 128;                      // threads per block (4 warps)
+constexpr int kPack16MaxH = 2047;                   // the largest H of the 16-bit cells (ksw_group16.cuh)
 
 static_assert(kNumTiles == BSB_NUM_TILES, "tile list and public header disagree");
 static_assert(kNumTiles <= 64, "tile sets are 64-bit masks");
@@ -85,7 +86,7 @@ constexpr KswTileMap kDefaultTileMap = make_default_tile_map();
 // follow one another.  Jobs of 10-140 bases, us (default map in brackets): 64 jobs 129 (328), 3000
 // 181 (490), 10,000 220 (537), 30,000 300 (586), 130,000 774 (792), 260,000 1362 (1349).
 // Queries beyond the bands given here keep the default's shapes.
-constexpr int kBuiltinMaps = 4;
+constexpr int kBuiltinMaps = 5;
 constexpr KswTileMap with_band(KswTileMap m, int lo, int hi, int G, int C)
 {
     for (int need = lo; need <= hi; ++need) m.tile[need] = (uint8_t)tile_index(G, C);
@@ -96,11 +97,51 @@ constexpr KswTileMap kBuiltinTileMaps[kBuiltinMaps] = {
     with_band(with_band(kDefaultTileMap, 1, 64, 4, 16), 65, 144, 8, 18),
     with_band(kDefaultTileMap, 1, 160, 16, 10),
     with_band(with_band(kDefaultTileMap, 1, 192, 32, 6), 193, 256, 32, 8),
+    with_band(with_band(kDefaultTileMap, 1, 192, 32, 6), 193, 256, 32, 8),     // (with the other ring, below)
 };
 // The built-in map of a batch of n jobs (lines between the measured sizes where two maps meet).
 inline int ksw_builtin_of(int64_t n, int n_sm)
 {
-    return n <= 50 * (int64_t)n_sm ? 3 : n <= 90 * (int64_t)n_sm ? 2 : n <= 1300 * (int64_t)n_sm ? 1 : 0;
+    return n <= 30 * (int64_t)n_sm ? 4 : n <= 50 * (int64_t)n_sm ? 3 : n <= 90 * (int64_t)n_sm ? 2 : n <= 1300 * (int64_t)n_sm ? 1 : 0;
+}
+
+// Queries wider than a ring's columns whose band is narrower run on it (ksw_group16.cuh): registers for G*C columns
+// that move along with the band.  Taken on the built-in maps only (an installed map's shapes are the caller's);
+// their jobs are listed, and their time is reported, under a shape no built-in map uses.  A row costs what its
+// lanes hold, so a 600-base query with a band of 201 pays for 224 columns instead of 640, two jobs a warp:
+// 50k jobs of 500-600 bases 14.4 ms -> 6.7, 50k of 100-600 6.9 -> 4.3, 20k of 230-300 1.68 -> 1.44; 16x16, 8x30 and
+// 8x32 rings 4.6, 4.6 and 4.6 where 16x14 takes 4.3.  The smallest batches are bound by the rows one after the
+// other, where a warp a job is faster: 64 jobs of 300-600 bases 0.77 ms -> 0.54 (16x14 0.64), 3000 of 100-600 1.05
+// -> 0.76 (0.95), but 7500 of 300-600 1.34 (1.16), 10,000 of 300-400 1.55 -> 1.38 (1.12).
+constexpr KswTile kRings[2] = {{16, 14}, {32, 8}};
+__host__ __device__ __forceinline__ constexpr int ring_of(int builtin) { return builtin == kBuiltinMaps - 1 ? 1 : 0; }
+__host__ __device__ __forceinline__ constexpr int ring_cols(int ring) { return ring ? 32 * 8 : 16 * 14; }
+__host__ __device__ __forceinline__ constexpr int ring_block(int ring) { return ring ? 8 : 14; }
+static_assert(ring_cols(0) == kRings[0].G * kRings[0].C && ring_cols(1) == kRings[1].G * kRings[1].C &&
+              ring_block(0) == kRings[0].C && ring_block(1) == kRings[1].C, "the rings' sizes");
+constexpr int kRingTile = tile_index(32, 5);
+constexpr bool ring_tile_is_free()
+{
+    for (int b = 0; b < kBuiltinMaps; ++b)
+        for (int need = 1; need <= kMaxNeed; ++need)
+            if (kBuiltinTileMaps[b].tile[need] == kRingTile) return false;
+    return true;
+}
+static_assert(ring_tile_is_free(), "a built-in map uses the ring's place");
+// The job's cells fit 16 bits, no column passes the row-maximum key's 10 bits, and a block of columns beside
+// the band of a row (w as ksw.c:399-407 cuts it) holds all columns that row and the next write.
+__host__ __device__ __forceinline__ bool ksw_ring_fits(const KswParams &P, const bsb_ext_job_t &j, int ring)
+{
+    const int cols = ring_cols(ring), block = ring_block(ring);
+    if (j.qlen < cols || j.qlen + block >= 1024 ||
+        (long long)j.h0 + (long long)j.qlen * P.mat_max > kPack16MaxH)
+        return false;
+    const int mi = band_cap(j.qlen * P.mat_max + j.end_bonus - P.o_ins, P.e_ins);
+    const int md = band_cap(j.qlen * P.mat_max + j.end_bonus - P.o_del, P.e_del);
+    int w = j.w;
+    w = w < mi ? w : mi > 1 ? mi : 1;
+    w = w < md ? w : md > 1 ? md : 1;
+    return 2 * (long long)w + block + 1 <= cols;
 }
 
 // Launches the persistent kernel of one tile shape over a range of the scheduled
@@ -121,6 +162,7 @@ KswTileLaunch ksw_tiles16_g32(int C);
 // The kernels of an alignment batch's jobs exist for the shapes of the built-in maps.
 KswTileLaunch ksw_packed16_g4(int C);
 KswTileLaunch ksw_packed16_wide(int G, int C);
+KswTileLaunch ksw_ring16(int ring);
 inline KswTileLaunch ksw_packed16_launcher(int t)
 {
     if (t < 0 || t >= kNumTiles) return nullptr;

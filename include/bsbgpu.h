@@ -131,7 +131,8 @@ int bsb_set_tile_map(bsb_ctx *ctx, const uint8_t *map, int n);
  * t < min(n, BSB_NUM_TILES); 0 for shapes not launched.  Batches below 2^20
  * jobs run their shapes on four streams at once, so a shape's time there
  * includes sharing the GPU; a host batch extended in pieces reports its last
- * piece.  Valid after bsb_sync. */
+ * piece.  Without an installed map, long queries with a narrow band run on a
+ * kernel of their own, reported under the 32 x 5 shape.  Valid after bsb_sync. */
 int bsb_last_tile_ms(const bsb_ctx *ctx, float *ms, int n);
 
 /* Copies the context's current tile map into map (n >= BSB_TILE_MAP_LEN);
