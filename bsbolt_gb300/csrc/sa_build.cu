@@ -317,18 +317,13 @@ __global__ void tails_rev(const uint64_t *__restrict__ key, int64_t N, int from,
 // New ranks of a sorted chunk, the position of the last row of each suffix's group: base + that
 // row in round 0 (base = the chunk's first position); later, the old group's rank (its last row)
 // less the rows of the old group after the new group's last row.
-// list (optional): receives the suffixes whose group has more members, n_open counting them.
-template <class V>
-__global__ void write_ranks(const uint64_t *__restrict__ key, const V *__restrict__ val, int64_t N,
+__global__ void write_ranks(const uint64_t *__restrict__ key, const uint64_t *__restrict__ val, int64_t N,
                             const uint32_t *__restrict__ ek, const uint32_t *__restrict__ eo, int rbits,
                             uint64_t base, int round0, uint64_t *__restrict__ rank,
-                            unsigned long long *__restrict__ n_open, V *__restrict__ list)
+                            unsigned long long *__restrict__ n_open)
 {
     unsigned open = 0;
-    const int lane = threadIdx.x & 31;
-    for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; j0 < N; j0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = min(j0 + lane, N - 1);
-        const bool in = j0 + lane < N;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = key[j];
         const int64_t end = N - 1 - (int64_t)ek[N - 1 - j];
         const bool alone = end == j && (j == 0 || key[j - 1] != k);
@@ -339,58 +334,208 @@ __global__ void write_ranks(const uint64_t *__restrict__ key, const V *__restric
             const int64_t oend = N - 1 - (int64_t)eo[N - 1 - j];
             r = base + (k >> rbits) - (uint64_t)(oend - end);
         }
-        const V i = val[j];
-        if (in) rank[i] = r | (alone ? kAlone : 0);
-        if (list) {
-            const unsigned m = __ballot_sync(BSB_FULL_MASK, in && !alone);
-            unsigned long long at = 0;
-            if (m && lane == 0) at = atomicAdd(n_open, (unsigned long long)__popc(m));
-            at = __shfl_sync(BSB_FULL_MASK, at, 0) + __popc(m & ((1u << lane) - 1u));
-            if (in && !alone) list[at] = i;
-        } else {
-            open += in && !alone;
-        }
+        rank[val[j]] = r | (alone ? kAlone : 0);
+        open += !alone;
     }
     open = __reduce_add_sync(0xffffffffu, open);
     if ((threadIdx.x & 31) == 0 && open) atomicAdd(n_open, (unsigned long long)open);
 }
 
-// ---- one chunk holds all suffixes
-// Every suffix's first key, eight suffixes a thread (a key is the one before, shifted by a symbol).
-__global__ void all_keys(const uint8_t *__restrict__ text, int64_t n, uint64_t *__restrict__ keys,
-                         uint32_t *__restrict__ vals)
+// ---- one chunk holds all suffixes: 32-bit ranks (bit 31: alone)
+//
+// Round 0 sorts every suffix by its first 20 symbols in 2 bits (5 passes of the radix sort against 8 for 21
+// symbols in 3 bits, 0.15 ms each for a 10 Mb text).  A suffix with fewer symbols is padded with A; those 20 come
+// first in the sort's input, the shortest foremost, and the sort is stable, so each stands in front of the longer
+// suffixes with its padded key, where it belongs, and it is taken as alone.
+//
+// From then on nearly all groups are small (the copies of a repeat), and a radix sort of all open suffixes by
+// (group, rank[i + h]) does 7 passes to order pairs.  So the open suffixes of groups of up to kSmall members are
+// kept side by side, group by group, and a round is one gather of rank[i + h] and one pass in which a suffix
+// counts the members before it and equal to it (its new rank) and the first of each new group writes the group to
+// the next list.  Groups of more members go through the radix sort and join the list once they are small.
+// A 10 Mb text of three letters with repeats (2.2M of 20M suffixes open, 9 rounds): SMALL_NOTE
+constexpr int kFirstSyms = 20;
+constexpr uint32_t kAlone32 = 1u << 31;
+constexpr int kSmall = 32;
+struct SmallGroups {                     // per entry: suffix, its group's last row, members << 16 | place in the group
+    uint32_t *sfx, *last, *span;         // (no members: an entry left free)
+};
+
+// 32 symbols a word, the first in the top bits, A past the end; a word more than the text has
+__global__ void pack_text(const uint8_t *__restrict__ text, int64_t n, uint64_t *__restrict__ words, int64_t n_words)
 {
-    constexpr int kRun = 8;
-    const int64_t m = n + 1;
-    for (int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * kRun; i0 < m;
-         i0 += (int64_t)gridDim.x * blockDim.x * kRun) {
-        uint64_t k = key21(text, n, i0);
+    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < n_words; w += (int64_t)gridDim.x * blockDim.x) {
+        uint64_t v = 0;
+        if (w * 32 + 32 <= n) {
+            const uint4 *src = (const uint4 *)(text + w * 32);      // (the text starts on 256 bytes)
+            const uint4 x = src[0], y = src[1];
+            const uint32_t part[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
-        for (int j = 0; j < kRun; ++j) {
-            if (i0 + j < m) keys[i0 + j] = k, vals[i0 + j] = (uint32_t)(i0 + j);
-            k = (k << 3 & ~0ull >> 1) | code_at(text, n, i0 + j + kPrefixSyms);
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) v = v << 2 | (part[k] >> 8 * b & 3);
+        } else {
+            for (int k = 0; k < 32; ++k) v = v << 2 | (w * 32 + k < n ? text[w * 32 + k] : 0);
         }
+        words[w] = v;
     }
 }
 
-// A later round's keys of the suffixes still open, straight from their list.
-__global__ void open_keys(const uint64_t *__restrict__ rank, int64_t m, int64_t h, int rbits,
+// Every suffix's first key, in the order described above.
+__global__ void all_keys(const uint64_t *__restrict__ words, int64_t n, uint64_t *__restrict__ keys,
+                         uint32_t *__restrict__ vals)
+{
+    const int64_t m = n + 1, n_short = m < kFirstSyms ? m : kFirstSyms;
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < m; p += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = p < n_short ? n - p : p - n_short;
+        const int b = (int)(i & 31) * 2;
+        const uint64_t hi = words[i >> 5], lo = words[(i >> 5) + 1];
+        keys[p] = (b ? hi << b | lo >> (64 - b) : hi) >> (64 - 2 * kFirstSyms);
+        vals[p] = (uint32_t)i;
+    }
+}
+
+// A later round's keys of the suffixes in large groups, from their list.
+__global__ void open_keys(const uint32_t *__restrict__ rank, int64_t m, int64_t h, int rbits,
                           const uint32_t *__restrict__ list, int64_t N, uint64_t *__restrict__ keys)
 {
     const uint64_t mask = (1ull << rbits) - 1;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = list[j];
-        keys[j] = rank[i] << rbits | (i + h < m ? rank[i + h] & mask : 0);
+        keys[j] = (uint64_t)rank[i] << rbits | (i + h < m ? rank[i + h] & mask : 0);
+    }
+}
+
+// The last row whose key agrees with row j's above bit `from` (the keys are sorted): the next rows are looked
+// at, then steps that double, then halve.
+__device__ __forceinline__ int64_t last_alike(const uint64_t *__restrict__ key, int64_t j, int64_t N, int from,
+                                              uint64_t k)
+{
+    int64_t step = 1;
+    while (j + step < N && key[j + step] >> from == k) j += step, step *= 2;
+    for (; step > 0; step >>= 1)
+        if (j + step < N && key[j + step] >> from == k) j += step;
+    return j;
+}
+
+// Room for `want` entries of each lane (0: none) at the counter, one addition a warp.
+__device__ __forceinline__ uint32_t warp_room(uint32_t want, unsigned long long *count, int lane)
+{
+    uint32_t incl = want;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(BSB_FULL_MASK, incl, d);
+        if (lane >= d) incl += v;
+    }
+    const uint32_t total = __shfl_sync(BSB_FULL_MASK, incl, 31);
+    uint32_t base = 0;
+    if (lane == 0 && total) base = (uint32_t)atomicAdd(count, (unsigned long long)total);
+    return __shfl_sync(BSB_FULL_MASK, base, 0) + incl - want;
+}
+
+// write_ranks, with the open suffixes listed: small groups in `out` (from entry base on, cap entries in all, cnt[1] counting), the members of
+// larger ones, and of groups that find no room there, in `large` (cnt[2]).  Bound by the scattered writes of the ranks,
+// which the sorted rows, read past the L2, leave there (20M suffixes: WRITE_NOTE).
+__global__ void whole_ranks(const uint64_t *__restrict__ key, const uint32_t *__restrict__ val, int64_t N, int round0,
+                            int rbits, int64_t n, uint32_t *__restrict__ rank, unsigned long long *__restrict__ cnt,
+                            SmallGroups out, uint32_t base, uint32_t cap, uint32_t *__restrict__ large)
+{
+    const int lane = threadIdx.x & 31;
+    const auto is_short = [&](int64_t j) { return round0 && val[j] + (int64_t)kFirstSyms > n; };
+    for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; j0 < N; j0 += (int64_t)gridDim.x * blockDim.x) {
+        const bool in = j0 + lane < N;
+        const int64_t j = in ? j0 + lane : N - 1;
+        const uint64_t k = __ldcs(key + j);
+        const uint32_t i = __ldcs(val + j);
+        // a short suffix stands alone in front of its key's rows
+        const int64_t end = is_short(j) ? j : last_alike(key, j, N, 0, k);
+        const bool head = j == 0 || key[j - 1] != k || is_short(j - 1);
+        const bool alone = head && end == j;
+        const uint32_t r = round0 ? (uint32_t)end
+                                  : (uint32_t)(k >> rbits) - (uint32_t)(last_alike(key, end, N, rbits, k >> rbits) - end);
+        if (in) rank[i] = r | (alone ? kAlone32 : 0);
+        const bool is_large = !alone && end >= kSmall && key[end - kSmall] == k && !is_short(end - kSmall);
+        const uint32_t len = in && head && !alone && !is_large ? (uint32_t)(end - j) + 1 : 0;
+        const uint32_t at = base + (__any_sync(BSB_FULL_MASK, len) ? warp_room(len, cnt + 1, lane) : 0);
+        uint32_t spill = 0;
+        if (len) {
+            if (at + len <= cap) {
+                for (uint32_t t = 0; t < len; ++t)
+                    out.sfx[at + t] = val[j + t], out.last[at + t] = r, out.span[at + t] = len << 16 | t;
+            } else {
+                for (uint32_t t = at; t < cap; ++t) out.span[t] = 0;
+                spill = len;
+            }
+        }
+        if (in && is_large) spill = 1;
+        if (__any_sync(BSB_FULL_MASK, spill)) {
+            const uint32_t to = warp_room(spill, cnt + 2, lane);
+            for (uint32_t t = 0; t < spill; ++t) large[to + t] = val[j + t];
+        }
+    }
+}
+
+// A round's keys of the small groups' suffixes: rank[i + h].
+__global__ void small_keys(const uint32_t *__restrict__ rank, int64_t m, int64_t h, SmallGroups g, int64_t N,
+                           uint32_t *__restrict__ keys)
+{
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x)
+        if (g.span[j]) {
+            const int64_t i = g.sfx[j] + h;
+            keys[j] = i < m ? rank[i] & ~kAlone32 : 0;
+        }
+}
+
+// The round itself: ranks of the small groups' suffixes; the entries in their new order to `out`, those now alone
+// free.  cnt[0] counts the open ones.
+__global__ void small_round(SmallGroups g, const uint32_t *__restrict__ keys, int64_t N, uint32_t *__restrict__ rank,
+                            unsigned long long *__restrict__ cnt, SmallGroups out)
+{
+    unsigned open = 0;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t span = g.span[j], len = span >> 16, at_in = span & 0xffff;
+        if (!len) {
+            out.span[j] = 0;
+            continue;
+        }
+        const int64_t first = j - at_in;
+        const uint32_t key = keys[j], sfx = g.sfx[j];
+        uint32_t less = 0, same = 0, before = 0;
+        for (uint32_t t = 0; t < len; ++t) {
+            const uint32_t x = keys[first + t];
+            less += x < key, same += x == key, before += x == key && t < at_in;
+        }
+        const uint32_t r = g.last[j] - len + less + same;
+        const int64_t p = first + less + before;
+        out.sfx[p] = sfx, out.last[p] = r, out.span[p] = same > 1 ? same << 16 | before : 0;
+        if (same < len) rank[sfx] = r | (same == 1 ? kAlone32 : 0);
+        open += same > 1;
+    }
+    open = __reduce_add_sync(BSB_FULL_MASK, open);
+    if ((threadIdx.x & 31) == 0 && open) atomicAdd(cnt, (unsigned long long)open);
+}
+
+// The list without its free entries (cnt[1] counting).
+__global__ void small_close_up(SmallGroups g, int64_t N, unsigned long long *__restrict__ cnt, SmallGroups out)
+{
+    const int lane = threadIdx.x & 31;
+    for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; j0 < N; j0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = j0 + lane;
+        const uint32_t span = j < N ? g.span[j] : 0;
+        const uint32_t len = span & 0xffff ? 0 : span >> 16;        // the first of a group moves it
+        const uint32_t at = warp_room(len, cnt + 1, lane);
+        for (uint32_t t = 0; t < len; ++t)
+            out.sfx[at + t] = g.sfx[j + t], out.last[at + t] = g.last[j + t], out.span[at + t] = g.span[j + t];
     }
 }
 
 // BWT symbols (2 bits, 16 to a word, first symbol in the top bits) and sampled rows, from the ranks
-__global__ void bwt_from_ranks(const uint8_t *__restrict__ text, const uint64_t *__restrict__ rank, int64_t n,
-                               uint64_t primary, int sa_intv, uint32_t *__restrict__ bwt, uint64_t *__restrict__ sa)
+template <class R>
+__global__ void bwt_from_ranks(const uint8_t *__restrict__ text, const R *__restrict__ rank, int64_t n, uint64_t primary, int sa_intv, uint32_t *__restrict__ bwt, uint64_t *__restrict__ sa)
 {
     const int64_t m = n + 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = rank[i] & ~kAlone;
+        const uint64_t r = rank[i] & (R)~((R)1 << (8 * sizeof(R) - 1));
         if (r % (uint64_t)sa_intv == 0) sa[r / (uint64_t)sa_intv] = (uint64_t)i;
         if (i == 0) continue;
         const uint64_t pos = r - (r > primary);
@@ -416,28 +561,25 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
     cudaStream_t st = ctx->stream;
     const size_t pb = (size_t)(l_pac + 3) / 4;
     const int64_t n_words = (n + 15) / 16, n_sa = (n + sa_intv) / sa_intv;
-    DevBuf d_pac, d_text, d_rank, d_hist, d_cnt, k0, k1, v0, v1, s0, s1, d_tmp;
+    DevBuf d_pac, d_text, d_rank, d_hist, d_cnt, k0, k1, v0, v1, s0, s1, d_tmp, d_small;
     // A text whose suffixes one chunk holds in kBuildKept bytes: everything in one buffer that the
     // context keeps (allocating and freeing 1 GB in 13 pieces took more than the sort of a 10 Mb text),
-    // no bins, after each round only the suffixes still open are looked at again, and suffixes are 32-bit
-    // values of the sorts.  10 Mb text of three letters with repeats: 9.65 -> 5.5 ms, of which the sorts
-    // are half (0.15 ms a pass of the first, 10-30 us of the later ones).
+    // no bins, and after round 0 only the suffixes still open are looked at again.  10 Mb text of three letters
+    // with repeats: 9.65 ms in chunks' form, 5.5 with radix sorts of the open suffixes, WHOLE_NOTE
     size_t lent_tmp = 0;
+    uint32_t small_cap = 0;
     bool whole = false;
     if (m <= 0x7fffffffLL / 2 && (chunk <= 0 || chunk >= m)) {
         cub::DoubleBuffer<uint64_t> kk((uint64_t *)nullptr, (uint64_t *)nullptr);
         cub::DoubleBuffer<uint32_t> vv((uint32_t *)nullptr, (uint32_t *)nullptr);
-        size_t ts = 0, tc = 0;
-        if (cub::DeviceRadixSort::SortPairs(nullptr, ts, kk, vv, (int)m, 0, 64, st) != cudaSuccess ||
-            cub::DeviceScan::InclusiveScan(nullptr, tc, (uint32_t *)nullptr, (uint32_t *)nullptr, cuda::maximum<>(),
-                                           (int)m, st) != cudaSuccess)
+        if (cub::DeviceRadixSort::SortPairs(nullptr, lent_tmp, kk, vv, (int)m, 0, 64, st) != cudaSuccess)
             return bsb_fail(ctx, BSB_ECUDA, "BWT build: sort set-up");
-        lent_tmp = std::max(ts, tc);
         struct Part { DevBuf *b; size_t bytes; };
         const size_t mm = (size_t)m;
-        const Part parts[] = {{&d_text, (size_t)n + 64}, {&d_rank, 8 * mm}, {&d_hist, 64}, {&d_cnt, 64}, {&d_pac, pb + 16},
-                              {&k0, 8 * mm}, {&k1, 8 * mm}, {&v0, 4 * mm}, {&v1, 4 * mm}, {&s0, 4 * mm}, {&s1, 4 * mm},
-                              {&d_tmp, lent_tmp + 256}};
+        small_cap = (uint32_t)(m / 4 + 1024);       // two sets of three words, and the keys
+        const Part parts[] = {{&d_text, (size_t)n + 64}, {&d_rank, 4 * mm}, {&d_hist, 64}, {&d_cnt, 64}, {&d_pac, pb + 16},
+                              {&k0, 8 * mm}, {&k1, 8 * mm}, {&v0, 4 * mm}, {&v1, 4 * mm}, {&s0, mm / 4 + 64},
+                              {&d_tmp, lent_tmp + 256}, {&d_small, 28 * (size_t)small_cap}};
         size_t need = 0;
         for (const Part &q : parts) need += (q.bytes + 255) & ~(size_t)255;
         if (need <= kBuildKept && !bsb_ensure(ctx, &ctx->build_buf, &ctx->build_bytes, need, "BWT build")) {
@@ -501,9 +643,7 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
 
     // sorts the gathered chunk of N suffixes on key bits [0, end_bit) and writes their ranks
     unsigned long long h_cnt[2];
-    // (listed: the open ones' list in the spare buffer of vals, suffixes in 32 bits)
-    auto sort_as = [&](auto vals, int64_t N, int end_bit, int round0, uint64_t base, bool listed, void **list) -> int {
-        cub::DoubleBuffer<uint64_t> keys((uint64_t *)k0.p, (uint64_t *)k1.p);
+    auto sort_pairs = [&](auto &keys, auto &vals, int64_t N, int end_bit) -> int {
         size_t t = 0;
         int r;
         if ((r = bsb_cuda(ctx, cub::DeviceRadixSort::SortPairs(nullptr, t, keys, vals, (int)N, 0, end_bit, st),
@@ -511,13 +651,18 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
             return r;
         if (t > tmp_bytes) return bsb_fail(ctx, BSB_ENOMEM, "BWT build: sort scratch of %zu bytes", t);
         t = tmp_bytes;
-        if ((r = bsb_cuda(ctx, cub::DeviceRadixSort::SortPairs(d_tmp.p, t, keys, vals, (int)N, 0, end_bit, st),
-                          "BWT build: sort")))
-            return r;
+        return bsb_cuda(ctx, cub::DeviceRadixSort::SortPairs(d_tmp.p, t, keys, vals, (int)N, 0, end_bit, st),
+                        "BWT build: sort");
+    };
+    auto sort_chunk = [&](int64_t N, int end_bit, int round0, uint64_t base) -> int {
+        cub::DoubleBuffer<uint64_t> keys((uint64_t *)k0.p, (uint64_t *)k1.p);
+        cub::DoubleBuffer<uint64_t> vals((uint64_t *)v0.p, (uint64_t *)v1.p);
+        int r;
+        if ((r = sort_pairs(keys, vals, N, end_bit))) return r;
         const int g = (int)std::min<int64_t>((N + 255) / 256, (int64_t)ctx->n_sm * 16);
         uint32_t *ek = (uint32_t *)s0.p, *eo = (uint32_t *)s1.p;
         tails_rev<<<g, 256, 0, st>>>(keys.Current(), N, 0, ek);
-        t = tmp_bytes;
+        size_t t = tmp_bytes;
         if ((r = bsb_cuda(ctx, cub::DeviceScan::InclusiveScan(d_tmp.p, t, ek, ek, cuda::maximum<>(), (int)N, st),
                           "BWT build: group scan")))
             return r;
@@ -528,15 +673,8 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                                                                   st), "BWT build: group scan")))
                 return r;
         }
-        write_ranks<<<g, 256, 0, st>>>(keys.Current(), vals.Current(), N, ek, eo, rbits, base, round0, rank,
-                                       cnt + 1, listed ? vals.Alternate() : nullptr);
-        *list = vals.Alternate();
+        write_ranks<<<g, 256, 0, st>>>(keys.Current(), vals.Current(), N, ek, eo, rbits, base, round0, rank, cnt + 1);
         return bsb_cuda(ctx, cudaGetLastError(), "BWT build: ranks");
-    };
-    auto sort_chunk = [&](int64_t N, int end_bit, int round0, uint64_t base) -> int {
-        void *list;
-        return sort_as(cub::DoubleBuffer<uint64_t>((uint64_t *)v0.p, (uint64_t *)v1.p), N, end_bit, round0, base, false,
-                       &list);
     };
 
     // the gather of a chunk appended exactly the suffixes its histogram counted
@@ -550,25 +688,56 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                                        (unsigned long long)N);
     };
 
+    uint32_t *const rank32 = (uint32_t *)d_rank.p;
     if (whole) {
-        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters"))) return rc;
-        all_keys<<<grid, 256, 0, st>>>(text, n, (uint64_t *)k0.p, (uint32_t *)v0.p);
-        int64_t N = m;
-        for (int64_t h = kPrefixSyms, round = 0;; h *= 2, ++round) {
-            // the open suffixes go to the spare buffer, which becomes the next round's list
-            void *list = nullptr;
-            if ((rc = sort_as(cub::DoubleBuffer<uint32_t>((uint32_t *)v0.p, (uint32_t *)v1.p), N,
-                              round == 0 ? 63 : 2 * rbits, round == 0, 0, true, &list)) ||
-                (rc = bsb_cuda(ctx, cudaMemcpyAsync(h_cnt, cnt, 16, cudaMemcpyDeviceToHost, st), "BWT build: count")) ||
-                (rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 16, st), "BWT build: counters")) ||
+        uint32_t *const sp = (uint32_t *)d_small.p;
+        SmallGroups now{sp, sp + small_cap, sp + 2 * (size_t)small_cap};
+        SmallGroups next{sp + 3 * (size_t)small_cap, sp + 4 * (size_t)small_cap, sp + 5 * (size_t)small_cap};
+        uint32_t *const skey = sp + 6 * (size_t)small_cap;
+        const auto blocks = [&](int64_t N) { return (int)std::min<int64_t>((N + 255) / 256, (int64_t)ctx->n_sm * 16); };
+        unsigned long long got[3];
+        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 24, st), "BWT build: counters"))) return rc;
+        pack_text<<<grid, 256, 0, st>>>(text, n, (uint64_t *)s0.p, n / 32 + 2);
+        all_keys<<<ctx->n_sm * 16, 256, 0, st>>>((const uint64_t *)s0.p, n, (uint64_t *)k0.p, (uint32_t *)v0.p);
+        int64_t N = m, n_small = 0;                  // N: suffixes of large groups, listed in v0; small ones' entries
+        for (int64_t h = kFirstSyms / 2, round = 0;; ++round) {
+            if (round > 40) return bsb_fail(ctx, BSB_EINVAL, "BWT build: no convergence");
+            // where there are small groups only, two rounds follow one another before the host looks
+            for (int sub = round && !N ? 2 : 1; sub > 0; --sub, h *= 2) {
+                if (round) {                                        // every rank is read before any is written
+                    if (n_small) small_keys<<<blocks(n_small), 256, 0, st>>>(rank32, m, h, now, n_small, skey);
+                    if (N) open_keys<<<blocks(N), 256, 0, st>>>(rank32, m, h, rbits, (const uint32_t *)v0.p, N,
+                                                                (uint64_t *)k0.p);
+                    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 24, st), "BWT build: counters"))) return rc;
+                    if (n_small) small_round<<<blocks(n_small), 256, 0, st>>>(now, skey, n_small, rank32, cnt, next);
+                    std::swap(now, next);
+                }
+                if (N) {
+                    cub::DoubleBuffer<uint64_t> keys((uint64_t *)k0.p, (uint64_t *)k1.p);
+                    cub::DoubleBuffer<uint32_t> vals((uint32_t *)v0.p, (uint32_t *)v1.p);
+                    if ((rc = sort_pairs(keys, vals, N, round ? 2 * rbits : 2 * kFirstSyms))) return rc;
+                    whole_ranks<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(
+                        keys.Current(), vals.Current(), N, round == 0, rbits, n, rank32, cnt, now, (uint32_t)n_small,
+                        small_cap, vals.Alternate());
+                    if (vals.Alternate() != v0.p) std::swap(v0.p, v1.p);
+                }
+            }
+            if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(got, cnt, 24, cudaMemcpyDeviceToHost, st), "BWT build: count")) ||
                 (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: round")))
                 return rc;
-            N = (int64_t)h_cnt[1];
-            if (N == 0) break;                                      // every suffix is alone: sorted
-            if (round > 40) return bsb_fail(ctx, BSB_EINVAL, "BWT build: no convergence");
-            if (list != v0.p) std::swap(v0.p, v1.p);                 // the next sort takes them from v0
-            open_keys<<<(int)std::min<int64_t>((N + 255) / 256, (int64_t)ctx->n_sm * 16), 256, 0, st>>>(
-                rank, m, h, rbits, (const uint32_t *)list, N, (uint64_t *)k0.p);
+            const int64_t joined = (int64_t)std::min<unsigned long long>(got[1], small_cap - (uint64_t)n_small);
+            const int64_t open = (int64_t)got[0] + joined;
+            n_small += joined, N = (int64_t)got[2];
+            if (open + N == 0) break;                               // every suffix is alone: sorted
+            if (2 * open < n_small) {
+                if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, 24, st), "BWT build: counters"))) return rc;
+                small_close_up<<<blocks(n_small), 256, 0, st>>>(now, n_small, cnt, next);
+                if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(got, cnt, 24, cudaMemcpyDeviceToHost, st), "BWT build: count")) ||
+                    (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: round")))
+                    return rc;
+                n_small = (int64_t)got[1];
+                std::swap(now, next);
+            }
         }
     }
     // round 0: buckets of the first five symbols, chunks of whole buckets, 21-symbol keys
@@ -639,10 +808,10 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
     }
     // the BWT without the row of suffix 0, and the sampled rows
     uint64_t r0 = 0;
-    if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(&r0, rank, 8, cudaMemcpyDeviceToHost, st), "BWT build: primary")) ||
+    if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(&r0, rank, whole ? 4 : 8, cudaMemcpyDeviceToHost, st), "BWT build: primary")) ||
         (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "BWT build: primary")))
         return rc;
-    *primary = r0 & ~kAlone;
+    *primary = whole ? r0 & ~(uint64_t)kAlone32 : r0 & ~kAlone;       // (little-endian)
     uint32_t *d_bwt = (uint32_t *)k0.p;
     uint64_t *d_sa = (uint64_t *)k1.p;
     DevBuf big_bwt, big_sa;                   // when a sort buffer is too small for them
@@ -655,7 +824,8 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
         d_sa = (uint64_t *)big_sa.p;
     }
     if ((rc = bsb_cuda(ctx, cudaMemsetAsync(d_bwt, 0, 4 * (size_t)n_words, st), "BWT build: BWT"))) return rc;
-    bwt_from_ranks<<<grid, 256, 0, st>>>(text, rank, n, *primary, sa_intv, d_bwt, d_sa);
+    if (whole) bwt_from_ranks<<<grid, 256, 0, st>>>(text, rank32, n, *primary, sa_intv, d_bwt, d_sa);
+    else bwt_from_ranks<<<grid, 256, 0, st>>>(text, rank, n, *primary, sa_intv, d_bwt, d_sa);
     if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(bwt, d_bwt, 4 * (size_t)n_words, cudaMemcpyDeviceToHost, st),
                        "BWT build: D2H BWT")) ||
         (rc = bsb_cuda(ctx, cudaMemcpyAsync(sa, d_sa, 8 * (size_t)n_sa, cudaMemcpyDeviceToHost, st),
