@@ -351,9 +351,11 @@ __global__ void write_ranks(const uint64_t *__restrict__ key, const uint64_t *__
 // From then on nearly all groups are small (the copies of a repeat), and a radix sort of all open suffixes by
 // (group, rank[i + h]) does 7 passes to order pairs.  So the open suffixes of groups of up to kSmall members are
 // kept side by side, group by group, and a round is one gather of rank[i + h] and one pass in which a suffix
-// counts the members before it and equal to it (its new rank) and the first of each new group writes the group to
-// the next list.  Groups of more members go through the radix sort and join the list once they are small.
-// A 10 Mb text of three letters with repeats (2.2M of 20M suffixes open, 9 rounds): SMALL_NOTE
+// counts the members before it and equal to it: its new rank and its place in the next list.  Groups of more
+// members go through the radix sort and join the list once they are small.
+// A 10 Mb text of three letters with repeats (2.2M of 20M suffixes open, 9 rounds): a round
+// 40 us (13 the gather, 27 the pass) instead of 360; moving the open groups together every round, with a
+// counter, cost 30 us more a round than leaving the places of sorted suffixes free and closing up when half are.
 constexpr int kFirstSyms = 20;
 constexpr uint32_t kAlone32 = 1u << 31;
 constexpr int kSmall = 32;
@@ -433,44 +435,78 @@ __device__ __forceinline__ uint32_t warp_room(uint32_t want, unsigned long long 
     return __shfl_sync(BSB_FULL_MASK, base, 0) + incl - want;
 }
 
-// write_ranks, with the open suffixes listed: small groups in `out` (from entry base on, cap entries in all, cnt[1] counting), the members of
-// larger ones, and of groups that find no room there, in `large` (cnt[2]).  Bound by the scattered writes of the ranks,
-// which the sorted rows, read past the L2, leave there (20M suffixes: WRITE_NOTE).
+// write_ranks, with the open suffixes listed: small groups in `out` (from entry base on, cap entries in all, cnt[1]
+// counting), the members of larger ones, and of groups that find no room there, in `large` (cnt[2]).  Bound by the
+// scattered writes of the ranks, one a suffix (20M: 255 us; with one addition a warp to the list's counter instead
+// of one a block of 1024 rows, 470).
 __global__ void whole_ranks(const uint64_t *__restrict__ key, const uint32_t *__restrict__ val, int64_t N, int round0,
                             int rbits, int64_t n, uint32_t *__restrict__ rank, unsigned long long *__restrict__ cnt,
                             SmallGroups out, uint32_t base, uint32_t cap, uint32_t *__restrict__ large)
 {
     const int lane = threadIdx.x & 31;
     const auto is_short = [&](int64_t j) { return round0 && val[j] + (int64_t)kFirstSyms > n; };
-    for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; j0 < N; j0 += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = j0 + lane < N;
-        const int64_t j = in ? j0 + lane : N - 1;
-        const uint64_t k = __ldcs(key + j);
-        const uint32_t i = __ldcs(val + j);
+    constexpr int kRows = 4;
+    __shared__ uint32_t warp_len[32], block_at;
+    const int64_t b0 = blockIdx.x * (int64_t)blockDim.x * kRows;
+    uint64_t k[kRows], ahead[kRows], after[kRows];
+    uint32_t v[kRows], len[kRows], r[kRows], spill[kRows], mine = 0;
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+        const int64_t j = min(b0 + u * blockDim.x + threadIdx.x, N - 1);
+        k[u] = key[j], v[u] = val[j];
+        ahead[u] = j ? key[j - 1] : ~0ull, after[u] = j + 1 < N ? key[j + 1] : ~0ull;     // (no key is ~0)
+    }
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+        const bool in = b0 + u * blockDim.x + threadIdx.x < N;
+        const int64_t j = min(b0 + u * blockDim.x + threadIdx.x, N - 1);
         // a short suffix stands alone in front of its key's rows
-        const int64_t end = is_short(j) ? j : last_alike(key, j, N, 0, k);
-        const bool head = j == 0 || key[j - 1] != k || is_short(j - 1);
+        const bool stays = after[u] == k[u] && !(round0 && v[u] + (int64_t)kFirstSyms > n);
+        const int64_t end = stays ? last_alike(key, j + 1, N, 0, k[u]) : j;
+        const bool head = ahead[u] != k[u] || is_short(j - 1);
         const bool alone = head && end == j;
-        const uint32_t r = round0 ? (uint32_t)end
-                                  : (uint32_t)(k >> rbits) - (uint32_t)(last_alike(key, end, N, rbits, k >> rbits) - end);
-        if (in) rank[i] = r | (alone ? kAlone32 : 0);
-        const bool is_large = !alone && end >= kSmall && key[end - kSmall] == k && !is_short(end - kSmall);
-        const uint32_t len = in && head && !alone && !is_large ? (uint32_t)(end - j) + 1 : 0;
-        const uint32_t at = base + (__any_sync(BSB_FULL_MASK, len) ? warp_room(len, cnt + 1, lane) : 0);
-        uint32_t spill = 0;
-        if (len) {
-            if (at + len <= cap) {
-                for (uint32_t t = 0; t < len; ++t)
-                    out.sfx[at + t] = val[j + t], out.last[at + t] = r, out.span[at + t] = len << 16 | t;
+        r[u] = round0 ? (uint32_t)end
+                      : (uint32_t)(k[u] >> rbits) - (uint32_t)(last_alike(key, end, N, rbits, k[u] >> rbits) - end);
+        if (in) rank[v[u]] = r[u] | (alone ? kAlone32 : 0);
+        const bool is_large = !alone && end >= kSmall && key[end - kSmall] == k[u] && !is_short(end - kSmall);
+        len[u] = in && head && !alone && !is_large ? (uint32_t)(end - j) + 1 : 0;
+        spill[u] = in && is_large;
+        mine += len[u];
+    }
+    uint32_t incl = mine;                    // the block's groups take their entries with one addition
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t x = __shfl_up_sync(BSB_FULL_MASK, incl, d);
+        if (lane >= d) incl += x;
+    }
+    if (lane == 31) warp_len[threadIdx.x >> 5] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t sum = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+            const uint32_t x = warp_len[w];
+            warp_len[w] = sum, sum += x;
+        }
+        block_at = sum ? (uint32_t)atomicAdd(cnt + 1, (unsigned long long)sum) : 0;
+    }
+    __syncthreads();
+    uint32_t at = base + block_at + warp_len[threadIdx.x >> 5] + incl - mine;
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+        const int64_t j = min(b0 + u * blockDim.x + threadIdx.x, N - 1);
+        if (len[u]) {
+            if (at + len[u] <= cap) {
+                for (uint32_t t = 0; t < len[u]; ++t)
+                    out.sfx[at + t] = val[j + t], out.last[at + t] = r[u], out.span[at + t] = len[u] << 16 | t;
             } else {
                 for (uint32_t t = at; t < cap; ++t) out.span[t] = 0;
-                spill = len;
+                spill[u] = len[u];
             }
+            at += len[u];
         }
-        if (in && is_large) spill = 1;
-        if (__any_sync(BSB_FULL_MASK, spill)) {
-            const uint32_t to = warp_room(spill, cnt + 2, lane);
-            for (uint32_t t = 0; t < spill; ++t) large[to + t] = val[j + t];
+        if (__any_sync(BSB_FULL_MASK, spill[u])) {
+            const uint32_t to = warp_room(spill[u], cnt + 2, lane);
+            for (uint32_t t = 0; t < spill[u]; ++t) large[to + t] = val[j + t];
         }
     }
 }
@@ -565,7 +601,8 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
     // A text whose suffixes one chunk holds in kBuildKept bytes: everything in one buffer that the
     // context keeps (allocating and freeing 1 GB in 13 pieces took more than the sort of a 10 Mb text),
     // no bins, and after round 0 only the suffixes still open are looked at again.  10 Mb text of three letters
-    // with repeats: 9.65 ms in chunks' form, 5.5 with radix sorts of the open suffixes, WHOLE_NOTE
+    // with repeats: 9.65 ms in chunks' form, 5.5 with radix sorts of the open suffixes, 2.0 as below, of which
+    // the first sort 0.8, its ranks 0.26, the rounds 0.4.
     size_t lent_tmp = 0;
     uint32_t small_cap = 0;
     bool whole = false;
@@ -716,7 +753,7 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                     cub::DoubleBuffer<uint64_t> keys((uint64_t *)k0.p, (uint64_t *)k1.p);
                     cub::DoubleBuffer<uint32_t> vals((uint32_t *)v0.p, (uint32_t *)v1.p);
                     if ((rc = sort_pairs(keys, vals, N, round ? 2 * rbits : 2 * kFirstSyms))) return rc;
-                    whole_ranks<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(
+                    whole_ranks<<<(unsigned)((N + 1023) / 1024), 256, 0, st>>>(
                         keys.Current(), vals.Current(), N, round == 0, rbits, n, rank32, cnt, now, (uint32_t)n_small,
                         small_cap, vals.Alternate());
                     if (vals.Alternate() != v0.p) std::swap(v0.p, v1.p);
