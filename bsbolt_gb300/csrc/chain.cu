@@ -10,6 +10,8 @@
 //   chain_kernel            the same by one thread, with the reference's B-tree of
 //                           chains (kbtree.h, t = 5), for reads where two chains start
 //                           at the same place and the tree's nodes decide;
+//   chain2aln_plain         one warp per read: mem_chain2aln (bwamem.c:636-790) for the reads whose
+//                           extensions were all run as batches before
 //   chain2aln_kernel        one warp per read: mem_chain2aln (bwamem.c:636-790),
 //                           each ksw_extend2 run by the warp (ksw_core.cuh) on the
 //                           read and the device 2-bit reference directly, so no
@@ -1325,8 +1327,8 @@ __device__ __forceinline__ void chain_window(const AlnOpt &opt, const DevBns &B,
 // results where it comes to such a seed; what it passes over (a seed inside an earlier region) was
 // extended for nothing.  A warp per extension of a few dozen rows took 8,100 warp instructions a
 // region.  One GB300, everything from the read order to the regions: 114k RRBS reads (450k regions)
-// 4.62 -> 1.98 ms, of which chain2aln_kernel 0.60; 67k reads of 150 bases 2.21 -> 1.18; 40k of 100 on
-// 2 Mb 0.46 -> 0.42.  (With the jobs' bytes written out first, RRBS 2.54.)
+// 4.62 -> 1.68 ms; 67k reads of 150 bases 2.21 -> 1.05; 40k of 100 on 2 Mb 0.46 -> 0.39.  (With the jobs'
+// bytes written out first, and chain2aln_kernel alone behind them, RRBS 2.54 against 1.98.)
 struct PreChain {
     int64_t rmax0, rmax1;
     int seed, pad;                      // the first seed to extend
@@ -1410,7 +1412,167 @@ __global__ void pre_right_kernel(AlnOpt opt, int64_t n_chains, const bsb_ext_job
     else right[t].flags |= kExtNone;
 }
 
-// One warp per read.  regs: the read's region slots start at its row offset.
+// Is seed s (almost) contained in region p of its read (bwamem.c:675-690)?
+struct RegSpan {
+    int64_t rb, re;
+    int qb, qe, w, seedlen0;
+};
+__device__ __forceinline__ bool seed_in_region(const AlnOpt &opt, int l_query, const RegSpan &p, int64_t rbeg, int qbeg,
+                                               int len)
+{
+    if (rbeg < p.rb || rbeg + len > p.re || qbeg < p.qb || qbeg + len > p.qe) return false;
+    if (len - p.seedlen0 > .1 * l_query) return false;
+    int qd = qbeg - p.qb;
+    int64_t rd = rbeg - p.rb;
+    int max_gap = cal_max_gap(opt, qd < rd ? qd : (int)rd);
+    int w = max_gap < p.w ? max_gap : p.w;
+    if (qd - rd < w && rd - qd < w) return true;
+    qd = p.qe - (qbeg + len);
+    rd = p.re - (rbeg + len);
+    max_gap = cal_max_gap(opt, qd < rd ? qd : (int)rd);
+    w = max_gap < p.w ? max_gap : p.w;
+    return qd - rd < w && rd - qd < w;
+}
+
+// Can seed s, contained in a region, lead elsewhere because of seed t, extended before it (bwamem.c:691-707)?
+__device__ __forceinline__ bool seeds_part(int64_t s_rbeg, int s_qbeg, int s_len, int64_t t_rbeg, int t_qbeg, int t_len)
+{
+    if (t_len < s_len * .95) return false;
+    return (s_qbeg <= t_qbeg && s_qbeg + s_len - t_qbeg >= s_len >> 2 && t_qbeg - s_qbeg != t_rbeg - s_rbeg) ||
+           (t_qbeg <= s_qbeg && t_qbeg + t_len - s_qbeg >= s_len >> 2 && s_qbeg - t_qbeg != s_rbeg - t_rbeg);
+}
+
+// The ends of seed s's region from its extensions (bwamem.c:736-775; left has no part where the seed starts the read,
+// right none where it ends it).
+__device__ __forceinline__ void left_end(const AlnOpt &opt, const DevSeed &s, const KswResult &x, bsb_reg_t &a)
+{
+    if (x.gscore <= 0 || x.gscore <= a.score - opt.pen_clip5) {
+        a.qb = s.qbeg - x.qle, a.rb = s.rbeg - x.tle;
+        a.truesc = a.score;
+    } else {
+        a.qb = 0, a.rb = s.rbeg - x.gtle;
+        a.truesc = x.gscore;
+    }
+}
+__device__ __forceinline__ void right_end(const AlnOpt &opt, int l_query, const DevSeed &s, const KswResult &x, int sc0,
+                                          bsb_reg_t &a)
+{
+    if (x.gscore <= 0 || x.gscore <= a.score - opt.pen_clip3) {
+        a.qe = s.qbeg + s.len + x.qle, a.re = s.rbeg + s.len + x.tle;
+        a.truesc += a.score - sc0;
+    } else {
+        a.qe = l_query, a.re = s.rbeg + s.len + x.gtle;
+        a.truesc += x.gscore - sc0;
+    }
+}
+
+// mem_chain2aln for the reads whose extensions are all known (PreResults), a warp a read: 32 chains at a time, each lane
+// one chain's first seed, its region and its record; then the chains in order, the seed of each against the regions so
+// far over the lanes, and the chain's other seeds over the lanes, which must all be contained in a region and not part
+// from the chain's first.  A read where one would be extended, or with more than kPlainRegs regions, goes to `left`
+// for chain2aln_kernel.  That kernel's loads follow one another chain by chain, on 16 warps an SM (it holds the DP).
+// 114k RRBS reads (450k regions): 617 us -> 199 and 175 for the reads left; 67k of 150 bases 292 -> 89 and 86.  At 10
+// blocks an SM, or a block for every four reads in place of 8 an SM: 20-80 us more.
+constexpr int kPlainWarps = 4, kPlainRegs = 64;
+__global__ void __launch_bounds__(kPlainWarps * 32, 8)
+chain2aln_plain(AlnOpt opt, int n_reads, const int64_t *__restrict__ read_off, const int64_t *__restrict__ seed_off,
+                const int64_t *__restrict__ row_off_of_seed, const DevSeed *__restrict__ seeds,
+                const DevChain *__restrict__ chains, const int *__restrict__ n_chains, bsb_reg_t *__restrict__ regs,
+                int *__restrict__ n_regs, PreResults pre, int *__restrict__ left, int *__restrict__ n_left)
+{
+    __shared__ RegSpan sm[kPlainWarps][kPlainRegs];
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    RegSpan *const list = sm[wb];
+    for (int r = blockIdx.x * kPlainWarps + wb; r < n_reads; r += gridDim.x * kPlainWarps) {
+        const int nc = n_chains[r];
+        const int64_t R0 = row_off_of_seed[seed_off[r]], P0 = pre.off[r];
+        const int l_query = (int)(read_off[r + 1] - read_off[r]);
+        const DevSeed *const sd = seeds + R0;
+        int nav = 0;
+        bool ok = true;
+        __syncwarp();
+        for (int base = 0; base < nc && ok; base += 32) {
+            const int ci = base + lane;
+            DevChain c;
+            c.n = 0;
+            if (ci < nc) c = chains[R0 + ci];
+            DevSeed s;
+            s.rbeg = 0, s.qbeg = s.len = s.score = 0;
+            bsb_reg_t a;
+            memset(&a, 0, sizeof a);
+            bool known = true;
+            int first = 0;
+            if (c.n > 0) {
+                first = pre.chains[P0 + ci].seed;
+                s = sd[c.seed_off + first];
+                a.w = opt.w, a.rid = c.rid, a.seedlen0 = s.len, a.frac_rep = c.frac_rep;
+                KswResult x;
+                if (s.qbeg) {
+                    known = pre_result(opt, pre.left[P0 + ci], x);
+                    a.score = x.score;
+                    left_end(opt, s, x, a);
+                } else {
+                    a.score = a.truesc = s.len * opt.a, a.qb = 0, a.rb = s.rbeg;
+                }
+                if (s.qbeg + s.len != l_query) {
+                    const int sc0 = a.score;
+                    known = pre_result(opt, pre.right[P0 + ci], x) && known;
+                    a.score = x.score;
+                    right_end(opt, l_query, s, x, sc0, a);
+                } else {
+                    a.qe = l_query, a.re = s.rbeg + s.len;
+                }
+                for (int i = 0; i < c.n; ++i) {          // seedcov (bwamem.c:779-783)
+                    const DevSeed t = c.n == 1 ? s : sd[c.seed_off + i];
+                    if (t.qbeg >= a.qb && t.qbeg + t.len <= a.qe && t.rbeg >= a.rb && t.rbeg + t.len <= a.re)
+                        a.seedcov += t.len;
+                }
+            }
+            int slot = -1;
+            for (unsigned todo = __ballot_sync(BSB_FULL_MASK, c.n > 0); todo; todo &= todo - 1) {
+                const int j = __ffs(todo) - 1;
+                const int64_t rbeg = __shfl_sync(BSB_FULL_MASK, s.rbeg, j);
+                const int qbeg = __shfl_sync(BSB_FULL_MASK, s.qbeg, j), len = __shfl_sync(BSB_FULL_MASK, s.len, j);
+                bool in = false;
+                for (int i = lane; i < nav; i += 32) in |= seed_in_region(opt, l_query, list[i], rbeg, qbeg, len);
+                const bool fresh = !__any_sync(BSB_FULL_MASK, in);
+                if (fresh) {
+                    ok = __shfl_sync(BSB_FULL_MASK, known, j) && nav < kPlainRegs;
+                    if (!ok) break;
+                    if (lane == j) list[nav] = RegSpan{a.rb, a.re, a.qb, a.qe, a.w, a.seedlen0}, slot = nav;
+                    ++nav;
+                    __syncwarp();
+                }
+                const int n = __shfl_sync(BSB_FULL_MASK, c.n, j);
+                if (n > 1) {
+                    const int f = __shfl_sync(BSB_FULL_MASK, first, j);
+                    const DevSeed *const cs = sd + __shfl_sync(BSB_FULL_MASK, c.seed_off, j);
+                    // (the reference marks an excluded seed by key 0, which a seed 0 of score 0 has in any case)
+                    const bool stands = fresh && (f != 0 || __shfl_sync(BSB_FULL_MASK, s.score, j) != 0);
+                    bool extends = false;
+                    for (int i = lane; i < n; i += 32) {
+                        if (i == f) continue;
+                        const DevSeed t = cs[i];
+                        bool held = false;
+                        for (int x = 0; x < nav && !held; ++x)
+                            held = seed_in_region(opt, l_query, list[x], t.rbeg, t.qbeg, t.len);
+                        extends |= !held || (stands && seeds_part(t.rbeg, t.qbeg, t.len, rbeg, qbeg, len));
+                    }
+                    ok = !__any_sync(BSB_FULL_MASK, extends);
+                    if (!ok) break;
+                }
+            }
+            if (ok && slot >= 0) regs[R0 + slot] = a;
+        }
+        if (lane == 0) {
+            if (ok) n_regs[r] = nav;
+            else left[atomicAdd(n_left, 1)] = r;
+        }
+    }
+}
+
+// One warp per read.  regs: the read's region slots start at its row offset.  n_list: the number of reads in `order`
+// where it is not all n_reads.
 // MaxC = 4, 5, 8 serve batches whose reads are at most 127, 159, 255 bases long (one DP
 // copy of that width), 16 every read the batch accepts; the 4- and 5-column variants are
 // held to 4 blocks (16 warps) per SM, the 8-column one to 3.
@@ -1421,8 +1583,10 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                  const int64_t *__restrict__ row_off_of_seed, const DevSeed *__restrict__ seeds,
                  const DevChain *__restrict__ chains, const int *__restrict__ n_chains, uint64_t *__restrict__ srt_buf,
                  bsb_reg_t *__restrict__ regs, int *__restrict__ n_regs, int *__restrict__ next,
-                 const int *__restrict__ order, int64_t *__restrict__ read_cells, PreResults pre)
+                 const int *__restrict__ order, const int *__restrict__ n_list, int64_t *__restrict__ read_cells,
+                 PreResults pre)
 {
+    if (n_list) n_reads = *n_list;
     __shared__ int8_t tab[kScoreTable];
     load_score_table(P, tab);
     __syncthreads();
@@ -1469,21 +1633,8 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                     bool ok = false;
                     if (i < nav) {
                         const bsb_reg_t p = av[i];
-                        if (!(s.rbeg < p.rb || s.rbeg + s.len > p.re || s.qbeg < p.qb || s.qbeg + s.len > p.qe) &&
-                            !(s.len - p.seedlen0 > .1 * l_query)) {
-                            int qd = s.qbeg - p.qb;
-                            int64_t rd = s.rbeg - p.rb;
-                            int max_gap = cal_max_gap(opt, qd < rd ? qd : (int)rd);
-                            int w = max_gap < p.w ? max_gap : p.w;
-                            if (qd - rd < w && rd - qd < w) ok = true;
-                            else {
-                                qd = p.qe - (s.qbeg + s.len);
-                                rd = p.re - (s.rbeg + s.len);
-                                max_gap = cal_max_gap(opt, qd < rd ? qd : (int)rd);
-                                w = max_gap < p.w ? max_gap : p.w;
-                                ok = qd - rd < w && rd - qd < w;
-                            }
-                        }
+                        ok = seed_in_region(opt, l_query, RegSpan{p.rb, p.re, p.qb, p.qe, p.w, p.seedlen0}, s.rbeg, s.qbeg,
+                                            s.len);
                     }
                     const unsigned m = __ballot_sync(BSB_FULL_MASK, ok);
                     if (m) hit = i0 + __ffs(m) - 1;
@@ -1495,14 +1646,7 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                         bool ok = false;
                         if (i < c.n && srt[i] != 0) {
                             const DevSeed t = cs[(uint32_t)srt[i]];
-                            if (!(t.len < s.len * .95)) {
-                                if (s.qbeg <= t.qbeg && s.qbeg + s.len - t.qbeg >= s.len >> 2 &&
-                                    t.qbeg - s.qbeg != t.rbeg - s.rbeg)
-                                    ok = true;
-                                else if (t.qbeg <= s.qbeg && t.qbeg + t.len - s.qbeg >= s.len >> 2 &&
-                                         s.qbeg - t.qbeg != s.rbeg - t.rbeg)
-                                    ok = true;
-                            }
+                            ok = seeds_part(s.rbeg, s.qbeg, s.len, t.rbeg, t.qbeg, t.len);
                         }
                         const unsigned m = __ballot_sync(BSB_FULL_MASK, ok);
                         if (m) found = i0 + __ffs(m) - 1;
@@ -1536,13 +1680,7 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                         a.score = x.score;
                         if (a.score == prev || x.max_off < (aw0 >> 1) + (aw0 >> 2)) break;
                     }
-                    if (x.gscore <= 0 || x.gscore <= a.score - opt.pen_clip5) {
-                        a.qb = s.qbeg - x.qle, a.rb = s.rbeg - x.tle;
-                        a.truesc = a.score;
-                    } else {
-                        a.qb = 0, a.rb = s.rbeg - x.gtle;
-                        a.truesc = x.gscore;
-                    }
+                    left_end(opt, s, x, a);
                 } else a.score = a.truesc = s.len * opt.a, a.qb = 0, a.rb = s.rbeg;
                 if (s.qbeg + s.len != l_query) {   // right extension (bwamem.c:750-775)
                     const int qe = s.qbeg + s.len, sc0 = a.score;
@@ -1562,13 +1700,7 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                         a.score = x.score;
                         if (a.score == prev || x.max_off < (aw1 >> 1) + (aw1 >> 2)) break;
                     }
-                    if (x.gscore <= 0 || x.gscore <= a.score - opt.pen_clip3) {
-                        a.qe = qe + x.qle, a.re = rmax0 + re + x.tle;
-                        a.truesc += a.score - sc0;
-                    } else {
-                        a.qe = l_query, a.re = rmax0 + re + x.gtle;
-                        a.truesc += x.gscore - sc0;
-                    }
+                    right_end(opt, l_query, s, x, sc0, a);
                 } else a.qe = l_query, a.re = s.rbeg + s.len;
                 int cov = 0;      // seedcov (bwamem.c:779-783)
                 for (int i = lane; i < c.n; i += 32) {
@@ -2437,6 +2569,7 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     const size_t o_ctrl = off; off += al(sizeof(int) * 4);
     const size_t o_regoff = off; off += al(sizeof(int64_t) * (n_reads + 1));
     const size_t o_out = off; off += al(sizeof(bsb_reg_t) * Rb);
+    const size_t o_bail = off; off += al(sizeof(int) * (size_t)n_reads);
     const size_t o_order = off; off += al(sizeof(int) * (n_reads + 1)) + al(sizeof(int) * 2 * kOrderBins);
     const size_t o_dtmp = off; off += dedup ? al(sizeof(bsb_reg_t) * Rb) : 0;
     const size_t o_dn = off; off += dedup ? al(sizeof(int) * (n_reads + 1)) : 0;
@@ -2541,22 +2674,30 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
         (rc = first_extensions(ctx, o, ao, B, P, n_reads, max_len, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
                                n_chains, reg_off, scan_tmp, &pre)))
         return rc;
+    const int *n_list = nullptr;
+    if (pre.chains) {           // the reads that need no other extension; the rest is chain2aln_kernel's
+        int *const bail = (int *)(A + o_bail);
+        const int pb = std::min((n_reads + kPlainWarps - 1) / kPlainWarps, ctx->n_sm * 8);
+        chain2aln_plain<<<pb, kPlainWarps * 32, 0, st>>>(ao, n_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
+                                                         n_chains, regs, n_regs, pre, bail, ctrl + 2);
+        order = bail, n_list = ctrl + 2;
+    }
     // every extension of these reads fits (max_len + 1) columns: the narrowest variant that holds them
     if (max_len <= 127)
         chain2aln_kernel<4><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
+                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else if (max_len <= 159)
         chain2aln_kernel<5><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
+                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else if (max_len <= 255)
         chain2aln_kernel<8><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
+                                                            cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else if (max_len <= 511)
         chain2aln_kernel<16><<<ctx->n_sm * 4, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
+                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else
         chain2aln_kernel<32><<<ctx->n_sm * 2, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
-                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, rcells_out, pre);
+                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     if ((rc = bsb_cuda(ctx, cudaEventRecord(ctx->stage_ev[4], st), "stage mark")) ||
         (rc = bsb_cuda(ctx, scan_i32_i64(n_regs, n_reads, reg_off, scan_tmp, st), "region offsets")))
         return rc;
