@@ -14,7 +14,7 @@
 //
 //   sw_pack_kernel<16, ..> byte-lane jobs of 1..16 segments (every mate of < 250 bases with
 //                          BWA's scoring), two SIMD lanes per thread (sw_pack.cuh): forward
-//                          passes in the order of a host counting sort by segments and length,
+//                          passes in the order of a counting sort by segments and length,
 //                          sw_rev_scatter grouping the jobs that want start positions by the
 //                          segment count of their reversed query, then their reverse passes
 //   sw_pack_kernel<8, ..>  the same for word-lane jobs of 1..40 segments whose scores stay
@@ -27,10 +27,11 @@
 // KSW_XSTART the same pass then runs over the reversed query and target prefixes.
 
 #include <algorithm>
+#include <climits>
 #include <cstring>
-#include <vector>
 
 #include "bsb_internal.cuh"
+#include "scan.cuh"
 #include "sw_pack.cuh"
 
 namespace {
@@ -287,6 +288,105 @@ sw_kernel(SwParams S, const bsb_sw_job_t *__restrict__ jobs, const uint8_t *__re
     }
 }
 
+// ---- the job lists
+//
+// Four lists one behind the other: packed byte lanes (1..16 segments), packed word lanes (1..40 segments, when
+// 16-bit arithmetic without saturation is exact: qlen * max score <= 32640 and penalties below 32768), then the
+// one-lane byte and word jobs.  The packed lists are in counting-sort order by segment count and then target length,
+// both descending: bins of kLenBins lengths per segment count.  Bin kBins - 2 and kBins - 1: the one-lane lists.
+// (On the host the check and the sort took 140 us of a call on 40k jobs; here they go on while the sequences are
+// copied.)
+constexpr int kLenBins = 64, kKeys8 = kPackMaxSeg8 * kLenBins, kKeys16 = kPackMaxSeg16 * kLenBins;
+constexpr int kBins = kKeys8 + kKeys16 + 2;
+constexpr int kPlanThreads = 256;
+
+// What the host needs of the lists: their sizes (n_hi: the word-lane jobs of more than 16 segments), the one-lane
+// jobs' longest queries, and the first unfit job.
+struct SwPlan {
+    int bad, n_p8, n_p16, n_hi, n_fb8, n_fb16, max8, max16;
+};
+
+// 1: bytes outside seq, 2: a query over the limit.
+__host__ __device__ __forceinline__ int job_fault(const bsb_sw_job_t &j, int64_t seq_bytes)
+{
+    if (j.qlen < 0 || j.tlen < 0 || j.qoff < 0 || j.toff < 0 || j.qoff > seq_bytes - j.qlen ||
+        j.toff > seq_bytes - j.tlen)
+        return 1;
+    return j.qlen > BSB_SW_MAX_QLEN ? 2 : 0;
+}
+
+// Every job's bin, the bins' sizes, and the rows of its suboptimal-score scratch.
+__global__ void __launch_bounds__(kPlanThreads)
+sw_plan_kernel(const bsb_sw_job_t *__restrict__ jobs, int n, int64_t seq_bytes, int qmax, int b8_ok, int w16_ok,
+               int *__restrict__ bin, int *__restrict__ rows, int *__restrict__ hist, SwPlan *__restrict__ plan)
+{
+    __shared__ int sh[kBins];
+    for (int k = threadIdx.x; k < kBins; k += kPlanThreads) sh[k] = 0;
+    __syncthreads();
+    for (int64_t i = blockIdx.x * (int64_t)kPlanThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kPlanThreads) {
+        const bsb_sw_job_t j = jobs[i];
+        bin[i] = kBins - 1, rows[i] = 0;
+        if (job_fault(j, seq_bytes)) {
+            atomicMin(&plan->bad, (int)i);
+            continue;
+        }
+        const int len = kLenBins - 1 - min(j.tlen >> 4, kLenBins - 1);
+        const bool byte = j.xtra & kXByte;
+        const int sl = byte ? (j.qlen + 15) >> 4 : (j.qlen + 7) >> 3;
+        int k;
+        if (byte && b8_ok && sl >= 1 && sl <= kPackMaxSeg8) k = (kPackMaxSeg8 - sl) * kLenBins + len;
+        else if (!byte && w16_ok && sl >= 1 && sl <= kPackMaxSeg16 && (int64_t)j.qlen * qmax <= 32640)
+            k = kKeys8 + (kPackMaxSeg16 - sl) * kLenBins + len;
+        else if (byte) k = kBins - 2, atomicMax(&plan->max8, j.qlen);
+        else k = kBins - 1, atomicMax(&plan->max16, j.qlen);
+        bin[i] = k;
+        if (j.xtra & kXSubo) rows[i] = j.tlen;
+        atomicAdd(&sh[k], 1);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kBins; k += kPlanThreads)
+        if (sh[k]) atomicAdd(&hist[k], sh[k]);
+}
+
+// The bins' first places (one block) and the lists' sizes.
+__global__ void __launch_bounds__(1024) sw_plan_scan(const int *__restrict__ hist, int *__restrict__ cursor,
+                                                     SwPlan *__restrict__ plan)
+{
+    constexpr int kPer = (kBins + 1023) / 1024;
+    __shared__ int tot[1024];
+    const int t = threadIdx.x;
+    int v[kPer], s = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) s += v[k] = t * kPer + k < kBins ? hist[t * kPer + k] : 0;
+    tot[t] = s;
+    __syncthreads();
+    for (int d = 1; d < 1024; d <<= 1) {
+        const int add = t >= d ? tot[t - d] : 0;
+        __syncthreads();
+        tot[t] += add;
+        __syncthreads();
+    }
+    int at = tot[t] - s;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int b = t * kPer + k;
+        if (b < kBins) cursor[b] = at;
+        // running totals at the lists' ends, taken apart on the host
+        if (b == kKeys8) plan->n_p8 = at;
+        if (b == kKeys8 + (kPackMaxSeg16 - 16) * kLenBins) plan->n_hi = at;
+        if (b == kBins - 2) plan->n_p16 = at;
+        if (b == kBins - 1) plan->n_fb8 = at, plan->n_fb16 = at + v[k];
+        at += v[k];
+    }
+}
+
+__global__ void __launch_bounds__(kPlanThreads)
+sw_plan_scatter(const int *__restrict__ bin, int n, int *__restrict__ cursor, int32_t *__restrict__ list)
+{
+    for (int64_t i = blockIdx.x * (int64_t)kPlanThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kPlanThreads)
+        list[atomicAdd(&cursor[bin[i]], 1)] = (int32_t)i;
+}
+
 }  // namespace
 
 extern "C" int bsb_align2_batch(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *jobs, int64_t n,
@@ -326,57 +426,11 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
         int rc0;
         if ((rc0 = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice"))) return rc0;
     }
-    // Four job lists: packed byte lanes (1..16 segments), packed word lanes (1..40 segments, when
-    // 16-bit arithmetic without saturation is exact: qlen * max score <= 32640 and penalties
-    // below 32768), then the one-lane byte and word jobs.  The packed lists are in counting-sort
-    // order by segment count and then target length, both descending.
-    constexpr int kLenBins = 64, kKeys8 = kPackMaxSeg8 * kLenBins, kKeys16 = kPackMaxSeg16 * kLenBins;
     const bool w16_ok = S.o_del + S.e_del <= 32767 && S.o_ins + S.e_ins <= 32767;
     // the packed passes read F in closed form, which needs oe_ins >= e_ins as the lanes hold them
     // (and byte lanes a matrix entry <= 0, see sw_pack.cuh)
     const bool b8_ok = (uint8_t)(S.o_ins + S.e_ins) >= (uint8_t)S.e_ins &&
                        *std::min_element(S.mat, S.mat + 25) <= 0;
-    std::vector<int64_t> boff((size_t)n);
-    std::vector<int32_t> key((size_t)n);
-    std::vector<int32_t> lists((size_t)n);
-    std::vector<int64_t> kcnt((size_t)(kKeys8 + kKeys16) + 1, 0);
-    int64_t nb = 0, n_fb8 = 0, n_fb16 = 0, n_p8 = 0, n_p16 = 0;
-    int max8 = 0, max16 = 0;
-    for (int64_t i = 0; i < n; ++i) {
-        const bsb_sw_job_t &j = jobs[i];
-        if (j.qlen < 0 || j.tlen < 0 || j.qoff < 0 || j.toff < 0 || j.qoff > seq_bytes - j.qlen ||
-            j.toff > seq_bytes - j.tlen)
-            return bsb_fail(ctx, BSB_EINVAL, "job %lld: bytes outside seq", (long long)i);
-        if (j.qlen > BSB_SW_MAX_QLEN)
-            return bsb_fail(ctx, BSB_ETOOLONG, "job %lld: qlen %d > %d", (long long)i, j.qlen, BSB_SW_MAX_QLEN);
-        boff[(size_t)i] = nb;
-        if (j.xtra & kXSubo) nb += j.tlen;
-        const int bin = kLenBins - 1 - std::min(j.tlen >> 4, kLenBins - 1);
-        const bool byte = j.xtra & kXByte;
-        const int sl = byte ? (j.qlen + 15) >> 4 : (j.qlen + 7) >> 3;
-        int k = -1;
-        if (byte && b8_ok && sl >= 1 && sl <= kPackMaxSeg8)
-            k = (kPackMaxSeg8 - sl) * kLenBins + bin, ++n_p8;
-        else if (!byte && w16_ok && sl >= 1 && sl <= kPackMaxSeg16 && (int64_t)j.qlen * S.qmax <= 32640)
-            k = kKeys8 + (kPackMaxSeg16 - sl) * kLenBins + bin, ++n_p16;
-        else if (byte)
-            ++n_fb8, max8 = std::max(max8, j.qlen);
-        else
-            ++n_fb16, max16 = std::max(max16, j.qlen);
-        key[(size_t)i] = k;
-        if (k >= 0) ++kcnt[(size_t)k + 1];
-    }
-    for (int k = 0; k < kKeys8 + kKeys16; ++k) kcnt[(size_t)k + 1] += kcnt[(size_t)k];
-    {   // lists: [packed byte | packed word | one-lane byte | one-lane word]
-        int64_t p8 = n_p8 + n_p16, p16 = n_p8 + n_p16 + n_fb8;
-        for (int64_t i = 0; i < n; ++i) {
-            const int k = key[(size_t)i];
-            if (k >= 0) lists[(size_t)kcnt[(size_t)k]++] = (int32_t)i;
-            else if (jobs[i].xtra & kXByte) lists[(size_t)p8++] = (int32_t)i;
-            else lists[(size_t)p16++] = (int32_t)i;
-        }
-    }
-    S.slen8 = std::max(1, (max8 + 15) / 16), S.slen16 = std::max(1, (max16 + 7) / 8);
     PackParams P8, P16;
     {
         for (int tc = 0; tc < 5; ++tc) {
@@ -404,7 +458,7 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     if ((rc = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice"))) return rc;
     cudaStream_t st = ctx->stream;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t jb = al(sizeof(bsb_sw_job_t) * (size_t)n), sb = al((size_t)seq_bytes), ob = al(8 * (size_t)n);
+    const size_t jb = al(sizeof(bsb_sw_job_t) * (size_t)n), sb = al((size_t)seq_bytes), ob = al(8 * ((size_t)n + 1));
     const size_t lb = al(sizeof(int32_t) * (size_t)n);
     if ((rc = bsb_ensure(ctx, in_buf, in_bytes, jb + sb + ob + lb + 256, "SW input staging"))) return rc;
     char *in = (char *)*in_buf;
@@ -412,6 +466,43 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     uint8_t *d_seq = (uint8_t *)(in + jb);
     int64_t *d_boff = (int64_t *)(in + jb + sb);
     int32_t *d_list = (int32_t *)(in + jb + sb + ob);
+    // the plan's scratch is the output's: a bin and a row count per job, the scan's sums, the bins
+    const size_t hb = al(sizeof(int) * kBins), tb = al(8 * (size_t)scan_tmp_words(n));
+    if ((rc = bsb_ensure(ctx, out_buf, out_bytes,
+                         std::max(sizeof(bsb_kswr_t) * (size_t)n, 2 * lb + 2 * hb + tb + 256) + 256, "SW output")))
+        return rc;
+    bsb_kswr_t *d_out = (bsb_kswr_t *)*out_buf;
+    char *pl = (char *)*out_buf;
+    int *d_bin = (int *)pl, *d_rows = (int *)(pl + lb), *d_hist = (int *)(pl + 2 * lb), *d_cur = (int *)(pl + 2 * lb + hb);
+    int64_t *d_tmp = (int64_t *)(pl + 2 * lb + 2 * hb);
+    SwPlan *d_plan = (SwPlan *)(pl + 2 * lb + 2 * hb + tb);
+    SwPlan plan{INT_MAX, 0, 0, 0, 0, 0, 0, 0};
+    const int pb = (int)std::min<int64_t>((n + kPlanThreads - 1) / kPlanThreads, (int64_t)ctx->n_sm * 4);
+    if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_jobs, jobs, sizeof(bsb_sw_job_t) * n, cudaMemcpyHostToDevice, st),
+                       "H2D jobs")) ||
+        (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_plan, &plan, sizeof plan, cudaMemcpyHostToDevice, st), "SW plan")) ||
+        (rc = bsb_cuda(ctx, cudaMemsetAsync(d_hist, 0, sizeof(int) * kBins, st), "SW plan")))
+        return rc;
+    sw_plan_kernel<<<pb, kPlanThreads, 0, st>>>(d_jobs, (int)n, seq_bytes, S.qmax, b8_ok, w16_ok, d_bin, d_rows, d_hist,
+                                                d_plan);
+    sw_plan_scan<<<1, 1024, 0, st>>>(d_hist, d_cur, d_plan);
+    sw_plan_scatter<<<pb, kPlanThreads, 0, st>>>(d_bin, (int)n, d_cur, d_list);
+    int64_t nb = 0;
+    if ((rc = bsb_cuda(ctx, scan_i32_i64(d_rows, n, d_boff, d_tmp, st), "SW plan")) ||
+        (seq_bytes && (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_seq, seq, seq_bytes, cudaMemcpyHostToDevice, st), "H2D seq"))) ||
+        (rc = bsb_cuda(ctx, cudaMemcpyAsync(&plan, d_plan, sizeof plan, cudaMemcpyDeviceToHost, st), "SW plan")) ||
+        (rc = bsb_cuda(ctx, cudaMemcpyAsync(&nb, d_boff + n, 8, cudaMemcpyDeviceToHost, st), "SW plan")) ||
+        (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "SW plan")))
+        return rc;
+    if (plan.bad != INT_MAX) {
+        const bsb_sw_job_t &j = jobs[plan.bad];
+        if (job_fault(j, seq_bytes) == 1)
+            return bsb_fail(ctx, BSB_EINVAL, "job %lld: bytes outside seq", (long long)plan.bad);
+        return bsb_fail(ctx, BSB_ETOOLONG, "job %lld: qlen %d > %d", (long long)plan.bad, j.qlen, BSB_SW_MAX_QLEN);
+    }
+    const int64_t n_p8 = plan.n_p8, n_hi16 = plan.n_hi - plan.n_p8, n_p16 = plan.n_p16 - plan.n_p8;
+    const int64_t n_fb8 = plan.n_fb8 - plan.n_p16, n_fb16 = plan.n_fb16 - plan.n_fb8;
+    S.slen8 = std::max(1, (plan.max8 + 15) / 16), S.slen16 = std::max(1, (plan.max16 + 7) / 8);
     const size_t bb = al(sizeof(int2) * (size_t)(nb > 0 ? nb : 1)), rb = al((size_t)n);
     constexpr size_t kCtrBytes = 4096;
     if ((rc = bsb_ensure(ctx, &ctx->arena2, &ctx->arena2_bytes, lb + rb + kCtrBytes + bb, "SW scratch"))) return rc;
@@ -422,15 +513,7 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     int *cnt = (int *)(a2 + lb + rb);
     int *ctr8 = cnt + 64, *ctr16 = cnt + 64 + kCtrInts;
     int2 *d_b = (int2 *)(a2 + lb + rb + kCtrBytes);
-    if ((rc = bsb_ensure(ctx, out_buf, out_bytes, sizeof(bsb_kswr_t) * (size_t)n + 256, "SW output"))) return rc;
-    bsb_kswr_t *d_out = (bsb_kswr_t *)*out_buf;
-    if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_jobs, jobs, sizeof(bsb_sw_job_t) * n, cudaMemcpyHostToDevice, st),
-                       "H2D jobs")) ||
-        (seq_bytes && (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_seq, seq, seq_bytes, cudaMemcpyHostToDevice, st), "H2D seq"))) ||
-        (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_boff, boff.data(), 8 * n, cudaMemcpyHostToDevice, st), "H2D offsets")) ||
-        (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_list, lists.data(), 4 * n, cudaMemcpyHostToDevice, st), "H2D lists")) ||
-        (rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, kCtrBytes, st), "SW counters")))
-        return rc;
+    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, kCtrBytes, st), "SW counters"))) return rc;
     // the word-lane and one-lane jobs on a second stream, beside the packed byte-lane jobs
     const bool side = n_p16 + n_fb8 + n_fb16 > 0;
     cudaStream_t st2 = ctx->ms.aux[0];
@@ -441,7 +524,7 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
         if (n_p16) {   // word lanes: the 17..40-segment part of the list, then the 1..16 part
             const int32_t *l16 = d_list + n_p8;
             int32_t *r16 = d_rlist + n_p8;
-            const int n_hi = (int)(kcnt[(size_t)(kKeys8 + (kPackMaxSeg16 - 16) * kLenBins - 1)] - n_p8), n16 = (int)n_p16;
+            const int n_hi = (int)n_hi16, n16 = (int)n_p16;
             if ((rc = bsb_cuda(ctx, sw_pack16_run_hi(false, P16, d_jobs, d_seq, l16, n_hi, d_boff, d_b, d_out, d_rsl,
                                                      ctr16, 0, ctx->n_sm, st2), "SW word-lane kernels")) ||
                 (rc = bsb_cuda(ctx, sw_pack16_run_lo(false, P16, d_jobs, d_seq, l16 + n_hi, n16 - n_hi, d_boff, d_b,
