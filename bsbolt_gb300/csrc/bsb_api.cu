@@ -224,13 +224,6 @@ struct JobScan {
     int64_t need;
 };
 
-static bool job_ok(const bsb_ext_job_t &j, int64_t seq_bytes, int qmax)
-{
-    return j.qlen >= 0 && j.tlen >= 0 && j.w >= 0 && j.flags == 0 && j.h0 > 0 && j.h0 <= (1 << 20) &&
-           j.qlen <= qmax && j.qoff >= 0 && j.toff >= 0 && j.qoff + j.qlen <= seq_bytes &&
-           j.toff + j.tlen <= seq_bytes && (int64_t)j.qlen + j.tlen <= (1 << 30);
-}
-
 // builtin: the number of the built-in map, -1 where tile_map is an installed one.
 static JobScan scan_jobs(const KswParams &P, const bsb_ext_job_t *jobs, int64_t lo, int64_t hi, int64_t seq_bytes,
                          const uint8_t *tile_map, int builtin)
@@ -239,7 +232,7 @@ static JobScan scan_jobs(const KswParams &P, const bsb_ext_job_t *jobs, int64_t 
     JobScan r{hi, 0, 0};
     for (int64_t i = lo; i < hi; ++i) {
         const bsb_ext_job_t &j = jobs[i];
-        if (!job_ok(j, seq_bytes, qmax)) {
+        if (!ext_job_ok(j, seq_bytes, qmax)) {
             r.first_bad = i;
             break;
         }
@@ -418,9 +411,13 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     const int builtin = ksw_builtin(per, ctx->n_sm);      // one map for all pieces
     P.pack16 = ksw_pack16(P);
     const bool installed = ctx->d_tile_map != nullptr;
-    scan_pieces(P, jobs, n_jobs, per, nck, seq_bytes, installed ? ctx->tile_map : ksw_builtin_tile_map(builtin),
+    // Batches of one piece, from a few thousand jobs on: the scan is a kernel over the copied jobs, which goes on while
+    // the sequences follow.  On one host thread it took 165 of 835 us for 64k jobs of 10-140 bases and 280 of 4300
+    // for 50k of 100-600.  It would also have told how much of seq the jobs use, so not where seq may be mostly others'.
+    const bool on_device = nck == 1 && n_jobs >= 4096 && seq_bytes / 2048 <= n_jobs;
+    if (!on_device) scan_pieces(P, jobs, n_jobs, per, nck, seq_bytes, installed ? ctx->tile_map : ksw_builtin_tile_map(builtin),
                 installed ? -1 : builtin, piece);
-    for (int k = 0; k < nck; ++k)          // every job is checked before any device work
+    for (int k = 0; k < nck && !on_device; ++k)          // every job is checked before any other use of it
         if (piece[k].first_bad < n_jobs) return check_jobs(ctx, jobs + piece[k].first_bad, 1, seq_bytes,
                                                            piece[k].first_bad);
     if ((rc = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice"))) return rc;
@@ -442,6 +439,20 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     // the stream must not still read the staging buffers from an earlier call when h2d overwrites them
     if ((rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "stream synchronize"))) return rc;
     int64_t done = 0;
+    if (on_device) {
+        ExtScan sc;
+        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_jobs, jobs, jb, cudaMemcpyHostToDevice, ctx->h2d), "H2D jobs")) ||
+            (rc = bsb_cuda(ctx, ksw_scan_jobs(P, d_jobs, n_jobs, seq_bytes, ctx->d_tile_map, builtin,
+                                              (ExtScan *)ctx->scratch, ctx->n_sm, ctx->h2d), "job scan")) ||
+            (seq_bytes && (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_seq, seq, seq_bytes, cudaMemcpyHostToDevice, ctx->h2d),
+                                         "H2D seq"))) ||
+            (rc = bsb_cuda(ctx, cudaMemcpyAsync(&sc, ctx->scratch, sizeof sc, cudaMemcpyDeviceToHost, ctx->h2d),
+                           "job scan")) ||
+            (rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->h2d), "job scan")))
+            return rc;
+        if (sc.bad) return check_jobs(ctx, jobs + (n_jobs - (int64_t)sc.bad), 1, seq_bytes, n_jobs - (int64_t)sc.bad);
+        piece[0].tiles = sc.tiles, piece[0].need = done = (int64_t)sc.need;
+    }
     for (int k = 0; k < nck; ++k) {
         const int64_t lo = k * per, cnt = n_jobs - lo < per ? n_jobs - lo : per;
         const int64_t need = piece[k].need;
@@ -452,8 +463,9 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
                            "H2D seq")))
             return rc;
         done = need > done ? need : done;
-        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_jobs + lo, jobs + lo, sizeof(bsb_ext_job_t) * cnt,
-                                                cudaMemcpyHostToDevice, ctx->h2d), "H2D jobs")) ||
+        if ((!on_device &&
+             (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_jobs + lo, jobs + lo, sizeof(bsb_ext_job_t) * cnt,
+                                                 cudaMemcpyHostToDevice, ctx->h2d), "H2D jobs"))) ||
             (rc = bsb_cuda(ctx, cudaEventRecord(ev[0], ctx->h2d), "event")) ||
             (rc = bsb_cuda(ctx, cudaStreamWaitEvent(ctx->stream, ev[0], 0), "event")))
             return rc;

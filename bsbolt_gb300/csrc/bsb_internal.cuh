@@ -183,6 +183,20 @@ uint64_t ksw_map_tiles(const uint8_t *map);
 // The same for a built-in map, with the place ksw_ring_tile() of the ring's jobs (ksw_tiles.cuh); and whether
 // ksw_launch puts job j there on that map (P.pack16 as ksw_pack16 has it), queries below ksw_ring_from() never.
 uint64_t ksw_builtin_tiles(int builtin);
+// What the host entry needs of a batch before it can run: n less the first job that fails the preconditions (0: none
+// does), the shapes its jobs map to, and the end of the sequence bytes they reference.
+struct ExtScan {
+    unsigned long long bad, tiles, need;
+};
+__host__ __device__ __forceinline__ bool ext_job_ok(const bsb_ext_job_t &j, int64_t seq_bytes, int qmax)
+{
+    return j.qlen >= 0 && j.tlen >= 0 && j.w >= 0 && j.flags == 0 && j.h0 > 0 && j.h0 <= (1 << 20) &&
+           j.qlen <= qmax && j.qoff >= 0 && j.toff >= 0 && j.qoff + j.qlen <= seq_bytes &&
+           j.toff + j.tlen <= seq_bytes && (int64_t)j.qlen + j.tlen <= (1 << 30);
+}
+// The scan on the device: *out from d_jobs (out zeroed on st first).  d_map, builtin as in ksw_launch.
+cudaError_t ksw_scan_jobs(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
+                          const uint8_t *d_map, int builtin, ExtScan *out, int n_sm, cudaStream_t st);
 int ksw_ring_tile();
 int ksw_ring_from(int builtin);
 bool ksw_takes_ring(const KswParams &P, const bsb_ext_job_t &j, int builtin);

@@ -261,6 +261,40 @@ ksw_sched_scatter_tiles(const int32_t *__restrict__ key, int n, int *__restrict_
         if (k[u] != kDoneKey) order[sh[k[u]] + at[u]] = (int32_t)(base + u * kScatterThreads + threadIdx.x);
 }
 
+__global__ void __launch_bounds__(256)
+ksw_scan_kernel(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int64_t n, int64_t seq_bytes,
+                const uint8_t *__restrict__ map, int builtin, ExtScan *__restrict__ out)
+{
+    const int lane = threadIdx.x & 31, ring = ring_of(builtin);
+    unsigned long long bad = 0, need = 0;
+    unsigned lo = 0, hi = 0;
+    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + lane;
+        if (i >= n) continue;
+        const bsb_ext_job_t j = jobs[i];
+        if (!ext_job_ok(j, seq_bytes, kMaxNeed - 1)) {
+            bad = max(bad, (unsigned long long)(n - i));
+            continue;
+        }
+        const int t = map ? map[j.qlen + 1]
+                      : P.pack16 && ksw_ring_fits(P, j, ring) ? kRingTile : c_tile_maps[builtin].tile[j.qlen + 1];
+        if (t < 32) lo |= 1u << t;
+        else hi |= 1u << (t - 32);
+        need = max(need, (unsigned long long)max(j.qoff + j.qlen, j.toff + j.tlen));
+    }
+    lo = __reduce_or_sync(BSB_FULL_MASK, lo), hi = __reduce_or_sync(BSB_FULL_MASK, hi);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        bad = max(bad, __shfl_xor_sync(BSB_FULL_MASK, bad, d));
+        need = max(need, __shfl_xor_sync(BSB_FULL_MASK, need, d));
+    }
+    if (lane == 0) {
+        if (bad) atomicMax(&out->bad, bad);
+        atomicOr(&out->tiles, (unsigned long long)hi << 32 | lo);
+        atomicMax(&out->need, need);
+    }
+}
+
 }  // namespace
 
 static_assert(kRejectKey % kClasses == 0, "the reject slot starts a bin");
@@ -311,6 +345,16 @@ uint64_t ksw_map_tiles(const uint8_t *map)
 }
 
 uint64_t ksw_builtin_tiles(int builtin) { return ksw_map_tiles(kBuiltinTileMaps[builtin].tile) | 1ull << kRingTile; }
+
+cudaError_t ksw_scan_jobs(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
+                          const uint8_t *d_map, int builtin, ExtScan *out, int n_sm, cudaStream_t st)
+{
+    cudaError_t e = cudaMemsetAsync(out, 0, sizeof *out, st);
+    if (e != cudaSuccess) return e;
+    ksw_scan_kernel<<<(int)min((n + 255) / 256, (int64_t)n_sm * 2), 256, 0, st>>>(P, d_jobs, n, seq_bytes, d_map, builtin,
+                                                                                  out);
+    return cudaGetLastError();
+}
 
 int ksw_ring_from(int builtin) { return ring_cols(ring_of(builtin)); }
 

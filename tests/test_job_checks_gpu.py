@@ -70,3 +70,24 @@ def test_mate_rescue_jobs(gpu_ctx, field, value, code, at):
     for f in want.dtype.names:
         if f in got.dtype.names:
             assert np.array_equal(got[f], want[f]), f
+
+
+@pytest.mark.parametrize("field,value,code", [("qoff", -1, "EINVAL"), ("toff", 1 << 40, "EINVAL"), ("qlen", -1, "EINVAL"),
+                                              ("qlen", 1024, "ETOOLONG"), ("tlen", -1, "EINVAL"), ("w", -1, "EINVAL"),
+                                              ("h0", 0, "EINVAL"), ("h0", (1 << 20) + 1, "EINVAL"), ("flags", 1, "EINVAL")])
+@pytest.mark.parametrize("n", [4095, 4096])              # checked on the host, on the device
+def test_extension_jobs(gpu_ctx, field, value, code, n):
+    from bsbolt_gb300 import extend
+    jobs, seq = synth.ksw_jobs(n, seed=3, qmin=1, qmax=300)
+    mat = synth.fill_scmat(1, 4)
+    for at in (0, 1000, n - 1):
+        bad = jobs.copy()
+        bad[field][at:] = value
+        with pytest.raises(_lib.BsbError, match=f"job {at}:") as e:
+            extend.ksw_extend2_batch(gpu_ctx, bad, np.concatenate([seq, np.zeros(2000, np.uint8)]), mat, 6, 1, 6, 1, 100)
+        assert e.value.code == getattr(_lib, "BSB_" + code)
+    want, _ = oracle.ksw_batch(jobs, seq, mat, 6, 1, 6, 1, 100, n_threads=8)
+    assert np.array_equal(extend.ksw_extend2_batch(gpu_ctx, jobs, seq, mat, 6, 1, 6, 1, 100), want)
+    # a buffer of which the jobs use a small part
+    wide = np.concatenate([seq, np.zeros(4096 * 2048 + (1 << 20), np.uint8)])
+    assert np.array_equal(extend.ksw_extend2_batch(gpu_ctx, jobs, wide, mat, 6, 1, 6, 1, 100), want)
