@@ -558,7 +558,8 @@ chain_kernel(AlnOpt opt, DevBns B, const int *__restrict__ list, const int *__re
 // rows, 20 chains a read), some 20,000 cycles a row; a warp per read with chain_general on shared
 // memory 1.03 ms (75,000 cycles a read: 960 a row, 12,500 the sort, 14,800 the filter); this 0.63 ms
 // (114k RRBS reads 1.78 -> 0.74 ms, 64 reads 78 -> 19 us), 6000 instructions a read with the issue
-// slots 71 % busy.  40 warps per SM (48 registers): 24 at 80 registers 0.68, 32 at 64 0.65.
+// slots 71 % busy; with the longest reads first (order_hist_rows) and chain_general's filter by kept chains 0.50
+// and 0.51.  40 warps per SM (48 registers): 24 at 80 registers 0.68, 32 at 64 0.65.
 constexpr int kFastRows = 128, kFastChains = 64, kChainWarps = 4;
 
 struct FastChain {
@@ -929,6 +930,11 @@ __device__ __forceinline__ float repeat_share(const AlnOpt &opt, int len, const 
     return (float)l_rep / len;
 }
 
+// Chains as weight << 20 | place, descending weight.
+struct PackedWeightLt {
+    __device__ bool operator()(int x, int y) const { return x >> 20 > y >> 20; }
+};
+
 // False: left to chain_kernel.  n_out: kept chains.
 __device__ __noinline__ bool chain_general(const AlnOpt &opt, const DevBns &B, float frac_rep, const DevIntv *seeds,
                                            int ns, const int64_t *roff, int64_t R0, int R, const uint64_t *pos,
@@ -1092,56 +1098,65 @@ __device__ __noinline__ bool chain_general(const AlnOpt &opt, const DevBns &B, f
         __syncwarp();
         if (!equal) {
             for (int k = lane; k < n; k += 32) A.order[k] = A.row_at[k];
-        } else if (lane == 0) {
-            int stk_l[64], stk_r[64], stk_d[64];
-            KsSort<FltLt> fs{A.order, FltLt{A.weight}};
-            fs.sort(n, stk_l, stk_r, stk_d);
+        } else {
+            // one word for weight and chain where they fit (a weight is at most the read's length): a comparison
+            // is then one load
+            bool fits = n_chn <= 1 << 20;
+            for (int k = lane; k < n; k += 32) fits &= A.weight[A.order[k]] < 1 << 11;
+            fits = __all_sync(BSB_FULL_MASK, fits);
+            if (fits) {
+                for (int k = lane; k < n; k += 32) A.order[k] |= A.weight[A.order[k]] << 20;
+                __syncwarp();
+            }
+            if (lane == 0) {
+                int stk_l[64], stk_r[64], stk_d[64];
+                if (fits) KsSort<PackedWeightLt>{A.order, PackedWeightLt{}}.sort(n, stk_l, stk_r, stk_d);
+                else KsSort<FltLt>{A.order, FltLt{A.weight}}.sort(n, stk_l, stk_r, stk_d);
+            }
+            __syncwarp();
+            if (fits)
+                for (int k = lane; k < n; k += 32) A.order[k] &= (1 << 20) - 1;
         }
         __syncwarp();
     }
-    int *const kept = A.row_chain, *const first = A.row_at, *const list = A.row_q;
+    // the kept chains one after the other, as in chain_fast: all chains behind one at once.  kept: first the marks
+    // (1 overlaps a kept chain, 2 is a first, 4 dropped)
+    int *const kept = A.row_chain, *const first = A.row_at;
     for (int k = lane; k < n; k += 32) kept[k] = 0, first[k] = -1;
     __syncwarp();
-    if (lane == 0) kept[0] = 3, list[0] = 0;
-    __syncwarp();
-    int n_kept = 1;
-    for (int i = 1; i < n; ++i) {
-        const int ci = A.order[i], wi = A.weight[ci];
-        const int bi = A.first_qbeg[ci], ei = A.last_qbeg[ci] + A.last_len[ci];
-        bool large = false, drop = false;
-        for (int base = 0; base < n_kept && !drop; base += 32) {
-            bool ovl = false, end = false;
-            int j = 0;
-            if (base + lane < n_kept) {
-                j = list[base + lane];
-                const int cj = A.order[j], wj = A.weight[cj];
-                const int bj = A.first_qbeg[cj], ej = A.last_qbeg[cj] + A.last_len[cj];
-                const int b_max = bj > bi ? bj : bi, e_min = ej < ei ? ej : ei;
+    for (int j = 0; j < n;) {
+        const int cj = A.order[j], wj = A.weight[cj];
+        const int bj = A.first_qbeg[cj], ej = A.last_qbeg[cj] + A.last_len[cj];
+        int f = -1, next = n;
+        for (int base = (j + 1) & ~31; base < n; base += 32) {
+            const int k = base + lane;
+            bool ovl = false, live = false;
+            if (k > j && k < n && !(kept[k] & 4)) {
+                live = true;
+                const int ck = A.order[k], wk = A.weight[ck];
+                const int bk = A.first_qbeg[ck], ek = A.last_qbeg[ck] + A.last_len[ck];
+                const int b_max = bj > bk ? bj : bk, e_min = ej < ek ? ej : ek;
                 if (e_min > b_max) {                     // no ALT contigs: the is_alt test always passes
-                    const int li = ei - bi, lj = ej - bj, min_l = li < lj ? li : lj;
+                    const int lk = ek - bk, lj = ej - bj, min_l = lk < lj ? lk : lj;
                     if (e_min - b_max >= min_l * opt.mask_level && min_l < opt.max_chain_gap) {
                         ovl = true;
-                        end = wi < wj * opt.drop_ratio && wj - wi >= opt.min_seed_len << 1;
+                        live = !(wk < wj * opt.drop_ratio && wj - wk >= opt.min_seed_len << 1);
+                        kept[k] |= live ? 1 : 5;
                     }
                 }
             }
-            // the reference stops at the first chain that drops this one: those after it see nothing
-            const unsigned me = __ballot_sync(BSB_FULL_MASK, end);
-            const unsigned seen = me ? (2u << (__ffs(me) - 1)) - 1u : 0xffffffffu;
-            ovl = ovl && (seen >> lane & 1u);
-            if (ovl && first[j] < 0) first[j] = i;
-            large |= __any_sync(BSB_FULL_MASK, ovl);
-            drop = me != 0;
-        }
-        if (!drop) {
-            if (lane == 0) list[n_kept] = i, kept[i] = large ? 2 : 3;
-            ++n_kept;
+            const unsigned mo = __ballot_sync(BSB_FULL_MASK, ovl), ml = __ballot_sync(BSB_FULL_MASK, live);
+            if (mo && f < 0) f = base + __ffs(mo) - 1;
+            if (ml && next == n) next = base + __ffs(ml) - 1;
         }
         __syncwarp();
+        if (lane == 0 && f >= 0) first[j] = f, kept[f] |= 2;
+        __syncwarp();
+        j = next;
     }
-    for (int k = lane; k < n_kept; k += 32) {
-        const int f = first[list[k]];
-        if (f >= 0) kept[f] = 1;
+    for (int k = lane; k < n; k += 32) {
+        const int m = kept[k];
+        kept[k] = m & 2 ? 1 : m & 4 ? 0 : m & 1 ? 2 : 3;
     }
     __syncwarp();
     if (n >= opt.max_chain_extend) {
@@ -1180,12 +1195,14 @@ chain_warp_kernel(AlnOpt opt, DevBns B, int n_reads, const int64_t *__restrict__
                   const int64_t *__restrict__ row_off_of_seed, const uint64_t *__restrict__ pos,
                   ChainRec *__restrict__ chains, BtNode *__restrict__ nodes, int *__restrict__ row_chain,
                   int *__restrict__ iwork, DevSeed *__restrict__ out_seeds, DevChain *__restrict__ out_chains,
-                  int *__restrict__ n_chains, int *__restrict__ left, int *__restrict__ n_left)
+                  int *__restrict__ n_chains, int *__restrict__ left, int *__restrict__ n_left,
+                  const int *__restrict__ order)
 {
     __shared__ ChainSmem sm[kChainWarps];
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
-    const int r = blockIdx.x * kChainWarps + wb;
+    int r = blockIdx.x * kChainWarps + wb;
     if (r >= n_reads) return;
+    if (order) r = order[r];
     const int len = (int)(read_off[r + 1] - read_off[r]);
     const int64_t s0 = seed_off[r], s1 = seed_off[r + 1];
     const int64_t R0 = row_off_of_seed[s0];
@@ -1984,6 +2001,30 @@ order_scatter(const int *__restrict__ n_chains, int n_reads, const int *__restri
     order_place(n_reads, cnt, cur, order, [=](int r) { return order_bin(n_chains[r]); });
 }
 
+// The order chain_warp_kernel takes a large batch's reads in: most rows first, in steps of four.  A read on
+// chain_general takes up to 0.25 ms, and a few such among 67k reads, met anywhere in the batch, set the end of the
+// kernel; and the four reads of a block then take about as long as one another.  67k reads of 150 bases 0.64 -> 0.50
+// ms, 114k RRBS reads 0.74 -> 0.51, the sort 11 us of it.
+__device__ __forceinline__ int rows_bin(const int64_t *__restrict__ seed_off, const int64_t *__restrict__ row_off_of_seed,
+                                        int r)
+{
+    const int64_t q = (row_off_of_seed[seed_off[r + 1]] - row_off_of_seed[seed_off[r]]) >> 2;
+    return kOrderBins - 1 - (int)(q < kOrderBins - 1 ? q : kOrderBins - 1);
+}
+constexpr int kRowOrderReads = 2048;    // smaller batches fit the GPU at once
+__global__ void __launch_bounds__(kOrderThreads)
+order_hist_rows(const int64_t *__restrict__ seed_off, const int64_t *__restrict__ row_off_of_seed, int n_reads,
+                int *__restrict__ cnt)
+{
+    order_count(n_reads, cnt, [=](int r) { return rows_bin(seed_off, row_off_of_seed, r); });
+}
+__global__ void __launch_bounds__(kOrderThreads)
+order_scatter_rows(const int64_t *__restrict__ seed_off, const int64_t *__restrict__ row_off_of_seed, int n_reads,
+                   const int *__restrict__ cnt, int *__restrict__ cur, int *__restrict__ order)
+{
+    order_place(n_reads, cnt, cur, order, [=](int r) { return rows_bin(seed_off, row_off_of_seed, r); });
+}
+
 // One warp per read (reads hold a few regions each).
 __global__ void compact_regs(const bsb_reg_t *__restrict__ regs, const int64_t *__restrict__ seed_off,
                              const int64_t *__restrict__ row_off_of_seed, int n_reads, const int *__restrict__ n_regs,
@@ -2613,9 +2654,18 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     P.mat_max = mx;
     P.pack16 = 0;
     int *const left = (int *)(A + o_order);                  // reads for chain_kernel (the read order comes after)
+    int *by_rows = nullptr;
+    if (n_reads >= kRowOrderReads) {
+        int *const cnt = (int *)(A + o_order + al(sizeof(int) * (n_reads + 1)));
+        by_rows = (int *)(A + o_bail);
+        const int ob = std::min((n_reads + kOrderThreads - 1) / kOrderThreads, ctx->n_sm * 4);
+        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, sizeof(int) * 2 * kOrderBins, st), "read order"))) return rc;
+        order_hist_rows<<<ob, kOrderThreads, 0, st>>>(d_seed_off, roff, n_reads, cnt);
+        order_scatter_rows<<<ob, kOrderThreads, 0, st>>>(d_seed_off, roff, n_reads, cnt, cnt + kOrderBins, by_rows);
+    }
     chain_warp_kernel<<<(n_reads + kChainWarps - 1) / kChainWarps, kChainWarps * 32, 0, st>>>(
         ao, B, n_reads, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos, chains, nodes, row_chain, iwork,
-        cseeds, cchains, n_chains, left, ctrl);
+        cseeds, cchains, n_chains, left, ctrl, by_rows);
     chain_kernel<<<ctx->n_sm, 128, 0, st>>>(ao, B, left, ctrl, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos,
                                             chains, nodes, row_chain, iwork, cseeds, cchains, n_chains);
     if (h_min_hsp &&
