@@ -2543,7 +2543,10 @@ static int first_extensions(bsb_ctx *ctx, const bsb_align_opt_t *o, const AlnOpt
     const size_t o_right = off; off += al(sizeof(bsb_ext_job_t) * T);
     const size_t o_out = off; off += al(sizeof(bsb_ext_out_t) * 2 * T);
     const size_t o_scr = off; off += al(ksw_scratch_bytes(T));
-    if ((rc = bsb_ensure(ctx, &ctx->pre_buf, &ctx->pre_bytes, off, "chain extensions"))) return rc;
+    if (bsb_ensure(ctx, &ctx->pre_buf, &ctx->pre_bytes, off, "chain extensions")) {
+        cudaGetLastError();              // no room: chain2aln_kernel extends every seed itself
+        return 0;
+    }
     char *const D = (char *)ctx->pre_buf;
     PreChain *const pc = (PreChain *)(D + o_pre);
     bsb_ext_job_t *const left = (bsb_ext_job_t *)(D + o_left), *const right = (bsb_ext_job_t *)(D + o_right);
