@@ -156,6 +156,71 @@ __device__ __forceinline__ bool ksw_diagonal(const int8_t *tab, int a, int lim, 
     return on;
 }
 
+// ksw_diagonal for jobs of a byte buffer, 8 lanes a job: a lane takes 4 columns side by side as one word of each
+// sequence (two aligned loads, both inside the buffer, else bytes), and where the words agree on bases 0..3 that
+// score `a` on themselves (plain) nothing is lost and nothing looked up.  Losses are never negative, so the job is on
+// while the total is below lim, and the diagonal's best prefix is the largest of its values just before the
+// columns that lose and at its end, the first of equals.
+__device__ __forceinline__ uint32_t word_at(const uint8_t *p)
+{
+    const uint32_t *const w = (const uint32_t *)((uintptr_t)p & ~(uintptr_t)3);
+    return __funnelshift_r(w[0], w[1], 8 * (unsigned)((uintptr_t)p & 3));
+}
+__device__ __forceinline__ bool ksw_diagonal_words(const int8_t *tab, int a, bool plain, int lim, int qlen, int tlen,
+                                                   int h0, const uint8_t *q, const uint8_t *t, const uint8_t *buf,
+                                                   const uint8_t *buf_end, int lane, int &best, int &best_j, int &last)
+{
+    const int gl = lane & 7;
+    bool on = lim > 0 && qlen >= 1 && tlen >= qlen;
+    int loss = 0, key = 0;                       // key: the best prefix above h0 so far, << 11, and 2047 less its length
+    for (int c0 = 0; __any_sync(BSB_FULL_MASK, on && c0 < qlen); c0 += 32) {
+        const int j = c0 + 4 * gl;
+        int l[4] = {0, 0, 0, 0};
+        if (on && j < qlen) {
+            uint32_t x = 0, y = 0;
+            const int n = min(qlen - j, 4);
+            if (((max((uintptr_t)q, (uintptr_t)t) + j) | 3) + 4 < (uintptr_t)buf_end &&
+                ((min((uintptr_t)q, (uintptr_t)t) + j) & ~(uintptr_t)3) >= (uintptr_t)buf) {
+                x = word_at(q + j), y = word_at(t + j);
+            } else {
+                for (int k = 0; k < n; ++k) x |= (uint32_t)q[j + k] << 8 * k, y |= (uint32_t)t[j + k] << 8 * k;
+            }
+            const uint32_t in = n == 4 ? 0xffffffffu : (1u << 8 * n) - 1u;
+            if (!plain || (((x ^ y) | (x & 0xfcfcfcfcu)) & in)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < n) l[k] = a - tab[min(y >> 8 * k & 255u, 4u) << 3 | min(x >> 8 * k & 255u, 4u)];
+            }
+        }
+        const int sum = l[0] + l[1] + l[2] + l[3];
+        if (!__any_sync(BSB_FULL_MASK, sum != 0)) continue;
+        int incl = sum;
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) {
+            const int v = __shfl_up_sync(BSB_FULL_MASK, incl, d, 8);
+            if (gl >= d) incl += v;
+        }
+        int before = loss + incl - sum;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int v = a * (j + k) - before;
+            if (l[k] && v > 0) key = max(key, v << 11 | (2047 - (j + k)));
+            before += l[k];
+        }
+        loss += __shfl_sync(BSB_FULL_MASK, incl, 7, 8);
+        on = on && loss < lim;
+    }
+    {
+        const int v = a * qlen - loss;
+        if (v > 0) key = max(key, v << 11 | (2047 - qlen));
+    }
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) key = max(key, __shfl_xor_sync(BSB_FULL_MASK, key, d, 8));
+    best = h0 + (key >> 11), best_j = key ? 2047 - (key & 2047) - 1 : -1;
+    last = h0 + a * qlen - loss;
+    return on;
+}
+
 // Rows that can no longer change a result.  After row i every cell of a later row is reached from
 // H(i, j-1) or E(i+1, j) of some column j (stale cells beyond the band included: the band can grow
 // back over them), gaining at most a = max(mat) per remaining column, and from nothing where both

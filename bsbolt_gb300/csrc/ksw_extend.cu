@@ -108,6 +108,7 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+    const bool plain = tab[0] == P.mat_max && tab[9] == P.mat_max && tab[18] == P.mat_max && tab[27] == P.mat_max;
     for (long long i0 = (long long)((int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; i0 < n;
          i0 += (long long)warps * per) {
         const int i = (int)(i0 + lane);
@@ -156,7 +157,13 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
                 const int qlen = __shfl_sync(BSB_FULL_MASK, jb.qlen, b), tlen = __shfl_sync(BSB_FULL_MASK, jb.tlen, b);
                 const int h0 = __shfl_sync(BSB_FULL_MASK, jb.h0, b), lm = __shfl_sync(BSB_FULL_MASK, lim, b);
                 int best, best_j, last;
-                const bool known = ksw_diagonal<8>(tab, P.mat_max, lm, qlen, tlen, h0, acc, lane, best, best_j, last);
+                bool known;
+                if constexpr (Packed) {
+                    known = ksw_diagonal<8>(tab, P.mat_max, lm, qlen, tlen, h0, acc, lane, best, best_j, last);
+                } else {
+                    known = ksw_diagonal_words(tab, P.mat_max, plain, lm, qlen, tlen, h0, acc.qs.p, acc.ts.p,
+                                               seq, seq + seq_bytes, lane, best, best_j, last);
+                }
                 if (known && (lane & 7) == 0) {
                     bsb_ext_out_t o;
                     o.score = best; o.qle = o.tle = best_j + 1;
