@@ -160,7 +160,8 @@ __device__ __forceinline__ bool ksw_diagonal(const int8_t *tab, int a, int lim, 
 // sequence (two aligned loads, both inside the buffer, else bytes), and where the words agree on bases 0..3 that
 // score `a` on themselves (plain) nothing is lost and nothing looked up.  Losses are never negative, so the job is on
 // while the total is below lim, and the diagonal's best prefix is the largest of its values just before the
-// columns that lose and at its end, the first of equals.
+// columns that lose and at its end, the first of equals.  loss: the whole diagonal's (where the job is on); lowest: the
+// smallest of h0 and the diagonal's values just behind the columns that lose.
 __device__ __forceinline__ uint32_t word_at(const uint8_t *p)
 {
     const uint32_t *const w = (const uint32_t *)((uintptr_t)p & ~(uintptr_t)3);
@@ -168,11 +169,13 @@ __device__ __forceinline__ uint32_t word_at(const uint8_t *p)
 }
 __device__ __forceinline__ bool ksw_diagonal_words(const int8_t *tab, int a, bool plain, int lim, int qlen, int tlen,
                                                    int h0, const uint8_t *q, const uint8_t *t, const uint8_t *buf,
-                                                   const uint8_t *buf_end, int lane, int &best, int &best_j, int &last)
+                                                   const uint8_t *buf_end, int lane, int &best, int &best_j, int &last,
+                                                   int &loss, int &lowest)
 {
     const int gl = lane & 7;
     bool on = lim > 0 && qlen >= 1 && tlen >= qlen;
-    int loss = 0, key = 0;                       // key: the best prefix above h0 so far, << 11, and 2047 less its length
+    int low = h0, key = 0;                       // key: the best prefix above h0 so far, << 11, and 2047 less its length
+    loss = 0;
     for (int c0 = 0; __any_sync(BSB_FULL_MASK, on && c0 < qlen); c0 += 32) {
         const int j = c0 + 4 * gl;
         int l[4] = {0, 0, 0, 0};
@@ -206,6 +209,7 @@ __device__ __forceinline__ bool ksw_diagonal_words(const int8_t *tab, int a, boo
             const int v = a * (j + k) - before;
             if (l[k] && v > 0) key = max(key, v << 11 | (2047 - (j + k)));
             before += l[k];
+            if (l[k]) low = min(low, h0 + a * (j + k + 1) - before);
         }
         loss += __shfl_sync(BSB_FULL_MASK, incl, 7, 8);
         on = on && loss < lim;
@@ -215,10 +219,32 @@ __device__ __forceinline__ bool ksw_diagonal_words(const int8_t *tab, int a, boo
         if (v > 0) key = max(key, v << 11 | (2047 - qlen));
     }
 #pragma unroll
-    for (int d = 4; d > 0; d >>= 1) key = max(key, __shfl_xor_sync(BSB_FULL_MASK, key, d, 8));
+    for (int d = 4; d > 0; d >>= 1) {
+        key = max(key, __shfl_xor_sync(BSB_FULL_MASK, key, d, 8));
+        low = min(low, __shfl_xor_sync(BSB_FULL_MASK, low, d, 8));
+    }
+    lowest = low;
     best = h0 + (key >> 11), best_j = key ? 2047 - (key & 2047) - 1 : -1;
     last = h0 + a * qlen - loss;
     return on;
+}
+
+// How far a job's band can be cut without changing its result.  Notation and bound of ksw_diagonal: with L the whole
+// diagonal's loss and D such that o + e(D+1) > L for both gaps, a path that leaves the 2D + 1 diagonals around the main
+// one is worth less than the main diagonal in the same row or column from there on.  So it is never a row's maximum
+// (nor ties with it), and never the last column's best, up to row qlen-1; behind it nothing but those diagonals can
+// reach D(qlen-1) in the last column, and they end by row qlen-1+D.  A cell of those diagonals whose value comes
+// from such a path is itself below the main diagonal, and so are the cells it leads to.  What is left is that the
+// reference computes all 2D + 1 diagonals in every row, whatever its band w >= D (the band follows the non-zero cells: so
+// the main diagonal has to exceed o + eD everywhere, which keeps the gaps from it non-zero that far), and that no
+// row up to qlen-1+D ends the job: it is non-zero by the same condition, and its drop is at most L + o_del + e_del D.
+// Then every band from D on gives the same six results.  Returns D, or -1 where the conditions do not hold.
+__device__ __forceinline__ int cut_band(const KswParams &P, int loss, int lowest)
+{
+    const int D = max(0, max((loss - P.o_del) / P.e_del, (loss - P.o_ins) / P.e_ins));
+    if (lowest <= max(P.o_del + P.e_del * D, P.o_ins + P.e_ins * D)) return -1;
+    if (P.zdrop > 0 && loss + P.o_del + P.e_del * D > P.zdrop) return -1;
+    return D;
 }
 
 // Rows that can no longer change a result.  After row i every cell of a later row is reached from

@@ -30,7 +30,8 @@
 // (h0 + qlen * max(mat) > kPack16MaxH) is binned last in its shape and runs on
 // the 32-bit kernel.  Results never depend on the shape, the cell width or the
 // order.  Long queries with a narrow band run on registers that move along with the band
-// (ksw_ring16.cu) where the scheduler's own maps are in use.
+// (ksw_ring16.cu) where the scheduler's own maps are in use; so do, in large batches, jobs whose band can be cut
+// (cut_band, ksw_core.cuh).
 
 #include <climits>
 #include <cstdio>
@@ -85,6 +86,14 @@ struct JobAcc {
     __device__ __forceinline__ int t(int i) const { return (int)ts.base(P, i); }
 };
 
+// A job's band as ksw.c:399-407 cuts it.
+__device__ __forceinline__ int clamped_band(const KswParams &P, const bsb_ext_job_t &j)
+{
+    const int mi = band_cap(j.qlen * P.mat_max + j.end_bonus - P.o_ins, P.e_ins);
+    const int md = band_cap(j.qlen * P.mat_max + j.end_bonus - P.o_del, P.e_del);
+    return min(min(j.w, max(mi, 1)), max(md, 1));
+}
+
 // Keys and their histogram; and, unless cells are counted, the jobs whose result the main
 // diagonal decides (ksw_diagonal): these are answered here, get the key kDoneKey and are never
 // issued.  A warp takes `per` jobs at a time: a lane each for the checks and the key, then four
@@ -98,7 +107,7 @@ template <bool Packed>
 __global__ void __launch_bounds__(kHistThreads)
 ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long long seq_bytes,
                const uint8_t *__restrict__ seq, const int32_t *__restrict__ cost, const uint8_t *__restrict__ map,
-               int builtin, int ring, int diagonals, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist,
+               int builtin, int ring, int diagonals, int cuts, int per, bsb_ext_out_t *__restrict__ out, int *__restrict__ hist,
                int32_t *__restrict__ key_out)
 {
     __shared__ int sh[kHistSlots];
@@ -143,6 +152,17 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
         }
         if (diagonals) {
             const int lim = key != kRejectKey && in ? diagonal_limit(P, jb.h0) : 0;
+            // the widest ring a job's query pays for, and how far its diagonal is followed for that
+            int cut = -1, band = 0, far = lim;
+            if (!Packed && cuts && lim > 0 && key % kClasses != kWideClass) {
+                band = clamped_band(P, jb);
+#pragma unroll
+                for (int c = 0; c < kCutRings; ++c)
+                    if (cuts >> c & 1 && jb.qlen + 1 >= cut_from(c, builtin) && band > cut_width(c)) cut = c;
+                if (jb.qlen + 32 >= 1024) cut = -1;
+                if (cut >= 0)
+                    far = max(lim, min(P.o_del + P.e_del * (cut_width(cut) + 1), P.o_ins + P.e_ins * (cut_width(cut) + 1)));
+            }
             const JobText<Packed> qt = job_query<Packed>(seq, jb), tt = job_target<Packed>(seq, jb);
             for (int r = 0; r < per; r += 4) {
                 const int b = r + (lane >> 3);
@@ -158,17 +178,36 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
                 const int h0 = __shfl_sync(BSB_FULL_MASK, jb.h0, b), lm = __shfl_sync(BSB_FULL_MASK, lim, b);
                 int best, best_j, last;
                 bool known;
+                int cls = 0;
                 if constexpr (Packed) {
                     known = ksw_diagonal<8>(tab, P.mat_max, lm, qlen, tlen, h0, acc, lane, best, best_j, last);
                 } else {
-                    known = ksw_diagonal_words(tab, P.mat_max, plain, lm, qlen, tlen, h0, acc.qs.p, acc.ts.p,
-                                               seq, seq + seq_bytes, lane, best, best_j, last);
+                    const int fr = __shfl_sync(BSB_FULL_MASK, far, b), most = __shfl_sync(BSB_FULL_MASK, cut, b);
+                    int loss, lowest;
+                    const bool followed = ksw_diagonal_words(tab, P.mat_max, plain, fr, qlen, tlen, h0, acc.qs.p, acc.ts.p,
+                                                             seq, seq + seq_bytes, lane, best, best_j, last, loss, lowest);
+                    known = followed && loss < lm;
+                    if (followed && !known && most >= 0) {
+                        const int D = cut_band(P, loss, lowest);
+                        if (D >= 0) {
+#pragma unroll
+                            for (int c = kCutRings - 1; c >= 0; --c)
+                                if (c <= most && cuts >> c & 1 && D <= cut_width(c)) cls = c + 1;
+                        }
+                    }
                 }
                 if (known && (lane & 7) == 0) {
                     bsb_ext_out_t o;
                     o.score = best; o.qle = o.tle = best_j + 1;
                     o.gtle = qlen; o.gscore = last; o.max_off = 0;
                     out[i0 + b] = o;
+                }
+                if constexpr (!Packed) {
+                    const unsigned c0 = __ballot_sync(BSB_FULL_MASK, cls & 1), c1 = __ballot_sync(BSB_FULL_MASK, cls & 2);
+                    if (lane >= r && lane < r + 4) {
+                        const int c = (int)(c0 >> ((lane - r) * 8) & 1u) | (int)(c1 >> ((lane - r) * 8) & 1u) << 1;
+                        if (c) key = cut_tile(c - 1) * kClasses + key % kClasses;
+                    }
                 }
                 const unsigned done = __ballot_sync(BSB_FULL_MASK, known);
                 if (lane >= r && lane < r + 4 && (done >> ((lane - r) * 8) & 1)) key = kDoneKey;
@@ -393,6 +432,15 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
     Q.pack16 = ksw_pack16(P);
     const bool ring = !d_map && !Q.pac && Q.pack16 && (tiles >> kRingTile & 1);
     if (!d_map && !ring) tiles &= ~(1ull << kRingTile);
+    // the rings for cut bands that queries of the batch's shapes are wide enough for
+    int cuts = 0;
+    if (!d_map && !Q.pac && Q.pack16 && !d_cells && builtin <= 1) {
+        for (int t = 0; t < kNumTiles; ++t)
+            for (int c = 0; c < kCutRings; ++c)
+                if (tiles >> t & 1 && (t == kRingTile || kTileList[t].G * kTileList[t].C >= cut_from(c, builtin))) cuts |= 1 << c;
+        for (int c = 0; c < kCutRings; ++c)
+            if (cuts >> c & 1) tiles |= 1ull << cut_tile(c);
+    }
     cudaError_t e;
     if (ev0) cudaEventRecord(ev0, st);
     e = cudaMemsetAsync(scratch, 0, sizeof(int) * (3 * kNumTiles + 1 + kHistSlots), st);
@@ -405,7 +453,7 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
         const int hb = (int)min((int64_t)n_sm * 8, (n + per * (kHistThreads / 32) - 1) / (per * (kHistThreads / 32)));
         const auto hist_kernel = Q.pac ? ksw_sched_hist<true> : ksw_sched_hist<false>;
         hist_kernel<<<hb, kHistThreads, 0, st>>>(Q, d_jobs, (int)n, (long long)seq_bytes, d_seq, d_cost, d_map, builtin,
-                                                 ring, d_cells == nullptr, per, d_out, hist, key);
+                                                 ring, d_cells == nullptr, cuts, per, d_out, hist, key);
         ksw_sched_scan<<<1, kScanThreads, 0, st>>>(hist, cursor, ranges, rejected);
         if (n >= 8 * kScatterTile)
             ksw_sched_scatter_tiles<<<(unsigned)((n + kScatterTile - 1) / kScatterTile), kScatterThreads, 0, st>>>(
@@ -432,8 +480,11 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
             cudaStream_t s = conc && lane ? ms->aux[lane - 1] : st;
             const int32_t *r = ranges + kRangeInts * t;
             if (tile_ev) cudaEventRecord(tile_ev[2 * t], s);
-            if (ring && t == kRingTile) {
-                e = ksw_ring16(ring_of(builtin))(Q, d_jobs, d_seq, order, r + 4, counter + 3 * t, d_out, d_cells, n_sm, s);
+            int cut = -1;
+            for (int c = 0; c < kCutRings; ++c)
+                if (cuts >> c & 1 && t == cut_tile(c)) cut = c;
+            if ((ring && t == kRingTile) || cut >= 0) {
+                e = ksw_ring16(cut >= 0 ? kFirstCut + cut : ring_of(builtin))(Q, d_jobs, d_seq, order, r + 4, counter + 3 * t, d_out, d_cells, n_sm, s);
             } else if (f16) {
                 // the wide class is rare (very large h0): one block per SM drains it
                 e = f16(Q, d_jobs, d_seq, order, r, counter + 3 * t, d_out, d_cells, n_sm, s);

@@ -208,6 +208,7 @@ __device__ __forceinline__ void ksw_group16_run(const KswParams &P, const bsb_ex
                     max_del = max_del > 1 ? max_del : 1;
                     w = w < max_del ? w : max_del;
                 }
+                if constexpr (Ring) w = min(w, (G * C - C - 1) / 2);     // the cut rings' jobs (cut_band)
                 best = h0; best_i = best_j = -1; max_ie = -1; gscore = -1; max_off = 0;
                 beg = 0; end = qlen; i = 0; ncell = 0;
                 q_lane = qlen / C & (G - 1); q_slot = qlen % C;

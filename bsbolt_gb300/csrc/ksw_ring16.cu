@@ -30,4 +30,13 @@ cudaError_t ksw_ring16_launch(const KswParams &P, const bsb_ext_job_t *jobs, con
 
 }  // namespace
 
-KswTileLaunch ksw_ring16(int ring) { return ring ? ksw_ring16_launch<1> : ksw_ring16_launch<0>; }
+KswTileLaunch ksw_ring16(int ring)
+{
+    switch (ring) {
+    case 0: return ksw_ring16_launch<0>;
+    case 1: return ksw_ring16_launch<1>;
+    case 2: return ksw_ring16_launch<2>;
+    case 3: return ksw_ring16_launch<3>;
+    default: return ksw_ring16_launch<4>;
+    }
+}

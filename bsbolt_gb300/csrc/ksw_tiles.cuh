@@ -113,18 +113,38 @@ inline int ksw_builtin_of(int64_t n, int n_sm)
 // 8x32 rings 4.6, 4.6 and 4.6 where 16x14 takes 4.3.  The smallest batches are bound by the rows one after the
 // other, where a warp a job is faster: 64 jobs of 300-600 bases 0.77 ms -> 0.54 (16x14 0.64), 3000 of 100-600 1.05
 // -> 0.76 (0.95), but 7500 of 300-600 1.34 (1.16), 10,000 of 300-400 1.55 -> 1.38 (1.12).
-constexpr KswTile kRings[2] = {{16, 14}, {32, 8}};
+constexpr KswTile kRings[] = {{16, 14}, {32, 8}, {4, 8}, {4, 16}, {4, 32}};
 __host__ __device__ __forceinline__ constexpr int ring_of(int builtin) { return builtin == kBuiltinMaps - 1 ? 1 : 0; }
 __host__ __device__ __forceinline__ constexpr int ring_cols(int ring) { return ring ? 32 * 8 : 16 * 14; }
 __host__ __device__ __forceinline__ constexpr int ring_block(int ring) { return ring ? 8 : 14; }
 static_assert(ring_cols(0) == kRings[0].G * kRings[0].C && ring_cols(1) == kRings[1].G * kRings[1].C &&
               ring_block(0) == kRings[0].C && ring_block(1) == kRings[1].C, "the rings' sizes");
+// Jobs whose band can be cut (cut_band, ksw_core.cuh: most of those with a few mismatches) run on rings of their own, by
+// the band they need, where the query is wider than its ring pays for: 4 lanes of 8, 16 and 32 columns, eight jobs a
+// warp.  Only in batches that come near to filling the GPU with 4-lane groups (the first two built-in maps; on the
+// second, beyond its 8 x 18 shape: 64k jobs of 10-140 bases 658 us, 674 with the shorter ones cut), on byte jobs, and not
+// where cells are counted.  2M jobs of 10-140 bases 7.92 ms -> 6.84, 50k of 100-600 4.03 -> 3.30 (half of them cut).
+constexpr int kCutRings = 3, kFirstCut = 2;
+__host__ __device__ __forceinline__ constexpr int cut_from(int c, int builtin)          // query + 1
+{
+    return builtin == 1 || c == 2 ? 145 : c == 1 ? 97 : 65;
+}
+__host__ __device__ __forceinline__ constexpr int cut_width(int c) { return c == 0 ? 11 : c == 1 ? 23 : 47; }
+static_assert(2 * cut_width(0) + 8 + 1 <= 32 && 2 * cut_width(1) + 16 + 1 <= 64 && 2 * cut_width(2) + 32 + 1 <= 128,
+              "the cut rings' bands");
 constexpr int kRingTile = tile_index(32, 5);
+constexpr int kCutTile0 = tile_index(32, 7), kCutTile1 = tile_index(32, 9), kCutTile2 = tile_index(32, 11);
+__host__ __device__ __forceinline__ constexpr int cut_tile(int c)
+{
+    return c == 0 ? kCutTile0 : c == 1 ? kCutTile1 : kCutTile2;
+}
 constexpr bool ring_tile_is_free()
 {
     for (int b = 0; b < kBuiltinMaps; ++b)
         for (int need = 1; need <= kMaxNeed; ++need)
-            if (kBuiltinTileMaps[b].tile[need] == kRingTile) return false;
+            if (kBuiltinTileMaps[b].tile[need] == kRingTile || kBuiltinTileMaps[b].tile[need] == kCutTile0 ||
+                kBuiltinTileMaps[b].tile[need] == kCutTile1 || kBuiltinTileMaps[b].tile[need] == kCutTile2)
+                return false;
     return true;
 }
 static_assert(ring_tile_is_free(), "a built-in map uses the ring's place");
