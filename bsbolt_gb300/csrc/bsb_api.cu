@@ -307,9 +307,8 @@ static int extend_device(bsb_ctx *ctx, const bsb_ext_param_t *param, const bsb_e
         return rc;
     cudaError_t e = ksw_launch(P, d_jobs, n_jobs, seq_bytes, d_seq, d_cost, ctx->d_tile_map, builtin, tiles, d_out, d_cells,
                                ctx->scratch, ctx->n_sm, ctx->stream, e0 ? e0 : ctx->ev0, e1 ? e1 : ctx->ev1,
-                               ctx->tile_ev, &ctx->ms);
-    ctx->pending_ksw = 1;
-    ctx->last_tiles = tiles;
+                               ctx->tile_ev, &ctx->last_tiles, &ctx->ms);
+    if (e == cudaSuccess) ctx->pending_ksw = 1;
     return bsb_cuda(ctx, e, "extension launch");
 }
 
@@ -321,6 +320,7 @@ extern "C" int bsb_extend_batch_device(bsb_ctx *ctx, const bsb_ext_param_t *para
     if (!ctx) return BSB_EINVAL;
     const int builtin = ksw_builtin(n_jobs, ctx->n_sm);
     const uint64_t tiles = ctx->d_tile_map ? ctx->map_tiles : ksw_builtin_tiles(builtin);
+    ctx->n_chunks = 0;
     return extend_device(ctx, param, d_jobs, n_jobs, d_seq, seq_bytes, d_cost, d_out, d_cells, builtin, tiles);
 }
 
@@ -472,6 +472,7 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
         if ((rc = extend_device(ctx, param, d_jobs + lo, cnt, d_seq, seq_bytes, nullptr, d_out + lo,
                                 d_cells ? d_cells + lo : nullptr, builtin, tiles, ev[2], ev[3])))
             return rc;
+        ctx->n_chunks = k + 1;
         if ((rc = bsb_cuda(ctx, cudaEventRecord(ev[1], ctx->stream), "event")) ||
             (rc = bsb_cuda(ctx, cudaStreamWaitEvent(ctx->d2h, ev[1], 0), "event")) ||
             (rc = bsb_cuda(ctx, cudaMemcpyAsync(out + lo, d_out + lo, sizeof(bsb_ext_out_t) * cnt,
@@ -481,9 +482,16 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
                                                              cudaMemcpyDeviceToHost, ctx->d2h), "D2H cells")))
             return rc;
     }
-    ctx->n_chunks = nck;
     if ((rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->d2h), "D2H synchronize"))) return rc;
     return bsb_sync(ctx);
+}
+
+// The time between two marks; an error is reported, not left behind as the thread's last one.
+static int elapsed(bsb_ctx *ctx, float *ms, cudaEvent_t a, cudaEvent_t b)
+{
+    const cudaError_t e = cudaEventElapsedTime(ms, a, b);
+    if (e != cudaSuccess) cudaGetLastError();
+    return bsb_cuda(ctx, e, "extension times");
 }
 
 extern "C" int bsb_sync(bsb_ctx *ctx)
@@ -494,19 +502,22 @@ extern "C" int bsb_sync(bsb_ctx *ctx)
     if (ctx->pending_ksw) {
         ctx->pending_ksw = 0;
         if (ctx->n_chunks) {        // a host batch in pieces: the sum of the pieces' extension times
+            const int n_chunks = ctx->n_chunks;
+            ctx->n_chunks = 0;
             ctx->last_kernel_ms = 0.f;
-            for (int k = 0; k < ctx->n_chunks; ++k) {
+            for (int k = 0; k < n_chunks; ++k) {
                 float m = 0.f;
-                cudaEventElapsedTime(&m, ctx->chunk_ev[4 * k + 2], ctx->chunk_ev[4 * k + 3]);
+                if ((rc = elapsed(ctx, &m, ctx->chunk_ev[4 * k + 2], ctx->chunk_ev[4 * k + 3]))) return rc;
                 ctx->last_kernel_ms += m;
             }
-            ctx->n_chunks = 0;
-        } else {
-            cudaEventElapsedTime(&ctx->last_kernel_ms, ctx->ev0, ctx->ev1);
+        } else if ((rc = elapsed(ctx, &ctx->last_kernel_ms, ctx->ev0, ctx->ev1))) {
+            return rc;
         }
         for (int t = 0; t < BSB_NUM_TILES; ++t) {
             ctx->tile_ms[t] = 0.f;
-            if (ctx->last_tiles >> t & 1) cudaEventElapsedTime(&ctx->tile_ms[t], ctx->tile_ev[2 * t], ctx->tile_ev[2 * t + 1]);
+            if (ctx->last_tiles >> t & 1 &&
+                (rc = elapsed(ctx, &ctx->tile_ms[t], ctx->tile_ev[2 * t], ctx->tile_ev[2 * t + 1])))
+                return rc;
         }
         int rej = 0;
         if ((rc = bsb_cuda(ctx, cudaMemcpy(&rej, ksw_rejected_counter(ctx->scratch), sizeof(int),

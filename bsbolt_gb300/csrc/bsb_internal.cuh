@@ -158,14 +158,16 @@ int *ksw_rejected_counter(void *scratch);
 // d_map: the tile map in device memory (BSB_TILE_MAP_LEN bytes), or NULL for
 // the built-in map number `builtin`; tiles: bit t set = launch tile shape t (the shapes that
 // map gives the batch's query lengths; a shape left out leaves its jobs unrun).
-// tile_ev (optional, 2 * BSB_NUM_TILES events): per-shape timing marks as in bsb_ctx.
+// tile_ev (optional, 2 * BSB_NUM_TILES events): per-shape timing marks as in bsb_ctx; launched (optional): the shapes
+// whose marks were recorded, which is not `tiles` (the ring is left out where the scoring needs 32-bit cells, the cut
+// rings come in).
 // ms (optional): run the shape kernels of batches below ksw_concurrent_below() jobs
 // on st and ms->aux (joined back into st before ev1).
 cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
                        const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
                        cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev = nullptr,
-                       const KswStreams *ms = nullptr, bool all_narrow = false);
+                       uint64_t *launched = nullptr, const KswStreams *ms = nullptr, bool all_narrow = false);
 // all_narrow: the caller knows that no job's h0 + qlen * max(mat) exceeds this, so that no job needs
 // 32-bit cells where the scoring allows 16-bit ones.
 int ksw_pack16_max();

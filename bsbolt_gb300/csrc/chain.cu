@@ -2565,7 +2565,7 @@ static int first_extensions(bsb_ctx *ctx, const bsb_align_opt_t *o, const AlnOpt
         if (side) pre_right_kernel<<<tb, 128, 0, st>>>(ao, T, left, out, right);
         if ((rc = bsb_cuda(ctx, ksw_launch(Q, side ? right : left, T, 0, d_reads, nullptr, nullptr, builtin, tiles,
                                            out + side * T, nullptr, D + o_scr, ctx->n_sm, st, nullptr, nullptr, nullptr,
-                                           &ctx->ms, true), "chain extensions")))
+                                           nullptr, &ctx->ms, true), "chain extensions")))
             return rc;
     }
     pre->chains = pc, pre->off = chain_off, pre->left = out, pre->right = out + T;

@@ -414,9 +414,10 @@ int ksw_ring_tile() { return kRingTile; }
 cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
                        const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
-                       cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev, const KswStreams *ms,
-                       bool all_narrow)
+                       cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev, uint64_t *launched,
+                       const KswStreams *ms, bool all_narrow)
 {
+    if (launched) *launched = 0;
     char *p = (char *)scratch;
     int *counter = (int *)p;                // 3 per tile: 16-bit range, wide range, whole tile
     int *rejected = counter + 3 * kNumTiles;
@@ -495,6 +496,7 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
             }
             if (e != cudaSuccess) return e;
             if (tile_ev) cudaEventRecord(tile_ev[2 * t + 1], s);
+            if (launched) *launched |= 1ull << t;
         }
         if (conc) {
             for (int a = 0; a < BSB_AUX_STREAMS; ++a) {

@@ -132,7 +132,9 @@ int bsb_set_tile_map(bsb_ctx *ctx, const uint8_t *map, int n);
  * jobs run their shapes on four streams at once, so a shape's time there
  * includes sharing the GPU; a host batch extended in pieces reports its last
  * piece.  Without an installed map, long queries with a narrow band run on a
- * kernel of their own, reported under the 32 x 5 shape.  Valid after bsb_sync. */
+ * kernel of their own, reported under the 32 x 5 shape, and large batches run the
+ * jobs whose band can be cut on three more, reported under the 32 x 7, 32 x 9 and
+ * 32 x 11 shapes.  Valid after bsb_sync. */
 int bsb_last_tile_ms(const bsb_ctx *ctx, float *ms, int n);
 
 /* Copies the context's current tile map into map (n >= BSB_TILE_MAP_LEN);
