@@ -39,6 +39,7 @@ EXPORTS = (
     "bsb_index_upload_opac", "bsb_gen_cigar_batch", "bsb_align2_batch",
     "bsb_last_seed_extensions", "bsb_read_cost_log", "bsb_last_read_costs", "bsb_set_read_cost_model",
     "bsb_build_suffix_array", "bsb_last_stage_ms", "bsb_set_read_order_keys", "bsb_build_bwt",
+    "bsb_last_read_order",
 )
 
 
@@ -177,6 +178,8 @@ def load(path: str = LIB_PATH):
     L.bsb_last_seed_extensions.restype = I32
     L.bsb_set_read_order_keys.argtypes = [P, P, I32]
     L.bsb_set_read_order_keys.restype = I32
+    L.bsb_last_read_order.argtypes = [P, P, I32, ctypes.POINTER(ctypes.c_int32)]
+    L.bsb_last_read_order.restype = I32
     L.bsb_last_stage_ms.argtypes = [P, P, I32]
     L.bsb_last_stage_ms.restype = I32
     L.bsb_read_cost_log.argtypes = [P, I32]

@@ -101,6 +101,7 @@ struct bsb_ctx {
     // the last batch when logging
     const void *read_model = nullptr;
     int read_log = 0, rc_n = 0;
+    const int32_t *queue_reads = nullptr, *queue_count = nullptr;      // the last batch's read queue, in arena1
     std::vector<int32_t> order_keys;   // per-read order keys for the next alignment batch
     void *rc_buf = nullptr;
     size_t rc_bytes = 0;

@@ -1486,8 +1486,8 @@ __device__ __forceinline__ void right_end(const AlnOpt &opt, int l_query, const 
 // mem_chain2aln for the reads whose extensions are all known (PreResults), a warp a read: 32 chains at a time, each lane
 // one chain's first seed, its region and its record; then the chains in order, the seed of each against the regions so
 // far over the lanes, and the chain's other seeds over the lanes, which must all be contained in a region and not part
-// from the chain's first.  A read where one would be extended, or with more than kPlainRegs regions, goes to `left`
-// for chain2aln_kernel.  That kernel's loads follow one another chain by chain, on 16 warps an SM (it holds the DP).
+// from the chain's first.  A read where one would be extended, or with more than kPlainRegs regions, gets n_regs -1:
+// it is left for chain2aln_kernel, in the read order.  That kernel's loads follow one another chain by chain, on 16 warps an SM (it holds the DP).
 // 114k RRBS reads (450k regions): 617 us -> 199 and 175 for the reads left; 67k of 150 bases 292 -> 89 and 86.  At 10
 // blocks an SM, or a block for every four reads in place of 8 an SM: 20-80 us more.
 constexpr int kPlainWarps = 4, kPlainRegs = 64;
@@ -1495,7 +1495,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, 8)
 chain2aln_plain(AlnOpt opt, int n_reads, const int64_t *__restrict__ read_off, const int64_t *__restrict__ seed_off,
                 const int64_t *__restrict__ row_off_of_seed, const DevSeed *__restrict__ seeds,
                 const DevChain *__restrict__ chains, const int *__restrict__ n_chains, bsb_reg_t *__restrict__ regs,
-                int *__restrict__ n_regs, PreResults pre, int *__restrict__ left, int *__restrict__ n_left)
+                int *__restrict__ n_regs, PreResults pre)
 {
     __shared__ RegSpan sm[kPlainWarps][kPlainRegs];
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
@@ -1581,21 +1581,17 @@ chain2aln_plain(AlnOpt opt, int n_reads, const int64_t *__restrict__ read_off, c
             }
             if (ok && slot >= 0) regs[R0 + slot] = a;
         }
-        if (lane == 0) {
-            if (ok) n_regs[r] = nav;
-            else left[atomicAdd(n_left, 1)] = r;
-        }
+        if (lane == 0) n_regs[r] = ok ? nav : -1;
     }
 }
 
-// One warp per read.  regs: the read's region slots start at its row offset.  n_list: the number of reads in `order`
-// where it is not all n_reads.
+// One warp per read, the *n_list reads of `order`.  regs: the read's region slots start at its row offset.
 // MaxC = 4, 5, 8 serve batches whose reads are at most 127, 159, 255 bases long (one DP
 // copy of that width), 16 every read the batch accepts; the 4- and 5-column variants are
 // held to 4 blocks (16 warps) per SM, the 8-column one to 3.
 template <int MaxC>
 __global__ void __launch_bounds__(128, MaxC <= 5 ? 4 : MaxC <= 8 ? 3 : 1)
-chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *__restrict__ reads,
+chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, const uint8_t *__restrict__ reads,
                  const int64_t *__restrict__ read_off, const int64_t *__restrict__ seed_off,
                  const int64_t *__restrict__ row_off_of_seed, const DevSeed *__restrict__ seeds,
                  const DevChain *__restrict__ chains, const int *__restrict__ n_chains, uint64_t *__restrict__ srt_buf,
@@ -1603,7 +1599,7 @@ chain2aln_kernel(AlnOpt opt, KswParams P, DevBns B, int n_reads, const uint8_t *
                  const int *__restrict__ order, const int *__restrict__ n_list, int64_t *__restrict__ read_cells,
                  PreResults pre)
 {
-    if (n_list) n_reads = *n_list;
+    const int n_reads = *n_list;
     __shared__ int8_t tab[kScoreTable];
     load_score_table(P, tab);
     __syncthreads();
@@ -1936,7 +1932,8 @@ __device__ __forceinline__ int key_bin(int32_t key)
     const int half = 2 * msb + (msb > 0 ? (int)(k >> (msb - 1) & 1u) : 0);
     return 63 - (half < 63 ? half : 63);
 }
-// Counting sort into 64 bins in two kernels: the bins' sizes, then the places.  A block counts in shared
+// Counting sort into 64 bins in two kernels: the bins' sizes, then the places (bin -1: the read is left out; n_placed,
+// optional: how many were not).  A block counts in shared
 // memory and touches each global counter once (one global atomic per read on a few busy counters took
 // 84 us for 67k reads, the two kernels together).
 constexpr int kOrderBins = 64, kOrderThreads = 256;
@@ -1947,18 +1944,19 @@ __device__ __forceinline__ void order_count(int n_reads, int *__restrict__ cnt, 
     if (threadIdx.x < kOrderBins) sh[threadIdx.x] = 0;
     __syncthreads();
     for (int r = blockIdx.x * kOrderThreads + threadIdx.x; r < n_reads; r += gridDim.x * kOrderThreads)
-        atomicAdd(&sh[bin(r)], 1);
+        if (const int b = bin(r); b >= 0) atomicAdd(&sh[b], 1);
     __syncthreads();
     if (threadIdx.x < kOrderBins && sh[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], sh[threadIdx.x]);
 }
 template <class Bin>
 __device__ __forceinline__ void order_place(int n_reads, const int *__restrict__ cnt, int *__restrict__ cur,
-                                            int *__restrict__ order, Bin bin)
+                                            int *__restrict__ order, int *__restrict__ n_placed, Bin bin)
 {
     __shared__ int off[kOrderBins], sh[kOrderBins];
     if (threadIdx.x == 0) {
         int acc = 0;
         for (int b = 0; b < kOrderBins; ++b) off[b] = acc, acc += cnt[b];
+        if (n_placed && blockIdx.x == 0) *n_placed = acc;
     }
     for (int base = blockIdx.x * kOrderThreads; base < n_reads; base += gridDim.x * kOrderThreads) {
         if (threadIdx.x < kOrderBins) sh[threadIdx.x] = 0;
@@ -1973,32 +1971,35 @@ __device__ __forceinline__ void order_place(int n_reads, const int *__restrict__
         __syncthreads();
     }
 }
+
+// The order chain2aln_kernel takes reads in, by the keys given or else most chains first (reads are independent, so the
+// order changes no result; it shortens the tail a few repeat-laden reads would otherwise set).  Where chain2aln_plain
+// has gone before, only the reads it left: n_regs below 0 (NULL: all reads).
 __global__ void __launch_bounds__(kOrderThreads)
-order_hist_key(const int32_t *__restrict__ key, int n_reads, int *__restrict__ cnt)
+order_hist_key(const int32_t *__restrict__ key, const int *__restrict__ n_regs, int n_reads, int *__restrict__ cnt)
 {
-    order_count(n_reads, cnt, [=](int r) { return key_bin(key[r]); });
+    order_count(n_reads, cnt, [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : key_bin(key[r]); });
 }
 __global__ void __launch_bounds__(kOrderThreads)
-order_scatter_key(const int32_t *__restrict__ key, int n_reads, const int *__restrict__ cnt, int *__restrict__ cur,
-                  int *__restrict__ order)
+order_scatter_key(const int32_t *__restrict__ key, const int *__restrict__ n_regs, int n_reads,
+                  const int *__restrict__ cnt, int *__restrict__ cur, int *__restrict__ order, int *__restrict__ n_placed)
 {
-    order_place(n_reads, cnt, cur, order, [=](int r) { return key_bin(key[r]); });
+    order_place(n_reads, cnt, cur, order, n_placed, [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : key_bin(key[r]); });
 }
 
-// The order chain2aln_kernel takes reads in: most chains first (reads are independent, so the
-// order changes no result; it shortens the tail a few repeat-laden reads would otherwise set).
 __device__ __forceinline__ int order_bin(int nc) { return kOrderBins - 1 - (nc < kOrderBins - 1 ? nc : kOrderBins - 1); }
 
 __global__ void __launch_bounds__(kOrderThreads)
-order_hist(const int *__restrict__ n_chains, int n_reads, int *__restrict__ cnt)
+order_hist(const int *__restrict__ n_chains, const int *__restrict__ n_regs, int n_reads, int *__restrict__ cnt)
 {
-    order_count(n_reads, cnt, [=](int r) { return order_bin(n_chains[r]); });
+    order_count(n_reads, cnt, [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : order_bin(n_chains[r]); });
 }
 __global__ void __launch_bounds__(kOrderThreads)
-order_scatter(const int *__restrict__ n_chains, int n_reads, const int *__restrict__ cnt, int *__restrict__ cur,
-              int *__restrict__ order)
+order_scatter(const int *__restrict__ n_chains, const int *__restrict__ n_regs, int n_reads, const int *__restrict__ cnt,
+              int *__restrict__ cur, int *__restrict__ order, int *__restrict__ n_placed)
 {
-    order_place(n_reads, cnt, cur, order, [=](int r) { return order_bin(n_chains[r]); });
+    order_place(n_reads, cnt, cur, order, n_placed,
+                [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : order_bin(n_chains[r]); });
 }
 
 // The order chain_warp_kernel takes a large batch's reads in: most rows first, in steps of four.  A read on
@@ -2022,7 +2023,7 @@ __global__ void __launch_bounds__(kOrderThreads)
 order_scatter_rows(const int64_t *__restrict__ seed_off, const int64_t *__restrict__ row_off_of_seed, int n_reads,
                    const int *__restrict__ cnt, int *__restrict__ cur, int *__restrict__ order)
 {
-    order_place(n_reads, cnt, cur, order, [=](int r) { return rows_bin(seed_off, row_off_of_seed, r); });
+    order_place(n_reads, cnt, cur, order, nullptr, [=](int r) { return rows_bin(seed_off, row_off_of_seed, r); });
 }
 
 // One warp per read (reads hold a few regions each).
@@ -2613,7 +2614,7 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     const size_t o_ctrl = off; off += al(sizeof(int) * 4);
     const size_t o_regoff = off; off += al(sizeof(int64_t) * (n_reads + 1));
     const size_t o_out = off; off += al(sizeof(bsb_reg_t) * Rb);
-    const size_t o_bail = off; off += al(sizeof(int) * (size_t)n_reads);
+    const size_t o_by_rows = off; off += al(sizeof(int) * (size_t)n_reads);
     const size_t o_order = off; off += al(sizeof(int) * (n_reads + 1)) + al(sizeof(int) * 2 * kOrderBins);
     const size_t o_dtmp = off; off += dedup ? al(sizeof(bsb_reg_t) * Rb) : 0;
     const size_t o_dn = off; off += dedup ? al(sizeof(int) * (n_reads + 1)) : 0;
@@ -2660,7 +2661,7 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     int *by_rows = nullptr;
     if (n_reads >= kRowOrderReads) {
         int *const cnt = (int *)(A + o_order + al(sizeof(int) * (n_reads + 1)));
-        by_rows = (int *)(A + o_bail);
+        by_rows = (int *)(A + o_by_rows);
         const int ob = std::min((n_reads + kOrderThreads - 1) / kOrderThreads, ctx->n_sm * 4);
         if ((rc = bsb_cuda(ctx, cudaMemsetAsync(cnt, 0, sizeof(int) * 2 * kOrderBins, st), "read order"))) return rc;
         order_hist_rows<<<ob, kOrderThreads, 0, st>>>(d_seed_off, roff, n_reads, cnt);
@@ -2676,15 +2677,27 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
                              n_chains, ao)))
         return rc;
     if ((rc = bsb_cuda(ctx, cudaEventRecord(ctx->stage_ev[3], st), "stage mark"))) return rc;
-    int *order = (int *)(A + o_order);
-    int *ocnt = (int *)(A + o_order + al(sizeof(int) * (n_reads + 1)));
+    int *const order = (int *)(A + o_order);
+    int *const n_list = ctrl + 2, *const ocnt = (int *)(A + o_order + al(sizeof(int) * (n_reads + 1)));
+    // the reads that need no other extension than their chains' first; the rest is chain2aln_kernel's
+    const bool logging = ctx->read_log != 0;
+    PreResults pre{};
+    if (!logging && n_reads >= kPreReads &&
+        (rc = first_extensions(ctx, o, ao, B, P, n_reads, max_len, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
+                               n_chains, reg_off, scan_tmp, &pre)))
+        return rc;
+    if (pre.chains) {
+        const int pb = std::min((n_reads + kPlainWarps - 1) / kPlainWarps, ctx->n_sm * 8);
+        chain2aln_plain<<<pb, kPlainWarps * 32, 0, st>>>(ao, n_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
+                                                         n_chains, regs, n_regs, pre);
+    }
     // per-read features / extension cells for the learned read order (kept for bsb_last_read_costs)
     float *d_feat = nullptr;
     int64_t *d_rcells = nullptr;
     int32_t *d_rkey = nullptr;
     const bool keyed = !ctx->order_keys.empty() && (int64_t)ctx->order_keys.size() == n_reads;
     if (!keyed) ctx->order_keys.clear();          // keys for another batch size are dropped
-    const bool learned = ctx->read_model != nullptr && !keyed, logging = ctx->read_log != 0;
+    const bool learned = ctx->read_model != nullptr && !keyed;
     if (learned || logging || keyed) {
         const size_t nr = (size_t)n_reads;
         if ((rc = bsb_ensure(ctx, &ctx->rc_buf, &ctx->rc_bytes, al(32 * nr) + al(8 * nr) + al(4 * nr) + 256,
@@ -2700,6 +2713,7 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
         ctx->rc_n = logging ? n_reads : 0;
     }
     {
+        const int *const open = pre.chains ? n_regs : nullptr;
         const int ob = (int)((n_reads + 255) / 256) < ctx->n_sm * 4 ? (int)((n_reads + 255) / 256) : ctx->n_sm * 4;
         if ((rc = bsb_cuda(ctx, cudaMemsetAsync(ocnt, 0, sizeof(int) * 2 * kOrderBins, st), "read order"))) return rc;
         if (keyed) {         // the caller's keys, once (the copy is done before they are cleared)
@@ -2708,48 +2722,36 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
                 (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "read order keys")))
                 return rc;
             ctx->order_keys.clear();
-            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt);
-            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt, ocnt + kOrderBins, order);
+            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt);
+            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt, ocnt + kOrderBins, order, n_list);
         } else if (learned) {   // predicted cells of every read, most expensive first
             if ((rc = bsb_mlp_forward(ctx, (const bsb_mlp_weights_t *)ctx->read_model, d_feat, n_reads, nullptr,
                                       d_rkey)))
                 return rc;
-            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt);
-            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, n_reads, ocnt, ocnt + kOrderBins, order);
+            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt);
+            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt, ocnt + kOrderBins, order, n_list);
         } else {
-            order_hist<<<ob, kOrderThreads, 0, st>>>(n_chains, n_reads, ocnt);
-            order_scatter<<<ob, kOrderThreads, 0, st>>>(n_chains, n_reads, ocnt, ocnt + kOrderBins, order);
+            order_hist<<<ob, kOrderThreads, 0, st>>>(n_chains, open, n_reads, ocnt);
+            order_scatter<<<ob, kOrderThreads, 0, st>>>(n_chains, open, n_reads, ocnt, ocnt + kOrderBins, order, n_list);
         }
     }
+    ctx->queue_reads = order, ctx->queue_count = n_list;
     int64_t *const rcells_out = logging ? d_rcells : nullptr;
-    PreResults pre{};
-    if (!logging && n_reads >= kPreReads &&
-        (rc = first_extensions(ctx, o, ao, B, P, n_reads, max_len, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
-                               n_chains, reg_off, scan_tmp, &pre)))
-        return rc;
-    const int *n_list = nullptr;
-    if (pre.chains) {           // the reads that need no other extension; the rest is chain2aln_kernel's
-        int *const bail = (int *)(A + o_bail);
-        const int pb = std::min((n_reads + kPlainWarps - 1) / kPlainWarps, ctx->n_sm * 8);
-        chain2aln_plain<<<pb, kPlainWarps * 32, 0, st>>>(ao, n_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
-                                                         n_chains, regs, n_regs, pre, bail, ctrl + 2);
-        order = bail, n_list = ctrl + 2;
-    }
     // every extension of these reads fits (max_len + 1) columns: the narrowest variant that holds them
     if (max_len <= 127)
-        chain2aln_kernel<4><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
+        chain2aln_kernel<4><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, d_reads, d_read_off, d_seed_off, roff,
                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else if (max_len <= 159)
-        chain2aln_kernel<5><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
+        chain2aln_kernel<5><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, d_reads, d_read_off, d_seed_off, roff,
                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else if (max_len <= 255)
-        chain2aln_kernel<8><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
+        chain2aln_kernel<8><<<ctx->n_sm * 8, 128, 0, st>>>(ao, P, B, d_reads, d_read_off, d_seed_off, roff,
                                                             cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else if (max_len <= 511)
-        chain2aln_kernel<16><<<ctx->n_sm * 4, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
+        chain2aln_kernel<16><<<ctx->n_sm * 4, 128, 0, st>>>(ao, P, B, d_reads, d_read_off, d_seed_off, roff,
                                                              cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     else
-        chain2aln_kernel<32><<<ctx->n_sm * 2, 128, 0, st>>>(ao, P, B, n_reads, d_reads, d_read_off, d_seed_off, roff,
+        chain2aln_kernel<32><<<ctx->n_sm * 2, 128, 0, st>>>(ao, P, B, d_reads, d_read_off, d_seed_off, roff,
                                                              cseeds, cchains, n_chains, srt, regs, n_regs, ctrl + 1, order, n_list, rcells_out, pre);
     if ((rc = bsb_cuda(ctx, cudaEventRecord(ctx->stage_ev[4], st), "stage mark")) ||
         (rc = bsb_cuda(ctx, scan_i32_i64(n_regs, n_reads, reg_off, scan_tmp, st), "region offsets")))
@@ -2830,6 +2832,7 @@ static int align_batch(bsb_ctx *ctx, const bsb_align_opt_t *o, int32_t n_reads, 
     std::vector<int64_t> rel(n_reads + 1);
     for (int r = 0; r <= n_reads; ++r) rel[r] = offs[r] - offs[0];
     ctx->stage_valid = false;
+    ctx->queue_reads = ctx->queue_count = nullptr;
     cudaEvent_t *const sev = ctx->stage_ev;
     if ((rc = bsb_cuda(ctx, cudaEventRecord(sev[0], ctx->stream), "stage mark")) ||
         (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_reads, seqs + offs[0], total, cudaMemcpyHostToDevice, ctx->stream), "H2D reads")))
@@ -2933,6 +2936,25 @@ extern "C" int bsb_last_read_costs(bsb_ctx *ctx, int32_t n_reads, float *feat, i
                                                      ctx->stream), "D2H")))
         return rc;
     return bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "read costs");
+}
+
+extern "C" int bsb_last_read_order(bsb_ctx *ctx, int32_t *reads, int32_t max, int32_t *n)
+{
+    if (!ctx) return BSB_EINVAL;
+    if (!n || max < 0 || (max > 0 && !reads)) return bsb_fail(ctx, BSB_EINVAL, "read order: NULL or negative count");
+    if (!ctx->queue_reads) return bsb_fail(ctx, BSB_EINVAL, "no alignment batch on this context");
+    int rc;
+    if ((rc = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice")) ||
+        (rc = bsb_cuda(ctx, cudaMemcpyAsync(n, ctx->queue_count, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream),
+                       "read order")) ||
+        (rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "read order")))
+        return rc;
+    const size_t got = std::min(*n, max);
+    if (got && ((rc = bsb_cuda(ctx, cudaMemcpyAsync(reads, ctx->queue_reads, sizeof(int32_t) * got, cudaMemcpyDeviceToHost,
+                                                    ctx->stream), "read order")) ||
+                (rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "read order"))))
+        return rc;
+    return 0;
 }
 
 extern "C" int bsb_set_read_cost_model(bsb_ctx *ctx, const bsb_mlp_weights_t *d_w)

@@ -59,6 +59,14 @@ def set_read_order_keys(ctx: Context, keys) -> None:
     _lib.check(ctx.handle, ctx.L.bsb_set_read_order_keys(ctx.handle, _ptr(k), len(k)))
 
 
+def last_read_order(ctx: Context, n_reads: int) -> np.ndarray:
+    """The reads of the context's last alignment batch (n_reads reads) that went through its queue, in the
+    order they were taken (bsb_last_read_order)."""
+    reads, n = np.zeros(n_reads, np.int32), ctypes.c_int32()
+    _lib.check(ctx.handle, ctx.L.bsb_last_read_order(ctx.handle, _ptr(reads), n_reads, ctypes.byref(n)))
+    return reads[: n.value]
+
+
 ALIGN_STAGES = ("seeding", "sa_rows", "chains", "chain2aln", "dedup", "d2h")
 
 

@@ -426,7 +426,10 @@ int bsb_mlp_adam(bsb_ctx *ctx, bsb_mlp_weights_t *d_w, float *d_master, float *d
 /* No reference counterpart: BWA runs mem_chain2aln read by read on CPU threads.  Inside
  * bsb_align_regs_batch / bsb_mem_align1_batch one warp extends one read's chains at a
  * time, taking reads from a queue; by default the queue holds the reads with the most
- * chains first.  A 2 x 64 cost model (the bsb_mlp_* kernels above, BSB_MLP_FEATURES
+ * chains first.  In batches of 4096 reads and more whose scoring and lengths fit 16-bit
+ * cells, the first extension of every chain is run ahead, and the queue holds the reads
+ * that need further ones; without a log, that is (bsb_read_cost_log), under which it holds
+ * every read.  A 2 x 64 cost model (the bsb_mlp_* kernels above, BSB_MLP_FEATURES
  * features per read: read length, kept chains and their seeds, best chain weight, mean
  * seed offset, reverse-strand share, C+G content, the plain bound of the extension cells)
  * can order the queue by predicted DP cells instead.  The order never changes a result.
@@ -439,11 +442,14 @@ int bsb_mlp_adam(bsb_ctx *ctx, bsb_mlp_weights_t *d_w, float *d_master, float *d
  *   bsb_set_read_order_keys(ctx, keys, n): order the next batch, which must hold n reads,
  *     by the caller's per-read keys (host int32, larger first, in the model's half-octave
  *     bins) -- e.g. the cells a log recorded, the order a perfect model would give, which
- *     bounds what any learned order can gain; used once, over the model; n = 0 clears. */
+ *     bounds what any learned order can gain; used once, over the model; n = 0 clears;
+ *   bsb_last_read_order: the last batch's queue, *n reads of which the first min(*n, max) go
+ *     to reads (host buffer), in the order they were taken; until the context's next batch. */
 int bsb_read_cost_log(bsb_ctx *ctx, int enable);
 int bsb_last_read_costs(bsb_ctx *ctx, int32_t n_reads, float *feat, int64_t *cells);
 int bsb_set_read_cost_model(bsb_ctx *ctx, const bsb_mlp_weights_t *d_w);
 int bsb_set_read_order_keys(bsb_ctx *ctx, const int32_t *keys, int32_t n);
+int bsb_last_read_order(bsb_ctx *ctx, int32_t *reads, int32_t max, int32_t *n);
 
 /* ---- extension without any device allocation ---------------------------- */
 
