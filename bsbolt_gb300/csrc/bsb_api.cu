@@ -207,7 +207,7 @@ static int check_jobs(bsb_ctx *ctx, const bsb_ext_job_t *jobs, int64_t n, int64_
                             (long long)i);
         if (j.qlen > qmax)
             return bsb_fail(ctx, BSB_ETOOLONG, "job %lld: qlen %d exceeds %d", (long long)i, j.qlen, qmax);
-        if (j.qoff < 0 || j.toff < 0 || j.qoff + j.qlen > seq_bytes || j.toff + j.tlen > seq_bytes)
+        if (!span_inside(j.qoff, j.qlen, seq_bytes) || !span_inside(j.toff, j.tlen, seq_bytes))
             return bsb_fail(ctx, BSB_EINVAL, "job %lld: sequence range outside the buffer", (long long)i);
         if ((int64_t)j.qlen + j.tlen > (1 << 30))
             return bsb_fail(ctx, BSB_ETOOLONG, "job %lld: sequence too long", (long long)i);

@@ -191,11 +191,16 @@ uint64_t ksw_builtin_tiles(int builtin);
 struct ExtScan {
     unsigned long long bad, tiles, need;
 };
+// len bytes from off on lie inside a buffer of `bytes` (no sum that could overflow).
+__host__ __device__ __forceinline__ bool span_inside(int64_t off, int32_t len, int64_t bytes)
+{
+    return off >= 0 && len >= 0 && len <= bytes && off <= bytes - len;
+}
 __host__ __device__ __forceinline__ bool ext_job_ok(const bsb_ext_job_t &j, int64_t seq_bytes, int qmax)
 {
     return j.qlen >= 0 && j.tlen >= 0 && j.w >= 0 && j.flags == 0 && j.h0 > 0 && j.h0 <= (1 << 20) &&
-           j.qlen <= qmax && j.qoff >= 0 && j.toff >= 0 && j.qoff + j.qlen <= seq_bytes &&
-           j.toff + j.tlen <= seq_bytes && (int64_t)j.qlen + j.tlen <= (1 << 30);
+           j.qlen <= qmax && span_inside(j.qoff, j.qlen, seq_bytes) && span_inside(j.toff, j.tlen, seq_bytes) &&
+           (int64_t)j.qlen + j.tlen <= (1 << 30);
 }
 // The scan on the device: *out from d_jobs (out zeroed on st first).  d_map, builtin as in ksw_launch.
 cudaError_t ksw_scan_jobs(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,

@@ -30,8 +30,7 @@ __global__ void features_kernel(const bsb_ext_job_t *__restrict__ jobs, int64_t 
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const bsb_ext_job_t j = jobs[i];
         float *f = feat + i * F;
-        const bool ok = j.qlen >= 0 && j.tlen >= 0 && j.qoff >= 0 && j.toff >= 0 && j.qoff + j.qlen <= seq_bytes &&
-                        j.toff + j.tlen <= seq_bytes;
+        const bool ok = span_inside(j.qoff, j.qlen, seq_bytes) && span_inside(j.toff, j.tlen, seq_bytes);
         if (!ok) {
             for (int k = 0; k < F; ++k) f[k] = 0.f;
             continue;

@@ -128,8 +128,8 @@ ksw_sched_hist(KswParams P, const bsb_ext_job_t *__restrict__ jobs, int n, long 
         const bool ok = in && jb.qlen >= 0 && jb.qlen < kMaxNeed && jb.tlen >= 0 && jb.w >= 0 && jb.h0 > 0 &&
                         jb.h0 <= (1 << 20) &&
                         (Packed ? !(jb.flags & kExtNone)
-                                : jb.flags == 0 && jb.qoff >= 0 && jb.toff >= 0 && jb.qoff + jb.qlen <= seq_bytes &&
-                                      jb.toff + jb.tlen <= seq_bytes);
+                                : jb.flags == 0 && span_inside(jb.qoff, jb.qlen, seq_bytes) &&
+                                      span_inside(jb.toff, jb.tlen, seq_bytes));
         int key;
         if (!ok) {
             key = kRejectKey;
