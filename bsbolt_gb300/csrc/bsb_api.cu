@@ -414,7 +414,7 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     // Batches of one piece, from a few thousand jobs on: the scan is a kernel over the copied jobs, which goes on while
     // the sequences follow.  On one host thread it took 165 of 835 us for 64k jobs of 10-140 bases and 280 of 4300
     // for 50k of 100-600.  It would also have told how much of seq the jobs use, so not where seq may be mostly others'.
-    const bool on_device = nck == 1 && n_jobs >= 4096 && seq_bytes / 2048 <= n_jobs;
+    const bool on_device = nck == 1 && n_jobs >= 4096 && seq_bytes >= 0 && seq_bytes / 2048 <= n_jobs;
     if (!on_device) scan_pieces(P, jobs, n_jobs, per, nck, seq_bytes, installed ? ctx->tile_map : ksw_builtin_tile_map(builtin),
                 installed ? -1 : builtin, piece);
     for (int k = 0; k < nck && !on_device; ++k)          // every job is checked before any other use of it

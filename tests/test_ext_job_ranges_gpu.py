@@ -1,5 +1,7 @@
-"""Extension jobs whose offset plus length passes the largest 64-bit number are refused by every entry as any other
-range outside the buffer is."""
+"""Extension jobs whose offset plus length passes the largest 64-bit number, and sequence buffers of negative size, are
+refused by every entry as any other range outside the buffer is."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -22,6 +24,17 @@ def test_host_entry(gpu_ctx, field, n):
         with pytest.raises(_lib.BsbError, match=f"job {n - 3}: sequence range") as e:
             extend.ksw_extend2_batch(gpu_ctx, jobs, seq, MAT, 6, 1, 6, 1, 100)
         assert e.value.code == _lib.BSB_EINVAL
+
+
+@pytest.mark.parametrize("n", [40, 4096])
+def test_negative_buffer_size(gpu_ctx, n):
+    few, seq = synth.ksw_jobs(64, seed=9)
+    jobs, out = np.resize(few, n), np.zeros((n, 6), np.int32)
+    p = extend.make_param(MAT, 6, 1, 6, 1, 100)
+    for size in (-1, -257, -2**63):
+        rc = gpu_ctx.L.bsb_extend_batch(gpu_ctx.handle, ctypes.byref(p), ctypes.c_void_p(jobs.ctypes.data), n,
+                                        ctypes.c_void_p(seq.ctypes.data), size, ctypes.c_void_p(out.ctypes.data), None)
+        assert rc == _lib.BSB_EINVAL and not out.any()
 
 
 def test_device_entry_and_features(gpu_ctx):
