@@ -288,6 +288,18 @@ static void scan_pieces(const KswParams &P, const bsb_ext_job_t *jobs, int64_t n
     }
 }
 
+// Do the jobs use nearly all of seq, as far as 64 of them spread over the batch tell?
+static bool seq_mostly_used(const bsb_ext_job_t *jobs, int64_t n, int64_t seq_bytes)
+{
+    int64_t end = 0;
+    for (int k = 0; k < 64; ++k) {
+        const bsb_ext_job_t &j = jobs[(n - 1) * k / 63];
+        if (span_inside(j.qoff, j.qlen, seq_bytes)) end = std::max(end, j.qoff + j.qlen);
+        if (span_inside(j.toff, j.tlen, seq_bytes)) end = std::max(end, j.toff + j.tlen);
+    }
+    return seq_bytes - end <= seq_bytes / 8;
+}
+
 // Device-buffer extension with the tile shapes `tiles` launched (every shape
 // the context's map uses when the caller cannot tell which are needed).
 static int extend_device(bsb_ctx *ctx, const bsb_ext_param_t *param, const bsb_ext_job_t *d_jobs,
@@ -413,8 +425,9 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     const bool installed = ctx->d_tile_map != nullptr;
     // Batches of one piece, from a few thousand jobs on: the scan is a kernel over the copied jobs, which goes on while
     // the sequences follow.  On one host thread it took 165 of 835 us for 64k jobs of 10-140 bases and 280 of 4300
-    // for 50k of 100-600.  It would also have told how much of seq the jobs use, so not where seq may be mostly others'.
-    const bool on_device = nck == 1 && n_jobs >= 4096 && seq_bytes >= 0 && seq_bytes / 2048 <= n_jobs;
+    // for 50k of 100-600.  It also tells how much of seq the jobs use, which the device cannot before all of it is on the
+    // way: so not where seq may be mostly others' (300k jobs on the first MB of 600: 4.9 ms copied whole, 2.1).
+    const bool on_device = nck == 1 && n_jobs >= 4096 && seq_bytes >= 0 && seq_mostly_used(jobs, n_jobs, seq_bytes);
     if (!on_device) scan_pieces(P, jobs, n_jobs, per, nck, seq_bytes, installed ? ctx->tile_map : ksw_builtin_tile_map(builtin),
                 installed ? -1 : builtin, piece);
     for (int k = 0; k < nck && !on_device; ++k)          // every job is checked before any other use of it
