@@ -169,6 +169,9 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
                        cudaEvent_t ev0, cudaEvent_t ev1, const cudaEvent_t *tile_ev = nullptr,
                        uint64_t *launched = nullptr, const KswStreams *ms = nullptr, bool all_narrow = false);
+// Runs every kernel that ksw_launch can choose on the built-in maps once, on no jobs, so that the CUDA runtime has nothing
+// of them to load later.  scratch: the ksw_launch scratch of no jobs.
+cudaError_t ksw_load_kernels(void *scratch, cudaStream_t st);
 // all_narrow: the caller knows that no job's h0 + qlen * max(mat) exceeds this, so that no job needs
 // 32-bit cells where the scoring allows 16-bit ones.
 int ksw_pack16_max();

@@ -411,6 +411,48 @@ bool ksw_takes_ring(const KswParams &P, const bsb_ext_job_t &j, int builtin)
 
 int ksw_ring_tile() { return kRingTile; }
 
+namespace {
+
+// What the head of the scratch holds behind the counters.
+constexpr size_t kZeroedBytes = sizeof(int) * (3 * kNumTiles + 1 + kHistSlots);
+struct SchedScratch {
+    int *rejected, *hist, *cursor;
+    int32_t *ranges;
+    explicit SchedScratch(void *scratch)
+        : rejected((int *)scratch + 3 * kNumTiles), hist(rejected + 1), cursor(hist + kHistSlots), ranges(cursor + kHistSlots)
+    {
+    }
+};
+
+}  // namespace
+
+cudaError_t ksw_load_kernels(void *scratch, cudaStream_t st)
+{
+    const SchedScratch s(scratch);
+    KswParams P{};
+    P.e_del = P.e_ins = P.pack16 = 1;
+    cudaError_t e = cudaMemsetAsync(scratch, 0, kZeroedBytes, st);
+    if (e != cudaSuccess) return e;
+    ksw_sched_hist<false><<<1, kHistThreads, 0, st>>>(P, nullptr, 0, 0, nullptr, nullptr, nullptr, 0, 0, 0, 0, 4, nullptr,
+                                                      s.hist, nullptr);
+    ksw_sched_scan<<<1, kScanThreads, 0, st>>>(s.hist, s.cursor, s.ranges, s.rejected);
+    ksw_sched_scatter<<<1, 256, 0, st>>>(nullptr, 0, s.cursor, nullptr);
+    ksw_sched_scatter_tiles<<<1, kScatterThreads, 0, st>>>(nullptr, 0, s.cursor, nullptr);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const auto run = [&](KswTileLaunch f) {
+        return f ? f(P, nullptr, nullptr, nullptr, s.ranges, (int *)scratch, nullptr, nullptr, -1, st) : cudaSuccess;
+    };
+    uint64_t tiles = 0;
+    for (int b = 0; b < kBuiltinMaps; ++b) tiles |= ksw_map_tiles(kBuiltinTileMaps[b].tile);
+    for (int t = 0; t < kNumTiles; ++t)
+        if (tiles >> t & 1 &&
+            ((e = run(ksw_tile_launcher(t))) != cudaSuccess || (e = run(ksw_tile16_launcher(t))) != cudaSuccess))
+            return e;
+    for (int r = 0; r < (int)(sizeof(kRings) / sizeof(kRings[0])); ++r)
+        if ((e = run(ksw_ring16(r))) != cudaSuccess) return e;
+    return cudaSuccess;
+}
+
 cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t n, int64_t seq_bytes,
                        const uint8_t *d_seq, const int32_t *d_cost, const uint8_t *d_map, int builtin, uint64_t tiles,
                        bsb_ext_out_t *d_out, int64_t *d_cells, void *scratch, int n_sm, cudaStream_t st,
@@ -418,14 +460,10 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
                        const KswStreams *ms, bool all_narrow)
 {
     if (launched) *launched = 0;
-    char *p = (char *)scratch;
-    int *counter = (int *)p;                // 3 per tile: 16-bit range, wide range, whole tile
-    int *rejected = counter + 3 * kNumTiles;
-    int *hist = rejected + 1;
-    int *cursor = hist + kHistSlots;
-    int32_t *ranges = cursor + kHistSlots;
-    int32_t *key = (int32_t *)(p + fixed_bytes());
-    int32_t *order = key + n;
+    int *const counter = (int *)scratch;    // 3 per tile: 16-bit range, wide range, whole tile
+    const SchedScratch sched(scratch);
+    int *const rejected = sched.rejected, *const hist = sched.hist, *const cursor = sched.cursor;
+    int32_t *const ranges = sched.ranges, *const key = (int32_t *)((char *)scratch + fixed_bytes()), *const order = key + n;
     // 16-bit cells need every value of the packed arithmetic inside 16 bits: penalties
     // and their multiples by a lane's column count stay small, and scores at most
     // kPack16MaxScore (h0 + qlen * max score is checked per job)
@@ -444,7 +482,7 @@ cudaError_t ksw_launch(const KswParams &P, const bsb_ext_job_t *d_jobs, int64_t 
     }
     cudaError_t e;
     if (ev0) cudaEventRecord(ev0, st);
-    e = cudaMemsetAsync(scratch, 0, sizeof(int) * (3 * kNumTiles + 1 + kHistSlots), st);
+    e = cudaMemsetAsync(scratch, 0, kZeroedBytes, st);
     if (e != cudaSuccess) return e;
     if (n > 0) {
         const int nb = (int)min((int64_t)n_sm * 8, (n + 255) / 256);

@@ -468,16 +468,13 @@ int bsb_last_read_order(bsb_ctx *ctx, int32_t *reads, int32_t max, int32_t *n);
  *   - At most BSB_NOALLOC_MAX_JOBS jobs per call; a larger n_jobs returns
  *     BSB_ECAPACITY before any work is queued.
  *   - The first call on a device looks up the array's device address
- *     (cudaGetSymbolAddress), also when n_jobs is 0; make that first call
- *     before any stream capture.  The extension kernels themselves are
- *     loaded by the CUDA runtime on their first launch, which takes device
- *     memory for their code: a warm-up batch that reaches the shapes and
- *     cell widths the later calls use (16-bit cells need penalties and
- *     scores as bsb_extend_batch allows them, max score <= 15) leaves
- *     nothing to load later.
- *   - Every shape of the library's default tile map is launched on every
- *     call (those with no jobs exit at once): the tile map is not chosen
- *     per batch.
+ *     (cudaGetSymbolAddress) and runs every extension kernel once on no
+ *     jobs, also when n_jobs is 0: the CUDA runtime loads a kernel on its
+ *     first launch, which takes device memory for its code, and this leaves
+ *     nothing to load later, whatever the later calls' sizes, shapes and
+ *     cell widths.  Make that first call before any stream capture.
+ *   - The tile map is the built-in one for n_jobs, as in bsb_extend_batch;
+ *     every shape of it is launched (those with no jobs exit at once).
  *   - Every call shares the array and it keeps the last call's contents
  *     (the launch clears what must start at zero).  Calls whose work
  *     overlaps on the GPU race on it: order them on one stream.
