@@ -30,6 +30,7 @@ int bsb_fail(bsb_ctx *ctx, int code, const char *fmt, ...)
 int bsb_cuda(bsb_ctx *ctx, cudaError_t e, const char *what)
 {
     if (e == cudaSuccess) return 0;
+    cudaGetLastError();      // reported here: the thread's next launch check must not find it again
     if (e == cudaErrorMemoryAllocation)
         return bsb_fail(ctx, BSB_ENOMEM, "%s: %s", what, cudaGetErrorString(e));
     return bsb_fail(ctx, BSB_ECUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -499,12 +500,10 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     return bsb_sync(ctx);
 }
 
-// The time between two marks; an error is reported, not left behind as the thread's last one.
+// The time between two marks.
 static int elapsed(bsb_ctx *ctx, float *ms, cudaEvent_t a, cudaEvent_t b)
 {
-    const cudaError_t e = cudaEventElapsedTime(ms, a, b);
-    if (e != cudaSuccess) cudaGetLastError();
-    return bsb_cuda(ctx, e, "extension times");
+    return bsb_cuda(ctx, cudaEventElapsedTime(ms, a, b), "extension times");
 }
 
 extern "C" int bsb_sync(bsb_ctx *ctx)
