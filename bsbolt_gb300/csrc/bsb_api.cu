@@ -36,6 +36,15 @@ int bsb_cuda(bsb_ctx *ctx, cudaError_t e, const char *what)
     return bsb_fail(ctx, BSB_ECUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+void bsb_release_build(bsb_ctx *ctx)
+{
+    if (!ctx->build_buf) return;
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->build_buf);
+    ctx->build_buf = nullptr;
+    ctx->build_bytes = 0;
+}
+
 int bsb_ensure(bsb_ctx *ctx, void **buf, size_t *cur, size_t bytes, const char *what)
 {
     if (*cur >= bytes && *buf) return 0;
@@ -48,6 +57,11 @@ int bsb_ensure(bsb_ctx *ctx, void **buf, size_t *cur, size_t bytes, const char *
     }
     size_t want = bytes + bytes / 4 + 4096;   // grow with headroom
     cudaError_t e = cudaMalloc(buf, want);
+    if (e == cudaErrorMemoryAllocation && ctx->build_buf) {
+        cudaGetLastError();
+        bsb_release_build(ctx);
+        e = cudaMalloc(buf, want);
+    }
     if (e != cudaSuccess) {
         *buf = nullptr;
         return bsb_cuda(ctx, e, what);

@@ -102,6 +102,7 @@ extern "C" int bsb_index_full_sa(bsb_ctx *ctx, int enable)
         ctx->idx_sa_full = nullptr;
         return 0;
     }
+    if (!ctx->idx_sa_full) bsb_release_build(ctx);
     if ((rc = build_sa_full(ctx))) return rc;
     return ctx->idx_sa_full ? 0 : bsb_fail(ctx, BSB_ENOMEM, "the full suffix array does not fit in device memory");
 }
@@ -159,6 +160,7 @@ extern "C" int bsb_index_upload(bsb_ctx *ctx, const bsb_index_view_t *v)
     int rc;
     if ((rc = bsb_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice"))) return rc;
     bsb_index_release(ctx);
+    bsb_release_build(ctx);
     {
         // the reference blocks go to a zero-padded staging buffer of whole blocks, then are re-cut
         // into sectors (two per block, one extra block of padding past the last symbol)

@@ -93,7 +93,8 @@ struct bsb_ctx {
     // the chains' first extensions of an alignment batch: jobs, bytes, results, scheduler scratch
     void *pre_buf = nullptr;
     size_t pre_bytes = 0;
-    // workspace of bsb_build_bwt for texts that need at most 4 GB
+    // workspace of bsb_build_bwt for texts that need at most 4 GB; given back (bsb_release_build) where other calls need
+    // room: index uploads, builds of another form, an allocation of bsb_ensure that does not fit
     void *build_buf = nullptr;
     size_t build_bytes = 0;
     // learned read order of the alignment batches: the cost model (caller's device memory,
@@ -123,6 +124,7 @@ int bsb_fail(bsb_ctx *ctx, int code, const char *fmt, ...);
 // Maps a CUDA error to BSB_ECUDA with a message; returns 0 for cudaSuccess.
 int bsb_cuda(bsb_ctx *ctx, cudaError_t e, const char *what);
 // Ensures *buf holds at least bytes of device memory (grow-only).
+void bsb_release_build(bsb_ctx *ctx);
 int bsb_ensure(bsb_ctx *ctx, void **buf, size_t *cur, size_t bytes, const char *what);
 
 // Device-side scoring for one extension batch.

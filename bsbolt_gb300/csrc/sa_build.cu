@@ -121,6 +121,7 @@ extern "C" int bsb_build_suffix_array(bsb_ctx *ctx, const uint8_t *pac, int64_t 
                                        m, st) != cudaSuccess)
         return bsb_fail(ctx, BSB_ECUDA, "suffix array: sort set-up");
     const size_t tmp_bytes = tmp_sort > tmp_scan ? tmp_sort : tmp_scan;
+    bsb_release_build(ctx);
     if ((rc = bsb_cuda(ctx, cudaMalloc(&d_pac.p, pb + 16), "suffix array: pac")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&d_text.p, (size_t)n + 16), "suffix array: text")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&k0.p, 8 * (size_t)m), "suffix array: keys")) ||
@@ -619,14 +620,19 @@ extern "C" int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, in
                               {&d_tmp, lent_tmp + 256}, {&d_small, 28 * (size_t)small_cap}};
         size_t need = 0;
         for (const Part &q : parts) need += (q.bytes + 255) & ~(size_t)255;
-        if (need <= kBuildKept && !bsb_ensure(ctx, &ctx->build_buf, &ctx->build_bytes, need, "BWT build")) {
+        if (need <= kBuildKept && ctx->build_bytes < need) {
+            bsb_release_build(ctx);
+            const size_t want = std::min(need + need / 4, kBuildKept);       // headroom for the next text, under the limit
+            if (cudaMalloc(&ctx->build_buf, want) == cudaSuccess) ctx->build_bytes = want;
+            else ctx->build_buf = nullptr, cudaGetLastError();     // no room for it: in chunks, as large texts are
+        }
+        if (need <= ctx->build_bytes) {
             char *at = (char *)ctx->build_buf;
             for (const Part &q : parts) q.b->p = at, q.b->lent = true, at += (q.bytes + 255) & ~(size_t)255;
             whole = true;
-        } else {
-            cudaGetLastError();          // no room for it: in chunks, as large texts are
         }
     }
+    if (!whole) bsb_release_build(ctx);
     if (!whole && ((rc = bsb_cuda(ctx, cudaMalloc(&d_text.p, (size_t)n + 64), "BWT build: text")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&d_rank.p, 8 * (size_t)m), "BWT build: ranks")) ||
         (rc = bsb_cuda(ctx, cudaMalloc(&d_hist.p, 8 * (size_t)std::max(kBuckets, 1 << kBinBits)),

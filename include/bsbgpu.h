@@ -188,7 +188,9 @@ int bsb_build_suffix_array(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, int6
  * layout before the occurrence counts are interleaved); *primary, that row; sa[k] = SA[k *
  * sa_intv] for k < (2*l_pac + sa_intv)/sa_intv.  bsbolt_gb300.index.build_index writes
  * BWA's .bwt/.sa from them (bwtindex.c:256-321).  BSB_ENOMEM when one 5-symbol bucket of
- * suffixes does not fit a chunk.  No reference counterpart: bwa index sorts on the CPU. */
+ * suffixes does not fit a chunk.  For a text whose workspace takes at most 4 GB (some 36 bytes
+ * per symbol) and that `chunk` does not divide, the context keeps that workspace for the next
+ * build, until an index is uploaded, another call needs the memory or the context ends.  No reference counterpart: bwa index sorts on the CPU. */
 int bsb_build_bwt(bsb_ctx *ctx, const uint8_t *pac, int64_t l_pac, int sa_intv, int64_t chunk, uint32_t *bwt,
                   uint64_t *primary, uint64_t *sa);
 
