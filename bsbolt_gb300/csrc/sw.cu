@@ -428,9 +428,10 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     }
     const bool w16_ok = S.o_del + S.e_del <= 32767 && S.o_ins + S.e_ins <= 32767;
     // the packed passes read F in closed form, which needs oe_ins >= e_ins as the lanes hold them
-    // (and byte lanes a matrix entry <= 0, see sw_pack.cuh)
-    const bool b8_ok = (uint8_t)(S.o_ins + S.e_ins) >= (uint8_t)S.e_ins &&
-                       *std::min_element(S.mat, S.mat + 25) <= 0;
+    const bool b8_ok = (uint8_t)(S.o_ins + S.e_ins) >= (uint8_t)S.e_ins;
+    // byte lanes of a matrix without an entry <= 0: its smallest, m, gives a shift of 256 - m, so a column adds at most
+    // mat - m and then takes 256 - m off, and every H stays 0.  A score that no H of 0 survives does the same
+    const bool all_zero8 = *std::min_element(S.mat, S.mat + 25) > 0;
     PackParams P8, P16;
     {
         for (int tc = 0; tc < 5; ++tc) {
@@ -439,6 +440,7 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
             P8.prof[tc] = make_uint2((uint32_t)w[0] | (uint32_t)w[1] << 8 | (uint32_t)w[2] << 16 | (uint32_t)w[3] << 24,
                                      (uint32_t)w[4]);
             P16.prof[tc] = P8.prof[tc];
+            if (all_zero8) P8.prof[tc] = make_uint2(0x80808080u, 0x80u);
         }
         P8.prof[5] = P16.prof[5] = make_uint2(0u, 0u);
         // the penalties as _mm_set1_epi8 / _mm_set1_epi16 broadcast them, negated in both halves.  Word lanes: no

@@ -7,7 +7,8 @@
 // Here thread t of a group of P/2 plays SIMD lanes t (low 16 bits) and t + P/2 (high 16 bits):
 //   P = 16, byte lanes (ksw_u8), for matrices with an entry <= 0: then shift = -min, and a score that the
 //     reference's bytes would clip puts the row's maximum at 255 - shift or above, where the pass ends with
-//     score 255 whatever the rest of the row holds.  So signed scores in 16 bits, without a clip, are exact;
+//     score 255 whatever the rest of the row holds.  So signed scores in 16 bits, without a clip, are exact.
+//     (Matrices without one leave every H at 0: sw.cu hands in scores that do.)
 //   P = 8, word lanes (ksw_i16): the same instructions, for jobs whose scores
 //     cannot reach the reference's 16-bit saturation (qlen * max score <= 32640) and whose
 //     penalties stay below 32768, so that 16-bit arithmetic without saturation is exact.
