@@ -99,7 +99,7 @@ __device__ __forceinline__ void load_score_table(const KswParams &P, int8_t *tab
 __device__ __forceinline__ int diagonal_limit(const KswParams &P, int h0)
 {
     int lim = min(P.o_del + P.e_del, P.o_ins + P.e_ins);
-    if (P.zdrop > 0) lim = min(lim, P.zdrop + 1);
+    if (P.zdrop > 0 && P.zdrop < lim) lim = P.zdrop + 1;         // (zdrop + 1 may not exist)
     return P.mat_max > 0 ? min(lim, h0 + P.mat_max) : 0;
 }
 
