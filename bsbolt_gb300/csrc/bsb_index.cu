@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -23,7 +24,7 @@ cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, in
                         void *d_padded, int *d_count, int64_t *d_out_off, void *d_out,
                         const SeedPlan &p, void *d_lists, void *d_list_counts, int *d_ctrl, void *d_queue, int64_t queue_cap, int *d_tot,
                         int64_t *d_scan_tmp, int mult, int n_sm, cudaStream_t st);
-size_t kmer_bytes(uint64_t seq_len);
+size_t kmer_bytes(bool wide);
 cudaError_t kmer_build(const DevFM &F, void *out, cudaStream_t st);
 cudaError_t sa_launch(const DevFM &F, const uint64_t *d_rows, int64_t n, uint64_t *d_pos, int n_sm, cudaStream_t st);
 cudaError_t sa_full_build(const DevFM &F, int64_t n_sa, uint64_t *full, int *failed, int n_sm, cudaStream_t st);
@@ -62,6 +63,7 @@ static DevFM dev_fm(const bsb_ctx *ctx)
     int sh = 0;
     while ((1 << sh) < ctx->sa_intv) ++sh;
     F.sa_shift = sh;
+    F.wide = ctx->idx_wide;
     return F;
 }
 
@@ -219,14 +221,17 @@ extern "C" int bsb_index_upload(bsb_ctx *ctx, const bsb_index_view_t *v)
     ctx->primary = v->primary;
     for (int i = 0; i < 5; ++i) ctx->L2[i] = v->L2[i];
     ctx->seq_len = seq_len;
+    // (BSB_SEED_64BIT=1, read here: small indexes in 64 bits too, to test what otherwise takes 2^32 rows)
+    const char *const force = getenv("BSB_SEED_64BIT");
+    ctx->idx_wide = seq_len >= kNarrowRows || (force && force[0] == '1');
     ctx->sa_intv = v->sa_intv;
     ctx->n_sa = v->n_sa;
     ctx->l_pac = v->l_pac;
     if ((rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "index upload"))) return rc;
     if ((rc = build_sa_full(ctx))) return rc;
-    // the k-mer table, where it fits (seeding goes base by base without it); a text too short for
-    // every base to occur has none
-    if (seq_len > 0 && cudaMalloc(&ctx->idx_kmers, kmer_bytes(seq_len)) == cudaSuccess) {
+    // the k-mer table, where it fits (seeding goes base by base without it).  Strings that do not occur have empty
+    // intervals, those of a base the text does not hold among them
+    if (seq_len > 0 && cudaMalloc(&ctx->idx_kmers, kmer_bytes(ctx->idx_wide)) == cudaSuccess) {
         const DevFM F = dev_fm(ctx);
         if ((rc = bsb_cuda(ctx, kmer_build(F, ctx->idx_kmers, ctx->stream), "index: k-mer table")) ||
             (rc = bsb_cuda(ctx, cudaStreamSynchronize(ctx->stream), "index: k-mer table")))
@@ -352,7 +357,7 @@ int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_r
     const size_t padded = seed_padded_entries(total_bases, n_reads, mult) * sizeof(DevIntv);
     if (max_len > BSB_SEED_MAX_LEN) return bsb_fail(ctx, BSB_ETOOLONG, "max_len %d > %d", max_len, BSB_SEED_MAX_LEN);
     const DevFM F = dev_fm(ctx);
-    const SeedPlan plan = seed_plan(ctx->n_sm, total_bases, max_len, n_reads, F.seq_len);
+    const SeedPlan plan = seed_plan(ctx->n_sm, total_bases, max_len, n_reads, F.wide);
     const size_t lists = plan.list_bytes, counts_b = (plan.counts_bytes + 255) & ~(size_t)255;
     int64_t qn = 0;
     const size_t queue_b = (seed_queue_bytes(total_bases, n_reads, mult, &qn) + 255) & ~(size_t)255;
@@ -364,7 +369,7 @@ int bsb_seed_batch_device_m(bsb_ctx *ctx, const bsb_seed_opt_t *opt, int32_t n_r
     void *d_padded = s;
     void *d_lists = s + ((padded + 255) & ~(size_t)255);
     int *d_count = (int *)((char *)d_lists + ((lists + 255) & ~(size_t)255));
-    int *d_ctrl = d_count + ((2 * n_reads + 63) & ~63);     // two counts per read (seed_kernel's two parts)
+    int *d_ctrl = d_count + ((2 * n_reads + 63) & ~63);     // two counts per read (passes 1-2, pass 3)
     void *d_queue = d_ctrl + 64;                              // pass-2 work items
     int *d_tot = (int *)((char *)d_queue + queue_b);         // seeds kept per read
     void *d_list_counts = (char *)d_tot + tot_b;

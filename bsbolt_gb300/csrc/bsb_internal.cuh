@@ -50,6 +50,7 @@ struct bsb_ctx {
     void *idx_bwt = nullptr, *idx_sa = nullptr, *idx_pac = nullptr;
     void *idx_sb = nullptr;       // superblock counts of the occurrence array
     void *idx_kmers = nullptr;    // bi-intervals of all short strings (built at upload when they fit), or NULL
+    int idx_wide = 0;             // seeding in 64 bits (DevFM::wide)
     void *idx_sa_full = nullptr;  // every row's SA value (built at upload when it fits), or NULL
     void *idx_opac = nullptr;     // original (unconverted) reference, 2-bit, for the methylation calls
     uint64_t primary = 0, seq_len = 0, n_sa = 0;
@@ -236,4 +237,4 @@ struct SeedPlan {
     int64_t list_entries;
     size_t smem, counts_bytes, list_bytes;
 };
-SeedPlan seed_plan(int n_sm, int64_t total_bases, int max_len, int n_reads, uint64_t seq_len);
+SeedPlan seed_plan(int n_sm, int64_t total_bases, int max_len, int n_reads, bool wide);

@@ -28,7 +28,11 @@ struct DevFM {
     uint64_t seq_len;
     uint64_t L2[5];
     int sa_shift;            // log2(sa_intv)
+    int wide;                // seeding and its table in 64 bits
 };
+
+// An index below this many rows is seeded in 32 bits.
+constexpr uint64_t kNarrowRows = 0xfffffffdull;
 
 struct DevIntv {             // bwtintv_t (bwt.h:60-62)
     uint64_t x0, x1, x2, info;

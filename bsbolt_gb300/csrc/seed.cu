@@ -57,7 +57,6 @@ template <class P>
 struct Iv {
     P x0, x1, x2;
 };
-constexpr uint64_t kNarrowRows = 0xfffffffdull;
 
 // A match on a warp's list: its interval, and slot of the read << 21 | start << 11 | end (reads
 // have at most 1024 bases, so a start is below 2^10 and an end below 2^11).
@@ -837,15 +836,13 @@ __global__ void sa_fill_kernel(DevFM F, int64_t n_sa, uint64_t *__restrict__ ful
 
 }  // namespace
 
-static bool seed_narrow(uint64_t seq_len) { return seq_len < kNarrowRows; }
-
-// Builds the k-mer table of an index (kmer_bytes(seq_len) bytes) on the stream.
-size_t kmer_bytes(uint64_t seq_len) { return (size_t)kKmers * (seed_narrow(seq_len) ? 16 : 32); }
+// Builds the k-mer table of an index (kmer_bytes(F.wide) bytes) on the stream.
+size_t kmer_bytes(bool wide) { return (size_t)kKmers * (wide ? 32 : 16); }
 cudaError_t kmer_build(const DevFM &F, void *out, cudaStream_t st)
 {
     const unsigned blocks = kKmers / 16 / 128;
-    if (seed_narrow(F.seq_len)) kmer_kernel<uint32_t><<<blocks, 128, 0, st>>>(F, (uint4 *)out);
-    else kmer_kernel<uint64_t><<<blocks, 128, 0, st>>>(F, (uint4 *)out);
+    if (F.wide) kmer_kernel<uint64_t><<<blocks, 128, 0, st>>>(F, (uint4 *)out);
+    else kmer_kernel<uint32_t><<<blocks, 128, 0, st>>>(F, (uint4 *)out);
     return cudaGetLastError();
 }
 
@@ -863,9 +860,9 @@ static int again_blocks_per_sm(size_t smem)
 // matches: enough to fill the GPU, and at least four, which even out the lists (67k reads of 150
 // bases, seeding stage: 1.28 ms at 2, 1.30 at 3, 1.24 at 4, 1.26 at 6 and 8).  32 warps per SM at 64
 // registers: 40 at 48 registers 1.29, 48 at 40 2.1.  The lists of pass 1 and 2 share the memory.
-SeedPlan seed_plan(int n_sm, int64_t total_bases, int max_len, int n_reads, uint64_t seq_len)
+SeedPlan seed_plan(int n_sm, int64_t total_bases, int max_len, int n_reads, bool wide)
 {
-    const bool narrow = seed_narrow(seq_len);
+    const bool narrow = !wide;
     const size_t entry = narrow ? sizeof(Match32) : sizeof(Match64);
     SeedPlan p;
     p.slots = max_len <= 512 ? 32 : 16;
@@ -935,8 +932,8 @@ cudaError_t seed_launch(const DevFM &F, int min_seed_len, float split_factor, in
     S.mult = mult;
     S.offs = d_offs;
     int2 *const d_counts = (int2 *)d_list_counts;
-    if (seed_narrow(F.seq_len)) seed_passes<uint32_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, d_counts, p, st);
-    else seed_passes<uint64_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, d_counts, p, st);
+    if (F.wide) seed_passes<uint64_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, d_counts, p, st);
+    else seed_passes<uint32_t>(F, o, n_reads, max_len, d_seqs, S, d_lists, d_counts, p, st);
     read_totals<<<n_sm * 4, 256, 0, st>>>(d_count, d_offs, n_reads, mult, d_tot);
     e = scan_i32_i64(d_tot, n_reads, d_out_off, d_scan_tmp, st);
     if (e != cudaSuccess) return e;
