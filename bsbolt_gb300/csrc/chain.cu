@@ -1483,11 +1483,32 @@ __device__ __forceinline__ void right_end(const AlnOpt &opt, int l_query, const 
     }
 }
 
+// The learned order: reads by predicted cost, most expensive first, in 64 bins of half an
+// octave of the predicted cells (key).
+__device__ __forceinline__ int key_bin(int32_t key)
+{
+    if (key <= 0) return 63;
+    const uint32_t k = (uint32_t)key;
+    const int msb = 31 - __clz(k);
+    const int half = 2 * msb + (msb > 0 ? (int)(k >> (msb - 1) & 1u) : 0);
+    return 63 - (half < 63 ? half : 63);
+}
+
+// The order chain2aln_kernel takes reads in: by the keys given, or else (key NULL) most chains first (reads are
+// independent, so the order changes no result; it shortens the tail a few repeat-laden reads would otherwise set).
+// Where chain2aln_plain has gone before, only the reads it left.
+constexpr int kOrderBins = 64, kOrderThreads = 256;
+__device__ __forceinline__ int read_bin(const int32_t *key, const int *n_chains, int r)
+{
+    return key ? key_bin(key[r]) : kOrderBins - 1 - min(n_chains[r], kOrderBins - 1);
+}
+
 // mem_chain2aln for the reads whose extensions are all known (PreResults), a warp a read: 32 chains at a time, each lane
 // one chain's first seed, its region and its record; then the chains in order, the seed of each against the regions so
 // far over the lanes, and the chain's other seeds over the lanes, which must all be contained in a region and not part
 // from the chain's first.  A read where one would be extended, or with more than kPlainRegs regions, gets n_regs -1:
-// it is left for chain2aln_kernel, in the read order.  That kernel's loads follow one another chain by chain, on 16 warps an SM (it holds the DP).
+// it is left for chain2aln_kernel, in the read order, and counted in its bin of that (cnt; key as in read_bin).  That
+// kernel's loads follow one another chain by chain, on 16 warps an SM (it holds the DP).
 // 114k RRBS reads (450k regions): 617 us -> 199 and 175 for the reads left; 67k of 150 bases 292 -> 89 and 86.  At 10
 // blocks an SM, or a block for every four reads in place of 8 an SM: 20-80 us more.
 constexpr int kPlainWarps = 4, kPlainRegs = 64;
@@ -1495,7 +1516,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, 8)
 chain2aln_plain(AlnOpt opt, int n_reads, const int64_t *__restrict__ read_off, const int64_t *__restrict__ seed_off,
                 const int64_t *__restrict__ row_off_of_seed, const DevSeed *__restrict__ seeds,
                 const DevChain *__restrict__ chains, const int *__restrict__ n_chains, bsb_reg_t *__restrict__ regs,
-                int *__restrict__ n_regs, PreResults pre)
+                int *__restrict__ n_regs, PreResults pre, const int32_t *__restrict__ key, int *__restrict__ cnt)
 {
     __shared__ RegSpan sm[kPlainWarps][kPlainRegs];
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
@@ -1581,7 +1602,10 @@ chain2aln_plain(AlnOpt opt, int n_reads, const int64_t *__restrict__ read_off, c
             }
             if (ok && slot >= 0) regs[R0 + slot] = a;
         }
-        if (lane == 0) n_regs[r] = ok ? nav : -1;
+        if (lane == 0) {
+            n_regs[r] = ok ? nav : -1;
+            if (!ok) atomicAdd(&cnt[read_bin(key, n_chains, r)], 1);
+        }
     }
 }
 
@@ -1922,21 +1946,9 @@ __global__ void read_features_kernel(AlnOpt opt, DevBns B, int n_reads, const ui
     }
 }
 
-// The learned order: reads by predicted cost, most expensive first, in 64 bins of half an
-// octave of the predicted cells (key).
-__device__ __forceinline__ int key_bin(int32_t key)
-{
-    if (key <= 0) return 63;
-    const uint32_t k = (uint32_t)key;
-    const int msb = 31 - __clz(k);
-    const int half = 2 * msb + (msb > 0 ? (int)(k >> (msb - 1) & 1u) : 0);
-    return 63 - (half < 63 ? half : 63);
-}
-// Counting sort into 64 bins in two kernels: the bins' sizes, then the places (bin -1: the read is left out; n_placed,
-// optional: how many were not).  A block counts in shared
-// memory and touches each global counter once (one global atomic per read on a few busy counters took
-// 84 us for 67k reads, the two kernels together).
-constexpr int kOrderBins = 64, kOrderThreads = 256;
+// Counting sort into 64 bins in two kernels: the bins' sizes, then the places (bin -1: the read gets none; n_placed,
+// optional: how many did).  A block counts in shared memory and touches each global counter once (one global atomic
+// per read on a few busy counters took 84 us for 67k reads, the two kernels together).
 template <class Bin>
 __device__ __forceinline__ void order_count(int n_reads, int *__restrict__ cnt, Bin bin)
 {
@@ -1944,7 +1956,7 @@ __device__ __forceinline__ void order_count(int n_reads, int *__restrict__ cnt, 
     if (threadIdx.x < kOrderBins) sh[threadIdx.x] = 0;
     __syncthreads();
     for (int r = blockIdx.x * kOrderThreads + threadIdx.x; r < n_reads; r += gridDim.x * kOrderThreads)
-        if (const int b = bin(r); b >= 0) atomicAdd(&sh[b], 1);
+        atomicAdd(&sh[bin(r)], 1);
     __syncthreads();
     if (threadIdx.x < kOrderBins && sh[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], sh[threadIdx.x]);
 }
@@ -1972,34 +1984,19 @@ __device__ __forceinline__ void order_place(int n_reads, const int *__restrict__
     }
 }
 
-// The order chain2aln_kernel takes reads in, by the keys given or else most chains first (reads are independent, so the
-// order changes no result; it shortens the tail a few repeat-laden reads would otherwise set).  Where chain2aln_plain
-// has gone before, only the reads it left: n_regs below 0 (NULL: all reads).
+// Not where chain2aln_plain has gone before, which counts.
 __global__ void __launch_bounds__(kOrderThreads)
-order_hist_key(const int32_t *__restrict__ key, const int *__restrict__ n_regs, int n_reads, int *__restrict__ cnt)
+order_hist(const int32_t *__restrict__ key, const int *__restrict__ n_chains, int n_reads, int *__restrict__ cnt)
 {
-    order_count(n_reads, cnt, [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : key_bin(key[r]); });
+    order_count(n_reads, cnt, [=](int r) { return read_bin(key, n_chains, r); });
 }
+// n_regs: chain2aln_plain's (below 0: the read was left), or NULL.
 __global__ void __launch_bounds__(kOrderThreads)
-order_scatter_key(const int32_t *__restrict__ key, const int *__restrict__ n_regs, int n_reads,
-                  const int *__restrict__ cnt, int *__restrict__ cur, int *__restrict__ order, int *__restrict__ n_placed)
-{
-    order_place(n_reads, cnt, cur, order, n_placed, [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : key_bin(key[r]); });
-}
-
-__device__ __forceinline__ int order_bin(int nc) { return kOrderBins - 1 - (nc < kOrderBins - 1 ? nc : kOrderBins - 1); }
-
-__global__ void __launch_bounds__(kOrderThreads)
-order_hist(const int *__restrict__ n_chains, const int *__restrict__ n_regs, int n_reads, int *__restrict__ cnt)
-{
-    order_count(n_reads, cnt, [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : order_bin(n_chains[r]); });
-}
-__global__ void __launch_bounds__(kOrderThreads)
-order_scatter(const int *__restrict__ n_chains, const int *__restrict__ n_regs, int n_reads, const int *__restrict__ cnt,
-              int *__restrict__ cur, int *__restrict__ order, int *__restrict__ n_placed)
+order_scatter(const int32_t *__restrict__ key, const int *__restrict__ n_chains, const int *__restrict__ n_regs, int n_reads,
+              const int *__restrict__ cnt, int *__restrict__ cur, int *__restrict__ order, int *__restrict__ n_placed)
 {
     order_place(n_reads, cnt, cur, order, n_placed,
-                [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : order_bin(n_chains[r]); });
+                [=](int r) { return n_regs && n_regs[r] >= 0 ? -1 : read_bin(key, n_chains, r); });
 }
 
 // The order chain_warp_kernel takes a large batch's reads in: most rows first, in steps of four.  A read on
@@ -2679,18 +2676,7 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     if ((rc = bsb_cuda(ctx, cudaEventRecord(ctx->stage_ev[3], st), "stage mark"))) return rc;
     int *const order = (int *)(A + o_order);
     int *const n_list = ctrl + 2, *const ocnt = (int *)(A + o_order + al(sizeof(int) * (n_reads + 1)));
-    // the reads that need no other extension than their chains' first; the rest is chain2aln_kernel's
     const bool logging = ctx->read_log != 0;
-    PreResults pre{};
-    if (!logging && n_reads >= kPreReads &&
-        (rc = first_extensions(ctx, o, ao, B, P, n_reads, max_len, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
-                               n_chains, reg_off, scan_tmp, &pre)))
-        return rc;
-    if (pre.chains) {
-        const int pb = std::min((n_reads + kPlainWarps - 1) / kPlainWarps, ctx->n_sm * 8);
-        chain2aln_plain<<<pb, kPlainWarps * 32, 0, st>>>(ao, n_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
-                                                         n_chains, regs, n_regs, pre);
-    }
     // per-read features / extension cells for the learned read order (kept for bsb_last_read_costs)
     float *d_feat = nullptr;
     int64_t *d_rcells = nullptr;
@@ -2712,29 +2698,35 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
                                                      cchains, n_chains, d_feat);
         ctx->rc_n = logging ? n_reads : 0;
     }
-    {
-        const int *const open = pre.chains ? n_regs : nullptr;
-        const int ob = (int)((n_reads + 255) / 256) < ctx->n_sm * 4 ? (int)((n_reads + 255) / 256) : ctx->n_sm * 4;
-        if ((rc = bsb_cuda(ctx, cudaMemsetAsync(ocnt, 0, sizeof(int) * 2 * kOrderBins, st), "read order"))) return rc;
-        if (keyed) {         // the caller's keys, once (the copy is done before they are cleared)
-            if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_rkey, ctx->order_keys.data(), sizeof(int32_t) * (size_t)n_reads,
-                                                    cudaMemcpyHostToDevice, st), "read order keys")) ||
-                (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "read order keys")))
-                return rc;
-            ctx->order_keys.clear();
-            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt);
-            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt, ocnt + kOrderBins, order, n_list);
-        } else if (learned) {   // predicted cells of every read, most expensive first
-            if ((rc = bsb_mlp_forward(ctx, (const bsb_mlp_weights_t *)ctx->read_model, d_feat, n_reads, nullptr,
-                                      d_rkey)))
-                return rc;
-            order_hist_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt);
-            order_scatter_key<<<ob, kOrderThreads, 0, st>>>(d_rkey, open, n_reads, ocnt, ocnt + kOrderBins, order, n_list);
-        } else {
-            order_hist<<<ob, kOrderThreads, 0, st>>>(n_chains, open, n_reads, ocnt);
-            order_scatter<<<ob, kOrderThreads, 0, st>>>(n_chains, open, n_reads, ocnt, ocnt + kOrderBins, order, n_list);
-        }
+    const int32_t *key = nullptr;
+    if (keyed) {             // the caller's keys, once (the copy is done before they are cleared)
+        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_rkey, ctx->order_keys.data(), sizeof(int32_t) * (size_t)n_reads,
+                                                cudaMemcpyHostToDevice, st), "read order keys")) ||
+            (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "read order keys")))
+            return rc;
+        ctx->order_keys.clear();
+        key = d_rkey;
+    } else if (learned) {    // predicted cells of every read
+        if ((rc = bsb_mlp_forward(ctx, (const bsb_mlp_weights_t *)ctx->read_model, d_feat, n_reads, nullptr, d_rkey)))
+            return rc;
+        key = d_rkey;
     }
+    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(ocnt, 0, sizeof(int) * 2 * kOrderBins, st), "read order"))) return rc;
+    PreResults pre{};
+    if (!logging && n_reads >= kPreReads &&
+        (rc = first_extensions(ctx, o, ao, B, P, n_reads, max_len, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
+                               n_chains, reg_off, scan_tmp, &pre)))
+        return rc;
+    const int ob = std::min((n_reads + kOrderThreads - 1) / kOrderThreads, ctx->n_sm * 4);
+    if (pre.chains) {           // the reads that need no other extension than their chains' first
+        const int pb = std::min((n_reads + kPlainWarps - 1) / kPlainWarps, ctx->n_sm * 8);
+        chain2aln_plain<<<pb, kPlainWarps * 32, 0, st>>>(ao, n_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
+                                                         n_chains, regs, n_regs, pre, key, ocnt);
+    } else {
+        order_hist<<<ob, kOrderThreads, 0, st>>>(key, n_chains, n_reads, ocnt);
+    }
+    order_scatter<<<ob, kOrderThreads, 0, st>>>(key, n_chains, pre.chains ? n_regs : nullptr, n_reads, ocnt,
+                                                ocnt + kOrderBins, order, n_list);
     ctx->queue_reads = order, ctx->queue_count = n_list;
     int64_t *const rcells_out = logging ? d_rcells : nullptr;
     // every extension of these reads fits (max_len + 1) columns: the narrowest variant that holds them
