@@ -365,7 +365,9 @@ extern "C" int bsb_tile_shapes(int32_t *G, int32_t *C, int max)
 extern "C" int bsb_set_tile_map(bsb_ctx *ctx, const uint8_t *map, int n)
 {
     if (!ctx) return BSB_EINVAL;
-    if (!map) {
+    // the map bsb_get_tile_map gives where none is installed means the built-in ones, whatever the batch's size, rings and
+    // cut bands included: a caller that puts back what it read leaves the context as it was
+    if (!map || (n == BSB_TILE_MAP_LEN && !memcmp(map + 1, ksw_default_tile_map() + 1, BSB_TILE_MAP_LEN - 1))) {
         memcpy(ctx->tile_map, ksw_default_tile_map(), BSB_TILE_MAP_LEN);
         ctx->map_tiles = ksw_map_tiles(ctx->tile_map);
         if (ctx->d_tile_map) {

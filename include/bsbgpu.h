@@ -121,9 +121,10 @@ float bsb_last_kernel_ms(const bsb_ctx *ctx);
 int bsb_tile_shapes(int32_t *G, int32_t *C, int max);
 
 /* Installs map (BSB_TILE_MAP_LEN entries, shape index per qlen + 1) for this
- * context's later extension batches; NULL restores the default map.  Every
- * entry [need], need = 1..1024, must name a shape with G*C >= need
- * (BSB_EINVAL otherwise, and the current map stays). */
+ * context's later extension batches; NULL, or the map that bsb_get_tile_map
+ * gives without an installed one, restores the built-in maps.  Every entry
+ * [need], need = 1..1024, must name a shape with G*C >= need (BSB_EINVAL
+ * otherwise, and the current map stays). */
 int bsb_set_tile_map(bsb_ctx *ctx, const uint8_t *map, int n);
 
 /* Device time of each shape's kernel in the context's most recent extension
