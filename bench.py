@@ -1130,7 +1130,7 @@ def autotune_block(ctx, L, param, d_jobs, n, d_seq, seq_bytes, d_out, out_ref, s
         same = bool(np.array_equal(d_out.cpu().numpy(), out_ref))
     finally:
         autotune.set_map(ctx, None)
-    changed = [r for r in report if r["best"] != r["current"]]
+    changed = [r for r in report if r["best"] != r["current"] and r.get("kept", True)]
     return {"tuned_on": "1M held-out jobs of the same distribution (another seed), bands of need = qlen+1",
             "tune_s": round(tune_s, 2), "bands_tuned": len(report), "bands_changed": len(changed),
             "changes": [{"need": r["need"], "from": r["current"], "to": r["best"],

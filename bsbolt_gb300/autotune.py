@@ -104,7 +104,11 @@ def tune(ctx, jobs: np.ndarray, seq: np.ndarray, param, min_jobs: int = 4096, ma
     """Measure the candidate shapes of every band with at least `min_jobs` jobs.
 
     Returns (tile map, report); bands with too few jobs keep the context's
-    current shape.  The context's map is left as it was."""
+    current shape.  A map that takes another shape anywhere runs without what
+    only the built-in maps have (shapes by batch size, rings, cut bands), so it
+    is timed on all the jobs at last: where it is not faster there, the
+    context's current map is returned, and the report's bands say "kept": False.
+    The context's map is left as it was."""
     jobs = np.ascontiguousarray(jobs)
     if jobs.dtype != JOB_DTYPE:
         jobs = jobs.view(JOB_DTYPE).reshape(-1)
@@ -148,6 +152,15 @@ def tune(ctx, jobs: np.ndarray, seq: np.ndarray, param, min_jobs: int = 4096, ma
                            "best": list(shape_list[best]), "current_ms": round(times[cur], 4),
                            "best_ms": round(times[best], 4),
                            "ms": {f"{shape_list[t][0]}x{shape_list[t][1]}": round(v, 4) for t, v in times.items()}})
+        if not np.array_equal(tmap[1:], base[1:]):
+            whole = {}
+            for name, m in (("current", base), ("tuned", tmap)):
+                set_map(ctx, m)
+                whole[name] = float(np.median([_run(ctx, param, jobs, seq)[1] for _ in range(reps + 1)][1:]))
+            for r in report:
+                r["kept"] = whole["tuned"] < whole["current"]
+            if not report[0]["kept"]:
+                tmap = base.copy()
     finally:
         set_map(ctx, base)
     return tmap, report
