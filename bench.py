@@ -450,7 +450,7 @@ def measured_hbm_gbs():
 
 
 def seeding_roofline(ctx, reads, offs, reps=5):
-    """Device time of one seeding batch (seed_kernel's two launches, the offset scan and the
+    """Device time of one seeding batch (the three seeding kernels, the offset scan and the
     compaction: bsb_seed_batch_device) with CUDA events on the context stream, and the
     occurrence-query bytes it reads as algorithmic traffic: per bwt_extend one bwt_2occ4 =
     two queries, 32 B each in the device's sector layout (64 B each in the reference's

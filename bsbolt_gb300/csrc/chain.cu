@@ -2164,7 +2164,7 @@ __device__ __noinline__ int patch_reg_warp(const DedupOpt &O, const int8_t *smat
 // merge scan is taken by every lane in step (lane 0 writes), so that the warp can run a merge's global
 // alignment, and only at regions that reach the one before.
 // Both sorts on one lane with the records in global memory, all regions scanned: 0.50 ms for 114k RRBS
-// reads (450k regions), 0.20 ms for 67k of 150 bases; as here 0.24 and 0.13.  Time is a warp's own chain
+// reads (450k regions), 0.20 ms for 67k of 150 bases; as here 0.25 and 0.12.  Time is a warp's own chain
 // (10k clocks a read), so warps resident count up to where registers spill: at 6, 8, 10 and 12 blocks an SM the
 // stage takes 0.315, 0.288, 0.287, 0.350 ms on the RRBS reads and 0.190, 0.181, 0.207, 0.237 on the others.
 __global__ void __launch_bounds__(kDedupWarps * 32, 8)

@@ -99,8 +99,8 @@ __device__ __forceinline__ int clamped_band(const KswParams &P, const bsb_ext_jo
 // issued.  A warp takes `per` jobs at a time: a lane each for the checks and the key, then four
 // diagonals at once, eight lanes each (2M jobs of 10-140 bases: 0.38 ms, 26 us without the
 // diagonals; one diagonal after the other by the whole warp 0.52 ms; 64 jobs 9 against 46 us).
-// Half of those jobs end here: with the rows left out (ksw_core.cuh) the batch takes 8.0 ms
-// instead of 23.4.
+// Half of those jobs end here: with the rows left out (ksw_core.cuh) the batch takes 7.9 ms
+// instead of 23.4, and 6.8 with the others' bands cut (ksw_tiles.cuh).
 constexpr int32_t kDoneKey = -1;
 constexpr int kHistThreads = 256;
 template <bool Packed>

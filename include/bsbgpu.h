@@ -78,7 +78,8 @@ typedef struct {
  * the reference visits (sum over rows of end-beg).  Requires qlen <= 1023,
  * 1 <= e_del, e_ins <= 65535, 0 <= o_del, o_ins <= 65535, matrix entries in
  * [-63, 63] and 0 < h0 <= 2^20 (the reference asserts h0 > 0); violations
- * return BSB_EINVAL / BSB_ETOOLONG before any device work. */
+ * return BSB_EINVAL / BSB_ETOOLONG, with the first unfit job named, before any
+ * job is extended. */
 int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param,
                      const bsb_ext_job_t *jobs, int64_t n_jobs,
                      const uint8_t *seq, int64_t seq_bytes,
@@ -111,7 +112,7 @@ float bsb_last_kernel_ms(const bsb_ctx *ctx);
  * A batched extension job runs on a tile of G lanes x C query columns per
  * lane (32/G jobs per warp); the tile map assigns a compiled shape to every
  * query length.  The shape changes the time, never a result.  The library
- * ships a default map measured on GB300; an autotuner (bsbolt_gb300.autotune)
+ * ships maps measured on GB300, by batch size; an autotuner (bsbolt_gb300.autotune)
  * can measure the shapes on the caller's own jobs and install its map. */
 #define BSB_NUM_TILES 61
 #define BSB_TILE_MAP_LEN 1025    /* entry [qlen + 1] for qlen = 0..1023; [0] unused */
@@ -138,8 +139,11 @@ int bsb_set_tile_map(bsb_ctx *ctx, const uint8_t *map, int n);
  * 32 x 11 shapes.  Valid after bsb_sync. */
 int bsb_last_tile_ms(const bsb_ctx *ctx, float *ms, int n);
 
-/* Copies the context's current tile map into map (n >= BSB_TILE_MAP_LEN);
- * ctx = NULL gives the built-in default map (no device needed). */
+/* Copies the context's installed tile map into map (n >= BSB_TILE_MAP_LEN), or,
+ * where none is, the built-in map of the largest batches, as ctx = NULL does (no
+ * device needed).  Smaller batches run on other built-in maps, by their size, and
+ * all of them beside the kernels named above; an installed map, this one
+ * included, is used as it is for batches of every size. */
 int bsb_get_tile_map(bsb_ctx *ctx, uint8_t *map, int n);
 
 /* ---- FM-index (device resident) ----------------------------------------- */
