@@ -332,7 +332,13 @@ chain_kernel(AlnOpt opt, DevBns B, const int *__restrict__ list, const int *__re
              int *__restrict__ row_chain, int *__restrict__ iwork, DevSeed *__restrict__ out_seeds,
              DevChain *__restrict__ out_chains, int *__restrict__ n_chains)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < *n_list; t += gridDim.x * blockDim.x) {
+    // As few reads a warp as the list allows, one where there are no more reads than warps: the lanes' trees take different
+    // paths, one after the other.  4096 reads of 100 bases, a quarter of them from tandem repeats (up to 2000 chains each),
+    // the chaining stage: 1.02 s with 32 reads a warp, 0.38 with one.
+    const int n = *n_list, warps = (int)(gridDim.x * blockDim.x) >> 5, per = min(32, (n + warps - 1) / warps);
+    const int lane = threadIdx.x & 31;
+    if (lane >= per) return;
+    for (int t = ((int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per + lane; t < n; t += warps * per) {
         const int r = list[t];
         const int len = (int)(read_off[r + 1] - read_off[r]);
         const int64_t s0 = seed_off[r], s1 = seed_off[r + 1];
@@ -2667,7 +2673,7 @@ static int bsb_align_regs_run(bsb_ctx *ctx, const bsb_align_opt_t *o, int n_read
     chain_warp_kernel<<<(n_reads + kChainWarps - 1) / kChainWarps, kChainWarps * 32, 0, st>>>(
         ao, B, n_reads, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos, chains, nodes, row_chain, iwork,
         cseeds, cchains, n_chains, left, ctrl, by_rows);
-    chain_kernel<<<ctx->n_sm, 128, 0, st>>>(ao, B, left, ctrl, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos,
+    chain_kernel<<<ctx->n_sm * 4, 128, 0, st>>>(ao, B, left, ctrl, d_read_off, (const DevIntv *)d_seeds, d_seed_off, roff, pos,
                                             chains, nodes, row_chain, iwork, cseeds, cchains, n_chains);
     if (h_min_hsp &&
         (rc = seed_sw_filter(ctx, o, B, n_reads, h_min_hsp, d_reads, d_read_off, d_seed_off, roff, cseeds, cchains,
