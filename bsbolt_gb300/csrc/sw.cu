@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <vector>
 
 #include "bsb_internal.cuh"
 #include "scan.cuh"
@@ -295,7 +296,9 @@ sw_kernel(SwParams S, const bsb_sw_job_t *__restrict__ jobs, const uint8_t *__re
 // one-lane byte and word jobs.  The packed lists are in counting-sort order by segment count and then target length,
 // both descending: bins of kLenBins lengths per segment count.  Bin kBins - 2 and kBins - 1: the one-lane lists.
 // (On the host the check and the sort took 140 us of a call on 40k jobs; here they go on while the sequences are
-// copied.)
+// copied.  Up to kHostPlan jobs they are the host's: they take 4 ns a job there, and a call on one job was 50 us longer for
+// the kernels here and the wait for their result.)
+constexpr int kHostPlan = 8192;
 constexpr int kLenBins = 64, kKeys8 = kPackMaxSeg8 * kLenBins, kKeys16 = kPackMaxSeg16 * kLenBins;
 constexpr int kBins = kKeys8 + kKeys16 + 2;
 constexpr int kPlanThreads = 256;
@@ -315,6 +318,18 @@ __host__ __device__ __forceinline__ int job_fault(const bsb_sw_job_t &j, int64_t
     return j.qlen > BSB_SW_MAX_QLEN ? 2 : 0;
 }
 
+// A fit job's bin.
+__host__ __device__ __forceinline__ int job_bin(const bsb_sw_job_t &j, int qmax, int b8_ok, int w16_ok)
+{
+    const int rows = j.tlen >> 4, len = kLenBins - 1 - (rows < kLenBins - 1 ? rows : kLenBins - 1);
+    const bool byte = j.xtra & kXByte;
+    const int sl = byte ? (j.qlen + 15) >> 4 : (j.qlen + 7) >> 3;
+    if (byte && b8_ok && sl >= 1 && sl <= kPackMaxSeg8) return (kPackMaxSeg8 - sl) * kLenBins + len;
+    if (!byte && w16_ok && sl >= 1 && sl <= kPackMaxSeg16 && (int64_t)j.qlen * qmax <= 32640)
+        return kKeys8 + (kPackMaxSeg16 - sl) * kLenBins + len;
+    return byte ? kBins - 2 : kBins - 1;
+}
+
 // Every job's bin, the bins' sizes, and the rows of its suboptimal-score scratch.
 __global__ void __launch_bounds__(kPlanThreads)
 sw_plan_kernel(const bsb_sw_job_t *__restrict__ jobs, int n, int64_t seq_bytes, int qmax, int b8_ok, int w16_ok,
@@ -330,15 +345,9 @@ sw_plan_kernel(const bsb_sw_job_t *__restrict__ jobs, int n, int64_t seq_bytes, 
             atomicMin(&plan->bad, (int)i);
             continue;
         }
-        const int len = kLenBins - 1 - min(j.tlen >> 4, kLenBins - 1);
-        const bool byte = j.xtra & kXByte;
-        const int sl = byte ? (j.qlen + 15) >> 4 : (j.qlen + 7) >> 3;
-        int k;
-        if (byte && b8_ok && sl >= 1 && sl <= kPackMaxSeg8) k = (kPackMaxSeg8 - sl) * kLenBins + len;
-        else if (!byte && w16_ok && sl >= 1 && sl <= kPackMaxSeg16 && (int64_t)j.qlen * qmax <= 32640)
-            k = kKeys8 + (kPackMaxSeg16 - sl) * kLenBins + len;
-        else if (byte) k = kBins - 2, atomicMax(&plan->max8, j.qlen);
-        else k = kBins - 1, atomicMax(&plan->max16, j.qlen);
+        const int k = job_bin(j, qmax, b8_ok, w16_ok);
+        if (k == kBins - 2) atomicMax(&plan->max8, j.qlen);
+        if (k == kBins - 1) atomicMax(&plan->max16, j.qlen);
         bin[i] = k;
         if (j.xtra & kXSubo) rows[i] = j.tlen;
         atomicAdd(&sh[k], 1);
@@ -462,6 +471,39 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t jb = al(sizeof(bsb_sw_job_t) * (size_t)n), sb = al((size_t)seq_bytes), ob = al(8 * ((size_t)n + 1));
     const size_t lb = al(sizeof(int32_t) * (size_t)n);
+    SwPlan plan{INT_MAX, 0, 0, 0, 0, 0, 0, 0};
+    const auto refuse = [&]() -> int {
+        const bsb_sw_job_t &j = jobs[plan.bad];
+        if (job_fault(j, seq_bytes) == 1)
+            return bsb_fail(ctx, BSB_EINVAL, "job %lld: bytes outside seq", (long long)plan.bad);
+        return bsb_fail(ctx, BSB_ETOOLONG, "job %lld: qlen %d > %d", (long long)plan.bad, j.qlen, BSB_SW_MAX_QLEN);
+    };
+    int64_t nb = 0;
+    std::vector<char> lists;                 // the rows' offsets and the lists, as they lie on the device
+    if (n <= kHostPlan) {
+        lists.resize(ob + lb);
+        int64_t *const boff = (int64_t *)lists.data();
+        int32_t *const list = (int32_t *)(lists.data() + ob);
+        std::vector<int> bin((size_t)n), at(kBins + 1, 0);
+        for (int64_t i = 0; i < n && plan.bad == INT_MAX; ++i) {
+            const bsb_sw_job_t &job = jobs[i];
+            if (job_fault(job, seq_bytes)) {
+                plan.bad = (int)i;
+                break;
+            }
+            const int b = job_bin(job, S.qmax, b8_ok, w16_ok);
+            if (b == kBins - 2) plan.max8 = std::max(plan.max8, job.qlen);
+            if (b == kBins - 1) plan.max16 = std::max(plan.max16, job.qlen);
+            bin[(size_t)i] = b, ++at[(size_t)b + 1];
+            boff[i] = nb;
+            if (job.xtra & kXSubo) nb += job.tlen;
+        }
+        if (plan.bad != INT_MAX) return refuse();
+        for (int b = 0; b < kBins; ++b) at[(size_t)b + 1] += at[(size_t)b];
+        plan.n_p8 = at[kKeys8], plan.n_hi = at[kKeys8 + (kPackMaxSeg16 - 16) * kLenBins];
+        plan.n_p16 = at[kBins - 2], plan.n_fb8 = at[kBins - 1], plan.n_fb16 = at[kBins];
+        for (int64_t i = 0; i < n; ++i) list[at[(size_t)bin[(size_t)i]]++] = (int32_t)i;
+    }
     if ((rc = bsb_ensure(ctx, in_buf, in_bytes, jb + sb + ob + lb + 256, "SW input staging"))) return rc;
     char *in = (char *)*in_buf;
     bsb_sw_job_t *d_jobs = (bsb_sw_job_t *)in;
@@ -474,34 +516,37 @@ int bsb_align2_run(bsb_ctx *ctx, const bsb_ext_param_t *p, const bsb_sw_job_t *j
                          std::max(sizeof(bsb_kswr_t) * (size_t)n, 2 * lb + 2 * hb + tb + 256) + 256, "SW output")))
         return rc;
     bsb_kswr_t *d_out = (bsb_kswr_t *)*out_buf;
-    char *pl = (char *)*out_buf;
-    int *d_bin = (int *)pl, *d_rows = (int *)(pl + lb), *d_hist = (int *)(pl + 2 * lb), *d_cur = (int *)(pl + 2 * lb + hb);
-    int64_t *d_tmp = (int64_t *)(pl + 2 * lb + 2 * hb);
-    SwPlan *d_plan = (SwPlan *)(pl + 2 * lb + 2 * hb + tb);
-    SwPlan plan{INT_MAX, 0, 0, 0, 0, 0, 0, 0};
-    const int pb = (int)std::min<int64_t>((n + kPlanThreads - 1) / kPlanThreads, (int64_t)ctx->n_sm * 4);
     if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_jobs, jobs, sizeof(bsb_sw_job_t) * n, cudaMemcpyHostToDevice, st),
-                       "H2D jobs")) ||
-        (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_plan, &plan, sizeof plan, cudaMemcpyHostToDevice, st), "SW plan")) ||
-        (rc = bsb_cuda(ctx, cudaMemsetAsync(d_hist, 0, sizeof(int) * kBins, st), "SW plan")))
+                       "H2D jobs")))
         return rc;
-    sw_plan_kernel<<<pb, kPlanThreads, 0, st>>>(d_jobs, (int)n, seq_bytes, S.qmax, b8_ok, w16_ok, d_bin, d_rows, d_hist,
-                                                d_plan);
-    sw_plan_scan<<<1, 1024, 0, st>>>(d_hist, d_cur, d_plan);
-    sw_plan_scatter<<<pb, kPlanThreads, 0, st>>>(d_bin, (int)n, d_cur, d_list);
-    int64_t nb = 0;
-    if ((rc = bsb_cuda(ctx, scan_i32_i64(d_rows, n, d_boff, d_tmp, st), "SW plan")) ||
-        (seq_bytes && (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_seq, seq, seq_bytes, cudaMemcpyHostToDevice, st), "H2D seq"))) ||
-        (rc = bsb_cuda(ctx, cudaMemcpyAsync(&plan, d_plan, sizeof plan, cudaMemcpyDeviceToHost, st), "SW plan")) ||
-        (rc = bsb_cuda(ctx, cudaMemcpyAsync(&nb, d_boff + n, 8, cudaMemcpyDeviceToHost, st), "SW plan")) ||
-        (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "SW plan")))
-        return rc;
-    if (plan.bad != INT_MAX) {
-        const bsb_sw_job_t &j = jobs[plan.bad];
-        if (job_fault(j, seq_bytes) == 1)
-            return bsb_fail(ctx, BSB_EINVAL, "job %lld: bytes outside seq", (long long)plan.bad);
-        return bsb_fail(ctx, BSB_ETOOLONG, "job %lld: qlen %d > %d", (long long)plan.bad, j.qlen, BSB_SW_MAX_QLEN);
+    if (!lists.empty()) {
+        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_boff, lists.data(), lists.size(), cudaMemcpyHostToDevice, st), "SW plan")) ||
+            (seq_bytes &&
+             (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_seq, seq, seq_bytes, cudaMemcpyHostToDevice, st), "H2D seq"))))
+            return rc;
+    } else {
+        char *pl = (char *)*out_buf;
+        int *d_bin = (int *)pl, *d_rows = (int *)(pl + lb), *d_hist = (int *)(pl + 2 * lb),
+            *d_cur = (int *)(pl + 2 * lb + hb);
+        int64_t *d_tmp = (int64_t *)(pl + 2 * lb + 2 * hb);
+        SwPlan *d_plan = (SwPlan *)(pl + 2 * lb + 2 * hb + tb);
+        const int pb = (int)std::min<int64_t>((n + kPlanThreads - 1) / kPlanThreads, (int64_t)ctx->n_sm * 4);
+        if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(d_plan, &plan, sizeof plan, cudaMemcpyHostToDevice, st), "SW plan")) ||
+            (rc = bsb_cuda(ctx, cudaMemsetAsync(d_hist, 0, sizeof(int) * kBins, st), "SW plan")))
+            return rc;
+        sw_plan_kernel<<<pb, kPlanThreads, 0, st>>>(d_jobs, (int)n, seq_bytes, S.qmax, b8_ok, w16_ok, d_bin, d_rows,
+                                                    d_hist, d_plan);
+        sw_plan_scan<<<1, 1024, 0, st>>>(d_hist, d_cur, d_plan);
+        sw_plan_scatter<<<pb, kPlanThreads, 0, st>>>(d_bin, (int)n, d_cur, d_list);
+        if ((rc = bsb_cuda(ctx, scan_i32_i64(d_rows, n, d_boff, d_tmp, st), "SW plan")) ||
+            (seq_bytes &&
+             (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_seq, seq, seq_bytes, cudaMemcpyHostToDevice, st), "H2D seq"))) ||
+            (rc = bsb_cuda(ctx, cudaMemcpyAsync(&plan, d_plan, sizeof plan, cudaMemcpyDeviceToHost, st), "SW plan")) ||
+            (rc = bsb_cuda(ctx, cudaMemcpyAsync(&nb, d_boff + n, 8, cudaMemcpyDeviceToHost, st), "SW plan")) ||
+            (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "SW plan")))
+            return rc;
     }
+    if (plan.bad != INT_MAX) return refuse();
     const int64_t n_p8 = plan.n_p8, n_hi16 = plan.n_hi - plan.n_p8, n_p16 = plan.n_p16 - plan.n_p8;
     const int64_t n_fb8 = plan.n_fb8 - plan.n_p16, n_fb16 = plan.n_fb16 - plan.n_fb8;
     S.slen8 = std::max(1, (plan.max8 + 15) / 16), S.slen16 = std::max(1, (plan.max16 + 7) / 8);
