@@ -129,15 +129,17 @@ __host__ __device__ __forceinline__ int job_fault(const bsb_cigar_job_t &j, int6
     return !reject && j.re - j.rb > BSB_CIGAR_MAX_LEN ? 4 : 0;
 }
 
-// Also the check of the jobs, which goes before every other use of them: *bad receives the first unfit one.  (On the
-// host it took 93 us for 40k jobs, a fifth of the call; here it goes on while the sequences are copied.)
+// Also the check of the jobs, which goes before every other use of them: *bad receives the first unfit one (NULL: they
+// have been checked).  On the host it took 93 us for 40k jobs, a fifth of the call; here it goes on while the sequences are
+// copied, but its result takes a copy home: up to kHostChecked jobs are the host's (one job 12 us less).
+constexpr int kHostChecked = 4096;
 __global__ void plan_kernel(CigarParams P, const bsb_cigar_job_t *__restrict__ jobs, int n, int64_t q_bytes,
                             int64_t o_bytes, int *__restrict__ scratch_units, int *__restrict__ slot_units,
                             int *__restrict__ bad)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const bsb_cigar_job_t jb = jobs[i];
-        if (job_fault(jb, P.l_pac, q_bytes, o_bytes)) {
+        if (bad && job_fault(jb, P.l_pac, q_bytes, o_bytes)) {
             atomicMin(bad, i);
             scratch_units[i] = slot_units[i] = 0;
             continue;
@@ -494,7 +496,8 @@ extern "C" int bsb_gen_cigar_batch(bsb_ctx *ctx, const bsb_align_opt_t *o, int64
         }
     };
     int rc;
-    if (!qbuf || !obuf)
+    const bool checked = n <= kHostChecked || !qbuf || !obuf;
+    if (checked)
         for (int32_t i = 0; i < n; ++i)
             if ((rc = fault(i))) return rc;
     cudaStream_t st = ctx->stream;
@@ -516,13 +519,13 @@ extern "C" int bsb_gen_cigar_batch(bsb_ctx *ctx, const bsb_align_opt_t *o, int64
     int *d_scr_units = (int *)pl, *d_slot_units = (int *)(pl + ib), *d_bytes = (int *)(pl + 2 * ib);
     int64_t *d_scr_off = (int64_t *)(pl + 3 * ib), *d_slot_off = (int64_t *)(pl + 3 * ib + lb);
     int64_t *d_off = (int64_t *)(pl + 3 * ib + 2 * lb), *d_tmp = (int64_t *)(pl + 3 * ib + 3 * lb);
-    int *d_bad = (int *)(pl + 3 * ib + 3 * lb + tb);
+    int *d_bad = checked ? nullptr : (int *)(pl + 3 * ib + 3 * lb + tb);
     CigarParams P;
     memcpy(P.mat, o->mat, 25);
     P.o_del = o->o_del, P.e_del = o->e_del, P.o_ins = o->o_ins, P.e_ins = o->e_ins;
     P.l_pac = lp, P.crick_l = crick_l;
     const int blocks = (int)std::min<int64_t>(((int64_t)n + kCigarBlock - 1) / kCigarBlock, (int64_t)ctx->n_sm * 16);
-    if ((rc = bsb_cuda(ctx, cudaMemsetAsync(d_bad, 0x7f, sizeof(int), st), "CIGAR plan"))) return rc;
+    if (d_bad && (rc = bsb_cuda(ctx, cudaMemsetAsync(d_bad, 0x7f, sizeof(int), st), "CIGAR plan"))) return rc;
     plan_kernel<<<blocks, kCigarBlock, 0, st>>>(P, d_jobs, n, q_bytes, o_bytes, d_scr_units, d_slot_units, d_bad);
     if ((rc = bsb_cuda(ctx, scan_i32_i64(d_scr_units, n, d_scr_off, d_tmp, st), "CIGAR scratch offsets"))) return rc;
     if ((rc = bsb_cuda(ctx, scan_i32_i64(d_slot_units, n, d_slot_off, d_tmp, st), "CIGAR slot offsets"))) return rc;
@@ -532,10 +535,11 @@ extern "C" int bsb_gen_cigar_batch(bsb_ctx *ctx, const bsb_align_opt_t *o, int64
     if (o_bytes && (rc = bsb_cuda(ctx, cudaMemcpyAsync(d_o, obuf, o_bytes, cudaMemcpyHostToDevice, st), "H2D read")))
         return rc;
     int64_t tot[2] = {0, 0};
-    int bad = 0;
+    int bad = 0x7f7f7f7f;
     if ((rc = bsb_cuda(ctx, cudaMemcpyAsync(&tot[0], d_scr_off + n, 8, cudaMemcpyDeviceToHost, st), "D2H sizes")) ||
         (rc = bsb_cuda(ctx, cudaMemcpyAsync(&tot[1], d_slot_off + n, 8, cudaMemcpyDeviceToHost, st), "D2H sizes")) ||
-        (rc = bsb_cuda(ctx, cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H sizes")) ||
+        (d_bad &&
+         (rc = bsb_cuda(ctx, cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H sizes"))) ||
         (rc = bsb_cuda(ctx, cudaStreamSynchronize(st), "CIGAR plan")))
         return rc;
     if (bad != 0x7f7f7f7f) return fault(bad);
