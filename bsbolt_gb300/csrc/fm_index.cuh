@@ -118,17 +118,18 @@ __device__ __forceinline__ void occ_cumulative(const DevFM &F, const uint32_t (&
 
 // One LF step of bwt_sa (bwt_invPsi, bwt.c:53-59): the row of the suffix one text
 // position earlier; the primary row steps to row 0 (BWA's "$" convention).
-__device__ __forceinline__ uint64_t lf_step(const DevFM &F, uint64_t k)
+template <class P>
+__device__ __forceinline__ P lf_step(const DevFM &F, P k)
 {
-    if (k == F.primary) return 0;
+    if (k == (P)F.primary) return 0;
     // the symbol row (bwt_invPsi uses k > primary, bwt.c:55) equals the counted row here
-    const uint64_t kk = sym_row<uint64_t>(F, k);
+    const P kk = sym_row<P>(F, k);
     uint32_t w[8];
-    load32(sector_of<uint64_t>(F, kk), w);
+    load32(sector_of<P>(F, kk), w);
     const int n = (int)(kk & 31);
     const uint32_t lo = (kk & 32) ? w[5] : w[4], hi = (kk & 32) ? w[7] : w[6];
     const int c = (int)(lo >> n & 1u) | (int)(hi >> n & 1u) << 1;
-    uint64_t ge, gt;
-    occ_cumulative<uint64_t>(F, w, kk, c, ge, gt);
-    return l2_at(F, c) + ge - gt;
+    P ge, gt;
+    occ_cumulative<P>(F, w, kk, c, ge, gt);
+    return l2_at<P>(F, c) + ge - gt;
 }

@@ -787,24 +787,27 @@ constexpr uint64_t kMaxWalk = 1ull << 20;
 // bwt_sa: LF-walk to the nearest sampled row (bwt.c:53-59, 86-96), or one load when
 // the full suffix array is resident.  Rows beyond seq_len are answered with
 // (uint64_t)-2 and never walked; a walk longer than kMaxWalk with (uint64_t)-3.
+template <class P>
 __global__ void sa_kernel(DevFM F, const uint64_t *__restrict__ rows, int64_t n, uint64_t *__restrict__ pos)
 {
     const uint64_t mask = (1ull << F.sa_shift) - 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        uint64_t k = rows[i], steps = 0;
-        if (k > F.seq_len) {
+        const uint64_t row = rows[i];
+        if (row > F.seq_len) {
             pos[i] = ~(uint64_t)1;
             continue;
         }
         if (F.sa_full) {
-            pos[i] = __ldg(F.sa_full + k);
+            pos[i] = __ldg(F.sa_full + row);
             continue;
         }
-        while ((k & mask) && steps < kMaxWalk) {
+        P k = (P)row;
+        uint64_t steps = 0;
+        while ((k & (P)mask) && steps < kMaxWalk) {
             ++steps;
-            k = lf_step(F, k);
+            k = lf_step<P>(F, k);
         }
-        pos[i] = (k & mask) ? ~(uint64_t)2 : steps + __ldg(F.sa + (k >> F.sa_shift));
+        pos[i] = (k & (P)mask) ? ~(uint64_t)2 : steps + __ldg(F.sa + (k >> F.sa_shift));
     }
 }
 
@@ -813,6 +816,7 @@ __global__ void sa_kernel(DevFM F, const uint64_t *__restrict__ rows, int64_t n,
 // (bwt_sa's own walk, read backwards: every row's walk ends at the sampled row this
 // fill starts from, so each row gets the value bwt_sa gives it).  Row 0 answers BWA's
 // sample, (uint64_t)-1; the rows after it count down from seq_len.
+template <class P>
 __global__ void sa_fill_kernel(DevFM F, int64_t n_sa, uint64_t *__restrict__ full, int *__restrict__ failed)
 {
     const uint64_t mask = (1ull << F.sa_shift) - 1;
@@ -821,14 +825,15 @@ __global__ void sa_fill_kernel(DevFM F, int64_t n_sa, uint64_t *__restrict__ ful
         if (s > F.seq_len) continue;
         const uint64_t sv = F.sa[t];
         full[s] = sv;
-        uint64_t v = s == 0 ? F.seq_len : sv, k = s;
+        uint64_t v = s == 0 ? F.seq_len : sv;
+        P k = (P)s;
         for (uint64_t step = 0;; ++step) {
             if (step >= kMaxWalk) {                      // not a valid index: the walk is kept
                 atomicExch(failed, 1);
                 break;
             }
-            k = lf_step(F, k);
-            if (!(k & mask)) break;                     // the next sampled row starts its own run
+            k = lf_step<P>(F, k);
+            if (!(k & (P)mask)) break;                     // the next sampled row starts its own run
             full[k] = --v;
         }
     }
@@ -947,7 +952,7 @@ cudaError_t sa_full_build(const DevFM &F, int64_t n_sa, uint64_t *full, int *fai
 {
     const int64_t want = (n_sa + 255) / 256;
     const int blocks = (int)(want < (int64_t)n_sm * 32 ? want : (int64_t)n_sm * 32);
-    sa_fill_kernel<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(F, n_sa, full, failed);
+    (F.wide ? sa_fill_kernel<uint64_t> : sa_fill_kernel<uint32_t>)<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(F, n_sa, full, failed);
     return cudaGetLastError();
 }
 
@@ -956,6 +961,6 @@ cudaError_t sa_launch(const DevFM &F, const uint64_t *d_rows, int64_t n, uint64_
     if (n <= 0) return cudaSuccess;
     const int64_t want = (n + 255) / 256;
     const int blocks = (int)(want < (int64_t)n_sm * 16 ? want : (int64_t)n_sm * 16);
-    sa_kernel<<<blocks, 256, 0, st>>>(F, d_rows, n, d_pos);
+    (F.wide ? sa_kernel<uint64_t> : sa_kernel<uint32_t>)<<<blocks, 256, 0, st>>>(F, d_rows, n, d_pos);
     return cudaGetLastError();
 }

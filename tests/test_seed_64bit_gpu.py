@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import oracle
-from bsbolt_gb300 import extend, index, seed, synth
+from bsbolt_gb300 import _lib, extend, index, seed, synth
 
 from test_seed_forms_gpu import reads_of, references
 
@@ -85,3 +85,16 @@ def test_seeds_match_the_reference(form, tmp_path, name):
     for r in range(len(lens)):
         exp = ref[roff[r]:roff[r + 1]] if lens[r] >= int(o[10]) else ref[0:0]
         assert np.array_equal(got[off[r]:off[r + 1]], exp), f"read {r}: seeds differ"
+
+
+def test_suffix_array_rows(form, indexed):
+    """Every row through the full suffix array and through the walk."""
+    prefix, bi, _ = indexed
+    ctx = form(prefix)
+    pac = bi.pac_codes()
+    full = index.suffix_array(np.concatenate([pac, 3 - pac[::-1]]).astype(np.uint8)).astype(np.int64)
+    want = np.where(full == 2 * len(pac), -1, full)
+    rows = np.arange(len(full)).astype(np.uint64)
+    for resident in (1, 0):
+        _lib.check(ctx.handle, ctx.L.bsb_index_full_sa(ctx.handle, resident))
+        assert np.array_equal(seed.sa_batch(ctx, rows).astype(np.int64), want)
