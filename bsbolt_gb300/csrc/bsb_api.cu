@@ -345,7 +345,7 @@ extern "C" int bsb_extend_batch_device(bsb_ctx *ctx, const bsb_ext_param_t *para
                                        const int32_t *d_cost, bsb_ext_out_t *d_out, int64_t *d_cells)
 {
     if (!ctx) return BSB_EINVAL;
-    const int builtin = ksw_builtin(n_jobs, ctx->n_sm);
+    const int builtin = ksw_builtin(n_jobs, ctx->n_sm, d_cells != nullptr);
     const uint64_t tiles = ctx->d_tile_map ? ctx->map_tiles : ksw_builtin_tiles(builtin);
     ctx->n_chunks = 0;
     return extend_device(ctx, param, d_jobs, n_jobs, d_seq, seq_bytes, d_cost, d_out, d_cells, builtin, tiles);
@@ -439,7 +439,7 @@ extern "C" int bsb_extend_batch(bsb_ctx *ctx, const bsb_ext_param_t *param, cons
     JobScan piece[BSB_MAX_CHUNKS];
     // One map for all pieces: a piece's, or where cells are counted, and every one is computed, the batch's: the pieces
     // then keep the GPU full (2^20 jobs of 10-140 bases 16.3 ms, 18.5 on a piece's).
-    const int builtin = ksw_builtin(cells_out ? n_jobs : per, ctx->n_sm);
+    const int builtin = ksw_builtin(cells_out ? n_jobs : per, ctx->n_sm, cells_out != nullptr);
     P.pack16 = ksw_pack16(P);
     const bool installed = ctx->d_tile_map != nullptr;
     // Batches of one piece, from a few thousand jobs on: the scan is a kernel over the copied jobs, which goes on while

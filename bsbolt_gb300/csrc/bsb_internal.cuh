@@ -183,7 +183,7 @@ int64_t ksw_concurrent_below();
 // The built-in tile map (host copy, BSB_TILE_MAP_LEN entries); the number of the built-in map a
 // batch of n jobs runs on where the caller has set none, and that map.
 const uint8_t *ksw_default_tile_map();
-int ksw_builtin(int64_t n, int n_sm);
+int ksw_builtin(int64_t n, int n_sm, bool counting);      // counting: the batch counts cells
 const uint8_t *ksw_builtin_tile_map(int builtin);
 // Shape of tile t; -1 if t is out of range.
 int ksw_tile_shape(int t, int *G, int *C);

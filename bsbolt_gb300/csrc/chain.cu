@@ -2561,7 +2561,7 @@ static int first_extensions(bsb_ctx *ctx, const bsb_align_opt_t *o, const AlnOpt
     if ((rc = bsb_cuda(ctx, cudaMemsetAsync(out, 0x80, sizeof(bsb_ext_out_t) * 2 * T, st), "chain extensions"))) return rc;
     KswParams Q = P;
     Q.pac = B.pac, Q.l_pac = B.l_pac;
-    const int builtin = ksw_builtin(T, ctx->n_sm);
+    const int builtin = ksw_builtin(T, ctx->n_sm, false);
     const uint8_t *const map = ksw_builtin_tile_map(builtin);
     uint64_t tiles = 0;
     for (int need = 1; need <= max_len + 1 && need < BSB_TILE_MAP_LEN; ++need) tiles |= 1ull << map[need];

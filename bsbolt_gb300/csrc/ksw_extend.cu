@@ -369,7 +369,7 @@ bool ksw_pack16(const KswParams &P)
            P.mat_max <= kPack16MaxScore;
 }
 
-int ksw_builtin(int64_t n, int n_sm) { return ksw_builtin_of(n, n_sm); }
+int ksw_builtin(int64_t n, int n_sm, bool counting) { return ksw_builtin_of(n, n_sm, counting); }
 
 const uint8_t *ksw_builtin_tile_map(int builtin) { return kBuiltinTileMaps[builtin].tile; }
 

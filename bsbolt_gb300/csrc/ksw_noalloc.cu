@@ -84,7 +84,7 @@ extern "C" int bsb_extend_batch_noalloc(const bsb_ext_param_t *param, const bsb_
     int rc = setup_device(dev, &scratch, &n_sm, (cudaStream_t)stream);    // also for an empty batch: a warm-up call sets up
     if (rc) return rc;
     if (n_jobs == 0) return 0;
-    const int builtin = ksw_builtin(n_jobs, n_sm);
+    const int builtin = ksw_builtin(n_jobs, n_sm, d_cells != nullptr);
     const uint64_t tiles = ksw_builtin_tiles(builtin);
     cudaError_t e = ksw_launch(P, d_jobs, n_jobs, seq_bytes, d_seq, nullptr, nullptr, builtin, tiles, d_out, d_cells, scratch,
                                n_sm, (cudaStream_t)stream, nullptr, nullptr);

@@ -99,10 +99,13 @@ constexpr KswTileMap kBuiltinTileMaps[kBuiltinMaps] = {
     with_band(with_band(kDefaultTileMap, 1, 192, 32, 6), 193, 256, 32, 8),
     with_band(with_band(kDefaultTileMap, 1, 192, 32, 6), 193, 256, 32, 8),     // (with the other ring, below)
 };
-// The built-in map of a batch of n jobs (lines between the measured sizes where two maps meet).
-inline int ksw_builtin_of(int64_t n, int n_sm)
+// The built-in map of a batch of n jobs (lines between the measured sizes where two maps meet).  Counting cells means
+// computing all of them, with twice the jobs and more rows: such batches fill the GPU sooner (100,000 jobs of 10-140 bases
+// through the device entry 1.41 ms on the default map, 1.65 on the next; 45,000 0.96 and 0.85).
+inline int ksw_builtin_of(int64_t n, int n_sm, bool counting)
 {
-    return n <= 30 * (int64_t)n_sm ? 4 : n <= 50 * (int64_t)n_sm ? 3 : n <= 90 * (int64_t)n_sm ? 2 : n <= 1300 * (int64_t)n_sm ? 1 : 0;
+    const int64_t per = n / n_sm + (n % n_sm != 0);
+    return per <= 30 ? 4 : per <= 50 ? 3 : per <= 90 ? 2 : per <= (counting ? 450 : 1300) ? 1 : 0;
 }
 
 // Queries wider than a ring's columns whose band is narrower run on it (ksw_group16.cuh): registers for G*C columns
