@@ -90,8 +90,9 @@ __device__ __forceinline__ int global_rows_warp(const GlobalPen &P, const int8_t
 // only chain is F's, and a job takes tlen + band / C steps.  H, E and F stay in registers (a diagonal's first
 // H is the border's value; a cell outside leaves E and F at -inf), and scores are fetched a step ahead.
 // Needs 2w + 1 < 32 C, Z and stride multiples of 4.  The lanes' rows differ, so every byte of directions is a sector of
-// its own to write: a lane's C are one word where they lie side by side (5000 alignments of 250 bases in bands of 61,
-// the call: 1.42 ms by bytes, 0.74 by words; in rows 1.16).
+// its own to write: of four a lane makes one word where they lie side by side (5000 alignments of 250 bases in bands of
+// 61, the call: 1.42 ms by bytes, 0.82 by words; in rows 1.17).  Two to a lane stay bytes: most such bands hold theirs
+// in shared memory, and the words' branch costs more (40000 alignments of 100 bases: 120 us by bytes, 129 by words).
 template <int C, class TS>
 __device__ __forceinline__ int global_diagonals_warp(const GlobalPen &P, const int8_t *smat, const uint8_t *qs,
                                                      int qlen, const TS &ts, int tlen, int w, int stride, uint8_t *Z,
@@ -128,7 +129,6 @@ __device__ __forceinline__ int global_diagonals_warp(const GlobalPen &P, const i
         if (lane == 0) f = kNegInf;
         const bool row = (unsigned)i < (unsigned)tlen;
         const int z_at = i * stride + (i >= w ? d0 : j0);
-        const bool whole = row && i >= w && j0 >= 0 && j0 + C <= qlen && d0 + C - 1 <= last;
         uint32_t dirs = 0;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -147,14 +147,19 @@ __device__ __forceinline__ int global_diagonals_warp(const GlobalPen &P, const i
             f = on ? (fi > ti ? fi : ti) : kNegInf;
             if (on) {
                 h[c] = best;
-                if (Z && !whole) Z[z_at + c] = (uint8_t)dir;
+                if (C == 2 && Z) Z[z_at + c] = (uint8_t)dir;
             }
             dirs |= dir << 8 * c;
             sc[c] = next[c];
         }
-        if (Z && whole) {
-            if constexpr (C == 4) *(uint32_t *)(Z + z_at) = dirs;
-            else *(uint16_t *)(Z + z_at) = (uint16_t)dirs;
+        if (C == 4 && Z && row) {
+            if (i >= w && j0 >= 0 && j0 + C <= qlen && d0 + C - 1 <= last) {
+                *(uint32_t *)(Z + z_at) = dirs;
+            } else {
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+                    if ((unsigned)(j0 + c) < (unsigned)qlen && d0 + c <= last) Z[z_at + c] = (uint8_t)(dirs >> 8 * c);
+            }
         }
         f_out = f;
     }
