@@ -303,16 +303,18 @@ static void scan_pieces(const KswParams &P, const bsb_ext_job_t *jobs, int64_t n
     }
 }
 
-// Do the jobs use nearly all of seq, as far as 64 of them spread over the batch tell?
+// Do the jobs use nearly all of seq, as far as 64 of them spread over the batch tell?  (The last of them where the bytes
+// lie in job order: 64 cold lines cost 10 us and more.)
 static bool seq_mostly_used(const bsb_ext_job_t *jobs, int64_t n, int64_t seq_bytes)
 {
-    int64_t end = 0;
-    for (int k = 0; k < 64; ++k) {
+    const int64_t enough = seq_bytes - seq_bytes / 8;
+    bool used = enough <= 0;
+    for (int k = 63; k >= 0 && !used; --k) {
         const bsb_ext_job_t &j = jobs[(n - 1) * k / 63];
-        if (span_inside(j.qoff, j.qlen, seq_bytes)) end = std::max(end, j.qoff + j.qlen);
-        if (span_inside(j.toff, j.tlen, seq_bytes)) end = std::max(end, j.toff + j.tlen);
+        used = (span_inside(j.qoff, j.qlen, seq_bytes) && j.qoff + j.qlen >= enough) ||
+               (span_inside(j.toff, j.tlen, seq_bytes) && j.toff + j.tlen >= enough);
     }
-    return seq_bytes - end <= seq_bytes / 8;
+    return used;
 }
 
 // Device-buffer extension with the tile shapes `tiles` launched (every shape
